@@ -150,10 +150,12 @@ struct BlockState {
     unsigned failed;               // a block ran out of candidates: every later block's kernels return at once
     long long last_pivot;          // rank of the previous block's last pivot
     long long pred_tiles;          // tiles the streaming pass computes for this block
-    long long max_tile;            // deepest tile the previous block's pivot search touched
+    long long max_tile[2];         // by block parity: deepest tile the block's pivot search touched
     unsigned long long total;      // running 64-bit total weight of the basis
     unsigned tail_ok, pad_;        // the pivot kernel's CTA 0 resolved the block
     long long pair_tiles;          // tiles the grouped streaming pass computed for the group's later blocks
+    unsigned nz_count[3];          // by group (mod 3): coordinates whose T (Tg) words are not all zero
+    unsigned by_columns;           // the group's W come from the column index, not from the lists
     long long pivrank[64];
     unsigned long long pivW[64];   // the pivots' W as found (not reduced)
     unsigned long long mask[64];   // final S_{e0+k} as a combination of S^0_{e0+l}
@@ -182,6 +184,7 @@ __global__ void reset_state_kernel(IterSlot *slots, BlockState *bs, unsigned *st
         slots[1].next_tile = 0;
         bs->total = 0;  // epoch keeps counting across runs: old tile marks never match
         bs->failed = 0;
+        for (int i = 0; i < 3; i++) bs->nz_count[i] = 0;
         *status = 0;
     }
 }
@@ -246,6 +249,95 @@ __global__ void tile_minc_kernel(const int64_t *__restrict__ off, const int32_t 
             tile_minc[t] = v;
         }
         cta_sync();
+    }
+}
+
+// ---- column index: for each coordinate, the ranks of the candidates that hold it ----
+// Keys are (coordinate, segment of 2^seg_shift ranks): coordinate c's ranks lie at
+// ranks[start[c * segs]] .. ranks[start[(c + 1) * segs]], segment by segment, in any
+// order inside a segment.  A counting sort: counts per key, an exclusive scan, then
+// the ranks at their key's cursor.  kColLanes lanes share a list, so that the reads
+// of neighbouring lists are contiguous.
+constexpr int kColLanes = 8;
+constexpr int kColSegs = 64;                // segments per coordinate at most
+constexpr long long kColKeys = 16ll << 20;  // (coordinate, segment) keys at most (one per coordinate at least)
+constexpr int kColThreads = 256;
+constexpr int kScanCta = 1024, kScanItems = 8;
+
+template <bool kFill>
+__global__ void __launch_bounds__(kColThreads) columns_kernel(const int64_t *__restrict__ off,
+                                                             const int32_t *__restrict__ coords, long long K, int segs,
+                                                             int seg_shift, unsigned *start, unsigned *ranks) {
+    const long long g0 = ((long long)blockIdx.x * kColThreads + threadIdx.x) / kColLanes;
+    const long long ng = (long long)gridDim.x * kColThreads / kColLanes;
+    const int sub = threadIdx.x % kColLanes;
+    for (long long r = g0; r < K; r += ng) {
+        const int seg = (int)(r >> seg_shift);
+        const int64_t e = off[r + 1];
+        for (int64_t i = off[r] + sub; i < e; i += kColLanes) {
+            // start[key + 1] counts the key; after the scan it is the key's cursor, and
+            // once every rank is placed the next key's start
+            unsigned *at = start + (size_t)coords[i] * segs + seg + 1;
+            const unsigned pos = atomicAdd(at, 1u);
+            if (kFill) ranks[pos] = (unsigned)r;
+        }
+    }
+}
+
+// Exclusive scan of v[0, n) in place in three launches: per-CTA sums, one CTA's scan
+// of the sums, each CTA's items.
+__device__ __forceinline__ unsigned cta_exclusive(unsigned x, unsigned *s_part, unsigned &total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned v = x;
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += y;
+    }
+    if (lane == 31) s_part[warp] = v;
+    cta_sync();
+    unsigned before = 0;
+    total = 0;
+    for (int i = 0; i < kScanCta / 32; i++) {
+        before += i < warp ? s_part[i] : 0u;
+        total += s_part[i];
+    }
+    cta_sync();
+    return before + v - x;
+}
+
+__global__ void __launch_bounds__(kScanCta) scan_sums_kernel(const unsigned *__restrict__ v, long long n, unsigned *sums) {
+    __shared__ unsigned s_part[kScanCta / 32];
+    const long long i0 = ((long long)blockIdx.x * kScanCta + threadIdx.x) * kScanItems;
+    unsigned x = 0, total;
+    for (int q = 0; q < kScanItems; q++) x += i0 + q < n ? v[i0 + q] : 0u;
+    cta_exclusive(x, s_part, total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanCta) scan_top_kernel(unsigned *sums, int n) {
+    __shared__ unsigned s_part[kScanCta / 32];
+    unsigned carry = 0;
+    for (int base = 0; base < n; base += kScanCta) {
+        const int i = base + threadIdx.x;
+        unsigned total;
+        const unsigned x = cta_exclusive(i < n ? sums[i] : 0u, s_part, total);
+        if (i < n) sums[i] = carry + x;
+        carry += total;
+    }
+}
+
+__global__ void __launch_bounds__(kScanCta) scan_items_kernel(unsigned *v, long long n, const unsigned *__restrict__ sums) {
+    __shared__ unsigned s_part[kScanCta / 32];
+    const long long i0 = ((long long)blockIdx.x * kScanCta + threadIdx.x) * kScanItems;
+    unsigned a[kScanItems], x = 0, total;
+    for (int q = 0; q < kScanItems; q++) {
+        a[q] = i0 + q < n ? v[i0 + q] : 0u;
+        x += a[q];
+    }
+    unsigned run = sums[blockIdx.x] + cta_exclusive(x, s_part, total);
+    for (int q = 0; q < kScanItems; q++) {
+        if (i0 + q < n) v[i0 + q] = run;
+        run += a[q];
     }
 }
 
@@ -367,34 +459,44 @@ __global__ void cycle_vector_kernel(uint64_t *C, int W, const int64_t *__restric
 //
 // blk_transpose_kernel: T[64w + i] bit k = S[e0+k] bit (64w+i), for w < Wb.
 // One warp per word column; also resets the block state (runs first in the block).
-// The first block of a group also writes Tg[kGStride c + j] for the grouped streaming
-// pass: slot 0 = T[c], slot j = bit k of S[e0+64j+k] bit c (the group's j-th later
-// block's bj rows as they are now), for words w < Wbj of that block.
-// transpose_rows writes T[64w + i] (T may be NULL) and, with Tg, the same into
-// Tg[kGStride (64w + i) + slot].
-__device__ __forceinline__ void transpose_rows(const uint64_t *__restrict__ S, int P, int r0, int b, int Wb,
-                                               uint64_t *__restrict__ T, uint64_t *__restrict__ Tg, int slot) {
+// The first block of a group also writes Tg[kGStride c + j] for the group's W pass:
+// slot 0 = T[c], slot j = bit k of S[e0+64j+k] bit c (the group's j-th later block's
+// bj rows as they are now), for the words of the group's last block (a row is zero
+// beyond its own word), and lists the coordinates whose words are not all zero.
+//
+// How the group's W will be formed is decided here, from the previous group's list:
+// while fewer than 1 / kColumnShare of the coordinates are listed, from the column
+// index (blk_w_kernel), and then the W the pass will add to are zeroed here.
+#ifndef MCB_COLUMN_SHARE
+#define MCB_COLUMN_SHARE 16
+#endif
+// 100k-point planar-chain graph (N = 109k, 276M coordinates): 654 -> 226 ms per solve
+// against streaming alone (pass 530 -> 50 us per pair of blocks).  The line: a random
+// graph of 50k vertices, whose support vectors fill up, takes 298 ms with 8, 16 or 32
+// here and 308 ms with 4 (an atomic costs more than a streamed coordinate); the planar
+// and RGG families stay far below it and do not move.
+constexpr int kColumnShare = MCB_COLUMN_SHARE;
+
+struct GroupArgs {       // the first block of a group (b[0] >= 0); later blocks: nz = nullptr
+    int b1, b2;          // rows of the later blocks (0: none)
+    int Wlast;           // words of the group's last block
+    int slot;            // group number mod 3: its entry of BlockState::nz_count
+    int columns;         // the column index exists
+    int32_t *nz;         // the listed coordinates
+    uint64_t *W[3];      // the W arrays of the group's blocks
+};
+
+__device__ __forceinline__ void load_columns(const uint64_t *__restrict__ S, int P, int r0, int b, int w, uint64_t &a,
+                                             uint64_t &c) {
     const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < Wb; w += warps) {
-        uint64_t a = lane < b ? S[(size_t)(r0 + lane) * P + w] : 0ull;
-        uint64_t c = (32 + lane) < b ? S[(size_t)(r0 + 32 + lane) * P + w] : 0ull;
-        warp_transpose64(a, c);  // a: column 64w + lane, c: column 64w + 32 + lane
-        if (T) {
-            T[(size_t)w * 64 + lane] = a;
-            T[(size_t)w * 64 + 32 + lane] = c;
-        }
-        if (Tg) {
-            Tg[kGStride * ((size_t)w * 64 + lane) + slot] = a;
-            Tg[kGStride * ((size_t)w * 64 + 32 + lane) + slot] = c;
-        }
-    }
+    a = lane < b ? S[(size_t)(r0 + lane) * P + w] : 0ull;
+    c = (32 + lane) < b ? S[(size_t)(r0 + 32 + lane) * P + w] : 0ull;
 }
 
-__global__ void blk_transpose_kernel(const uint64_t *__restrict__ S, int P, int e0, int b, int Wb,
-                                     uint64_t *__restrict__ T, BlockState *bs, long long ntiles,
-                                     GridBar *gb, long long window_tiles, int stream_pct,
-                                     uint64_t *__restrict__ Tg, int b1, int Wb1, int b2, int Wb2) {
+__global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__restrict__ S, int P, int e0, int b, int Wb,
+                                                           uint64_t *__restrict__ T, BlockState *bs, long long ntiles,
+                                                           GridBar *gb, long long window_tiles, int stream_pct,
+                                                           uint64_t *__restrict__ Tg, GroupArgs ga) {
     griddep_wait();
     griddep_launch();
     if (*(volatile const unsigned *)&bs->failed) {  // set by an earlier block's pivot kernel (same stream)
@@ -404,29 +506,76 @@ __global__ void blk_transpose_kernel(const uint64_t *__restrict__ S, int P, int 
         }
         return;
     }
+    const int par = (e0 >> 6) & 1;
+    // stream stream_pct percent past the previous block's deepest pivot; the pivot
+    // kernel computes any further tile it needs
+    long long pred = ntiles;
+    if (e0 != 0) {
+        const long long lp = bs->last_pivot + 1;
+        const long long a = (lp + lp * stream_pct / 100) / kTile + 1, m = bs->max_tile[par ^ 1] + 1;
+        pred = (a > m ? a : m) + window_tiles;
+    }
+    const int later = (ga.b1 > 0 ? 1 : 0) + (ga.b2 > 0 ? 1 : 0);  // the pass serves the group's later blocks too
+    if (later > 0 && e0 != 0) pred += pred * MCB_PAIR_MARGIN * later / 100;
+    pred = pred < ntiles ? pred : ntiles;
+    const bool cols = ga.nz && ga.columns &&
+                      (long long)bs->nz_count[(ga.slot + 2) % 3] * kColumnShare <= (long long)e0 + 64 * kColumnShare;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         gb->count = 0;
         gb->abort = 0;
         bs->rank = 0;
         bs->epoch = bs->epoch + 1;
         bs->b = (unsigned)b;
-        // stream stream_pct percent past the previous block's deepest pivot; the
-        // pivot kernel computes any further tile it needs
-        long long pred = ntiles;
-        if (e0 != 0) {
-            const long long lp = bs->last_pivot + 1;
-            const long long a = (lp + lp * stream_pct / 100) / kTile + 1, m = bs->max_tile + 1;
-            pred = (a > m ? a : m) + window_tiles;
+        bs->pred_tiles = pred;
+        if (later > 0) bs->pair_tiles = pred;  // read by the later blocks' blk_wfix_kernel
+        bs->max_tile[par] = 0;                 // the pivot kernel's; the other one is read above
+        if (ga.nz) {
+            bs->nz_count[(ga.slot + 1) % 3] = 0;  // the next group's
+            bs->by_columns = cols ? 1u : 0u;
         }
-        const int later = (b1 > 0 ? 1 : 0) + (b2 > 0 ? 1 : 0);  // the pass serves the group's later blocks too
-        if (later > 0 && e0 != 0) pred += pred * MCB_PAIR_MARGIN * later / 100;
-        bs->pred_tiles = pred < ntiles ? pred : ntiles;
-        if (later > 0) bs->pair_tiles = bs->pred_tiles;  // read by the later blocks' blk_wfix_kernel
-        bs->max_tile = 0;
     }
-    transpose_rows(S, P, e0, b, Wb, T, b1 > 0 ? Tg : nullptr, 0);
-    if (b1 > 0) transpose_rows(S, P, e0 + 64, b1, Wb1, nullptr, Tg, 1);
-    if (b2 > 0) transpose_rows(S, P, e0 + 128, b2, Wb2, nullptr, Tg, 2);
+    if (cols) {
+        const size_t n = (size_t)pred * kTile / 2;
+        for (int j = 0; j <= later; j++) {
+            ulonglong2 *W = reinterpret_cast<ulonglong2 *>(ga.W[j]);
+            for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+                W[i] = make_ulonglong2(0ull, 0ull);
+        }
+    }
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ga.Wlast; w += warps) {
+        const size_t c0 = (size_t)w * 64 + lane, c1 = c0 + 32;
+        uint64_t x0, y0, x1 = 0, y1 = 0, x2 = 0, y2 = 0;
+        load_columns(S, P, e0, b, w, x0, y0);
+        if (ga.b1 > 0) load_columns(S, P, e0 + 64, ga.b1, w, x1, y1);
+        if (ga.b2 > 0) load_columns(S, P, e0 + 128, ga.b2, w, x2, y2);
+        warp_transpose64(x0, y0);  // x: column 64w + lane, y: column 64w + 32 + lane
+        if (w < Wb) {
+            T[c0] = x0;
+            T[c1] = y0;
+        }
+        if (ga.b1 > 0) {
+            warp_transpose64(x1, y1);
+            *reinterpret_cast<ulonglong2 *>(Tg + kGStride * c0) = make_ulonglong2(x0, x1);
+            *reinterpret_cast<ulonglong2 *>(Tg + kGStride * c1) = make_ulonglong2(y0, y1);
+        }
+        if (ga.b2 > 0) {
+            warp_transpose64(x2, y2);
+            Tg[kGStride * c0 + 2] = x2;
+            Tg[kGStride * c1 + 2] = y2;
+        }
+        if (ga.nz) {
+            const bool nx = (x0 | x1 | x2) != 0, ny = (y0 | y1 | y2) != 0;
+            const unsigned lo = __ballot_sync(0xffffffffu, nx), hi = __ballot_sync(0xffffffffu, ny);
+            unsigned at = 0;
+            if (lane == 0 && (lo | hi)) at = atomicAdd(&bs->nz_count[ga.slot], (unsigned)(__popc(lo) + __popc(hi)));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            const unsigned below = (1u << lane) - 1u;
+            if (nx) ga.nz[at + __popc(lo & below)] = (int32_t)c0;
+            if (ny) ga.nz[at + __popc(lo) + __popc(hi & below)] = (int32_t)c1;
+        }
+    }
 }
 
 // Reduce W by the basis held as Four-Russians tables: tab[g][pat] = XOR of the basis
@@ -688,6 +837,46 @@ __device__ __forceinline__ void w_of_group(long long r, const int64_t *__restric
     }
 }
 
+// W from the column index: W starts at zero, and every listed coordinate's T words are
+// added to the ranks of its column below the limit.  Warp w takes part w / n of the
+// listed coordinate w mod n's column (n listed).
+//
+// Support vectors are sparse for most of a solve: 181-235 listed coordinates of
+// 27k-82k for a pair of blocks of a planar-chain graph (100k points), 129-600 of an
+// RGG's, 1.7k of 12.6k up to 34k of 37.5k of a random graph's.  Reading only their
+// columns touches 0.3-7% of the lists, which the streaming pass reads whole.
+struct Columns {
+    const unsigned *start;  // (N x segs) + 1
+    const unsigned *ranks;
+    const int32_t *nz;
+    int segs, seg_shift, slot;
+};
+
+template <int kG>
+__device__ __forceinline__ void w_by_columns(const Columns &co, const uint64_t *__restrict__ Tt, unsigned n,
+                                             long long limit, uint64_t *W0, uint64_t *W1, uint64_t *W2) {
+    constexpr int kStride = kG == 1 ? 1 : kGStride;
+    if (n == 0 || limit <= 0) return;
+    const int lane = threadIdx.x & 31;
+    const unsigned gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const unsigned parts = nw / n > 0 ? nw / n : 1u;
+    const int seg_end = (int)((limit - 1) >> co.seg_shift) + 1 < co.segs ? (int)((limit - 1) >> co.seg_shift) + 1 : co.segs;
+    for (unsigned it = gw; it < n * parts; it += nw) {
+        const int c = co.nz[it % n];
+        const unsigned part = it / n;
+        const uint64_t *t = Tt + (size_t)kStride * c;
+        const uint64_t x = t[0], y = kG > 1 ? t[kG > 1 ? 1 : 0] : 0ull, z = kG > 2 ? t[kG - 1] : 0ull;
+        const unsigned e = co.start[(size_t)c * co.segs + seg_end];
+        for (unsigned i = co.start[(size_t)c * co.segs] + part * 32 + lane; i < e; i += parts * 32) {
+            const unsigned r = __ldg(co.ranks + i);
+            if ((long long)r >= limit) continue;
+            if (x) atomicXor((unsigned long long *)W0 + r, (unsigned long long)x);
+            if (kG > 1 && y) atomicXor((unsigned long long *)W1 + r, (unsigned long long)y);
+            if (kG > 2 && z) atomicXor((unsigned long long *)W2 + r, (unsigned long long)z);
+        }
+    }
+}
+
 // Streaming pass: W for tiles [0, bs->pred_tiles), one candidate per thread (1024
 // threads = one tile per CTA pass), written to Warr and tagged with the block's
 // epoch.  This is the bandwidth-bound part of the block's search.
@@ -704,12 +893,19 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
                                                     const uint64_t *__restrict__ T, int bound, const BlockState *bs,
                                                     uint64_t *Warr, unsigned *tile_epoch, unsigned long long *bytes,
                                                     const uint64_t *__restrict__ Tg, int bound1, int bound2,
-                                                    uint64_t *Wl1, uint64_t *Wl2) {
+                                                    uint64_t *Wl1, uint64_t *Wl2, Columns co) {
     griddep_wait();
     griddep_launch();
     const unsigned epoch = bs->epoch;
     const long long ntiles = bs->pred_tiles;
     unsigned long long nb = (blockIdx.x == 0 && threadIdx.x == 0) ? 8ull * (unsigned long long)bound : 0ull;
+    if (bs->by_columns) {
+        w_by_columns<kG>(co, kG > 1 ? Tg : T, bs->nz_count[co.slot], min(ntiles * kTile, K), Warr, Wl1, Wl2);
+        for (long long t = blockIdx.x + (long long)threadIdx.x * gridDim.x; t < ntiles;
+             t += (long long)blockDim.x * gridDim.x)
+            tile_epoch[t] = (epoch << 1) | (tile_minc[t] >= bound ? 1u : 0u);
+        return;
+    }
     if (kG > 1) {
         const int bd[3] = {bound, bound1, bound2};
         const int last = bd[kG - 1];
@@ -1745,7 +1941,7 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
     if (threadIdx.x == 0) {
         atomicMax(&diag[14], nbar);
         atomicMin(&diag[15], nbar);
-        atomicMax((unsigned long long *)&bs->max_tile, (unsigned long long)maxt);
+        atomicMax((unsigned long long *)&bs->max_tile[ta.par], (unsigned long long)maxt);
         atomicAdd(&diag[1], n_local);
         atomicAdd(&diag[3], n_loaded);
         atomicAdd(&diag[4], n_computed);
@@ -2416,6 +2612,11 @@ struct mcbgpu_solver {
     uint64_t *d_Warr2 = nullptr;   // W of a group's second block (the grouped pass, then its correction)
     uint64_t *d_Warr3 = nullptr;   // W of a group's third block
     uint64_t *d_Tg = nullptr;      // the group's blocks' rows transposed, kGStride words per coordinate
+    // column index (coordinate -> ranks); absent (segs = 0) when a size needs more than 32 bits or
+    // the memory is not there
+    unsigned *d_colstart = nullptr, *d_colranks = nullptr, *d_colsums = nullptr;
+    int col_segs = 0, col_shift = 0;
+    int32_t *d_nz = nullptr;       // 64 P: the coordinates whose T (Tg) words are not all zero
     uint64_t *d_beta = nullptr;    // 3 x 192: update bits of the near rows of a group's first blocks
     unsigned long long *d_nearD = nullptr;  // 2 x kNearMaxRows: D of the near rows by block parity (zero between uses)
     // far update: rows whose support vector is still the unit vector get D by scatter
@@ -2587,6 +2788,10 @@ void free_solver(mcbgpu_solver *s) {
     cudaFree(s->d_Warr2);
     cudaFree(s->d_Warr3);
     cudaFree(s->d_Tg);
+    cudaFree(s->d_nz);
+    cudaFree(s->d_colstart);
+    cudaFree(s->d_colranks);
+    cudaFree(s->d_colsums);
     cudaFree(s->d_beta);
     cudaFree(s->d_nearD);
     cudaFree(s->d_unit);
@@ -2692,6 +2897,7 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
         ALLOC(s->d_beta, sizeof(uint64_t) * 3 * 192);
         ALLOC(s->d_masks, sizeof(uint64_t) * 2 * 64);
     }
+    ALLOC(s->d_nz, sizeof(int32_t) * 64 * (size_t)s->P);
     ALLOC(s->d_nearD, sizeof(unsigned long long) * 2 * kNearMaxRows);
     ALLOC(s->d_unit, (size_t)N);
     ALLOC(s->d_Dfar, sizeof(unsigned long long) * (size_t)N);
@@ -2726,6 +2932,28 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
     if (e == cudaSuccess) e = cudaMemset(s->d_unit, 1, (size_t)N > 0 ? (size_t)N : 16);
     if (e == cudaSuccess) e = cudaMemset(s->d_fcnt, 0, sizeof(unsigned) * 8);
     if (e == cudaSuccess) e = cudaMemset(s->d_word_end, 0, sizeof(unsigned) * 2 * ((size_t)s->P + 1));
+    if (e == cudaSuccess && N > 0 && nnz > 0 && nnz < 0xffffffffll && K < 0xffffffffll) {
+        // at most kColKeys keys; segments of a power-of-two number of ranks, whole tiles
+        const long long want = std::max<long long>(1, std::min<long long>(kColSegs, kColKeys / N));
+        int shift = 10;
+        while (((K - 1) >> shift) >= want) shift++;
+        s->col_shift = shift;
+        s->col_segs = (int)((K - 1) >> shift) + 1;
+        const size_t keys = (size_t)N * s->col_segs;
+        const size_t sums = (keys + (size_t)kScanCta * kScanItems - 1) / ((size_t)kScanCta * kScanItems) + 1;
+        cudaError_t ec = cudaMalloc((void **)&s->d_colranks, sizeof(unsigned) * (size_t)nnz);
+        if (ec == cudaSuccess) ec = cudaMalloc((void **)&s->d_colstart, sizeof(unsigned) * (keys + 1));
+        if (ec == cudaSuccess) ec = cudaMalloc((void **)&s->d_colsums, sizeof(unsigned) * sums);
+        if (ec == cudaSuccess) {
+            bytes += (long long)(sizeof(unsigned) * ((size_t)nnz + keys + 1 + sums));
+        } else {  // the streaming pass does without
+            (void)cudaGetLastError();
+            cudaFree(s->d_colranks);
+            cudaFree(s->d_colstart);
+            s->d_colranks = s->d_colstart = nullptr;
+            s->col_segs = 0;
+        }
+    }
     // the far update fills every SM when it runs; with the critical path (transpose,
     // streaming pass, pivot search, near update) on a higher-priority stream, the
     // block scheduler gives that path's CTAs the SMs as they free up
@@ -2848,6 +3076,22 @@ static int solver_upload(mcbgpu_solver *s, const int32_t *weight, const int64_t 
             Launch L(s, KC_TILE_MINC, st);
             tile_minc_kernel<<<grid, 256, 0, st>>>(s->d_off, s->d_coords, s->K, s->d_tile_minc, ntiles);
         }
+        MCB_CUDA(cudaGetLastError());
+    }
+    if (s->col_segs > 0) {
+        const long long keys = (long long)s->N * s->col_segs;
+        const int cgrid = (int)std::min<long long>((s->K * kColLanes + kColThreads - 1) / kColThreads,
+                                                   (long long)(s->sm_count > 0 ? s->sm_count : 148) * 8);
+        const unsigned sgrid = (unsigned)((keys + (long long)kScanCta * kScanItems - 1) / ((long long)kScanCta * kScanItems));
+        Launch L(s, KC_VALIDATE, st, 5);
+        MCB_CUDA(cudaMemsetAsync(s->d_colstart, 0, sizeof(unsigned) * (size_t)(keys + 1), st));
+        columns_kernel<false><<<cgrid, kColThreads, 0, st>>>(s->d_off, s->d_coords, s->K, s->col_segs, s->col_shift,
+                                                             s->d_colstart, nullptr);
+        scan_sums_kernel<<<sgrid, kScanCta, 0, st>>>(s->d_colstart + 1, keys, s->d_colsums);
+        scan_top_kernel<<<1, kScanCta, 0, st>>>(s->d_colsums, (int)sgrid);
+        scan_items_kernel<<<sgrid, kScanCta, 0, st>>>(s->d_colstart + 1, keys, s->d_colsums);
+        columns_kernel<true><<<cgrid, kColThreads, 0, st>>>(s->d_off, s->d_coords, s->K, s->col_segs, s->col_shift,
+                                                            s->d_colstart, s->d_colranks);
         MCB_CUDA(cudaGetLastError());
     }
     s->uploaded = true;
@@ -3016,7 +3260,21 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             for (int jj = 1; jj < kGroup; jj++) bl[jj - 1] = (int)std::max<int64_t>(0, std::min<int64_t>(64, iters - e0 - 64 * jj));
         const int nl = (bl[0] > 0 ? 1 : 0) + (bl[1] > 0 ? 1 : 0);
         const int bd1 = (int)(e0 + 64 + bl[0]), bd2 = (int)(e0 + 128 + bl[1]);
-        const int Wb1 = bl[0] > 0 ? (bd1 + 63) / 64 : 0, Wb2 = bl[1] > 0 ? (bd2 + 63) / 64 : 0;
+        GroupArgs ga;
+        ga.b1 = bl[0];
+        ga.b2 = bl[1];
+        ga.Wlast = bl[1] > 0 ? (bd2 + 63) / 64 : bl[0] > 0 ? (bd1 + 63) / 64 : Wb;
+        ga.slot = (int)((e0 / 64 / kGroup) % 3);
+        ga.columns = s->col_segs > 0 ? 1 : 0;
+        ga.nz = pos == 0 ? s->d_nz : nullptr;
+        for (int jj = 0; jj < 3; jj++) ga.W[jj] = Wpos[jj];
+        Columns cols;
+        cols.start = s->d_colstart;
+        cols.ranks = s->d_colranks;
+        cols.nz = s->d_nz;
+        cols.segs = s->col_segs;
+        cols.seg_shift = s->col_shift;
+        cols.slot = ga.slot;
         // this block's search shape: by segment (tuned or default), forced, or while
         // tuning every candidate in turn, group by group (a group's blocks share one
         // streaming pass, so a group is the unit that is timed: from its first
@@ -3038,10 +3296,12 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
         }
         {
             Launch L(s, KC_TRANSPOSE, st);
-            MCB_CUDA(launch_k(pdl, blk_transpose_kernel, dim3((std::max(Wb, std::max(Wb1, Wb2)) + 7) / 8), dim3(256), 0,
-                              st, (const uint64_t *)s->d_S, s->P, (int)e0, b, Wb, s->d_T, s->d_bs, ntiles, s->d_gbar,
-                              (long long)s->pivot_grid * sh.win_mid, sh.stream_pct, s->d_Tg, bl[0], Wb1, bl[1],
-                              Wb2));
+            // where W may have to be zeroed, a CTA per tile up to one per SM at least
+            const int tgrid = std::max((ga.Wlast + 7) / 8,
+                                       ga.nz && ga.columns ? (int)std::min<long long>(sms, std::max(1ll, ntiles)) : 1);
+            MCB_CUDA(launch_k(pdl, blk_transpose_kernel, dim3(tgrid), dim3(256), 0, st, (const uint64_t *)s->d_S, s->P,
+                              (int)e0, b, Wb, s->d_T, s->d_bs, ntiles, s->d_gbar,
+                              (long long)s->pivot_grid * sh.win_mid, sh.stream_pct, s->d_Tg, ga));
         }
         if (ntiles > 0 && pos > 0) {
             Launch L(s, KC_WFIX, st);
@@ -3062,14 +3322,14 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             uint64_t *nul = nullptr;
             if (nl == 2)
                 MCB_CUDA(launch_k(pdl, blk_w_kernel<3>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
-                                  bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd2, Wpos[1], Wpos[2]));
+                                  bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd2, Wpos[1], Wpos[2], cols));
             else if (nl == 1)
                 MCB_CUDA(launch_k(pdl, blk_w_kernel<2>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
-                                  bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd1, Wpos[1], nul));
+                                  bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd1, Wpos[1], nul, cols));
             else
                 MCB_CUDA(launch_k(pdl, blk_w_kernel<1>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
                                   bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), (const uint64_t *)nullptr, 0, 0, nul,
-                                  nul));
+                                  nul, cols));
         }
         // this block's tail rewrites the parity buffers the far update two blocks back reads
         if (par_far[par]) MCB_CUDA(cudaStreamWaitEvent(st, s->ev_par[par], 0));
