@@ -218,9 +218,8 @@ int mcbgpu_solver_kernel_stats(mcbgpu_solver *s, mcbgpu_kernel_stat *out, int ma
 int mcbgpu_solver_diagnostics(mcbgpu_solver *s, int64_t *out, int n, int reset);
 /* Search shapes of the blocked run (no counterpart in the reference, whose host scan
  * has no shape).  A shape sets the pivot search's window (W tiles a CTA scans per
- * step, by how many of the block's 64 pivots are known), the local pivots after
- * which a CTA ends its step, and how far past the previous block's last pivot the
- * streaming pass reaches.  Every shape gives the same result; only the time
+ * step, by how many of the block's 64 pivots are known) and how far past the previous
+ * two blocks' last pivots the W pass reaches.  Every shape gives the same result; only the time
  * differs.  A solve is cut into MCBGPU_SHAPE_SEGMENTS segments of 64-iteration
  * blocks, each with its own shape (candidate 0, the built-in default, until tuned).
  *
@@ -234,8 +233,9 @@ int mcbgpu_solver_diagnostics(mcbgpu_solver *s, int64_t *out, int n, int reset);
  *   segment and shape the default stays.
  * set_shape: force one candidate for every block (-1: back to the per-segment choice).
  * shapes: the candidates' parameters, MCBGPU_SHAPE_INTS each (window early, rank it
- *   ends at, window middle, rank the tail window starts at, window tail, local-pivot
- *   limit, streaming reach in percent), their number, and each segment's shape. */
+ *   ends at, window middle, rank the tail window starts at, window tail, 8 (once the
+ *   local pivots after which a CTA ended its step; a step has no such limit any more),
+ *   reach of the W pass in percent), their number, and each segment's shape. */
 #define MCBGPU_SHAPE_SEGMENTS 4
 #define MCBGPU_SHAPE_INTS 7
 int mcbgpu_solver_tune(mcbgpu_solver *s, double *ms_per_block, int32_t *chosen, void *stream);

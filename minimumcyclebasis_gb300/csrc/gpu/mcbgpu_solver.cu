@@ -46,26 +46,14 @@ constexpr unsigned kSpinLimit = 1u << 24;
 constexpr int kDiagWords = 48;  // counters of mcbgpu_solver_diagnostics (the pivot kernel's check area follows)
 // Shape parameters of the blocked search; each can be overridden at build time
 // (-DMCB_LMAX=... and so on) to sweep them.
-#ifndef MCB_LMAX
-#define MCB_LMAX 6
-#endif
-#ifndef MCB_WIN_TILES
-#define MCB_WIN_TILES 6
-#endif
 #ifndef MCB_UPD_ROWS
 #define MCB_UPD_ROWS 8
 #endif
 #ifndef MCB_W_CHUNK
 #define MCB_W_CHUNK 8
 #endif
-#ifndef MCB_OTF_PAIRS
-#define MCB_OTF_PAIRS 1  // pivot kernel: walk two candidates per thread together on the fly
-#endif
 #ifndef MCB_W_PREFETCH
 #define MCB_W_PREFETCH 1  // streaming pass: bulk L2 prefetch of the CTA's next tile
-#endif
-#ifndef MCB_PIVOT_DIV
-#define MCB_PIVOT_DIV 1  // pivot kernel grid = SM count / MCB_PIVOT_DIV
 #endif
 #ifndef MCB_GROUP
 #define MCB_GROUP 2  // blocks per streaming pass (1..3); the later blocks' W by blk_wfix_kernel
@@ -80,39 +68,10 @@ constexpr int kGStride = kGroup == 3 ? 4 : kGroup;  // words per coordinate in t
 #define MCB_UPD_SPLIT 1  // warps per row group in the block update (1, 2, 4 or 8)
 #endif
 
-#ifndef MCB_EARLY_WIN
-#define MCB_EARLY_WIN 2  // window while the rank is below MCB_EARLY_RANK
-#endif
-#ifndef MCB_EARLY_RANK
-#define MCB_EARLY_RANK 48
-#endif
-#ifndef MCB_TAIL_WIN
-#define MCB_TAIL_WIN 8  // window once the rank is at least MCB_TAIL_RANK
-#endif
-#ifndef MCB_TAIL_RANK
-#define MCB_TAIL_RANK 60
-#endif
 #ifndef MCB_PDL
 #define MCB_PDL 1  // blocked run: critical-path kernels launched with programmatic stream serialisation
 #endif
-#ifndef MCB_MERGE_CHUNKED
-#define MCB_MERGE_CHUNKED 0  // merge echelon by chunks of 32 with a table rebuild per chunk (1) or serially (0)
-#endif
-#ifndef MCB_MERGE_FAST
-#define MCB_MERGE_FAST 1  // merge: skip the sort and echelon when no report lies below D
-#endif
-#ifndef MCB_LMAX_CAP
-#define MCB_LMAX_CAP 8  // report slots per CTA and step: the largest local-pivot limit a shape may use
-#endif
-#ifndef MCB_WIN_CAP
-#define MCB_WIN_CAP 12  // the largest window (tiles per CTA and step) a shape may use
-#endif
-constexpr int kLmax = MCB_LMAX_CAP;       // report slots per CTA and pivot step
-constexpr int kWinTiles = MCB_WIN_TILES;  // tiles a CTA scans per pivot step (default shape)
-static_assert(MCB_LMAX >= 1 && MCB_LMAX <= kLmax, "MCB_LMAX above MCB_LMAX_CAP");
-static_assert(MCB_EARLY_WIN <= MCB_WIN_CAP && MCB_WIN_TILES <= MCB_WIN_CAP && MCB_TAIL_WIN <= MCB_WIN_CAP &&
-                  MCB_WIN_CAP <= 32, "a window above MCB_WIN_CAP (at most 32)");
-
+constexpr int kMaxWin = 32;  // the largest window (tiles per CTA and step) a shape may use
 // The runtime shape of the blocked search (blk_pivot_kernel and the streaming pass's
 // reach).  Every shape gives the same pivots (the search is exact for any window
 // and local-pivot limit); only the time differs, by graph and by how far a solve has
@@ -121,14 +80,11 @@ struct PivotShape {
     int win_early, rank_early;  // tiles per CTA and step while fewer than rank_early pivots are known
     int win_mid;                // ... from rank_early on
     int rank_tail, win_tail;    // ... once rank_tail pivots are known
-    int lmax;                   // local pivots after which a CTA ends its step (<= kLmax)
     int stream_pct;             // the streaming pass reaches this percent past the last block's last pivot
 };
-constexpr PivotShape kDefaultShape = {MCB_EARLY_WIN, MCB_EARLY_RANK, MCB_WIN_TILES, MCB_TAIL_RANK,
-                                      MCB_TAIL_WIN,  MCB_LMAX,       25};
+constexpr PivotShape kDefaultShape = {2, 48, 8, 60, 16, 25};
 constexpr int kUpdRows = MCB_UPD_ROWS;    // rows per warp group in the block update (<= 32)
 constexpr unsigned long long kNone = 0xFFFFFFFFFFFFFFFFull;
-constexpr unsigned kNoIndex = 0xFFFFFFFFu;
 
 // Kernel classes for the optional per-launch profile (events + algorithmic bytes).
 enum KernelClass {
@@ -148,9 +104,8 @@ struct IterSlot {            // state of one per-iteration search
 struct BlockState {
     unsigned rank, epoch, b;
     unsigned failed;               // a block ran out of candidates: every later block's kernels return at once
-    long long last_pivot;          // rank of the previous block's last pivot
+    long long last_pivot[2];       // by block parity: rank of the block's last pivot
     long long pred_tiles;          // tiles the streaming pass computes for this block
-    long long max_tile[2];         // by block parity: deepest tile the block's pivot search touched
     unsigned long long total;      // running 64-bit total weight of the basis
     unsigned tail_ok, pad_;        // the pivot kernel's CTA 0 resolved the block
     long long pair_tiles;          // tiles the grouped streaming pass computed for the group's later blocks
@@ -495,7 +450,7 @@ __device__ __forceinline__ void load_columns(const uint64_t *__restrict__ S, int
 
 __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__restrict__ S, int P, int e0, int b, int Wb,
                                                            uint64_t *__restrict__ T, BlockState *bs, long long ntiles,
-                                                           GridBar *gb, long long window_tiles, int stream_pct,
+                                                           GridBar *gb, long long slack_tiles, int stream_pct,
                                                            uint64_t *__restrict__ Tg, GroupArgs ga) {
     griddep_wait();
     griddep_launch();
@@ -506,14 +461,12 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
         }
         return;
     }
-    const int par = (e0 >> 6) & 1;
-    // stream stream_pct percent past the previous block's deepest pivot; the pivot
-    // kernel computes any further tile it needs
+    // stream stream_pct percent past the last two blocks' deepest pivot and a tile per
+    // CTA of the pivot kernel, which computes any further tile it needs
     long long pred = ntiles;
     if (e0 != 0) {
-        const long long lp = bs->last_pivot + 1;
-        const long long a = (lp + lp * stream_pct / 100) / kTile + 1, m = bs->max_tile[par ^ 1] + 1;
-        pred = (a > m ? a : m) + window_tiles;
+        const long long lp = max(bs->last_pivot[0], e0 >= 128 ? bs->last_pivot[1] : 0ll) + 1;
+        pred = (lp + lp * stream_pct / 100) / kTile + 1 + slack_tiles;
     }
     const int later = (ga.b1 > 0 ? 1 : 0) + (ga.b2 > 0 ? 1 : 0);  // the pass serves the group's later blocks too
     if (later > 0 && e0 != 0) pred += pred * MCB_PAIR_MARGIN * later / 100;
@@ -528,7 +481,6 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
         bs->b = (unsigned)b;
         bs->pred_tiles = pred;
         if (later > 0) bs->pair_tiles = pred;  // read by the later blocks' blk_wfix_kernel
-        bs->max_tile[par] = 0;                 // the pivot kernel's; the other one is read above
         if (ga.nz) {
             bs->nz_count[(ga.slot + 1) % 3] = 0;  // the next group's
             bs->by_columns = cols ? 1u : 0u;
@@ -587,21 +539,16 @@ __device__ __forceinline__ uint64_t fr_reduce(uint64_t W, const uint64_t (*tab)[
     return r;
 }
 
-// Build tab from the basis held in shared memory (rank vectors, pivot bits).
-__device__ void fr_build(uint64_t (*tab)[256], const uint64_t *basis, const unsigned *pivbit, unsigned rank) {
-    __shared__ uint64_t byBit[64];
-    if (threadIdx.x < 64) byBit[threadIdx.x] = 0;
-    cta_sync();
-    for (unsigned q = threadIdx.x; q < rank; q += blockDim.x) byBit[pivbit[q] & 63] = basis[q];
-    cta_sync();
+// Build tab from a reduced basis held by pivot bit (0: no vector has that pivot).
+__device__ __forceinline__ void fr_build(uint64_t (*tab)[256], const uint64_t *by_bit) {
     for (int idx = threadIdx.x; idx < 8 * 256; idx += blockDim.x) {
-        int g = idx >> 8, pat = idx & 255;
+        const int g = idx >> 8, pat = idx & 255;
         uint64_t v = 0;
+#pragma unroll
         for (int i = 0; i < 8; i++)
-            if (pat & (1 << i)) v ^= byBit[8 * g + i];
+            if (pat & (1 << i)) v ^= by_bit[8 * g + i];
         tab[g][pat] = v;
     }
-    cta_sync();
 }
 
 // ---- grid-wide barrier for the cooperative pivot kernel ----------------------
@@ -1052,102 +999,156 @@ __global__ void __launch_bounds__(kTile) blk_wfix_kernel(const int32_t *__restri
     if ((tid & 31) == 0 && nb) atomicAdd(bytes, nb);
 }
 
-// Cooperative pivot extraction, several pivots per grid barrier.
+// Cooperative pivot extraction.
 //
-// Definitions: B = the pivots found so far (a reduced row-echelon basis, held by
-// every CTA as Four-Russians tables); s = scan start: every candidate before s has
-// its W in span(B).  A pivot is a candidate whose W is not in the span of all
-// earlier W's.
+// The block's pivots are the rank-first basis of the W's: the candidates, in rank
+// order, whose W is not in the span of all earlier W's.  Adding an earlier row to a
+// later one changes neither the rank of any prefix of the rows nor which rows are
+// pivots, so rows may be reduced by any earlier ones on the way.
 //
-// Step, part 1 (no communication): CTA c scans its own tiles t = c (mod G) from s
-// on, up to the shape's window of them.  It keeps a local basis B ∪ L_c and, in rank
-// order, turns every candidate whose residual against B ∪ L_c is non-zero into a
-// local pivot (appended to L_c).  It stops early after the shape's lmax local
-// pivots.  It reports
-// its local pivots (rank, W) and `end`: every candidate of its tiles below `end`
-// has been processed.
-// Part 2, after one grid barrier, in every CTA identically: D = min over CTAs of
-// `end`.  Every candidate z below D is in span(B ∪ L_c' before z) for its CTA c',
-// so span(W's below r) = span(B ∪ reported local pivots below r) for any r <= D.
-// Hence the global pivots below D are exactly the reported local pivots below D
-// that, taken in rank order, are not in the span of B and the ones accepted
-// before them.  Accept them that way (first non-zero residual against the global
-// tables, add, repeat), then s = D.
-// The reductions below leave one value per warp in a shared slot array (plain
-// stores by lane 0, no shared atomics) and every thread combines the slots after
-// the barrier.  A caller must pass a barrier between reading one call's slots and
-// the next call that writes the same slots.
+// Step, part 1 (no communication): the scan starts at tile t0 (every candidate before
+// it has its W in the span of B, the pivots found so far).  CTA c takes wsz tiles from
+// t0 + c wsz on, reduces their W's by B (Four-Russians tables of a reduced basis) and
+// eliminates what is left: its local pivots, as residuals.
+// Part 2, after one grid barrier, in every CTA identically: the pivots of the whole
+// window are among the CTAs' local pivots (a row spanned by earlier rows of its CTA is
+// spanned by earlier rows); eliminating the reported ones, which lie in rank order CTA
+// after CTA, finds them; B takes them in, and t0 moves past the window.
+//
+// What bounds a step is latency: the 64 picks in a row, barriers and L2 round trips.
+// The elimination (eliminate()) therefore runs warp after warp on rows in rank order,
+// where the next pivot is a ballot away (about 120 cycles per pick), instead of one
+// pick per two CTA barriers with the tables rebuilt for each, and a CTA reports all its
+// local pivots, so that a step's window is searched to its end.  Microseconds per
+// block, before / now: 32 x 32 grid 212 / 38 (10.3 steps / 1), 10k-vertex RGG 118 /
+// 30 (5.3 / 1), 100k-point planar-chain graph 88 / 31 (2.0 / 1.0), 50k-vertex
+// random graph 217 / 114 (6.9 / 3.9).  (Eliminating eight columns at a time, the first
+// row of each byte pattern by shared-memory atomics, took 17 us per merge of 465 rows.)
 constexpr int kPivotThreads = 512;        // threads of a pivot-kernel CTA
 constexpr int kWarps = kPivotThreads / 32;
-constexpr int kWinMax = MCB_WIN_CAP;  // largest window
-constexpr int kWinW = kWinMax * kTile;  // W's the window buffer holds
+constexpr int kMaxLocal = 64;             // local pivots a CTA can report per step (W has 64 columns)
+constexpr int kMaxGrid = 256;             // CTAs of a pivot kernel at most
+constexpr int kMissWin = 4;               // tiles per CTA and step where W is computed on the way
+constexpr int kChunkTiles = 4;            // tiles of the window loaded together (kChunkRows rows per thread)
+constexpr int kChunkRows = kChunkTiles * kTile / kPivotThreads;
 
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-    for (int d = 16; d > 0; d >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, d);
-        v = o < v ? o : v;
+// Rows of an elimination in rank order: rank (relative to the step's first candidate)
+// and residual, in shared memory.
+struct RowList {
+    uint64_t *w;
+    unsigned *key;
+};
+
+// Shared scratch of eliminate().
+struct ElimShared {
+    ulonglong2 pick[64];  // chosen rows' residuals and pivot bits, in order of choice
+    unsigned pos[64];     // their places in the row list
+    int np[2];            // how many, after even and odd warps' turns
+    uint64_t pw[64];      // the result in rank order: residuals
+    unsigned pkey[64];    // and ranks
+};
+
+__device__ __forceinline__ uint64_t join64(unsigned lo, unsigned hi) { return ((uint64_t)hi << 32) | lo; }
+
+// Adds chosen row (v) with its pivot bit (low) to w if w has that bit.
+__device__ __forceinline__ void add_pick(unsigned &wl, unsigned &wh, const ulonglong2 &p) {
+    const unsigned hit = (wl & (unsigned)p.y) | (wh & (unsigned)(p.y >> 32));
+    if (hit) {
+        wl ^= (unsigned)p.x;
+        wh ^= (unsigned)(p.x >> 32);
     }
-    return v;
 }
 
-// Minimum over the CTA (every thread gets it).
-__device__ __forceinline__ unsigned long long block_min_u64(unsigned long long v, unsigned long long *slots) {
-    v = warp_min_u64(v);
-    if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = v;
-    cta_sync();
-    unsigned long long m = slots[0];
-#pragma unroll
-    for (int w = 1; w < kWarps; w++) m = slots[w] < m ? slots[w] : m;
-    return m;
-}
-
-// Adds v (already reduced against the basis, v != 0) to an RREF basis held as
-// vectors + pivot bits + Four-Russians tables.  Called by the whole CTA; `slots`
-// holds kWarps words.
-__device__ void basis_add(uint64_t (*tab)[256], uint64_t *basis, unsigned *piv, int &rank, uint64_t v,
-                          unsigned long long *slots) {
-    const unsigned qb = (unsigned)(__ffsll((long long)v) - 1) & 63u;
-    const bool mine = threadIdx.x < (unsigned)rank && ((basis[threadIdx.x] >> qb) & 1ull);
-    unsigned long long m = mine ? (1ull << (piv[threadIdx.x] & 63u)) : 0ull;
-    for (int d = 16; d > 0; d >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, d);
-    if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = m;
-    cta_sync();
-    unsigned long long chg = 1ull << qb;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) chg |= slots[w];
-    for (int idx = threadIdx.x; idx < 8 * 256; idx += blockDim.x) {
-        const int g = idx >> 8, pat = idx & 255;
-        if (__popc(pat & (unsigned)((chg >> (8 * g)) & 255)) & 1) (&tab[0][0])[idx] ^= v;
-    }
-    if (mine) basis[threadIdx.x] ^= v;
-    if (threadIdx.x == 0 && rank < 64) {
-        basis[rank] = v;
-        piv[rank] = qb;
-    }
-    rank++;
-    cta_sync();
-}
-
-// First window position p in [from, valid) whose W has a non-zero residual against
-// tab, or kNoIndex.  Window positions are in rank order.  `slots` holds kWarps words.
-__device__ unsigned window_first_nonzero(const uint64_t *win, const uint64_t (*tab)[256], unsigned from,
-                                         unsigned valid, unsigned *slots) {
-    unsigned best = kNoIndex;
-    for (unsigned base = from & ~(unsigned)(kPivotThreads - 1); base < valid; base += kPivotThreads) {
-        const unsigned p = base + threadIdx.x;
-        const bool nz = p >= from && p < valid && fr_reduce(win[p], tab) != 0;
-        const unsigned bal = __ballot_sync(0xffffffffu, nz);
-        if (bal) {  // warp-uniform: this warp's first hit
-            best = base + (threadIdx.x & ~31u) + (unsigned)(__ffs(bal) - 1);
-            break;
+// The rank-first basis of rows[0, n); returns its size (at most 64), with es.pw / es.pkey
+// the chosen rows in rank order.  Every thread holds one row, every warp 32 consecutive
+// ones.  Warp after warp chooses: first among the rows with a bit in the low half (the
+// first such row is the next pivot and is added to the later rows with its lowest bit),
+// then among those left with a bit in the high half (fewer columns have a subset of the
+// pivots, so the low half may go first); then the later warps add the new pivots to
+// theirs.  A pick is one chain of vote, shuffle and select on 32-bit words; the loop is
+// kept short because a lone warp's time goes by the length of that chain (64-bit words,
+// two rows per lane: 260 cycles a pick; eight rows fetched and reduced per turn: slower
+// still, their code does not stay in the instruction buffer).
+// Called by the whole CTA with a barrier since the rows were written; ends with one.
+__device__ __noinline__ int eliminate(const RowList rows, unsigned n, int most, ElimShared &es) {
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int np = 0;
+    for (unsigned r0 = 0; r0 < n && np < most; r0 += kPivotThreads) {
+        const unsigned i = r0 + tid;
+        const uint64_t w = i < n ? rows.w[i] : 0ull;
+        unsigned wl = (unsigned)w, wh = (unsigned)(w >> 32);
+        const unsigned nwarps = min((unsigned)kWarps, (n - r0 + 31) / 32);
+        int added = 0;  // chosen rows already added to this warp's
+        for (unsigned ch = 0; ch < nwarps; ch++) {
+            if (warp >= ch) {
+#pragma unroll 4
+                for (; added < np; added++) add_pick(wl, wh, es.pick[added]);
+            }
+            if (warp == ch) {
+                int q = np;
+                for (unsigned m; (m = __ballot_sync(0xffffffffu, wl != 0)) != 0 && q < 64; q++) {
+                    const int at = __ffs(m) - 1;
+                    const unsigned vl = __shfl_sync(0xffffffffu, wl, at), vh = __shfl_sync(0xffffffffu, wh, at);
+                    const unsigned low = vl & (0u - vl);
+                    if (wl & low) {
+                        wl ^= vl;
+                        wh ^= vh;
+                    }
+                    if ((int)lane == at) {
+                        es.pick[q] = make_ulonglong2(join64(vl, vh), low);
+                        es.pos[q] = i;
+                    }
+                }
+                for (unsigned m; (m = __ballot_sync(0xffffffffu, wh != 0)) != 0 && q < 64; q++) {
+                    const int at = __ffs(m) - 1;
+                    const unsigned vh = __shfl_sync(0xffffffffu, wh, at);
+                    const unsigned low = vh & (0u - vh);
+                    if (wh & low) wh ^= vh;
+                    if ((int)lane == at) {
+                        es.pick[q] = make_ulonglong2(join64(0u, vh), join64(0u, low));
+                        es.pos[q] = i;
+                    }
+                }
+                if (lane == 0) es.np[ch & 1] = q;
+            }
+            cta_sync();
+            np = es.np[ch & 1];  // written again two barriers on
+            if (np >= most) break;
         }
     }
-    if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = best;
+    if ((int)tid < np) {  // in rank order
+        const unsigned at = es.pos[tid];
+        int place = 0;
+        for (int j = 0; j < np; j++) place += es.pos[j] < at;
+        es.pw[place] = es.pick[tid].x;
+        es.pkey[place] = rows.key[at];
+    }
     cta_sync();
-    unsigned r = slots[0];
-#pragma unroll
-    for (int w = 1; w < kWarps; w++) r = slots[w] < r ? slots[w] : r;
-    return r;
+    return np;
+}
+
+// Adds the np rows chosen last to a reduced basis held by pivot bit (every row was
+// reduced by it before the elimination).  Warp 0.
+__device__ void basis_add(uint64_t *by_bit, int np, const ElimShared &es) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t a0 = by_bit[lane], b0 = by_bit[lane + 32];
+    unsigned al = (unsigned)a0, ah = (unsigned)(a0 >> 32), bl = (unsigned)b0, bh = (unsigned)(b0 >> 32);
+#pragma unroll 4
+    for (int q = 0; q < np; q++) {
+        const ulonglong2 p = es.pick[q];
+        add_pick(al, ah, p);
+        add_pick(bl, bh, p);
+        if (((unsigned)p.y >> lane) & 1u) {
+            al = (unsigned)p.x;
+            ah = (unsigned)(p.x >> 32);
+        }
+        if (((unsigned)(p.y >> 32) >> lane) & 1u) {
+            bl = (unsigned)p.x;
+            bh = (unsigned)(p.x >> 32);
+        }
+    }
+    by_bit[lane] = join64(al, ah);
+    by_bit[lane + 32] = join64(bl, bh);
 }
 
 // Index of the j-th set bit of a window mask.
@@ -1165,6 +1166,7 @@ struct TailArgs {
     unsigned pair_cap;
     int P, e0, Wb;
     int par;  // block parity: which gcol / sorted pairs to write
+    int first;  // the first block of its group: its W pass is its own
 };
 
 // Named CTA barrier 1 over the warps 1.. of the CTA (warp 0 is busy elsewhere);
@@ -1234,39 +1236,67 @@ __device__ bool resolve_block(BlockState *bs, int rank, const int64_t *__restric
         // i < k are final, so gcol[k] bit i = A[i][p_k].
         uint64_t a0 = s_w[lane], a1 = s_w[32 + lane];
         warp_transpose64(a0, a1);  // row j of A = bit j of every W
-        // The loop carries only what the next iteration needs (row k + 1 after this
-        // iteration's XORs); the selections stay in the lane of their iteration and
-        // gcol is read off the final rows afterwards.
-        uint64_t m0 = 1ull << lane, m1 = 1ull << (32 + lane);
-        uint64_t used = 0;
-        int psel0 = 0, psel1 = 0;  // lane l: the pivots of iterations l and l + 32
+        // The loop is one chain per iteration (fetch row k, its first unused pivot as a bit,
+        // add it to the later rows with that bit), so it works on 32-bit halves and bits
+        // instead of indices; the selections stay in the lane of their iteration and gcol
+        // is read off the final rows afterwards.
+        unsigned al0 = (unsigned)a0, ah0 = (unsigned)(a0 >> 32), al1 = (unsigned)a1, ah1 = (unsigned)(a1 >> 32);
+        unsigned ml0 = 1u << lane, mh0 = 0, ml1 = 0, mh1 = 1u << lane;
+        unsigned freel = 0xffffffffu, freeh = 0xffffffffu;  // pivots not selected yet
+        unsigned sl0 = 0, sh0 = 0, sl1 = 0, sh1 = 0;        // lane l: the pivots (bits) of iterations l and l + 32
         bool fail = false;
-        for (int k = 0; k < b; k++) {
-            const uint64_t ak = __shfl_sync(0xffffffffu, k < 32 ? a0 : a1, k & 31);
-            const uint64_t mk = __shfl_sync(0xffffffffu, k < 32 ? m0 : m1, k & 31);
-            const uint64_t cand = ak & ~used;
-            if (!cand) {  // warp-uniform
+        const int b0 = b < 32 ? b : 32;
+        for (int k = 0; k < b0; k++) {
+            const unsigned rl = __shfl_sync(0xffffffffu, al0, k), rh = __shfl_sync(0xffffffffu, ah0, k);
+            const unsigned nl = __shfl_sync(0xffffffffu, ml0, k), nh = __shfl_sync(0xffffffffu, mh0, k);
+            const unsigned cl = rl & freel, chh = rh & freeh;
+            const unsigned bl = cl & (0u - cl), bh = cl ? 0u : chh & (0u - chh);
+            if (!(bl | bh)) {  // warp-uniform
                 fail = true;
                 break;
             }
-            const int p = __ffsll((long long)cand) - 1;
-            used |= 1ull << p;
-            if (lane == (k & 31)) {
-                if (k < 32)
-                    psel0 = p;
-                else
-                    psel1 = p;
+            freel &= ~bl;
+            freeh &= ~bh;
+            if (lane == k) {
+                sl0 = bl;
+                sh0 = bh;
             }
-            const bool h0 = (a0 >> p) & 1ull, h1 = (a1 >> p) & 1ull;
-            if (lane > k && h0) {
-                a0 ^= ak;
-                m0 ^= mk;
+            if (lane > k && ((al0 & bl) | (ah0 & bh))) {
+                al0 ^= rl;
+                ah0 ^= rh;
+                ml0 ^= nl;
+                mh0 ^= nh;
             }
-            if (32 + lane > k && h1) {
-                a1 ^= ak;
-                m1 ^= mk;
+            if ((al1 & bl) | (ah1 & bh)) {
+                al1 ^= rl;
+                ah1 ^= rh;
+                ml1 ^= nl;
+                mh1 ^= nh;
             }
         }
+        for (int k = 0; k < b - 32 && !fail; k++) {
+            const unsigned rl = __shfl_sync(0xffffffffu, al1, k), rh = __shfl_sync(0xffffffffu, ah1, k);
+            const unsigned nl = __shfl_sync(0xffffffffu, ml1, k), nh = __shfl_sync(0xffffffffu, mh1, k);
+            const unsigned cl = rl & freel, chh = rh & freeh;
+            const unsigned bl = cl & (0u - cl), bh = cl ? 0u : chh & (0u - chh);
+            fail = !(bl | bh);  // warp-uniform
+            freel &= ~bl;
+            freeh &= ~bh;
+            if (lane == k) {
+                sl1 = bl;
+                sh1 = bh;
+            }
+            if (lane > k && ((al1 & bl) | (ah1 & bh))) {
+                al1 ^= rl;
+                ah1 ^= rh;
+                ml1 ^= nl;
+                mh1 ^= nh;
+            }
+        }
+        a0 = join64(al0, ah0);
+        a1 = join64(al1, ah1);
+        const uint64_t m0 = join64(ml0, mh0), m1 = join64(ml1, mh1);
+        const int psel0 = __ffsll((long long)join64(sl0, sh0)) - 1, psel1 = __ffsll((long long)join64(sl1, sh1)) - 1;
         if (fail) {
             if (lane == 0) s_fail = 1;
         } else {
@@ -1420,50 +1450,29 @@ __device__ void materialize_rows(const TailArgs &ta, const BlockState *bs, int b
     }
 }
 
-#ifdef MCB_MERGE_PROFILE
-__device__ long long g_merge_prof[5];
-#define MERGE_STAMP(i)                                                  \
-    do {                                                                \
-        const long long mp1 = clock64();                                \
-        if (threadIdx.x == 0 && c == 0) g_merge_prof[i] += mp1 - mp0;  \
-        mp0 = mp1;                                                      \
-    } while (0)
-#else
-#define MERGE_STAMP(i) \
-    do {               \
-    } while (0)
-#endif
-#ifdef MCB_SCAN_PROFILE
-__device__ long long g_scan_prof[4];
-#endif
 #ifndef MCB_PIVOT_MINB
-#define MCB_PIVOT_MINB 1  // pivot-kernel CTAs the register budget is sized for per SM
+#define MCB_PIVOT_MINB 1  // pivot CTAs per SM the registers are budgeted for (2: spills, 8% slower)
 #endif
+// Dynamic shared memory: B's tables (16 KB) | the row list (G x kMaxLocal rows at
+// least), which the block tail reuses as scratch (P + 1 counters; kMatCols columns).
 __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kernel(
     long long K, const int64_t *__restrict__ off, const int32_t *__restrict__ coords,
     const int32_t *__restrict__ head, const int32_t *__restrict__ tile_minc, const uint64_t *__restrict__ T,
-    int bound, BlockState *bs,
-    uint64_t *Warr, unsigned *tile_epoch, unsigned long long *reports, GridBar *gb, unsigned *status,
-    unsigned long long *bytes, unsigned long long *diag, unsigned long long *dbg, TailArgs ta, PivotShape sh) {
-    // dynamic shared memory: global tables | local tables | window W's | merge buffers | report staging
+    int bound, BlockState *bs, uint64_t *Warr, unsigned *tile_epoch, uint64_t *rep_w, unsigned *rep_key, unsigned *rep_n, GridBar *gb,
+    unsigned *status, unsigned long long *bytes, unsigned long long *diag, unsigned long long *dbg, TailArgs ta,
+    PivotShape sh, unsigned list_cap) {
     extern __shared__ __align__(128) unsigned char dsm[];
     const unsigned G = gridDim.x;
     uint64_t(*gtab)[256] = reinterpret_cast<uint64_t(*)[256]>(dsm);
-    uint64_t(*ltab)[256] = reinterpret_cast<uint64_t(*)[256]>(dsm + 16384);
-    uint64_t *win = reinterpret_cast<uint64_t *>(dsm + 32768);                                      // kWinW
-    unsigned long long *mr = reinterpret_cast<unsigned long long *>(dsm + 32768 + 8 * (size_t)kWinW);  // 2 G kLmax
-    uint64_t *mw = reinterpret_cast<uint64_t *>(mr + 2 * (size_t)G * kLmax);                          // 3 G kLmax
-    unsigned long long *lr = mr + 5 * (size_t)G * kLmax;  // G (2 kLmax + 2)
-    __shared__ uint64_t gbasis[64], lbasis[64];
-    __shared__ unsigned gpiv[64], lpiv[64];
-    __shared__ unsigned s_first[kWarps], s_wcnt[kWarps];
-    __shared__ unsigned long long s_chg[kWarps], s_dmin[kWarps];
-    __shared__ unsigned s_tag[kWinMax];
-    __shared__ __align__(8) uint64_t s_bar;  // completion of the window's bulk copies
-    __shared__ uint64_t s_newv[64];
-    __shared__ unsigned s_newq[64];
-    __shared__ int s_nnew;
-    __shared__ unsigned long long sr_rank[kLmax], sr_w[kLmax];
+    RowList rows;
+    rows.w = reinterpret_cast<uint64_t *>(dsm + 16384);
+    rows.key = reinterpret_cast<unsigned *>(rows.w + list_cap);
+    __shared__ ElimShared es;
+    __shared__ uint64_t s_basis[64];               // B, reduced, by pivot bit
+    __shared__ long long s_prank[64];              // ranks of the pivots found
+    __shared__ unsigned s_tag[kMaxWin];
+    __shared__ __align__(16) unsigned s_part[kChunkRows * kWarps];  // nonzero rows by (row of the chunk, warp)
+    __shared__ unsigned s_off[kWarps], s_start[kMaxGrid];
 
     griddep_wait();
     griddep_launch();
@@ -1478,192 +1487,125 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
     const int b = (int)bs->b;
     const long long ntiles = (K + kTile - 1) / kTile;
     const long long c = blockIdx.x;
+    const long long pred = ta.first ? bs->pred_tiles : bs->pair_tiles;
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned gen = ld_acquire_u32(&gb->gen);
-    for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&gtab[0][0])[i] = 0;
-    if (threadIdx.x == 0) {
-        mbar_init(&s_bar, 1);
-        fence_mbar_init();
-    }
-    unsigned mphase = 0;  // uses of s_bar so far
-    long long maxt = 0;   // deepest tile this CTA touched
-    long long s = 0;
+    if (tid < 64) s_basis[tid] = 0;
+    long long t0 = 0;    // scan start
     int grank = 0;
     bool ok = true;
     unsigned k = 0;
-    cta_sync();
     while (grank < b) {
-        unsigned long long *rep_rank =
-            reports + (size_t)(k & 1) * G * (2 * kLmax + 2);
-        unsigned long long *rep_w = rep_rank + (size_t)G * kLmax;
-        unsigned long long *rep_end = rep_w + (size_t)G * kLmax;
-        unsigned long long *rep_n = rep_end + G;
         // ---- part 1: local pivots over this CTA's window ----
-        const long long c0 = clock64();
-        for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&ltab[0][0])[i] = (&gtab[0][0])[i];
-        if (threadIdx.x < 64) {
-            lbasis[threadIdx.x] = gbasis[threadIdx.x];
-            lpiv[threadIdx.x] = gpiv[threadIdx.x];
-        }
-        int lrank = grank;
-        // window: this CTA's tiles tf, tf + G, ... (t = c mod G) from the scan start on
-        const long long t0 = s / kTile;
-        const long long tf = t0 + (((long long)c - t0 % G) + G) % G;
-#ifdef MCB_SCAN_PROFILE
-        long long sp0 = clock64();
-#define SCAN_STAMP(i)                                                 \
-    do {                                                              \
-        const long long sp1 = clock64();                              \
-        if (threadIdx.x == 0 && c == 0) g_scan_prof[i] += sp1 - sp0; \
-        sp0 = sp1;                                                    \
-    } while (0)
-#else
-#define SCAN_STAMP(i) \
-    do {              \
-    } while (0)
-#endif
-        const int wsz = grank < sh.rank_early ? sh.win_early
-                        : grank >= sh.rank_tail ? sh.win_tail
-                                                : sh.win_mid;  // same in every CTA
-        const int nwin = tf >= ntiles ? 0 : (int)min((long long)wsz, (ntiles - 1 - tf) / G + 1);
-        if (threadIdx.x < (unsigned)nwin) s_tag[threadIdx.x] = ld_acquire_u32(&tile_epoch[tf + (long long)threadIdx.x * G]);
+        const long long cyc0 = clock64();
+        // the window, the same in every CTA: the shape's while it lies in the tiles the W
+        // pass computed, cut at their end; beyond it at most kMissWin tiles
+        int wsz = grank < sh.rank_early ? sh.win_early : grank >= sh.rank_tail ? sh.win_tail : sh.win_mid;
+        if (t0 >= pred) wsz = min(wsz, kMissWin);
+        const long long end = min(t0 + (long long)wsz * G, t0 < pred ? pred : ntiles);
+        wsz = (int)((end - t0 + G - 1) / G);
+        const long long tf = t0 + c * wsz;
+        const int nwin = tf >= end ? 0 : (int)min((long long)wsz, end - tf);
+        if (tid < (unsigned)nwin) s_tag[tid] = ld_acquire_u32(&tile_epoch[tf + tid]);
         cta_sync();
-        unsigned copymask = 0, zeromask = 0, missmask = 0;
-        for (int m = 0; m < nwin; m++) {
-            const unsigned tag = s_tag[m];
-            if ((tag >> 1) != epoch) missmask |= 1u << m;
-            else if (tag & 1u) zeromask |= 1u << m;
-            else copymask |= 1u << m;
-        }
-        maxt = nwin > 0 && tf + (long long)(nwin - 1) * G > maxt ? tf + (long long)(nwin - 1) * G : maxt;
-        // tiles the streaming pass computed: one bulk copy each into the window
-        if (copymask && threadIdx.x == 0) {
-            fence_proxy_async_smem();  // the previous step's reads of the window come first
-            mbar_arrive_expect_tx(&s_bar, (unsigned)__popc(copymask) * 8u * kTile);
-            for (unsigned mm = copymask; mm; mm &= mm - 1) {
-                const int m = __ffs(mm) - 1;
-                tma_load_1d(win + (size_t)m * kTile, Warr + (size_t)(tf + (long long)m * G) * kTile, 8u * kTile, &s_bar);
-            }
-            nb += 8ull * kTile * (unsigned)__popc(copymask);
-        }
-        for (unsigned mm = zeromask; mm; mm &= mm - 1) {
-            const int m = __ffs(mm) - 1;
-            for (int i = threadIdx.x; i < kTile; i += blockDim.x) win[(size_t)m * kTile + i] = 0;
-        }
-        n_loaded += (unsigned)__popc(copymask | zeromask);
-        SCAN_STAMP(0);
-        if (missmask) {  // tiles beyond the streaming pass: W's computed here by the whole CTA
+        unsigned missmask = 0;
+        for (int m = 0; m < nwin; m++)
+            if ((s_tag[m] >> 1) != epoch) missmask |= 1u << m;
+        if (missmask) {  // tiles beyond the W pass: their W computed here, two candidates per thread in lockstep
             const unsigned nm = (unsigned)__popc(missmask);
             unsigned nread = 0;
-#if MCB_OTF_PAIRS
-            // two candidates per thread walked together (positions idx and idx + half)
-            const unsigned tot = nm * kTile, half = (tot + 1) / 2;
-            for (unsigned idx = threadIdx.x; idx < half; idx += blockDim.x) {
+            const unsigned tot = nm * kTile, half = tot / 2;
+            for (unsigned idx = tid; idx < half; idx += kPivotThreads) {
                 const unsigned jdx = idx + half;
-                const int ma = nth_bit(missmask, idx / kTile);
-                const long long ta_ = tf + (long long)ma * G, ra = ta_ * kTile + idx % kTile;
-                const bool va = ra < K && tile_minc[ta_] < bound;
-                long long rb = -1;
-                int mb = 0;
-                if (jdx < tot) {
-                    mb = nth_bit(missmask, jdx / kTile);
-                    const long long tb_ = tf + (long long)mb * G;
-                    rb = tb_ * kTile + jdx % kTile;
-                    if (!(rb < K && tile_minc[tb_] < bound)) rb = -2;
-                }
+                const int ma = nth_bit(missmask, idx / kTile), mb = nth_bit(missmask, jdx / kTile);
+                const long long ta_ = tf + ma, tb_ = tf + mb;
+                const long long ra = ta_ * kTile + idx % kTile, rb = tb_ * kTile + jdx % kTile;
+                const bool va = ra < K && tile_minc[ta_] < bound, vb = rb < K && tile_minc[tb_] < bound;
                 uint64_t Wa = 0, Wb = 0;
-                if (va || rb >= 0) w_of_two(va ? ra : rb, va ? (rb >= 0 ? rb : -1) : -1, off, coords, head, T, bound, nread, Wa, Wb);
+                if (va || vb) w_of_two(va ? ra : rb, va && vb ? rb : -1, off, coords, head, T, bound, nread, Wa, Wb);
                 if (!va) {  // the walk ran on rb alone
                     Wb = Wa;
                     Wa = 0;
                 }
-                win[(size_t)ma * kTile + idx % kTile] = Wa;
                 Warr[ra] = Wa;
-                if (jdx < tot) {
-                    win[(size_t)mb * kTile + jdx % kTile] = rb >= 0 ? Wb : 0ull;
-                    Warr[(tf + (long long)mb * G) * kTile + jdx % kTile] = rb >= 0 ? Wb : 0ull;
-                }
+                Warr[rb] = vb ? Wb : 0ull;
             }
-#else
-            for (unsigned idx = threadIdx.x; idx < nm * kTile; idx += blockDim.x) {
-                const int m = nth_bit(missmask, idx / kTile);
-                const unsigned i = idx % kTile;
-                const long long t = tf + (long long)m * G;
-                const long long r = t * kTile + i;
-                uint64_t W = 0;
-                if (r < K && tile_minc[t] < bound) W = w_of_candidate(r, off, coords, head, T, bound, nread);
-                win[(size_t)m * kTile + i] = W;
-                Warr[r] = W;
-            }
-#endif
-            fence_proxy_async_global();  // a later step may bulk-copy these tiles
-            nb += 4ull * nread + (threadIdx.x == 0 ? 16ull * kTile * nm : 0ull);
+            nb += 4ull * nread + (tid == 0 ? 8ull * kTile * nm : 0ull);
             n_computed += nm;
+            cta_sync();  // the CTA reads its tiles back below
         }
-        SCAN_STAMP(1);
-        if (copymask) {
-            bool done = mbar_wait_bounded(&s_bar, mphase & 1u, 1u << 22);
-            mphase++;
-            if (!cta_sync_and(done)) {
-                if (threadIdx.x == 0) {
-                    mbar_wait_bounded(&s_bar, (mphase - 1) & 1u, 1u << 22);  // copies still in flight
-                    atomicOr(status, ST_WAIT_TIMEOUT);
-                    atomicExch(&gb->abort, 1u);
-                }
-                ok = false;
-                break;
-            }
-        }
-        cta_sync();
-        if (missmask && threadIdx.x == 0) {
-            __threadfence();
-            for (unsigned mm = missmask; mm; mm &= mm - 1)
-                tile_epoch[tf + (long long)(__ffs(mm) - 1) * G] = epoch << 1;
-        }
-        SCAN_STAMP(2);
-        // local echelon over the window in rank order
-        const unsigned valid = (unsigned)nwin * kTile;
-        unsigned from = (nwin > 0 && tf == t0) ? (unsigned)(s - t0 * kTile) : 0u;
+        n_loaded += (unsigned)(nwin - __popc(missmask));
         int nloc = 0;
-        long long end = K;
-        bool trunc = false;
-        for (;;) {
-            const unsigned p = window_first_nonzero(win, ltab, from, valid, s_first);
-            if (p >= valid) break;
-            const uint64_t w = win[p];
-            const uint64_t x = fr_reduce(w, ltab);
-            const long long rank = (tf + (long long)(p / kTile) * G) * kTile + (p % kTile);
-            if (threadIdx.x == 0) {
-                sr_rank[nloc] = (unsigned long long)rank;
-                sr_w[nloc] = w;
+        unsigned cnt = 0;  // rows in the list
+        for (int m0 = 0; m0 < nwin; m0 += kChunkTiles) {
+            uint64_t w[kChunkRows];
+#pragma unroll
+            for (int q = 0; q < kChunkRows; q++) {
+                const int m = m0 + q * kPivotThreads / kTile;
+                const unsigned i = (q * kPivotThreads + tid) % kTile;
+                // a computed tile's tag bit 0: every W of the tile is 0 and none is written
+                const bool in = m < nwin && (((missmask >> m) & 1u) || !(s_tag[m] & 1u));
+                w[q] = in ? __ldcg(Warr + (tf + m) * kTile + i) : 0ull;
+            }
+            nb += 8ull * kChunkRows;
+            // what B leaves, appended to the list in rank order
+            unsigned nz[kChunkRows];
+#pragma unroll
+            for (int q = 0; q < kChunkRows; q++) {
+                if (grank > 0 && w[q]) w[q] = fr_reduce(w[q], gtab);
+                nz[q] = __ballot_sync(0xffffffffu, w[q] != 0);
+                if (lane == 0) s_part[q * kWarps + warp] = __popc(nz[q]);
             }
             cta_sync();
-            basis_add(ltab, lbasis, lpiv, lrank, x, s_chg);
-            nloc++;
-            from = p + 1;
-            if (nloc == sh.lmax) {
-                end = rank + 1;
-                trunc = true;
-                break;
+            static_assert(kChunkRows * kWarps == 128, "four counts per lane");
+            const uint4 pc = reinterpret_cast<const uint4 *>(s_part)[lane];
+            const unsigned own = pc.x + pc.y + pc.z + pc.w;
+            unsigned incl = own;
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= (unsigned)d) incl += y;
+            }
+            const unsigned excl = cnt + incl - own;
+            const unsigned e1 = excl + pc.x, e2 = e1 + pc.y, e3 = e2 + pc.z;
+            const unsigned my = (warp & 2u) ? ((warp & 1u) ? e3 : e2) : ((warp & 1u) ? e1 : excl);
+#pragma unroll
+            for (int q = 0; q < kChunkRows; q++) {
+                const unsigned at = __shfl_sync(0xffffffffu, my, q * (kWarps / 4) + (warp >> 2)) +
+                                    __popc(nz[q] & ((1u << lane) - 1u));
+                if (w[q]) {
+                    rows.w[at] = w[q];
+                    rows.key[at] = (unsigned)(c * wsz + m0) * kTile + q * kPivotThreads + tid;
+                }
+            }
+            cnt += __shfl_sync(0xffffffffu, incl, 31);
+            cta_sync();
+            // eliminate when the window is through, or when the next chunk might not fit;
+            // the local pivots so far then go on as the list's first rows
+            if (m0 + kChunkTiles >= nwin || cnt + kChunkTiles * kTile > list_cap) {
+                nloc = cnt ? eliminate(rows, cnt, 64 - grank, es) : 0;
+                if (m0 + kChunkTiles < nwin) {
+                    if ((int)tid < nloc) {
+                        rows.w[tid] = es.pw[tid];
+                        rows.key[tid] = es.pkey[tid];
+                    }
+                    cnt = (unsigned)nloc;
+                    cta_sync();
+                }
             }
         }
-        SCAN_STAMP(3);
-        if (!trunc && nwin == wsz) {  // a shorter window reached the last tile: end = K
-            const long long tl = tf + (long long)(wsz - 1) * G;
-            end = (tl + 1) * kTile < K ? (tl + 1) * kTile : K;
-        }
+        if (missmask && tid < kMaxWin && ((missmask >> tid) & 1u)) tile_epoch[tf + tid] = epoch << 1;
         n_local += nloc;
-        if (threadIdx.x == 0) {
-            for (int j = 0; j < nloc; j++) {
-                rep_rank[c * kLmax + j] = sr_rank[j];
-                rep_w[c * kLmax + j] = sr_w[j];
-            }
-            rep_end[c] = (unsigned long long)end;
-            rep_n[c] = (unsigned long long)nloc;
+        uint64_t *sw = rep_w + (size_t)(k & 1) * G * kMaxLocal;
+        unsigned *sk = rep_key + (size_t)(k & 1) * G * kMaxLocal, *sn = rep_n + (size_t)(k & 1) * G;
+        if ((int)tid < nloc) {
+            sw[c * kMaxLocal + tid] = es.pw[tid];
+            sk[c * kMaxLocal + tid] = es.pkey[tid];
         }
-        const long long c1 = clock64();
+        if (tid == 0) sn[c] = (unsigned)nloc;
+        const long long cyc1 = clock64();
         nbar++;
         if (!grid_barrier(gb, G, gen)) {
-            if (threadIdx.x == 0) {  // where the wait gave up
+            if (tid == 0) {  // where the wait gave up
                 atomicExch(&diag[9], (unsigned long long)c + 1);
                 atomicExch(&diag[10], (unsigned long long)k);
                 atomicExch(&diag[11], (unsigned long long)grank);
@@ -1673,245 +1615,93 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
             ok = false;
             break;
         }
-        const long long c2 = clock64();
-        cyc_scan += c1 - c0;
-        cyc_bar += c2 - c1;
-        if (k > 0 && c == 0 && threadIdx.x < G) {  // compare the previous step's merge results
+        const long long cyc2 = clock64();
+        cyc_scan += cyc1 - cyc0;
+        cyc_bar += cyc2 - cyc1;
+        if (k > 0 && c == 0 && tid < G) {  // compare the previous step's merge results
             const unsigned long long *prev = dbg + (size_t)((k - 1) & 1) * G;
-            if (__ldcg(prev + threadIdx.x) != __ldcg(prev)) {
+            if (__ldcg(prev + tid) != __ldcg(prev)) {
                 atomicOr(status, ST_DIVERGED);
                 if (atomicCAS(&diag[16], 0ull, 1ull) == 0ull) {
                     diag[17] = (unsigned long long)(k - 1);
-                    diag[18] = (unsigned long long)threadIdx.x;
+                    diag[18] = (unsigned long long)tid;
                     diag[19] = epoch;
                 }
             }
         }
         // ---- part 2: merge (identical in every CTA) ----
-#ifdef MCB_MERGE_PROFILE
-        long long mp0 = clock64();
-#endif
-        // all reports into shared memory with independent loads (one round trip)
-        const unsigned words = G * (2 * kLmax + 2);
-        for (unsigned i = threadIdx.x; i < words; i += blockDim.x) lr[i] = __ldcg(rep_rank + i);
-        cta_sync();
-        const unsigned long long *l_rank = lr, *l_w = lr + (size_t)G * kLmax, *l_end = l_w + (size_t)G * kLmax,
-                                 *l_n = l_end + G;
-        unsigned long long dmin = kNone;
-        for (unsigned i = threadIdx.x; i < G; i += blockDim.x) dmin = l_end[i] < dmin ? l_end[i] : dmin;
-        const unsigned long long D = block_min_u64(dmin, s_dmin);
-        MERGE_STAMP(0);
-        // the reports below D, CTA by CTA (a CTA's ranks ascend): per-CTA counts,
-        // block prefix sum, copy
-        unsigned cnt = 0;
-        const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        for (unsigned cb = 0; cb < G; cb += blockDim.x) {
-            const unsigned cc = cb + threadIdx.x;
-            unsigned n = 0;
-            if (cc < G) {
-                const unsigned ln = l_n[cc] < (unsigned long long)kLmax ? (unsigned)l_n[cc] : (unsigned)kLmax;
-                while (n < ln && l_rank[(size_t)cc * kLmax + n] < D) n++;
-            }
+        // the reports, CTA after CTA: a prefix sum of the counts gives the places
+        unsigned total = 0;
+        for (unsigned cb = 0; cb < G; cb += kPivotThreads) {
+            const unsigned cc = cb + tid;
+            const unsigned n = cc < G ? min(__ldcg(sn + cc), (unsigned)kMaxLocal) : 0u;
             unsigned incl = n;
             for (int d = 1; d < 32; d <<= 1) {
-                const unsigned v = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= (unsigned)d) incl += v;
+                const unsigned y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= (unsigned)d) incl += y;
             }
-            if (lane == 31) s_wcnt[wid] = incl;
+            if (lane == 31) s_off[warp] = incl;
             cta_sync();
-            unsigned before = 0, all = 0;
-#pragma unroll
-            for (int x = 0; x < kWarps; x++) {
-                const unsigned v = s_wcnt[x];
-                before += (unsigned)x < wid ? v : 0u;
-                all += v;
+            unsigned before = total;
+            for (unsigned x = 0; x < kWarps; x++) {
+                before += x < warp ? s_off[x] : 0u;
+                total += s_off[x];
             }
-            const unsigned o = cnt + before + incl - n;
-            for (unsigned j = 0; j < n && o + j < G * kLmax; j++) {
-                mr[o + j] = l_rank[(size_t)cc * kLmax + j];
-                mw[o + j] = l_w[(size_t)cc * kLmax + j];
-            }
-            cnt += all;
+            if (cc < G) s_start[cc] = before + incl - n;
             cta_sync();
         }
-        if (cnt > G * kLmax) cnt = G * kLmax;
-        n_cand += cnt;
-        MERGE_STAMP(1);
-        int nnew = 0;
-#if MCB_MERGE_CHUNKED
-        if (!MCB_MERGE_FAST || cnt > 0) {  // no report below D: no new pivot (uniform)
-            // rank order: each candidate's position = number of smaller ranks (ranks are distinct)
-            unsigned long long *sr = mr + cnt;  // sorted ranks
-            uint64_t *sw = mw + cnt;            // sorted W
-            for (unsigned i = threadIdx.x; i < cnt; i += blockDim.x) {
-                const unsigned long long r = mr[i];
-                unsigned pos = 0;
-                for (unsigned j = 0; j < cnt; j++) pos += mr[j] < r;
-                sr[pos] = r;
-                sw[pos] = mw[i];
+        for (unsigned i = tid; i < total; i += kPivotThreads) {
+            unsigned lo = 0, hi = G - 1;  // the last CTA whose place is at most i
+            while (lo < hi) {
+                const unsigned mid = (lo + hi + 1) >> 1;
+                if (s_start[mid] <= i)
+                    lo = mid;
+                else
+                    hi = mid - 1;
             }
-            cta_sync();
-            MERGE_STAMP(2);
-            // greedy echelon in rank order, 32 candidates at a time.  Warp 0 reduces the
-            // chunk against the basis (its Four-Russians tables hold every pivot
-            // accepted so far, this step's included), accepts in order the candidates
-            // whose residual is not in the span of the basis and of the chunk's accepted
-            // ones before them, and brings those to reduced form among themselves
-            // (latest first); then the whole CTA clears their pivot bits from the basis,
-            // appends them and rebuilds the tables for the next chunk.
-            for (unsigned base = 0; base < cnt && grank < b; base += 32) {
-                if (threadIdx.x < 32) {
-                    int nn = 0;
-                    uint64_t z = base + lane < cnt ? fr_reduce(sw[base + lane], gtab) : 0ull;
-                    for (;;) {
-                        const unsigned bal = __ballot_sync(0xffffffffu, z != 0);
-                        if (!bal || grank + nn >= b) break;
-                        const int pl = __ffs(bal) - 1;
-                        const uint64_t v = __shfl_sync(0xffffffffu, z, pl);
-                        const unsigned qb = (unsigned)(__ffsll((long long)v) - 1);
-                        if (lane == 0) {
-                            s_newv[nn] = v;
-                            s_newq[nn] = qb;
-                            if (c == 0) {
-                                bs->pivrank[grank + nn] = (long long)sr[base + pl];
-                                bs->pivW[grank + nn] = sw[base + pl];
-                            }
-                        }
-                        nn++;
-                        if ((z >> qb) & 1ull) z ^= v;
-                    }
-                    __syncwarp();
-                    uint64_t va = lane < (unsigned)nn ? s_newv[lane] : 0ull;  // nn <= 32
-                    for (int j = nn - 1; j >= 1; j--) {
-                        const uint64_t vj = __shfl_sync(0xffffffffu, va, j);
-                        const unsigned qj = s_newq[j];
-                        if ((int)lane < j && ((va >> qj) & 1ull)) va ^= vj;
-                    }
-                    __syncwarp();
-                    if (lane < (unsigned)nn) s_newv[lane] = va;
-                    if (lane == 0) s_nnew = nn;
+            const size_t from = (size_t)lo * kMaxLocal + (i - s_start[lo]);
+            rows.w[i] = __ldcg(sw + from);
+            rows.key[i] = __ldcg(sk + from);
+        }
+        cta_sync();
+        n_cand += total;
+        const int nnew = total ? eliminate(rows, total, 64 - grank, es) : 0;
+        if (tid < (unsigned)nnew) s_prank[grank + tid] = t0 * kTile + (long long)es.pkey[tid];
+        grank += nnew;
+        t0 = end;
+        if (grank < b) {
+            if (t0 >= ntiles) {  // every candidate scanned
+                if (c == 0 && tid == 0) {
+                    atomicOr(status, ST_RANK_DEFICIT);
+                    bs->failed = 1;
                 }
+                ok = false;
+                break;
+            }
+            if (nnew) {
+                if (warp == 0) basis_add(s_basis, nnew, es);
                 cta_sync();
-                const int nc = s_nnew;
-                if (nc > 0) {
-                    if (threadIdx.x < (unsigned)grank) {
-                        uint64_t v = gbasis[threadIdx.x];
-                        for (int j = 0; j < nc; j++)
-                            if ((v >> s_newq[j]) & 1ull) v ^= s_newv[j];
-                        gbasis[threadIdx.x] = v;
-                    }
-                    if (threadIdx.x < (unsigned)nc && grank + threadIdx.x < 64) {
-                        gbasis[grank + threadIdx.x] = s_newv[threadIdx.x];
-                        gpiv[grank + threadIdx.x] = s_newq[threadIdx.x];
-                    }
-                    grank += nc;
-                    nnew += nc;
-                    cta_sync();
-                    fr_build(gtab, gbasis, gpiv, (unsigned)grank);  // ends with a barrier: s_new* are free
-                } else {
-                    cta_sync();  // s_nnew is read by every thread before warp 0 writes it again
-                }
+                fr_build(gtab, s_basis);
             }
-            MERGE_STAMP(3);
         }
-#else
-        if (!MCB_MERGE_FAST || cnt > 0) {  // no report below D: no new pivot (uniform)
-            // rank order: each candidate's position = number of smaller ranks (ranks are distinct)
-            unsigned long long *sr = mr + cnt;  // sorted ranks
-            uint64_t *sz = mw + cnt;            // sorted residuals against the global basis
-            uint64_t *sw = sz + cnt;            // sorted W
-            for (unsigned i = threadIdx.x; i < cnt; i += blockDim.x) {
-                const unsigned long long r = mr[i];
-                unsigned pos = 0;
-                for (unsigned j = 0; j < cnt; j++) pos += mr[j] < r;
-                sr[pos] = r;
-                sw[pos] = mw[i];
-                sz[pos] = fr_reduce(mw[i], gtab);
-            }
-            cta_sync();
-            MERGE_STAMP(2);
-            // greedy echelon in rank order (warp 0): a candidate is a new global pivot iff
-            // its residual is not in the span of the new pivots before it; then the new
-            // vectors are brought to reduced form among themselves, latest first (lane l
-            // holds vectors l and l + 32)
-            if (threadIdx.x < 32) {
-                int nn = 0;
-                for (unsigned base = 0; base < cnt && grank + nn < b; base += 32) {
-                    uint64_t z = base + lane < cnt ? sz[base + lane] : 0ull;
-                    for (int j = 0; j < nn; j++)
-                        if ((z >> s_newq[j]) & 1ull) z ^= s_newv[j];
-                    for (;;) {
-                        const unsigned bal = __ballot_sync(0xffffffffu, z != 0);
-                        if (!bal || grank + nn >= b) break;
-                        const int pl = __ffs(bal) - 1;
-                        const uint64_t v = __shfl_sync(0xffffffffu, z, pl);
-                        const unsigned qb = (unsigned)(__ffsll((long long)v) - 1);
-                        if (lane == 0) {
-                            s_newv[nn] = v;
-                            s_newq[nn] = qb;
-                            if (c == 0) {
-                                bs->pivrank[grank + nn] = (long long)sr[base + pl];
-                                bs->pivW[grank + nn] = sw[base + pl];
-                            }
-                        }
-                        nn++;
-                        if ((z >> qb) & 1ull) z ^= v;
-                    }
-                    __syncwarp();
-                }
-                uint64_t va = lane < (unsigned)nn ? s_newv[lane] : 0ull;
-                uint64_t vb = lane + 32 < (unsigned)nn ? s_newv[lane + 32] : 0ull;
-                for (int j = nn - 1; j >= 1; j--) {
-                    const uint64_t vj = __shfl_sync(0xffffffffu, j < 32 ? va : vb, j & 31);
-                    const unsigned qj = s_newq[j];
-                    if ((int)lane < j && ((va >> qj) & 1ull)) va ^= vj;
-                    if ((int)lane + 32 < j && ((vb >> qj) & 1ull)) vb ^= vj;
-                }
-                __syncwarp();
-                if (lane < (unsigned)nn) s_newv[lane] = va;
-                if (lane + 32 < (unsigned)nn) s_newv[lane + 32] = vb;
-                if (lane == 0) s_nnew = nn;
-            }
-            cta_sync();
-            nnew = s_nnew;
-            MERGE_STAMP(3);
-        }
-        if (nnew > 0) {
-            // clear the new pivot bits from the old basis vectors, append, rebuild tables
-            if (threadIdx.x < (unsigned)grank) {
-                uint64_t v = gbasis[threadIdx.x];
-                for (int j = 0; j < nnew; j++)
-                    if ((v >> s_newq[j]) & 1ull) v ^= s_newv[j];
-                gbasis[threadIdx.x] = v;
-            }
-            if (threadIdx.x < (unsigned)nnew && grank + threadIdx.x < 64) {
-                gbasis[grank + threadIdx.x] = s_newv[threadIdx.x];
-                gpiv[grank + threadIdx.x] = s_newq[threadIdx.x];
-            }
-            grank += nnew;
-            cta_sync();
-            fr_build(gtab, gbasis, gpiv, (unsigned)grank);
-            MERGE_STAMP(4);
-        }
-#endif
-        if (nnew == 0 && D >= (unsigned long long)K) {
-            if (c == 0 && threadIdx.x == 0) {
-                atomicOr(status, ST_RANK_DEFICIT);
-                bs->failed = 1;
-            }
-            ok = false;
-            break;
-        }
-        s = (long long)D;
-        if (threadIdx.x == 0) {  // self-check: every CTA must reach the same merge result
+        if (tid == 0) {  // self-check: every CTA must reach the same merge result
             unsigned long long h = 1469598103934665603ull;
             h = (h ^ (unsigned long long)grank) * 1099511628211ull;
-            h = (h ^ D) * 1099511628211ull;
-            h = (h ^ (unsigned long long)cnt) * 1099511628211ull;
+            h = (h ^ (unsigned long long)t0) * 1099511628211ull;
+            h = (h ^ (unsigned long long)total) * 1099511628211ull;
+            if (nnew > 0) h = (h ^ es.pw[nnew - 1] ^ es.pkey[nnew - 1]) * 1099511628211ull;
             dbg[(size_t)(k & 1) * G + c] = h;
         }
         k++;
-        cyc_merge += clock64() - c2;
+        cta_sync();  // the tables and the ranks are in place
+        cyc_merge += clock64() - cyc2;
+    }
+    if (ok && c == 0) {  // the pivots, in rank order as they were found, with their W
+        if ((int)tid < grank) {
+            bs->pivrank[tid] = s_prank[tid];
+            bs->pivW[tid] = __ldcg(Warr + s_prank[tid]);
+        }
+        cta_sync();
     }
     // ---- block tail: CTA 0 resolves the block; then every CTA materialises its
     // column groups of the final rows and their tables ----
@@ -1919,7 +1709,7 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
     if (ok) {
         const long long c3 = clock64();
         if (c == 0) {
-            const bool done = resolve_block(bs, grank, off, coords, ta, reinterpret_cast<unsigned *>(win), status);
+            const bool done = resolve_block(bs, grank, off, coords, ta, reinterpret_cast<unsigned *>(rows.w), status);
             if (threadIdx.x == 0) bs->tail_ok = done ? 1u : 0u;
         }
         const long long c4 = clock64();
@@ -1928,7 +1718,7 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
             ok = false;
         } else {
             const long long c5 = clock64();
-            if (*((volatile unsigned *)&bs->tail_ok)) materialize_rows(ta, bs, b, win);
+            if (*((volatile unsigned *)&bs->tail_ok)) materialize_rows(ta, bs, b, rows.w);
             cta_sync();
             cyc_tailbar = c5 - c4;
             cyc_mat = clock64() - c5;
@@ -1941,14 +1731,13 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
     if (threadIdx.x == 0) {
         atomicMax(&diag[14], nbar);
         atomicMin(&diag[15], nbar);
-        atomicMax((unsigned long long *)&bs->max_tile[ta.par], (unsigned long long)maxt);
         atomicAdd(&diag[1], n_local);
         atomicAdd(&diag[3], n_loaded);
         atomicAdd(&diag[4], n_computed);
     }
     if (c == 0 && threadIdx.x == 0) {
         bs->rank = (unsigned)grank;
-        bs->last_pivot = grank > 0 ? bs->pivrank[grank - 1] : 0;
+        bs->last_pivot[ta.par] = grank > 0 && ok ? bs->pivrank[grank - 1] : 0;
         atomicAdd(&diag[0], (unsigned long long)k);
         atomicAdd(&diag[2], n_cand);
         atomicAdd(&diag[5], 1ull);
@@ -1958,23 +1747,20 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
         atomicAdd(&diag[20], (unsigned long long)cyc_resolve);
         atomicAdd(&diag[21], (unsigned long long)cyc_tailbar);
         atomicAdd(&diag[22], (unsigned long long)cyc_mat);
-#ifdef MCB_MERGE_PROFILE
-        for (int i = 0; i < 5; i++) diag[33 + i] = (unsigned long long)g_merge_prof[i];
-#endif
-#ifdef MCB_SCAN_PROFILE
-        for (int i = 0; i < 4; i++) diag[24 + i] = (unsigned long long)g_scan_prof[i];
-#endif
 #ifdef MCB_TAIL_PROFILE
         for (int i = 0; i < 6; i++) diag[24 + i] = g_tail_prof[i];
 #endif
     }
 }
 
-// Dynamic shared memory of blk_pivot_kernel for a grid of G CTAs: two sets of
-// Four-Russians tables, the window of kWinMax tiles of W's, the merge buffers
-// (5 x G x kLmax words) and the report staging (G x (2 kLmax + 2) words).
-size_t pivot_smem_bytes(int G) {
-    return 32768 + 8 * (size_t)kWinW + 8 * 5 * (size_t)G * kLmax + 8 * (size_t)G * (2 * kLmax + 2);
+// Row list entries for a grid of G CTAs: every CTA's largest report, and the local
+// list's carried pivots plus two chunks.
+unsigned pivot_list_cap(int G) {
+    return (unsigned)std::max(G * kMaxLocal, 64 + 2 * kChunkTiles * kTile);
+}
+// Dynamic shared memory: the tables and the row list, or the tail's P + 1 counters.
+size_t pivot_smem_bytes(int G, int P) {
+    return 16384 + std::max(12 * (size_t)pivot_list_cap(G), sizeof(unsigned) * ((size_t)P + 1));
 }
 
 // Rows j >= e0+b in groups of kUpdRows consecutive rows, kUpdSplit warps per group.
@@ -2577,24 +2363,25 @@ __global__ void __launch_bounds__(256) cert_check_kernel(const unsigned long lon
 
 // ===========================================================================
 // The candidate search shapes a solver times (mcbgpu_solver_tune): the compiled-in
-// default, more local pivots per step, wider windows, deeper streaming passes.  A
-// solve is cut into kShapeSegs segments of blocks, each with its own shape (the
-// pivots of later blocks lie deeper in the rank order).  On the 1M-vertex
-// planar-chain graph's prefix solve the wider windows with 8 local pivots (candidate
-// 2) take 0.113-0.146 ms per block against 0.128-0.164 ms for the default, from the
-// first quarter of the solve to the last (a one-tile early window was 10x slower
-// there and is not a candidate).
+// default, narrower and wider windows, deeper W passes.  A solve is cut into kShapeSegs
+// segments of blocks, each with its own shape (the pivots of later blocks lie deeper
+// in the rank order).
 constexpr int kShapeSegs = 4;
 constexpr int kShapeInts = 7;  // ints per shape in mcbgpu_solver_shapes
+constexpr int kShapeLmax = 8;  // their local-pivot limit: the search has none any more, the field stays
 const PivotShape kCandidateShapes[] = {
     kDefaultShape,
-    {2, 48, 6, 60, 8, 8, 25},
-    {4, 48, 8, 56, 12, 8, 25},
-    {3, 40, 8, 56, 12, 8, 60},
-    {2, 40, 8, 56, 12, 8, 40},
-    {3, 40, 8, 56, 12, 8, 40},
+    {1, 40, 8, 60, 16, 25},
+    {2, 48, 4, 60, 8, 25},
+    {4, 48, 16, 60, 32, 25},
+    {2, 40, 8, 56, 16, 60},
+    {4, 40, 16, 56, 32, 60},
 };
 constexpr int kNumShapes = (int)(sizeof(kCandidateShapes) / sizeof(kCandidateShapes[0]));
+
+// Dynamic shared memory a pivot kernel may ask for (its static arrays add 6 KB): an S
+// row of up to 168,832 bytes of word counters, as far as the block tail ever took.
+constexpr int kPivotSmemMax = 16384 + 168832;
 
 struct mcbgpu_solver {
     int N = 0, W = 0, P = 0, words_cap = 0;
@@ -2635,7 +2422,9 @@ struct mcbgpu_solver {
     uint64_t *d_masks = nullptr;   // 2 x 64: final masks of a group's first blocks
     unsigned *d_tile_epoch = nullptr;
     int32_t *d_tile_minc = nullptr;
-    unsigned long long *d_reports = nullptr;  // two step parities of G x (2 kLmax + 2) words
+    uint64_t *d_rep_w = nullptr;   // two step parities of G x kMaxLocal reported local pivots: residuals
+    unsigned *d_rep_key = nullptr;  // ranks, and 2 x G counts
+    unsigned *d_rep_n = nullptr;
     GridBar *d_gbar = nullptr;
     int pivot_grid = 0;
     unsigned *d_pairs = nullptr;     // 3 x pair_cap: resolve scratch, sorted pairs of the two block parities
@@ -2809,7 +2598,9 @@ void free_solver(mcbgpu_solver *s) {
     cudaFree(s->d_masks);
     cudaFree(s->d_tile_epoch);
     cudaFree(s->d_tile_minc);
-    cudaFree(s->d_reports);
+    cudaFree(s->d_rep_w);
+    cudaFree(s->d_rep_key);
+    cudaFree(s->d_rep_n);
     cudaFree(s->d_gbar);
     cudaFree(s->d_pairs);
     cudaFree(s->d_word_end);
@@ -2968,21 +2759,23 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
     for (int i = 0; i < 2 && e == cudaSuccess; i++) e = cudaEventCreateWithFlags(&s->ev_par[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMemset(s->d_coords, 0, sizeof(int32_t) * (size_t)(nnz + 16));
     if (e == cudaSuccess) {
-        const int G = s->sm_count > 0 ? std::max(1, s->sm_count / MCB_PIVOT_DIV) : 1;  // one CTA per SM
-        const size_t smem = pivot_smem_bytes(G);
-        e = cudaFuncSetAttribute(blk_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        // the block tail sorts the pairs in shared memory past the tables (P + 1 counters)
-        // and materialises 2 x 64 x (kMatCols + 1) words there
-        if (e == cudaSuccess && sizeof(unsigned) * ((size_t)s->P + 1) > smem - 32768) e = cudaErrorInvalidValue;
+        const int G = std::max(1, std::min(s->sm_count, kMaxGrid));  // one CTA per SM
+        const size_t smem = pivot_smem_bytes(G, s->P);
+        if (smem > (size_t)kPivotSmemMax) e = cudaErrorInvalidValue;
+        // the attribute is the kernel's, shared by all handles: never lowered
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(blk_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmemMax);
         int per_sm = 0;
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, blk_pivot_kernel, kPivotThreads, smem);
         if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
-        s->pivot_grid = G;
-        // two step-parity halves of: ranks + W's (G x kLmax each), ends, counts (G each)
-        const size_t rb = sizeof(unsigned long long) * 2 * (size_t)G * (2 * kLmax + 2);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_reports, rb);
-        bytes += (long long)rb;
+        // CTAs beyond one per tile have nothing to scan; a few more take the tail's columns
+        s->pivot_grid = (int)std::min<long long>(G, std::max<long long>((K + kTile - 1) / kTile, 8));
+        const size_t rows = 2 * (size_t)G * kMaxLocal;
+        if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_rep_w, sizeof(uint64_t) * rows);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_rep_key, sizeof(unsigned) * rows);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_rep_n, sizeof(unsigned) * 2 * (size_t)G);
+        bytes += (long long)(12 * rows + sizeof(unsigned) * 2 * (size_t)G);
     }
     if (e == cudaSuccess) e = cudaMemset(s->d_bs, 0, sizeof(BlockState));
     if (e == cudaSuccess) e = cudaMemset(s->d_status, 0, sizeof(unsigned));
@@ -3301,7 +3094,7 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
                                        ga.nz && ga.columns ? (int)std::min<long long>(sms, std::max(1ll, ntiles)) : 1);
             MCB_CUDA(launch_k(pdl, blk_transpose_kernel, dim3(tgrid), dim3(256), 0, st, (const uint64_t *)s->d_S, s->P,
                               (int)e0, b, Wb, s->d_T, s->d_bs, ntiles, s->d_gbar,
-                              (long long)s->pivot_grid * sh.win_mid, sh.stream_pct, s->d_Tg, ga));
+                              (long long)s->pivot_grid, sh.stream_pct, s->d_Tg, ga));
         }
         if (ntiles > 0 && pos > 0) {
             Launch L(s, KC_WFIX, st);
@@ -3346,7 +3139,9 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             unsigned *te = s->d_tile_epoch;
             GridBar *gb = s->d_gbar;
             unsigned *stt = s->d_status;
-            unsigned long long *rp = s->d_reports;
+            uint64_t *rw = s->d_rep_w;
+            unsigned *rk = s->d_rep_key, *rn = s->d_rep_n;
+            unsigned lcap = pivot_list_cap(s->pivot_grid);
             unsigned long long *nb = L.bytes();
             unsigned long long *dg = s->d_diag;
             unsigned long long *db = s->d_diag + kDiagWords;
@@ -3362,11 +3157,12 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             ta.e0 = (int)e0;
             ta.Wb = Wb;
             ta.par = par;
+            ta.first = pos == 0 ? 1 : 0;
             PivotShape shv = sh;
-            void *args[] = {&K, &off, &co, &hd, &tm, &T, (void *)&bound, &bs, &Wa, &te, &rp, &gb, &stt, &nb, &dg, &db, &ta,
-                            &shv};
+            void *args[] = {&K, &off, &co, &hd, &tm, &T, (void *)&bound, &bs, &Wa, &te, &rw, &rk, &rn, &gb, &stt, &nb, &dg, &db,
+                            &ta, &shv, &lcap};
             MCB_CUDA(launch_coop(pdl, (const void *)blk_pivot_kernel, dim3(s->pivot_grid), dim3(kPivotThreads), args,
-                                 pivot_smem_bytes(s->pivot_grid), st));
+                                 pivot_smem_bytes(s->pivot_grid, s->P), st));
         }
         if (s->tuning && (pos == kGroup - 1 || e0 + b >= iters)) {  // the group's last block
             cudaEvent_t tev_b = s->tpool[tnext++];
@@ -3705,7 +3501,7 @@ int mcbgpu_solver_shapes(const mcbgpu_solver *s, int32_t *params, int32_t max_sh
     }
     for (int k = 0; k < kNumShapes && k < max_shapes; k++) {
         const PivotShape &h = kCandidateShapes[k];
-        const int32_t v[kShapeInts] = {h.win_early, h.rank_early, h.win_mid, h.rank_tail, h.win_tail, h.lmax,
+        const int32_t v[kShapeInts] = {h.win_early, h.rank_early, h.win_mid, h.rank_tail, h.win_tail, kShapeLmax,
                                        h.stream_pct};
         for (int i = 0; i < kShapeInts; i++) params[k * kShapeInts + i] = v[i];
     }
