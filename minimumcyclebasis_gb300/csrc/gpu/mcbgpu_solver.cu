@@ -396,6 +396,133 @@ __global__ void update_kernel(uint64_t *S, int N, int P, int e, const int64_t *_
     }
 }
 
+// The whole per-iteration loop, one launch per iteration.  Search e needs only row e of
+// iteration e - 1's update, so every CTA forms that row for itself in shared memory
+// (S_e, and S_{e-1} if <C_{e-1}, S_e> is odd), searches with it, and then takes its share
+// of the other rows of the update of iteration e - 1, which nothing of search e waits
+// for.  A finished row goes through fin (two rows by iteration parity): S itself is not
+// written where another CTA may still read it.
+// What bounds an iteration is a chain of L2 round trips (previous rank, its list, the
+// candidates' heads and lists); the two launches per iteration it replaces had it twice
+// with a launch in between.  Random graph of 2k vertices: 15.5 -> 4.8 us per iteration.
+// search: 0 for the last launch, which only updates.
+struct PlainSlot {           // ring of four: read one launch after it was written, cleared two later
+    unsigned long long best;
+};
+constexpr int kPlainThreads = 256;
+
+__global__ void __launch_bounds__(kPlainThreads) plain_kernel(
+    uint64_t *S, uint64_t *fin, int N, int P, int e, int search, const int64_t *__restrict__ off,
+    const int32_t *__restrict__ coords, const int32_t *__restrict__ head, const int32_t *__restrict__ weight,
+    long long K, PlainSlot *ring, IterSlot *slots, long long *selected, BlockState *bs, unsigned *status) {
+    extern __shared__ __align__(16) uint64_t s_S[];
+    __shared__ unsigned s_par[kPlainThreads / 32];
+    griddep_wait();
+    griddep_launch();
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int we = (e >> 6) + 1;  // words of S_e; S_{e-1} has no bit beyond them
+    unsigned long long rp = kNone;
+    if (e > 0) rp = *((volatile unsigned long long *)&ring[(e - 1) & 3].best);
+    const bool upd = rp != kNone;
+    const uint64_t *prev = fin + (size_t)((e - 1) & 1) * P;  // S_{e-1}, final
+    const uint64_t *Se = S + (size_t)e * P;
+    if (search)
+        for (int w = tid; w < we; w += kPlainThreads) s_S[w] = Se[w];
+    int64_t c0 = 0, c1 = 0;
+    if (upd) {
+        c0 = off[rp];
+        c1 = off[rp + 1];
+    }
+    if (blockIdx.x == 0) {
+        if (tid == 0) {
+            if (e > 0) {
+                if (!upd) {
+                    atomicOr(status, ST_NO_CANDIDATE);
+                    selected[e - 1] = -1;
+                } else {
+                    selected[e - 1] = (long long)rp;
+                    bs->total += (unsigned long long)(long long)weight[rp];
+                }
+            }
+            ring[(e + 1) & 3].best = kNone;  // the next search's; last read two launches ago
+            if (!search) {  // as a last select and update leave them
+                slots[(e + 1) & 1].best = rp;
+                slots[e & 1].best = kNone;
+                slots[e & 1].next_tile = 0;
+            }
+        }
+        if (e > 0)
+            for (int w = tid; w < ((e - 1) >> 6) + 1; w += kPlainThreads) S[(size_t)(e - 1) * P + w] = prev[w];
+    }
+    cta_sync();
+    if (search) {
+        if (upd) {
+            unsigned par = 0;  // <C_{e-1}, S_e>
+            for (int64_t i = c0 + tid; i < c1; i += kPlainThreads) {
+                const int c = i - c0 < kHead ? __ldg(head + (size_t)rp * kHead + (i - c0)) : __ldg(coords + i);
+                if (c <= e) par ^= (unsigned)(s_S[c >> 6] >> (c & 63)) & 1u;
+            }
+            par = __reduce_xor_sync(0xffffffffu, par);
+            if (lane == 0) s_par[tid >> 5] = par;
+            cta_sync();
+            par = 0;
+#pragma unroll
+            for (int w = 0; w < kPlainThreads / 32; w++) par ^= s_par[w];
+            if (par)
+                for (int w = tid; w < ((e - 1) >> 6) + 1; w += kPlainThreads) s_S[w] ^= prev[w];
+            cta_sync();
+        }
+        if (blockIdx.x == 0)
+            for (int w = tid; w < we; w += kPlainThreads) fin[(size_t)(e & 1) * P + w] = s_S[w];
+        PlainSlot *slot = ring + (e & 3);
+        for (long long r0 = (long long)blockIdx.x * kPlainThreads; r0 < K; r0 += (long long)gridDim.x * kPlainThreads) {
+            if ((unsigned long long)r0 > *((volatile unsigned long long *)&slot->best)) break;  // nothing earlier is left here
+            const long long r = r0 + tid;
+            unsigned par = 0;
+            if (r < K) {
+                int hv[kHead];
+                const int4 a = __ldg(reinterpret_cast<const int4 *>(head + (size_t)r * kHead));
+                const int4 b = __ldg(reinterpret_cast<const int4 *>(head + (size_t)r * kHead) + 1);
+                hv[0] = a.x, hv[1] = a.y, hv[2] = a.z, hv[3] = a.w, hv[4] = b.x, hv[5] = b.y, hv[6] = b.z, hv[7] = b.w;
+#pragma unroll
+                for (int q = 0; q < kHead; q++)
+                    if (hv[q] <= e) par ^= (unsigned)(s_S[hv[q] >> 6] >> (hv[q] & 63)) & 1u;
+                if (hv[kHead - 1] <= e) {
+                    const int64_t en = __ldg(off + r + 1);
+                    for (int64_t i = __ldg(off + r) + kHead; i < en; i += kHead) {
+                        int v[kHead];
+#pragma unroll
+                        for (int q = 0; q < kHead; q++) v[q] = i + q < en ? __ldg(coords + i + q) : 0x7fffffff;
+#pragma unroll
+                        for (int q = 0; q < kHead; q++)
+                            if (v[q] <= e) par ^= (unsigned)(s_S[v[q] >> 6] >> (v[q] & 63)) & 1u;
+                        if (v[kHead - 1] > e) break;
+                    }
+                }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, par);
+            if (m) {  // ranks only rise from here: this warp's first
+                if (lane == 0) atomicMin(&slot->best, (unsigned long long)(r + __ffs(m) - 1));
+                break;
+            }
+        }
+    }
+    if (!upd) return;
+    // the other rows of iteration e - 1's update (all of them in the last launch)
+    const int warps = (gridDim.x * kPlainThreads) >> 5, wp = ((e - 1) >> 6) + 1;
+    for (int j = e + (search ? 1 : 0) + ((blockIdx.x * kPlainThreads + tid) >> 5); j < N; j += warps) {
+        uint64_t *Sj = S + (size_t)j * P;
+        unsigned par = 0;
+        for (int64_t i = lane; i < c1 - c0; i += 32) {
+            const int c = i < kHead ? __ldg(head + (size_t)rp * kHead + i) : __ldg(coords + c0 + i);
+            par ^= (unsigned)(Sj[c >> 6] >> (c & 63)) & 1u;
+        }
+        par = __reduce_xor_sync(0xffffffffu, par);
+        if (par)
+            for (int w = lane; w < wp; w += 32) Sj[w] ^= prev[w];
+    }
+}
+
 // C_e of the selected candidate as a bit vector (include/cycles.h:144-195).
 __global__ void cycle_vector_kernel(uint64_t *C, int W, const int64_t *__restrict__ off,
                                     const int32_t *__restrict__ coords, const IterSlot *slot) {
@@ -2435,6 +2562,8 @@ struct mcbgpu_solver {
     cudaEvent_t ev_join = nullptr;   // the end of a blocked run, for the caller's stream
     cudaEvent_t ev_fork = nullptr, ev_tail = nullptr, ev_upd[4] = {}, ev_par[2] = {};
     IterSlot *d_slots = nullptr;   // 2
+    PlainSlot *d_ring = nullptr;   // 4: the whole per-iteration loop's
+    uint64_t *d_fin = nullptr;     // 2 P: its finished rows by iteration parity
     BlockState *d_bs = nullptr;
     long long *d_selected = nullptr;
     unsigned *d_status = nullptr;
@@ -2614,6 +2743,8 @@ void free_solver(mcbgpu_solver *s) {
     for (cudaEvent_t e : s->ev_upd)
         if (e) cudaEventDestroy(e);
     cudaFree(s->d_slots);
+    cudaFree(s->d_ring);
+    cudaFree(s->d_fin);
     cudaFree(s->d_bs);
     cudaFree(s->d_selected);
     cudaFree(s->d_status);
@@ -2707,6 +2838,8 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
     ALLOC(s->d_gbar, sizeof(GridBar));
     ALLOC(s->d_word_end, sizeof(unsigned) * 2 * ((size_t)s->P + 1));
     ALLOC(s->d_slots, sizeof(IterSlot) * 2);
+    ALLOC(s->d_ring, sizeof(PlainSlot) * 4);
+    ALLOC(s->d_fin, sizeof(uint64_t) * 2 * (size_t)s->P);
     ALLOC(s->d_bs, sizeof(BlockState));
     ALLOC(s->d_selected, sizeof(long long) * (size_t)(N > 0 ? N : 1));
     ALLOC(s->d_status, sizeof(unsigned));
@@ -2988,12 +3121,36 @@ int mcbgpu_solver_run_plain(mcbgpu_solver *s, int64_t max_iterations, void *stre
         return MCBGPU_E_ARG;
     }
     int64_t iters = (max_iterations >= 0 && max_iterations < s->N) ? max_iterations : s->N;
-    for (int64_t e = 0; e < iters; e++) {
-        int rc = mcbgpu_select(s, (int32_t)e, nullptr, stream);
-        if (rc) return rc;
-        rc = mcbgpu_update(s, (int32_t)e, stream);
-        if (rc) return rc;
+    if (s->profiling || !s->uploaded || s->K == 0) {  // launch by launch (K = 0: no candidate, at once)
+        for (int64_t e = 0; e < iters; e++) {
+            int rc = mcbgpu_select(s, (int32_t)e, nullptr, stream);
+            if (rc) return rc;
+            rc = mcbgpu_update(s, (int32_t)e, stream);
+            if (rc) return rc;
+        }
+        return MCBGPU_OK;
     }
+    if (iters == 0) return MCBGPU_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int sms = s->sm_count > 0 ? s->sm_count : 64;
+    const long long chunks = (s->K + kPlainThreads - 1) / kPlainThreads;
+    const int grid = (int)std::min<long long>(std::max<long long>(chunks, (s->N + 7) / 8), (long long)sms * 4);
+    MCB_CUDA(cudaMemsetAsync(s->d_ring, 0xff, sizeof(PlainSlot) * 4, st));
+    for (int64_t e = 0; e <= iters; e++) {
+        const int search = e < iters ? 1 : 0;
+        const size_t smem = search ? sizeof(uint64_t) * (size_t)search_smem_words(s, (int)e) : 0;
+        if (smem > 200 * 1024) {
+            set_error("mcbgpu_solver_run_plain: support vector prefix too large for shared memory");
+            return MCBGPU_E_ARG;
+        }
+        if (smem > 48 * 1024) MCB_CUDA(cudaFuncSetAttribute(plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        Launch L(s, KC_SEARCH, st);
+        MCB_CUDA(launch_k(s->pdl, plain_kernel, dim3(grid), dim3(kPlainThreads), smem, st, s->d_S, s->d_fin, s->N, s->P,
+                          (int)e, search, (const int64_t *)s->d_off, (const int32_t *)s->d_coords,
+                          (const int32_t *)s->d_head, (const int32_t *)s->d_weight, s->K, s->d_ring, s->d_slots,
+                          s->d_selected, s->d_bs, s->d_status));
+    }
+    s->iters_run = iters;
     return MCBGPU_OK;
 }
 
