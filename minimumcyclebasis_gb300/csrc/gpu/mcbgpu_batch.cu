@@ -4,60 +4,61 @@
 // The reference solves one graph per process and, for a graph split into
 // biconnected components, runs the whole driver once per component file
 // (main.sh:19-32 loops `run.sh` over bicc's output).  Here every problem is a
-// (N, candidates, coordinate lists) triple as mcbgpu_solver takes it; one CTA owns
-// one problem at a time and pulls the next from a device work counter (problems
-// in order of decreasing N, so the longest start first).
+// (N, candidates, coordinate lists) triple as mcbgpu_solver takes it; a cluster of csz
+// CTAs owns one problem at a time and pulls the next from a device work counter
+// (problems in order of decreasing N, so the longest start first).
 //
-// Per problem the CTA runs the blocked loop of mcbgpu_solver_run (64 iterations per
-// block) with everything block-local in shared memory:
-//   1. T[c] = bits i of S_{e0+i}[c] for the block's rows (64x64 bit transposes of
-//      the rows' words by warp ballots; unit bits for c in [e0, bound));
-//   2. the rank-ordered scan: W_r = XOR of T over C_r's coordinates below the
-//      bound; the first b candidates whose W is independent of the earlier ones'
-//      (a reduced row echelon basis keyed by lead bit) are the pivots;
+// Per problem the cluster runs the blocked loop of mcbgpu_solver_run (64 iterations per
+// block), every CTA with the block's state in its own shared memory:
+//   1. T[c] = bits i of S_{e0+i}[c] for the block's rows (64x64 bit transposes; unit
+//      bits for c in [e0, bound));
+//   2. the rank-ordered scan, a chunk of candidates per round, a slice of it per CTA:
+//      W_r = XOR of T over C_r's coordinates below the bound, reduced by the pivots
+//      found so far (Four-Russians tables); what is left is compacted in rank order and
+//      eliminated (mcbgpu_elim.cuh).  With several CTAs each one's pivots go to all of
+//      them through distributed shared memory and are eliminated once more;
 //   3. resolve: the reference's loop restricted to the block on 64-bit masks
 //      (iteration k takes the first pivot with parity(W_p & m_k) = 1, later masks
 //      with odd parity absorb m_k), which selects the reference's candidate for
 //      every iteration (mcb/mcb_cycle_deg_two_remove.cpp:329-358);
-//   4. the block's final rows S_{e0+k} = XOR_{l in m_k} S^0_{e0+l}, computed from T;
+//   4. the block's final rows S_{e0+k} = XOR_{l in m_k} S^0_{e0+l}, computed from T, a
+//      share per CTA;
 //   5. every later row j: D_j[k] = <C_sel_k, S_j>, beta = the sequential effect of
 //      the 64 updates (a 64x64 GF(2) matrix applied to D), S_j ^= XOR_{k in beta}
-//      S_{e0+k} (mcb/mcb_cycle_deg_two_remove.cpp:371-390 for 64 iterations).
-// There is no inter-CTA synchronisation: the only shared word is the work counter.
+//      S_{e0+k} (mcb/mcb_cycle_deg_two_remove.cpp:371-390 for 64 iterations), a residue
+//      class of rows per warp.  A row that is still its unit vector and whose
+//      coordinate lies on none of the block's cycles is not read.
+// Clusters wait for nobody but themselves: the only shared word is the work counter.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <vector>
 
-#include "mcbgpu_internal.cuh"
+#include "mcbgpu_elim.cuh"
 
 using namespace mcbgpu;
+using namespace mcbgpu::elim;
+namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int kBThreads = 512;
+constexpr int kBThreads = kElimThreads;
 constexpr int kBWarps = kBThreads / 32;
-#ifndef MCB_BATCH_Q0
-#define MCB_BATCH_Q0 2  // candidates per thread per scan round, problems with N <= 1024
-#endif
-#ifndef MCB_BATCH_Q
-#define MCB_BATCH_Q 4   // the same for the larger classes
-#endif
-#ifndef MCB_BATCH_SINGLE
-#define MCB_BATCH_SINGLE 1  // one launch for the whole batch (0: one launch per size class)
-#endif
-#ifndef MCB_BATCH_PREFETCH
-#define MCB_BATCH_PREFETCH 1  // bulk L2 prefetch of the next scan chunk's offsets and lists
-#endif
-#ifndef MCB_BATCH_CHUNK
-#define MCB_BATCH_CHUNK 4
-#endif
-constexpr int kBChunk = MCB_BATCH_CHUNK;  // coordinates of each candidate loaded together in a W walk
+constexpr int kSmallQ = 2;               // candidates per thread and scan round, problems of N <= kSmallN
+constexpr int kLargeQ = 4;               // the same for larger ones
+constexpr int kSmallN = 1024;            // largest N of the small form (two CTAs per SM)
+constexpr int kBChunk = 4;               // coordinates of each candidate loaded together beyond its head
+constexpr int kBHead = 8;                // coordinates of a list's head (one aligned 32-byte slot per candidate)
 constexpr int kBatchMaxN = 12288;        // largest N a CTA holds (T and the final rows in shared memory)
+constexpr int kClasses = 4;              // launches of a batch: 8, 4, 2 or 1 CTAs per problem
 constexpr unsigned kPairSmemMax = 8192;  // pairs kept in shared memory (more go to the CTA's global scratch)
-constexpr size_t kSmemBudget = 220 * 1024;  // dynamic shared memory per CTA at most (static adds 3.4 KB)
-constexpr int kClasses = 3;
-constexpr int kClassMaxN[kClasses] = {1024, 4096, kBatchMaxN};
+constexpr size_t kSmemBudget = 214 * 1024;  // dynamic shared memory per CTA at most (static adds 12 KB)
 
 constexpr int kBProf = 13;  // profile words per problem (mcbgpu_batch_profile)
+
+// Words of the region that holds the scan's tables and row list and later the block's
+// final rows.
+constexpr size_t scan_words(int q) { return 2048 + (20 * (size_t)(kBThreads * q + 64) + 7) / 8; }
 
 struct BatchGraph {
     long long cand;  // first candidate (index into weight / offsets)
@@ -69,36 +70,52 @@ struct BatchGraph {
 
 __device__ __forceinline__ int ffs64(uint64_t x) { return __ffsll((long long)x) - 1; }
 
-// W of the kBQ consecutive candidates r0 .. r0 + kBQ - 1 (0 past K) from the block's
-// T in shared memory.  The lists are walked in lockstep, kBChunk coordinates of each
-// per step, so kBQ x kBChunk independent loads are in flight per thread.  `walked`
-// counts the offsets and coordinates read (for the profile's byte count).
+// W of the kBQ candidates r0 + q * kBThreads (0 past `end`) from the block's T in shared
+// memory.  The heads come in one coalesced read; the lists that go on below the bound
+// are walked in lockstep, kBChunk coordinates of each per step, so kBQ x kBChunk
+// independent loads are in flight per thread.  `walked` counts the bytes read.
 template <int kBQ>
-__device__ __forceinline__ void w_smem_q(long long r0, long long K, long long cand,
-                                         const int64_t *__restrict__ off, const int32_t *__restrict__ coords,
-                                         const uint64_t *T, int bound, uint64_t (&W)[kBQ],
-                                         unsigned long long &walked) {
+__device__ __forceinline__ void w_smem_q(long long r0, long long end, long long cand, const int64_t *__restrict__ off,
+                                         const int32_t *__restrict__ coords, const int32_t *__restrict__ head,
+                                         const uint64_t *T, int bound, uint64_t (&W)[kBQ], unsigned long long &walked) {
     long long ia[kBQ], ea[kBQ];
+    int4 ha[kBQ], hb[kBQ];
 #pragma unroll
     for (int q = 0; q < kBQ; q++) {
-        W[q] = 0;
-        ia[q] = ea[q] = 0;
-        if (r0 + q < K) {
-            ia[q] = __ldg(off + cand + r0 + q);
-            ea[q] = __ldg(off + cand + r0 + q + 1);
-            walked += 16;
+        const long long r = r0 + (long long)q * kBThreads;
+        ha[q] = hb[q] = make_int4(0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff);
+        if (r < end) {
+            const int4 *h = reinterpret_cast<const int4 *>(head + (size_t)(cand + r) * kBHead);
+            ha[q] = __ldg(h);
+            hb[q] = __ldg(h + 1);
+            walked += 4 * kBHead;
         }
     }
-    for (;;) {
-        bool any = false;
+    bool any = false;
 #pragma unroll
-        for (int q = 0; q < kBQ; q++) any |= ia[q] < ea[q];
-        if (!any) break;
+    for (int q = 0; q < kBQ; q++) {
+        const int c[kBHead] = {ha[q].x, ha[q].y, ha[q].z, ha[q].w, hb[q].x, hb[q].y, hb[q].z, hb[q].w};
+        uint64_t w = 0;
+#pragma unroll
+        for (int t = 0; t < kBHead; t++)
+            if (c[t] < bound) w ^= T[c[t]];
+        W[q] = w;
+        ia[q] = ea[q] = 0;
+        if (c[kBHead - 1] < bound) {
+            const long long r = cand + r0 + (long long)q * kBThreads;
+            ia[q] = __ldg(off + r) + kBHead;
+            ea[q] = __ldg(off + r + 1);
+            walked += 16;
+            any = true;
+        }
+    }
+    while (any) {
         int cv[kBQ][kBChunk];
 #pragma unroll
         for (int q = 0; q < kBQ; q++)
 #pragma unroll
             for (int t = 0; t < kBChunk; t++) cv[q][t] = ia[q] + t < ea[q] ? __ldg(coords + ia[q] + t) : 0x7fffffff;
+        any = false;
 #pragma unroll
         for (int q = 0; q < kBQ; q++) {
             walked += 4ull * (unsigned long long)min((long long)kBChunk, ea[q] - ia[q] > 0 ? ea[q] - ia[q] : 0);
@@ -106,50 +123,77 @@ __device__ __forceinline__ void w_smem_q(long long r0, long long K, long long ca
             for (int t = 0; t < kBChunk; t++)
                 if (cv[q][t] < bound) W[q] ^= T[cv[q][t]];
             ia[q] = cv[q][kBChunk - 1] >= bound ? ea[q] : ia[q] + kBChunk;
+            any |= ia[q] < ea[q];
         }
     }
 }
 
 // kBQ: candidates per thread in one scan round; kRowRegs: row words per lane in the
-// update (ceil(largest N of the class / 2048)).
+// update (ceil(largest N of the form / 2048)).
 template <int kBQ, int kRowRegs, int kMinBlocks>
 __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
     const BatchGraph *__restrict__ graphs, const int *__restrict__ order, int count, unsigned *next,
     const int32_t *__restrict__ weight, const int64_t *__restrict__ off, const int32_t *__restrict__ coords,
-    uint64_t *S, long long *selected, long long *total, unsigned *gstatus, unsigned *status, unsigned *pair_scratch,
-    unsigned pair_cap, int ncap, unsigned pcap, long long *prof) {
+    const int32_t *__restrict__ head, const unsigned *__restrict__ bad, uint64_t *S, long long *selected,
+    long long *total, unsigned *gstatus, unsigned *status, unsigned *pair_scratch, unsigned pair_cap, int ncap,
+    unsigned pcap, long long *prof) {
     extern __shared__ __align__(16) uint64_t smem[];
     const int wcap = ncap >> 6;                       // ncap is a multiple of 64
+    constexpr unsigned kListCap = kBThreads * kBQ + 64;
+    constexpr size_t kScanWords = 2048 + (20 * (size_t)kListCap + 7) / 8;  // scan_words(kBQ)
+    const size_t xw = kScanWords > (size_t)ncap ? kScanWords : (size_t)ncap;
     uint64_t *T = smem;                               // ncap words (the row buffers of the update alias it)
-    uint64_t *F = smem + ncap;                        // 64 x wcap words: the block's final rows
-    unsigned *sPairs = (unsigned *)(F + 64 * wcap);   // pcap pairs
+    uint64_t *F = smem + ncap;                        // 64 x wcap words: the block's final rows; before them:
+    uint64_t(*tab)[256] = reinterpret_cast<uint64_t(*)[256]>(F);  // the pivots' tables
+    RowList rows;                                     // and the rows of a round
+    rows.w = F + 2048;
+    uint64_t *row_w0 = rows.w + kListCap;      // their W as found
+    rows.key = reinterpret_cast<unsigned *>(row_w0 + kListCap);
+    unsigned *sPairs = (unsigned *)(F + xw);          // pcap pairs
     unsigned *gPairs = pair_scratch + (size_t)blockIdx.x * pair_cap;
 
-    __shared__ uint64_t sB[64];     // reduced echelon basis, by lead bit
-    __shared__ uint64_t sPivW[64];  // W of the pivots, in rank order
-    __shared__ int sPivR[64];       // their ranks
-    __shared__ uint64_t sMask[64];  // final masks m_k
-    __shared__ uint64_t sGcol[64];  // bit i of gcol[k] = <C_sel_k, S_{e0+i}> (i < k)
-    __shared__ uint64_t sMrow[64];  // beta of a row = XOR of sMrow[k] over the k with D bit k
-    __shared__ int sSel[64];        // rank selected at iteration e0 + k
-    __shared__ unsigned sPre[65];   // pair offsets of the selected lists
-    __shared__ int sWmin[kBWarps];
-    __shared__ uint64_t sNewRes, sNewW;
-    __shared__ int sGi;
+    __shared__ ElimShared es;
+    __shared__ uint64_t sBasis[64];  // reduced basis of the pivots, by pivot bit
+    __shared__ uint64_t sPivW[64];   // W of the pivots, in rank order
+    __shared__ int sPivR[64];        // their ranks
+    __shared__ uint64_t sMask[64];   // final masks m_k
+    __shared__ uint64_t sGcol[64];   // bit i of gcol[k] = <C_sel_k, S_{e0+i}> (i < k)
+    __shared__ uint64_t sMrow[64];   // beta of a row = XOR of sMrow[k] over the k with D bit k
+    __shared__ int sSel[64];         // rank selected at iteration e0 + k
+    __shared__ unsigned sPre[65];    // pair offsets of the selected lists
+    __shared__ __align__(8) unsigned sPart[kBQ * kBWarps];
+    __shared__ uint64_t sRepV[2][64], sRepW[2][64];  // this CTA's report of a round: residuals, W's,
+    __shared__ unsigned sRepKey[2][64], sRepN[2];    // ranks, number (by round parity)
+    __shared__ uint32_t sUnit[kRowRegs * 64], sHit[kRowRegs * 64];  // bit j: S_j = e_j; j on a cycle of the block
+    __shared__ int sGi[2];
     __shared__ unsigned sFail;
-    // profile (thread 0): cycles in T, scan, resolve, final rows, update; candidates
-    // scanned; cycles of the scan's list walks; pivot rounds; cycles of warp 0 in the
-    // update's D + beta and in its row writes
+    // profile (thread 0 of the first CTA): cycles in T, scan, resolve, final rows, update;
+    // candidates scanned; cycles of the scan's list walks; scan rounds; cycles of warp 0
+    // in the update's D + beta and in its row writes
     __shared__ long long pc[10];
     __shared__ unsigned long long s_walked;
 
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned csz = cluster.num_blocks(), crank = cluster.block_rank();
+    auto cluster_sync = [&] {
+        if (csz > 1) {
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        } else {
+            cta_sync();
+        }
+    };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gwarp = (int)crank * kBWarps + warp, nwarp = (int)csz * kBWarps;
     const unsigned full = 0xffffffffu;
 
-    for (;;) {
-        if (tid == 0) sGi = (int)atomicAdd(next, 1u);
-        cta_sync();
-        const int gi = sGi;
+    for (unsigned turn = 0;; turn ^= 1) {
+        if (crank == 0 && tid == 0) {
+            const int g = (int)atomicAdd(next, 1u);
+            for (unsigned i = 0; i < csz; i++) *cluster.map_shared_rank(&sGi[turn], i) = g;
+        }
+        cluster_sync();  // also: everyone is done with the previous problem
+        const int gi = sGi[turn];
         if (gi >= count) break;
         const int gx = order[gi];
         const BatchGraph g = graphs[gx];
@@ -157,40 +201,30 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
         const long long K = g.K, cand = g.cand;
         uint64_t *Sg = S + g.srow;
 
-        // the problem's coordinate lists: ascending, in [0, N); lengths fit the pair scratch
-        bool ok = N <= ncap;
-        for (long long r = tid; ok && r < K; r += kBThreads) {
-            const long long a = off[cand + r], e = off[cand + r + 1];
-            if (e - a > (long long)(pair_cap / 64)) ok = false;
-            int prev = -1;
-            for (long long i = a; ok && i < e; i++) {
-                const int c = coords[i];
-                if (c <= prev || c >= N) ok = false;
-                prev = c;
-            }
-        }
-        if (!cta_sync_and(ok)) {
-            if (tid == 0) {
+        // the problem's coordinate lists: ascending, in [0, N) (checked by the upload)
+        if (bad[gx] || N > ncap) {
+            if (crank == 0 && tid == 0) {
                 gstatus[gx] |= ST_BAD_INPUT;
                 atomicOr(status, ST_BAD_INPUT);
             }
             continue;  // the loop head's barrier separates the problems
         }
         // S_j = e_j; only words [0, j/64] of row j are ever read or written
-        for (int j = warp; j < N; j += kBWarps) {
+        for (int j = gwarp; j < N; j += nwarp) {
             uint64_t *row = Sg + (size_t)j * P;
             for (int w = lane; w <= (j >> 6); w += 32) row[w] = w == (j >> 6) ? 1ull << (j & 63) : 0ull;
         }
+        for (int i = tid; i < (N + 31) >> 5; i += kBThreads) sUnit[i] = 0xffffffffu;
         long long tot = 0;
         unsigned long long t_start = 0;
-        unsigned long long walked = 0;  // this thread's list-walk bytes (offsets + coordinates)
+        unsigned long long walked = 0;  // this thread's list-walk bytes
         if (prof && tid == 0) s_walked = 0;
         if (prof && tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
         if (tid == 0) {
             sFail = 0;
             for (int q = 0; q < 10; q++) pc[q] = 0;
         }
-        cta_sync();
+        cluster_sync();
 
         for (int e0 = 0; e0 < N; e0 += 64) {
             const int b = min(64, N - e0), bound = e0 + b, wl = e0 >> 6, Wb = wl + 1;
@@ -199,23 +233,14 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
             for (int c = e0 + tid; c < bound; c += kBThreads) T[c] = 1ull << (c - e0);
             for (int w = warp; w < wl; w += kBWarps) {
                 const uint64_t *r0 = Sg + (size_t)(e0 + lane) * P + w;
-                const uint64_t x0 = lane < b ? r0[0] : 0ull;
-                const uint64_t x1 = lane + 32 < b ? r0[(size_t)32 * P] : 0ull;
-                uint64_t v0 = 0, v1 = 0;
-#pragma unroll 8
-                for (int t = 0; t < 32; t++) {
-                    const unsigned lo = __ballot_sync(full, (x0 >> t) & 1), hi = __ballot_sync(full, (x1 >> t) & 1);
-                    if (lane == t) v0 = ((uint64_t)hi << 32) | lo;
-                }
-#pragma unroll 8
-                for (int t = 0; t < 32; t++) {
-                    const unsigned lo = __ballot_sync(full, (x0 >> (t + 32)) & 1),
-                                   hi = __ballot_sync(full, (x1 >> (t + 32)) & 1);
-                    if (lane == t) v1 = ((uint64_t)hi << 32) | lo;
-                }
-                T[(w << 6) + lane] = v0;
-                T[(w << 6) + 32 + lane] = v1;
+                uint64_t x0 = lane < b ? __ldcg(r0) : 0ull;
+                uint64_t x1 = lane + 32 < b ? __ldcg(r0 + (size_t)32 * P) : 0ull;
+                warp_transpose64(x0, x1);
+                T[(w << 6) + lane] = x0;
+                T[(w << 6) + 32 + lane] = x1;
             }
+            if (tid < 64) sBasis[tid] = 0;
+            for (int i = tid; i < (N + 31) >> 5; i += kBThreads) sHit[i] = 0;
             cta_sync();
             if (prof && tid == 0) {
                 const long long c = clock64();
@@ -225,94 +250,101 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
 
             // ---- 2. pivots: the first b rank-ordered candidates with independent W
             int npiv = 0;
-            uint64_t lead = 0;
-            for (long long base = 0; npiv < b; base += (long long)kBThreads * kBQ) {
+            const long long slice = (long long)kBThreads * kBQ;
+            unsigned par = 0;
+            for (long long base = 0; npiv < b; base += slice * csz, par ^= 1) {
                 if (base >= K) {  // fewer than b independent candidates
                     if (tid == 0) sFail = 1;
                     break;
                 }
-#if MCB_BATCH_PREFETCH
-                if (tid == 0) {  // the next chunk's offsets and lists into L2 while this one is walked
-                    const long long nb = base + (long long)kBThreads * kBQ;
-                    if (nb < K) {
-                        const long long ne = min(nb + (long long)kBThreads * kBQ, K);
-                        prefetch_l2(off + cand + nb, 8ull * (unsigned long long)(ne - nb + 1));
-                        const long long c0 = off[cand + nb], c1 = off[cand + ne];
-                        prefetch_l2(coords + c0, 4ull * (unsigned long long)(c1 - c0));
-                    }
+                const long long mine = base + (long long)crank * slice;
+                if (tid == 0) {  // the next slice's heads into L2 while this one is walked
+                    const long long nb = mine + slice * csz;
+                    if (nb < K) prefetch_l2(head + (size_t)(cand + nb) * kBHead, 4ull * kBHead * (unsigned long long)(min(nb + slice, K) - nb));
                 }
-#endif
-                // thread tid holds ranks base + tid * kBQ + q: key tid * kBQ + q is rank order
                 const long long cw = prof ? clock64() : 0;
-                bool first_round = true;
                 uint64_t W[kBQ], res[kBQ];
-                w_smem_q<kBQ>(base + (long long)tid * kBQ, K, cand, off, coords, T, bound, W, walked);
+                w_smem_q<kBQ>(mine + tid, K, cand, off, coords, head, T, bound, W, walked);
+                if (prof && tid == 0) {
+                    pc[6] += clock64() - cw;
+                    pc[7]++;
+                }
+                // what the pivots leave, in rank order
+                unsigned nz[kBQ];
 #pragma unroll
                 for (int q = 0; q < kBQ; q++) {
-                    res[q] = W[q];
-                    for (uint64_t m = W[q] & lead; m; m &= m - 1) res[q] ^= sB[ffs64(m)];
-                }
-                for (;;) {
-                    int myq = kBQ;
-#pragma unroll
-                    for (int q = kBQ - 1; q >= 0; q--)
-                        if (res[q]) myq = q;
-                    const unsigned bal = __ballot_sync(full, myq < kBQ);
-                    if (bal) {
-                        const int fl = __ffs(bal) - 1;
-                        const int fq = __shfl_sync(full, myq, fl);
-                        if (lane == 0) sWmin[warp] = (warp * 32 + fl) * kBQ + fq;
-                    } else if (lane == 0) {
-                        sWmin[warp] = 0x7fffffff;
-                    }
-                    cta_sync();
-                    if (prof && tid == 0) {
-                        if (first_round) pc[6] += clock64() - cw;
-                        pc[7]++;
-                    }
-                    first_round = false;
-                    int best = 0x7fffffff;
-#pragma unroll
-                    for (int q = 0; q < kBWarps; q++) best = min(best, sWmin[q]);
-                    if (best == 0x7fffffff) break;
-                    {
-                        uint64_t sr = 0, sw = 0;  // selects, not an indexed access (keeps res / W in registers)
-#pragma unroll
-                        for (int q = 0; q < kBQ; q++) {
-                            const bool h = tid * kBQ + q == best;
-                            sr = h ? res[q] : sr;
-                            sw = h ? W[q] : sw;
-                        }
-                        if (tid == best / kBQ) {
-                            sNewRes = sr;
-                            sNewW = sw;
-                        }
-                    }
-                    cta_sync();
-                    const uint64_t nr = sNewRes;
-                    const int L = ffs64(nr);
-                    if (warp == 0) {  // keep the basis reduced: clear bit L from the older vectors
-                        if (((lead >> lane) & 1) && ((sB[lane] >> L) & 1)) sB[lane] ^= nr;
-                        if (((lead >> (lane + 32)) & 1) && ((sB[lane + 32] >> L) & 1)) sB[lane + 32] ^= nr;
-                        if (lane == 0) {
-                            sB[L] = nr;
-                            sPivW[npiv] = sNewW;
-                            sPivR[npiv] = (int)(base + best);
-                        }
-                    }
-                    lead |= 1ull << L;
-                    npiv++;
-#pragma unroll
-                    for (int q = 0; q < kBQ; q++) {
-                        if (tid * kBQ + q == best)
-                            res[q] = 0;
-                        else if ((res[q] >> L) & 1)
-                            res[q] ^= nr;
-                    }
-                    if (npiv == b) break;
+                    res[q] = npiv > 0 && W[q] ? fr_reduce(W[q], tab) : W[q];
+                    nz[q] = __ballot_sync(full, res[q] != 0);
+                    if (lane == 0) sPart[q * kBWarps + warp] = __popc(nz[q]);
                 }
                 cta_sync();
-                if (tid == 0) pc[5] += kBThreads * kBQ;
+                constexpr int kPer = kBQ * kBWarps / 32;  // counts per lane
+                unsigned pc_[kPer], own = 0;
+#pragma unroll
+                for (int i = 0; i < kPer; i++) {
+                    pc_[i] = own;
+                    own += sPart[lane * kPer + i];
+                }
+                unsigned incl = own;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const unsigned y = __shfl_up_sync(full, incl, d);
+                    if (lane >= d) incl += y;
+                }
+                const unsigned cnt = __shfl_sync(full, incl, 31);
+#pragma unroll
+                for (int q = 0; q < kBQ; q++) {
+                    unsigned at = 0;
+#pragma unroll
+                    for (int i = 0; i < kPer; i++) {
+                        const unsigned v = __shfl_sync(full, incl - own + pc_[i], (q * kBWarps + warp) / kPer);
+                        if ((q * kBWarps + warp) % kPer == i) at = v;
+                    }
+                    at += __popc(nz[q] & ((1u << lane) - 1u));
+                    if (res[q]) {
+                        rows.w[at] = res[q];
+                        row_w0[at] = W[q];
+                        rows.key[at] = (unsigned)(mine - base) + q * kBThreads + tid;
+                    }
+                }
+                cta_sync();
+                int nnew = cnt ? eliminate(rows, cnt, b - npiv, es) : 0;
+                if (csz > 1) {
+                    if (tid < nnew) {
+                        sRepV[par][tid] = es.pw[tid];
+                        sRepW[par][tid] = row_w0[es.pat[tid]];
+                        sRepKey[par][tid] = es.pkey[tid];
+                    }
+                    if (tid == 0) sRepN[par] = (unsigned)nnew;
+                    cluster_sync();
+                    unsigned at = 0;
+                    for (unsigned i = 0; i < csz; i++) {
+                        const unsigned n = *cluster.map_shared_rank(&sRepN[par], i);
+                        if ((unsigned)warp / 2 == i) {  // two warps per CTA of the cluster
+                            const unsigned t = (unsigned)(warp & 1) * 32 + lane;
+                            if (t < n) {
+                                rows.w[at + t] = *cluster.map_shared_rank(&sRepV[par][t], i);
+                                row_w0[at + t] = *cluster.map_shared_rank(&sRepW[par][t], i);
+                                rows.key[at + t] = *cluster.map_shared_rank(&sRepKey[par][t], i);
+                            }
+                        }
+                        at += n;
+                    }
+                    cta_sync();
+                    nnew = at ? eliminate(rows, at, b - npiv, es) : 0;
+                }
+                if (nnew > 64 - npiv) nnew = 64 - npiv;
+                if (tid < nnew) {
+                    sPivW[npiv + tid] = row_w0[es.pat[tid]];
+                    sPivR[npiv + tid] = (int)(base + es.pkey[tid]);
+                }
+                npiv += nnew;
+                if (npiv < b && nnew > 0) {
+                    if (warp == 0) basis_add(sBasis, nnew, es);
+                    cta_sync();
+                    fr_build(tab, sBasis);
+                }
+                cta_sync();
+                if (tid == 0) pc[5] += slice * csz;
             }
             cta_sync();
             if (prof && tid == 0) {
@@ -324,75 +356,61 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
 
             // ---- 3. resolve (warp 0), gcol, the beta matrix, selected ranks, pair offsets
             if (warp == 0) {
-                const uint64_t W0 = lane < b ? sPivW[lane] : 0ull, W1 = lane + 32 < b ? sPivW[lane + 32] : 0ull;
-                uint64_t m0 = lane < b ? 1ull << lane : 0ull, m1 = lane + 32 < b ? 1ull << (lane + 32) : 0ull;
-                int p0 = 0, p1 = 0;  // pivot of iteration lane / lane + 32
-                bool bad = false;
-                for (int k = 0; k < b; k++) {
-                    const uint64_t mk = __shfl_sync(full, k < 32 ? m0 : m1, k & 31);
-                    const unsigned o0 = __ballot_sync(full, parity64(W0 & mk));
-                    const unsigned o1 = __ballot_sync(full, parity64(W1 & mk));
-                    const int p = o0 ? __ffs(o0) - 1 : (o1 ? 31 + __ffs(o1) : -1);
-                    if (p < 0) {  // cannot happen for independent pivots; guards the indexing
-                        bad = true;
-                        break;
-                    }
-                    const uint64_t Wp = __shfl_sync(full, p < 32 ? W0 : W1, p & 31);
-                    if (lane == (k & 31)) {
-                        if (k < 32)
-                            p0 = p;
-                        else
-                            p1 = p;
-                    }
-                    if (lane > k && parity64(Wp & m0)) m0 ^= mk;
-                    if (lane + 32 > k && parity64(Wp & m1)) m1 ^= mk;
-                }
-                sMask[lane] = m0;
-                sMask[lane + 32] = m1;
-                if (bad) {
+                uint64_t a0 = lane < b ? sPivW[lane] : 0ull, a1 = lane + 32 < b ? sPivW[lane + 32] : 0ull, m0, m1;
+                warp_transpose64(a0, a1);  // row j of A = bit j of every W
+                int p0, p1;                // pivot of iteration lane / lane + 32
+                const bool done = resolve_rows(b, a0, a1, m0, m1, p0, p1);
+                sMask[lane] = lane < b ? m0 : 0ull;
+                sMask[lane + 32] = lane + 32 < b ? m1 : 0ull;
+                if (!done) {  // cannot happen for independent pivots; guards the indexing
                     if (lane == 0) sFail = 1;
                 } else {
-                    __syncwarp();
-                    // gcol[k] bit i = parity(W_{p_k} & m_i), i < k
+                    // gcol[k] bit i = A[i][p_k] (i < k) of the final rows
+                    uint64_t col0 = a0, col1 = a1;
+                    warp_transpose64(col0, col1);
+#pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        const int k = lane + 32 * h;
-                        uint64_t gc = 0;
-                        if (k < b) {
-                            const uint64_t Wk = sPivW[h ? p1 : p0];
-                            for (int i = 0; i < k; i++) gc |= (uint64_t)parity64(Wk & sMask[i]) << i;
-                            sSel[k] = sPivR[h ? p1 : p0];
-                        }
-                        sGcol[k] = gc;
+                        const int k = lane + 32 * h, p = h ? p1 : p0;
+                        const uint64_t g0 = __shfl_sync(full, col0, p & 31), g1 = __shfl_sync(full, col1, p & 31);
+                        sGcol[k] = k < b ? (p < 32 ? g0 : g1) & ((1ull << k) - 1ull) : 0ull;
+                        if (k < b) sSel[k] = sPivR[p];
                     }
                     __syncwarp();
                     // beta for D = e_k: beta_i = 0 (i < k), 1 (i = k), parity(beta & gcol[i]) (i > k)
-                    for (int h = 0; h < 2; h++) {
-                        const int k = lane + 32 * h;
-                        uint64_t bt = 0;
-                        if (k < b) {
-                            bt = 1ull << k;
-                            for (int i = k + 1; i < b; i++) bt |= (uint64_t)parity64(bt & sGcol[i]) << i;
-                        }
-                        sMrow[k] = bt;
+                    uint64_t bt0 = 1ull << lane, bt1 = 1ull << (lane + 32);
+#pragma unroll 4
+                    for (int i = 1; i < b; i++) {
+                        const uint64_t gc = sGcol[i];
+                        if (i > lane) bt0 |= (uint64_t)parity64(bt0 & gc) << i;
+                        if (i > lane + 32) bt1 |= (uint64_t)parity64(bt1 & gc) << i;
                     }
+                    sMrow[lane] = lane < b ? bt0 : 0ull;
+                    sMrow[lane + 32] = lane + 32 < b ? bt1 : 0ull;
                     // pair offsets of the selected lists
                     long long l0 = 0, l1 = 0;
-                    if (lane < b) l0 = off[cand + sSel[lane] + 1] - off[cand + sSel[lane]];
-                    if (lane + 32 < b) l1 = off[cand + sSel[lane + 32] + 1] - off[cand + sSel[lane + 32]];
+                    unsigned long long wt = 0;
+                    if (lane < b) {
+                        l0 = off[cand + sSel[lane] + 1] - off[cand + sSel[lane]];
+                        wt += (unsigned long long)(long long)weight[cand + sSel[lane]];
+                    }
+                    if (lane + 32 < b) {
+                        l1 = off[cand + sSel[lane + 32] + 1] - off[cand + sSel[lane + 32]];
+                        wt += (unsigned long long)(long long)weight[cand + sSel[lane + 32]];
+                    }
                     unsigned s0 = (unsigned)l0, s1 = (unsigned)l1;
                     for (int d = 1; d < 32; d <<= 1) {
-                        const unsigned a0 = __shfl_up_sync(full, s0, d), a1 = __shfl_up_sync(full, s1, d);
+                        const unsigned a0_ = __shfl_up_sync(full, s0, d), a1_ = __shfl_up_sync(full, s1, d);
                         if (lane >= d) {
-                            s0 += a0;
-                            s1 += a1;
+                            s0 += a0_;
+                            s1 += a1_;
                         }
                     }
                     const unsigned t0 = __shfl_sync(full, s0, 31);
                     sPre[lane + 1] = s0;
                     sPre[lane + 33] = t0 + s1;
                     if (lane == 0) sPre[0] = 0;
-                    if (lane == 0)
-                        for (int k = 0; k < b; k++) tot += weight[cand + sSel[k]];
+                    for (int d = 16; d > 0; d >>= 1) wt += __shfl_xor_sync(full, wt, d);
+                    tot += (long long)wt;
                 }
             }
             cta_sync();
@@ -405,29 +423,39 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
             const unsigned np = sPre[b];
             unsigned *pairs = np <= pcap ? sPairs : gPairs;
 
-            // ---- 4. final rows of the block (shared F and global S), 5. pairs
-            for (int item = warp; item < b * wl; item += kBWarps) {
+            // ---- 4. final rows of the block: a share per CTA into S (and F, alone), 5. pairs
+            for (int item = gwarp; item < b * wl; item += nwarp) {
                 const int k = item / wl, w = item - k * wl;
                 const uint64_t mk = sMask[k];
                 const unsigned lo = __ballot_sync(full, parity64(T[(w << 6) + lane] & mk));
                 const unsigned hi = __ballot_sync(full, parity64(T[(w << 6) + 32 + lane] & mk));
                 if (lane == 0) {
                     const uint64_t v = ((uint64_t)hi << 32) | lo;
-                    F[k * Wb + w] = v;
+                    if (csz == 1) F[k * Wb + w] = v;
                     Sg[(size_t)(e0 + k) * P + w] = v;
                 }
             }
             for (int k = tid; k < b; k += kBThreads) {
                 F[k * Wb + wl] = sMask[k];
-                Sg[(size_t)(e0 + k) * P + wl] = sMask[k];
+                if (crank == 0) Sg[(size_t)(e0 + k) * P + wl] = sMask[k];
             }
             for (int k = warp; k < b; k += kBWarps) {
                 const long long a = off[cand + sSel[k]], e = off[cand + sSel[k] + 1];
                 const unsigned o = sPre[k];
-                for (long long i = a + lane; i < e; i += 32)
-                    pairs[o + (unsigned)(i - a)] = ((unsigned)coords[i] << 6) | (unsigned)k;
+                for (long long i = a + lane; i < e; i += 32) {
+                    const unsigned c = (unsigned)coords[i];
+                    pairs[o + (unsigned)(i - a)] = (c << 6) | (unsigned)k;
+                    if ((int)c >= bound) atomicOr(&sHit[c >> 5], 1u << (c & 31));
+                }
             }
-            cta_sync();
+            cluster_sync();
+            if (csz > 1) {  // the other CTAs' shares
+                for (int i = tid; i < b * wl; i += kBThreads) {
+                    const int k = i / wl, w = i - k * wl;
+                    F[k * Wb + w] = __ldcg(Sg + (size_t)(e0 + k) * P + w);
+                }
+                cta_sync();
+            }
             if (prof && tid == 0) {
                 const long long c = clock64();
                 pc[3] += c - c0;
@@ -437,16 +465,19 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
             // ---- 6. later rows: one warp per row.  The row's words [0, Wb) are loaded
             // once (coalesced) into registers and, below e0, into the warp's row buffer
             // (T's storage, free until the next block); D_j from the pairs against the
-            // buffer, beta = D_j x Mrow, then S_j ^= XOR_{k in beta} F_k.
+            // buffer, beta = D_j x Mrow, then S_j ^= XOR_{k in beta} F_k.  Row j belongs to
+            // warp j mod nwarp of the cluster throughout, which alone keeps its unit bit.
             uint64_t *rowbuf = T + (size_t)warp * wcap;
-            for (int j = bound + warp; j < N; j += kBWarps) {
+            for (int j = bound + ((gwarp - bound) % nwarp + nwarp) % nwarp; j < N; j += nwarp) {
+                const bool unit = (sUnit[j >> 5] >> (j & 31)) & 1u;
+                if (unit && !((sHit[j >> 5] >> (j & 31)) & 1u)) continue;  // D_j = 0
                 const long long cu0 = prof ? clock64() : 0;
                 uint64_t *Sj = Sg + (size_t)j * P;
                 uint64_t v[kRowRegs];
 #pragma unroll
                 for (int i = 0; i < kRowRegs; i++) {
                     const int w = lane + 32 * i;
-                    v[i] = w < Wb ? Sj[w] : 0ull;
+                    v[i] = w < Wb && !unit ? __ldcg(Sj + w) : 0ull;
                     if (w < wl) rowbuf[w] = v[i];
                 }
                 __syncwarp();
@@ -464,6 +495,7 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
                 const long long cu1 = prof ? clock64() : 0;
                 if (prof && tid == 0) pc[8] += cu1 - cu0;
                 if (beta) {
+                    if (unit && lane == 0) atomicAnd(&sUnit[j >> 5], ~(1u << (j & 31)));
 #pragma unroll
                     for (int i = 0; i < kRowRegs; i++) {
                         const int w = lane + 32 * i;
@@ -477,26 +509,23 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
                 if (prof && tid == 0) pc[9] += clock64() - cu1;
                 __syncwarp();
             }
-            if (tid == 0)
+            if (crank == 0 && tid == 0)
                 for (int k = 0; k < b; k++) selected[g.sel + e0 + k] = sSel[k];
-            cta_sync();
+            cluster_sync();
             if (prof && tid == 0) pc[4] += clock64() - c0;
         }
-        if (tid == 0) {
+        if (crank == 0 && tid == 0) {
             if (sFail) {
                 gstatus[gx] |= ST_RANK_DEFICIT;
                 atomicOr(status, ST_RANK_DEFICIT);
             }
-        }
-        if (warp == 0) {
-            // tot lives in lane 0 of warp 0
-            if (lane == 0) total[gx] = sFail ? -1 : tot;
+            total[gx] = sFail ? -1 : tot;  // tot lives in warp 0
         }
         if (prof) {
             atomicAdd(&s_walked, walked);
             cta_sync();
         }
-        if (prof && tid == 0) {
+        if (prof && crank == 0 && tid == 0) {
             unsigned long long t_end;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
             unsigned smid;
@@ -509,7 +538,7 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
             o[9] = pc[7];
             o[10] = pc[8];
             o[11] = pc[9];
-            o[12] = (long long)s_walked;
+            o[12] = (long long)(s_walked * csz);  // the other CTAs walk as much
         }
     }
 }
@@ -541,6 +570,45 @@ __global__ void batch_validate_kernel(const int64_t *__restrict__ off, long long
     }
 }
 
+// Behind it: each list's head (INT_MAX past its end), and bad[i] = 1 for a problem with
+// a list that is not ascending in [0, N).  `first` holds the problems' first candidates
+// (ascending; count entries).
+__global__ void __launch_bounds__(256) batch_lists_kernel(const int64_t *__restrict__ off, const int32_t *__restrict__ coords,
+                                                         long long K, const BatchGraph *__restrict__ graphs, int count,
+                                                         int32_t *head, unsigned *bad) {
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < K; r += (long long)gridDim.x * blockDim.x) {
+        int lo = 0, hi = count - 1;  // the last problem that starts at or before r
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (graphs[mid].cand <= r)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        const int N = graphs[lo].N;
+        const int64_t a = off[r], e = off[r + 1];
+        int v[kBHead], prev = -1;
+        bool ok = true;
+#pragma unroll
+        for (int q = 0; q < kBHead; q++) v[q] = a + q < e ? coords[a + q] : 0x7fffffff;
+#pragma unroll
+        for (int q = 0; q < kBHead; q++)
+            if (a + q < e) {
+                ok &= v[q] > prev && v[q] < N;
+                prev = v[q];
+            }
+        for (int64_t i = a + kBHead; i < e; i++) {
+            const int c = coords[i];
+            ok &= c > prev && c < N;
+            prev = c;
+        }
+        if (!ok) bad[lo] = 1u;
+        int4 *h = reinterpret_cast<int4 *>(head + (size_t)r * kBHead);
+        h[0] = make_int4(v[0], v[1], v[2], v[3]);
+        h[1] = make_int4(v[4], v[5], v[6], v[7]);
+    }
+}
+
 }  // namespace
 
 struct mcbgpu_batch {
@@ -548,28 +616,34 @@ struct mcbgpu_batch {
     int sm_count = 0;
     long long total_K = 0, nnz = 0, total_N = 0, s_words = 0;
     unsigned pair_cap = 0;   // pair scratch words per CTA (64 x the longest list)
-    int pair_slabs = 0;      // CTA slabs per class
     std::vector<BatchGraph> graphs;
-    std::vector<int> order;            // problems grouped by class, by decreasing N within a class
-    int class_off[kClasses + 1] = {};  // class c holds order[class_off[c], class_off[c + 1])
-    int class_ncap[kClasses] = {};     // largest N of the class (rounded up to 64)
-    int class_grid[kClasses] = {};
+    std::vector<int> order;  // problems with coordinates, class by class, each by decreasing N
+    struct Class {           // one launch: `cluster` CTAs per problem
+        int cluster, at = 0, count = 0;  // its problems in `order`
+        int ncap = 0;                    // largest N (rounded up to 64)
+        bool small = false;              // every problem fits the small form
+        int grid = 0, slab = 0;          // CTAs, and the first one's pair scratch
+        cudaStream_t st = nullptr;       // every class but the first launched runs beside the caller's stream
+        cudaEvent_t done = nullptr;
+    } cls[kClasses] = {{8}, {4}, {2}, {1}};
+    int slabs = 0;
+    cudaEvent_t ev_fork = nullptr;
     BatchGraph *d_graphs = nullptr;
     int *d_order = nullptr;
-    unsigned *d_next = nullptr;  // one work counter per class
+    unsigned *d_next = nullptr;  // the classes' work counters
     int32_t *d_weight = nullptr;
     int64_t *d_off = nullptr;
     int32_t *d_coords = nullptr;
+    int32_t *d_head = nullptr;   // kBHead per candidate
     uint64_t *d_S = nullptr;
     long long *d_selected = nullptr;
     long long *d_total = nullptr;
     unsigned *d_gstatus = nullptr;
+    unsigned *d_bad = nullptr;    // per problem: its lists are malformed
     unsigned *d_status = nullptr;
     unsigned *d_check = nullptr;  // [bad offsets, longest list]
     unsigned *d_pairs = nullptr;
-    long long *d_prof = nullptr;  // optional per-problem profile (count x 8)
-    cudaStream_t st[kClasses] = {};
-    cudaEvent_t ev_fork = nullptr, ev_join[kClasses] = {};
+    long long *d_prof = nullptr;  // optional per-problem profile (count x kBProf)
     bool uploaded = false;
     long long launches = 0;
     long long device_bytes = 0;
@@ -577,14 +651,20 @@ struct mcbgpu_batch {
 
 namespace {
 
-// Pairs kept in shared memory next to T and F for a class of largest N = ncap.
-unsigned batch_pair_smem(int ncap) {
-    const size_t tf = 16 * (size_t)ncap;
+size_t batch_region_words(bool small, int ncap) {
+    return std::max(scan_words(small ? kSmallQ : kLargeQ), (size_t)ncap);
+}
+
+// Pairs kept in shared memory next to T and the region of F.
+unsigned batch_pair_smem(bool small, int ncap) {
+    const size_t tf = 8 * ((size_t)ncap + batch_region_words(small, ncap));
     const size_t room = kSmemBudget > tf ? (kSmemBudget - tf) / 4 : 0;
     return (unsigned)std::min<size_t>(kPairSmemMax, room & ~(size_t)31);
 }
 
-size_t batch_smem_bytes(int ncap) { return 16 * (size_t)ncap + 4 * (size_t)batch_pair_smem(ncap); }
+size_t batch_smem_bytes(bool small, int ncap) {
+    return 8 * ((size_t)ncap + batch_region_words(small, ncap)) + 4 * (size_t)batch_pair_smem(small, ncap);
+}
 
 void free_batch(mcbgpu_batch *b) {
     if (!b) return;
@@ -594,47 +674,79 @@ void free_batch(mcbgpu_batch *b) {
     cudaFree(b->d_weight);
     cudaFree(b->d_off);
     cudaFree(b->d_coords);
+    cudaFree(b->d_head);
     cudaFree(b->d_S);
     cudaFree(b->d_selected);
     cudaFree(b->d_total);
     cudaFree(b->d_gstatus);
+    cudaFree(b->d_bad);
     cudaFree(b->d_status);
     cudaFree(b->d_check);
     cudaFree(b->d_pairs);
     cudaFree(b->d_prof);
-    for (int c = 0; c < kClasses; c++) {
-        if (b->st[c]) cudaStreamDestroy(b->st[c]);
-        if (b->ev_join[c]) cudaEventDestroy(b->ev_join[c]);
+    for (auto &c : b->cls) {
+        if (c.st) cudaStreamDestroy(c.st);
+        if (c.done) cudaEventDestroy(c.done);
     }
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     delete b;
 }
 
 using BatchKernel = void (*)(const BatchGraph *, const int *, int, unsigned *, const int32_t *, const int64_t *,
-                            const int32_t *, uint64_t *, long long *, long long *, unsigned *, unsigned *, unsigned *,
-                            unsigned, int, unsigned, long long *);
+                            const int32_t *, const int32_t *, const unsigned *, uint64_t *, long long *, long long *,
+                            unsigned *, unsigned *, unsigned *, unsigned, int, unsigned, long long *);
 
-// Class c's kernel: problems with N <= kClassMaxN[c] (row words per lane in the
-// update = kClassMaxN[c] / 2048, rounded up).
-BatchKernel class_kernel(int c) {
-    switch (c) {
-        case 0: return batch_solve_kernel<MCB_BATCH_Q0, 1, 2>;
-        case 1: return batch_solve_kernel<MCB_BATCH_Q, 2, 1>;
-        default: return batch_solve_kernel<MCB_BATCH_Q, (kBatchMaxN / 64 + 31) / 32, 1>;
+// A class is one queue in order of decreasing N: on the small form (two CTAs per SM)
+// when every problem has N <= kSmallN, else on the large one.
+BatchKernel batch_kernel(bool small) {
+    return small ? (BatchKernel)batch_solve_kernel<kSmallQ, (kSmallN / 64 + 31) / 32, 2>
+                 : (BatchKernel)batch_solve_kernel<kLargeQ, (kBatchMaxN / 64 + 31) / 32, 1>;
+}
+
+// CTAs per problem, as powers of two into `lg`.  One CTA each is the least work; but a
+// long problem alone can take longer than the whole batch spread over the GPU, and then
+// its scan and rows are split over a cluster.  With w = N x K (blocks times candidates)
+// for a problem's time on one CTA, a cluster of 2, 4, 8 takes 0.62, 0.365, 0.23 of it
+// (measured on problems of N = 5,700-6,400).  The least makespan M is sought for which
+// every problem on its smallest sufficient cluster takes at most M and all of them
+// together fill at most the GPU for M.  A CTA's slice of a scan round and some rows per
+// warp must be left, so short problems stay on one CTA.  384 graphs of 50-5000 vertices:
+// 69.5 ms on single CTAs (102 before), 43.0 / 25.3 / 32.9 with clusters of 2 / 4 / 8 for all,
+// 17.7 this way; 4096 such graphs and the components of a block tree stay on single CTAs.
+void choose_clusters(const std::vector<BatchGraph> &graphs, const std::vector<int> &order, int sms, std::vector<int> &lg) {
+    const double time_of[kClasses] = {1.0, 0.62, 0.365, 0.23};
+    lg.assign(graphs.size(), 0);
+    double all = 0;
+    auto weight = [&](int i) { return (double)graphs[i].N * (double)std::max<long long>(graphs[i].K, 2048); };
+    for (int i : order) all += weight(i);
+    for (double m = all / std::max(sms, 1);; m *= 1.1) {
+        double load = 0, longest = 0;
+        for (int i : order) {
+            const long long slice = (long long)kBThreads * kLargeQ;
+            int l = 0;
+            while (l + 1 < kClasses && weight(i) * time_of[l] > m && graphs[i].K > (slice << (l + 1)) &&
+                   graphs[i].N > (512 << l))
+                l++;
+            lg[i] = l;
+            load += weight(i) * time_of[l] * (1 << l);
+            longest = std::max(longest, weight(i) * time_of[l]);
+        }
+        // m has reached what the longest problem needs, or nothing can be split further
+        if (load / std::max(sms, 1) <= m || longest >= all) return;
     }
 }
 
-// The launch a problem goes to.  With MCB_BATCH_SINGLE (the default) a batch is one
-// queue in order of decreasing N: on the small-problem kernel (two CTAs per SM) when
-// every problem has N <= kClassMaxN[0], else on the largest-class kernel.  One queue
-// keeps the longest problems first across the whole batch (4096 graphs of the
-// batched configuration: 156 ms against 218 ms with a launch per size class, whose
-// large-problem CTAs take every SM first).
-int class_of(int N, int maxN) {
-    if (MCB_BATCH_SINGLE) return maxN <= kClassMaxN[0] ? 0 : kClasses - 1;
-    int c = 0;
-    while (c < kClasses - 1 && N > kClassMaxN[c]) c++;
-    return c;
+void batch_launch_config(const mcbgpu_batch::Class &c, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
+    cfg = {};
+    cfg.gridDim = dim3((unsigned)std::max(c.grid, c.cluster));
+    cfg.blockDim = dim3(kBThreads);
+    cfg.dynamicSmemBytes = batch_smem_bytes(c.small, c.ncap);
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)c.cluster;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
 }
 
 }  // namespace
@@ -675,24 +787,27 @@ int mcbgpu_batch_create(mcbgpu_batch **out, int32_t count, const int32_t *num_co
         b->total_N += g.N;
         b->s_words += (long long)g.N * g.P;
     }
-    // problems with no coordinate need no work; the rest by class, each by decreasing N
-    std::vector<int> idx;
+    // problems with no coordinate need no work; the rest by decreasing N
     for (int i = 0; i < count; i++)
-        if (b->graphs[i].N > 0) idx.push_back(i);
-    std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return b->graphs[x].N > b->graphs[y].N; });
-    const int maxN = idx.empty() ? 0 : b->graphs[idx[0]].N;
-    for (int c = 0; c < kClasses; c++) {
-        b->class_off[c] = (int)b->order.size();
-        for (int i : idx)
-            if (class_of(b->graphs[i].N, maxN) == c) {
-                b->order.push_back(i);
-                b->class_ncap[c] = std::max(b->class_ncap[c], (b->graphs[i].N + 63) & ~63);
-            }
-    }
-    b->class_off[kClasses] = (int)b->order.size();
+        if (b->graphs[i].N > 0) b->order.push_back(i);
+    std::stable_sort(b->order.begin(), b->order.end(),
+                     [&](int x, int y) { return b->graphs[x].N > b->graphs[y].N; });
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, dev);
+    {
+        std::vector<int> lg, sorted;
+        choose_clusters(b->graphs, b->order, b->sm_count, lg);
+        for (auto &c : b->cls) {
+            c.at = (int)sorted.size();
+            for (int i : b->order)
+                if ((1 << lg[i]) == c.cluster) sorted.push_back(i);
+            c.count = (int)sorted.size() - c.at;
+            if (c.count > 0) c.ncap = (b->graphs[sorted[c.at]].N + 63) & ~63;
+            c.small = c.ncap <= kSmallN;
+        }
+        b->order.swap(sorted);
+    }
     long long bytes = 0;
 #define ALLOC(ptr, sz)                                             \
     do {                                                           \
@@ -707,10 +822,12 @@ int mcbgpu_batch_create(mcbgpu_batch **out, int32_t count, const int32_t *num_co
     ALLOC(b->d_weight, sizeof(int32_t) * (size_t)b->total_K);
     ALLOC(b->d_off, sizeof(int64_t) * (size_t)(b->total_K + 1));
     ALLOC(b->d_coords, sizeof(int32_t) * (size_t)nnz);
+    ALLOC(b->d_head, sizeof(int32_t) * kBHead * (size_t)b->total_K);
     ALLOC(b->d_S, sizeof(uint64_t) * (size_t)b->s_words);
     ALLOC(b->d_selected, sizeof(long long) * (size_t)b->total_N);
     ALLOC(b->d_total, sizeof(long long) * (size_t)count);
     ALLOC(b->d_gstatus, sizeof(unsigned) * (size_t)count);
+    ALLOC(b->d_bad, sizeof(unsigned) * (size_t)count);
     ALLOC(b->d_status, sizeof(unsigned));
     ALLOC(b->d_check, 2 * sizeof(unsigned));
 #undef ALLOC
@@ -718,25 +835,29 @@ int mcbgpu_batch_create(mcbgpu_batch **out, int32_t count, const int32_t *num_co
         e = cudaMemcpy(b->d_graphs, b->graphs.data(), sizeof(BatchGraph) * (size_t)count, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !b->order.empty())
         e = cudaMemcpy(b->d_order, b->order.data(), sizeof(int) * b->order.size(), cudaMemcpyHostToDevice);
-    for (int c = 0; c < kClasses && e == cudaSuccess; c++) {
-        e = cudaStreamCreateWithFlags(&b->st[c], cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join[c], cudaEventDisableTiming);
+    // the attribute is per kernel, shared by all handles: the form's largest need
+    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+        const int most = k ? kBatchMaxN : kSmallN;
+        size_t need = batch_smem_bytes(!k, most);
+        for (int n = 64; n < most; n += 64) need = std::max(need, batch_smem_bytes(!k, n));
+        e = cudaFuncSetAttribute(batch_kernel(!k), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    }
+    for (auto &c : b->cls) {
+        if (e != cudaSuccess || c.count == 0) continue;
+        // as many clusters as are resident at once, at most one per problem
+        int clusters = 0;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        batch_launch_config(c, cfg, at);
+        e = cudaOccupancyMaxActiveClusters(&clusters, batch_kernel(c.small), &cfg);
+        if (e == cudaSuccess && clusters < 1) e = cudaErrorInvalidConfiguration;
+        c.grid = c.cluster * std::min(c.count, clusters);
+        c.slab = b->slabs;
+        b->slabs += c.grid;
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c.st, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
-    // one persistent grid per class: as many CTAs as are resident at once, at most one per problem
-    // the attribute is per kernel, shared by all handles: the class's largest need
-    for (int c = 0; c < kClasses && e == cudaSuccess; c++)
-        e = cudaFuncSetAttribute(class_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)batch_smem_bytes(kClassMaxN[c]));
-    for (int c = 0; c < kClasses && e == cudaSuccess; c++) {
-        const int n = b->class_off[c + 1] - b->class_off[c];
-        if (n == 0) continue;
-        int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, class_kernel(c), kBThreads,
-                                                          batch_smem_bytes(b->class_ncap[c]));
-        if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
-        b->class_grid[c] = (int)std::min<long long>(n, (long long)per_sm * std::max(b->sm_count, 1));
-    }
     if (e != cudaSuccess) {
         free_batch(b);
         return cuda_fail(e, "mcbgpu_batch_create");
@@ -783,18 +904,25 @@ int mcbgpu_batch_upload(mcbgpu_batch *b, const int32_t *weight, const int64_t *o
         return MCBGPU_E_ARG;
     }
     const unsigned cap = (unsigned)(64 * std::max<long long>(max_len, 1));
-    int slabs = 1;
-    for (int c = 0; c < kClasses; c++) slabs = std::max(slabs, b->class_grid[c]);
-    if (cap > b->pair_cap) {  // one slab per CTA of the widest class grid, for each class
+    if (cap > b->pair_cap) {  // one slab per CTA
         cudaFree(b->d_pairs);
         b->d_pairs = nullptr;
         b->pair_cap = 0;
-        const size_t n = (size_t)cap * (size_t)slabs * kClasses;
+        const size_t n = (size_t)cap * (size_t)std::max(b->slabs, 1);
         MCB_CUDA(cudaMalloc((void **)&b->d_pairs, sizeof(unsigned) * n));
         b->device_bytes += (long long)(sizeof(unsigned) * n);
         b->pair_cap = cap;
-        b->pair_slabs = slabs;
     }
+    // the offsets are good: heads, and the coordinate lists checked problem by problem
+    // (a bad one fails alone, when it is solved)
+    if (b->count > 0) MCB_CUDA(cudaMemsetAsync(b->d_bad, 0, sizeof(unsigned) * (size_t)b->count, st));
+    if (b->total_K > 0) {
+        const int grid = (int)std::min<long long>((b->total_K + 255) / 256, (long long)std::max(b->sm_count, 1) * 16);
+        batch_lists_kernel<<<grid, 256, 0, st>>>(b->d_off, b->d_coords, b->total_K, b->d_graphs, b->count, b->d_head,
+                                                 b->d_bad);
+        MCB_CUDA(cudaGetLastError());
+    }
+    MCB_CUDA(cudaStreamSynchronize(st));
     b->uploaded = true;
     return MCBGPU_OK;
 }
@@ -811,20 +939,32 @@ int mcbgpu_batch_run(mcbgpu_batch *b, void *stream) {
         MCB_CUDA(cudaMemsetAsync(b->d_gstatus, 0, sizeof(unsigned) * (size_t)b->count, st));
         MCB_CUDA(cudaMemsetAsync(b->d_total, 0, sizeof(long long) * (size_t)b->count, st));
     }
+    // the classes side by side, the widest clusters first: the first on the caller's
+    // stream, the others forked from it and joined
     MCB_CUDA(cudaEventRecord(b->ev_fork, st));
-    for (int c = 0; c < kClasses; c++) {
-        const int n = b->class_off[c + 1] - b->class_off[c];
-        if (n == 0) continue;
-        MCB_CUDA(cudaStreamWaitEvent(b->st[c], b->ev_fork, 0));
-        class_kernel(c)<<<b->class_grid[c], kBThreads, batch_smem_bytes(b->class_ncap[c]), b->st[c]>>>(
-            b->d_graphs, b->d_order + b->class_off[c], n, b->d_next + c, b->d_weight, b->d_off, b->d_coords, b->d_S,
-            b->d_selected, b->d_total, b->d_gstatus, b->d_status,
-            b->d_pairs + (size_t)c * b->pair_cap * (size_t)b->pair_slabs, b->pair_cap, b->class_ncap[c],
-            batch_pair_smem(b->class_ncap[c]), b->d_prof);
+    cudaStream_t on = st;
+    for (int k = 0; k < kClasses; k++) {
+        const auto &c = b->cls[k];
+        if (c.count == 0) continue;
+        if (on != st) MCB_CUDA(cudaStreamWaitEvent(on = c.st, b->ev_fork, 0));
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        batch_launch_config(c, cfg, at);
+        cfg.stream = on;
+        MCB_CUDA(cudaLaunchKernelEx(&cfg, batch_kernel(c.small), (const BatchGraph *)b->d_graphs,
+                                    (const int *)(b->d_order + c.at), c.count, b->d_next + k,
+                                    (const int32_t *)b->d_weight, (const int64_t *)b->d_off,
+                                    (const int32_t *)b->d_coords, (const int32_t *)b->d_head,
+                                    (const unsigned *)b->d_bad, b->d_S, b->d_selected, b->d_total, b->d_gstatus,
+                                    b->d_status, b->d_pairs + (size_t)c.slab * b->pair_cap, b->pair_cap, c.ncap,
+                                    batch_pair_smem(c.small, c.ncap), b->d_prof));
         MCB_CUDA(cudaGetLastError());
         b->launches++;
-        MCB_CUDA(cudaEventRecord(b->ev_join[c], b->st[c]));
-        MCB_CUDA(cudaStreamWaitEvent(st, b->ev_join[c], 0));
+        if (on != st) {
+            MCB_CUDA(cudaEventRecord(c.done, on));
+            MCB_CUDA(cudaStreamWaitEvent(st, c.done, 0));
+        }
+        on = c.st;
     }
     return MCBGPU_OK;
 }

@@ -303,7 +303,8 @@ class BatchSolver:
     def __init__(self, problems, stream=0, upload: bool = True):
         self.lib = gpu_lib()
         self.count = len(problems)
-        self.N = np.array([int(p[0]) for p in problems], np.int32)
+        self._counts = [int(p[0]) for p in problems]  # as Python integers: a slice per problem in results()
+        self.N = np.array(self._counts, np.int32)
         self.K = np.array([len(p[1]) for p in problems], np.int64)
         ws, offs, cos = [], [], []
         base = 0
@@ -347,12 +348,15 @@ class BatchSolver:
 
     def results(self, stream=0):
         """([selected ranks per problem], total weights int64[count]) after synchronising `stream`."""
-        sel = np.full(max(int(self.N.sum()), 1), -1, np.int64)
+        sel = np.empty(max(sum(self._counts), 1), np.int64)
         tot = np.zeros(max(self.count, 1), np.int64)
         check_gpu(self.lib.mcbgpu_batch_results(self._h, ptr(sel), ptr(tot), None, _stream(stream)),
                   "mcbgpu_batch_results")
-        bounds = np.concatenate([[0], np.cumsum(self.N.astype(np.int64))])
-        return [sel[bounds[i]:bounds[i + 1]] for i in range(self.count)], tot[: self.count]
+        at, sels = 0, []
+        for n in self._counts:
+            sels.append(sel[at:at + n])
+            at += n
+        return sels, tot[: self.count]
 
     def status(self, stream=0) -> np.ndarray:
         """Per-problem status words (0 = solved), without raising."""
