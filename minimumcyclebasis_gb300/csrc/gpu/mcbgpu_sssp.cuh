@@ -16,8 +16,12 @@
 //      the arcs of every dirty vertex nearer than lo + delta, marking improved heads
 //      dirty.  The dirty vertex at lo is final after its round (weights >= 1), so a
 //      root needs at most 2 (n + 1) rounds; the loop stops there and flags the root
-//      if it has not converged.  Distances and dirty bits live in shared memory up
-//      to kTreeSharedMaxN vertices, in a per-CTA global slice beyond.  delta (the
+//      if it has not converged.  A round first lists the vertices to relax, then gives
+//      each kTreeLanes lanes, one arc at a time each: one thread per dirty word with its
+//      vertices and arcs one after the other left a few threads with all of a frontier
+//      of neighbours (planar-chain graph of 65k points: 14.8 us per root, 5.2 now; random
+//      graph of 20k vertices 3.2, 1.0 now; 2 or 8 lanes are within 8%).  Distances and dirty bits live in shared
+//      memory up to kTreeSharedMaxN vertices, in a per-CTA global slice beyond.  delta (the
 //      bucket width) trades rounds (each a pass over the dirty bits and a barrier)
 //      against relaxations repeated inside a bucket; the callers time a few widths
 //      and CTA shapes on their first roots and keep the fastest.
@@ -37,6 +41,7 @@
 #pragma once
 
 #include <climits>
+#include <type_traits>
 #include <vector>
 
 #include "mcbgpu_internal.cuh"
@@ -48,7 +53,10 @@ namespace sssp {
 namespace {
 
 constexpr int kTreeThreads = 1024;      // the shared-memory form's CTA
-constexpr int kTreeSharedMaxN = 53248;  // 208 KB of distances + 6.5 KB of dirty bits (of 227 KB)
+constexpr int kTreeSharedMaxN = 53248;  // 208 KB of distances + 6.5 KB of dirty bits + 8 KB of list (of 227 KB)
+constexpr int kTreeLanes = 4;  // lanes that share a listed vertex's arcs
+constexpr int kTreeSharedList = 4096;   // vertices listed per round: shared form (16 bits each)
+constexpr int kTreeGlobalList = 1024;   // and global form
 constexpr int kTreeMaxCtasPerSm = 16;   // the global form's per-CTA slices are sized for this many
 
 struct TreeArgs {
@@ -71,31 +79,49 @@ struct TreeArgs {
 };
 
 // Threads per CTA: the shared-memory form runs one 1024-thread CTA per SM (its
-// distances fill the shared memory); the global form runs kThreads-thread CTAs,
-// several per SM, so that the bucket rounds of different roots overlap.
-template <bool kShared, int kThreads>
-__global__ void __launch_bounds__(kThreads) trees_kernel(TreeArgs a) {
+// distances fill the shared memory); the other forms run kThreads-thread CTAs, several
+// per SM, so that the bucket rounds of different roots overlap.  Their distances are
+// in the CTA's global slice; the dirty bits in shared memory while eight CTAs' fit an SM
+// (kTreeDirty, up to kTreeDirtyMaxN vertices), else beside the distances with a summary.
+// They wait on L2 half of their time, so a full SM of threads (32 registers, a few spills)
+// is worth more than registers: 5.2 us per root against 5.8 with 1536 threads.
+enum TreeForm { kTreeShared, kTreeDirty, kTreeGlobal };
+template <int kForm, int kThreads>
+__global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kThreads) trees_kernel(TreeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_next[3];
     __shared__ int s_root;
-    __shared__ int s_cnt[2];
+    __shared__ int s_cnt[2], s_nv[2];
     const int n = a.n;
     const int words = (n + 31) >> 5;
     const int swords = (words + 31) >> 5;  // summary: one bit per dirty word
     int32_t *dist;
     uint32_t *dirty, *summ;
+    constexpr bool kShared = kForm == kTreeShared, kSummary = kForm == kTreeGlobal;
+    using VertT = typename std::conditional<kShared, uint16_t, uint32_t>::type;
+    constexpr int kListCap = kShared ? kTreeSharedList : kTreeGlobalList;
+    VertT *s_verts;  // the vertices of a round
     if (kShared) {
         dist = reinterpret_cast<int32_t *>(smem);
         dirty = reinterpret_cast<uint32_t *>(smem + (((size_t)n * 4 + 15) & ~(size_t)15));
-        summ = dirty + words;
+        summ = nullptr;
+        s_verts = reinterpret_cast<VertT *>(dirty + words);
+    } else if (!kSummary) {
+        dist = a.gdist + (size_t)blockIdx.x * n;
+        dirty = reinterpret_cast<uint32_t *>(smem + 4 * kTreeGlobalList);
+        summ = nullptr;
+        s_verts = reinterpret_cast<VertT *>(smem);
     } else {
         dist = a.gdist + (size_t)blockIdx.x * n;
         dirty = a.gdirty + (size_t)blockIdx.x * words;
         summ = a.gsumm + (size_t)blockIdx.x * swords;
+        s_verts = reinterpret_cast<VertT *>(smem);
     }
     // global form: the dirty words of a round (words < 65536 entries, 16-bit)
-    uint16_t *s_list = reinterpret_cast<uint16_t *>(smem);
+    uint16_t *s_list = reinterpret_cast<uint16_t *>(smem + 4 * kTreeGlobalList);
     volatile int32_t *vdist = dist;
+    // a distance as the CTA's atomics left it; global ones from L2, loads free to overlap
+    auto get = [&](uint32_t v) -> int { return kShared ? vdist[v] : __ldcg(dist + v); };
     volatile uint32_t *vdirty = dirty;
     volatile uint32_t *vsumm = summ;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
@@ -108,22 +134,25 @@ __global__ void __launch_bounds__(kThreads) trees_kernel(TreeArgs a) {
         const uint32_t src = a.roots[r];  // < n, checked by the host
         for (int v = tid; v < n; v += nt) dist[v] = INT_MAX;
         for (int k = tid; k < words; k += nt) dirty[k] = 0;
-        for (int k = tid; k < swords; k += nt) summ[k] = 0;
+        if (kSummary)
+            for (int k = tid; k < swords; k += nt) summ[k] = 0;
         if (tid == 0) {
             s_next[0] = INT_MAX;
             s_next[1] = INT_MAX;
             s_cnt[0] = 0;
             s_cnt[1] = 0;
+            s_nv[0] = 0;
+            s_nv[1] = 0;
         }
         cta_sync();
         if (tid == 0) {
             dist[src] = 0;
             dirty[src >> 5] = 1u << (src & 31);
-            summ[src >> 10] = 1u << ((src >> 5) & 31);
+            if (kSummary) summ[src >> 10] = 1u << ((src >> 5) & 31);
         }
         cta_sync();
         // 1. distances.  One pass per round over the dirty bits: vertices nearer than
-        // hi = lo + delta are relaxed, the others skipped; the next round's lo is the
+        // hi = lo + delta are listed and relaxed, the others skipped; the next round's lo is the
         // smallest distance of a skipped vertex or of an improvement made in this
         // round (at most the smallest distance left dirty, so no vertex is missed;
         // an underestimate only costs a round).  The dirty vertex at the true lo is
@@ -142,50 +171,51 @@ __global__ void __launch_bounds__(kThreads) trees_kernel(TreeArgs a) {
             const int slot = round % 3;
             if (tid == 0) s_next[(round + 1) % 3] = INT_MAX;
             int mynext = INT_MAX;
-            // One dirty word: relax its vertices nearer than hi, keep the others (and
-            // their smallest distance for the next round).  Returns whether some
-            // vertex was left dirty.
-            auto scan_word = [&](int k) {
-                uint32_t bits = vdirty[k];
-                bool left = false;
-                while (bits) {
-                    const int b = __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    const int v = (k << 5) + b;
-                    const int d0 = vdist[v];
-                    if (d0 >= hi) {
-                        mynext = d0 < mynext ? d0 : mynext;
-                        left = true;
-                        continue;
+            int *nv = &s_nv[round & 1];
+            if (tid == 0) s_nv[(round + 1) & 1] = 0;  // read last in round - 1, before its barrier
+            // One dirty word: its vertices nearer than hi leave it for the round's list, the
+            // others stay (and their smallest distance counts for the next round), as do
+            // those that find the list full.  Returns whether some vertex was left dirty.
+            auto list_word = [&](int k) {
+                const uint32_t bits = vdirty[k];
+                uint32_t take = 0;
+                for (uint32_t m = bits; m;) {  // four distances in flight
+                    int b[4], d[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        b[q] = __ffs(m) - 1;
+                        m &= m - 1;
+                        d[q] = b[q] >= 0 ? get((uint32_t)((k << 5) + b[q])) : INT_MAX;
                     }
-                    atomicAnd(&dirty[k], ~(1u << b));
-                    // pairs with the fence between a writer's atomicMin and atomicOr:
-                    // a bit this atomicAnd cleared was set after its distance was
-                    // lowered, so the read below sees that distance; a later
-                    // improvement sets the bit again
-                    __threadfence_block();
-                    const int dv = vdist[v];
-                    for (uint32_t o = a.ro[v]; o < a.ro[v + 1]; o++) {
-                        const uint32_t x = a.cols[o];
-                        const int nd = dv + a.w[o];
-                        if (nd < vdist[x]) {
-                            const int old = atomicMin(&dist[x], nd);
-                            if (nd < old) {
-                                __threadfence_block();  // the new distance before the dirty bit
-                                atomicOr(&dirty[x >> 5], 1u << (x & 31));
-                                if (!kShared) {
-                                    __threadfence_block();  // the dirty bit before the summary bit
-                                    atomicOr(&summ[x >> 10], 1u << ((x >> 5) & 31));
-                                }
-                                mynext = nd < mynext ? nd : mynext;
-                            }
-                        }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (d[q] < hi)
+                            take |= 1u << b[q];
+                        else
+                            mynext = d[q] < mynext ? d[q] : mynext;
                     }
                 }
-                return left;
+                if (take) {
+                    int at = atomicAdd(nv, __popc(take));
+                    uint32_t listed = 0;
+                    for (uint32_t m = take; m; m &= m - 1, at++) {
+                        const int b = __ffs(m) - 1;
+                        if (at < kListCap) {
+                            s_verts[at] = (VertT)((k << 5) + b);
+                            listed |= 1u << b;
+                        } else {
+                            mynext = lo < mynext ? lo : mynext;
+                        }
+                    }
+                    // the bits go before the barrier, the distances are read after it: a
+                    // distance lowered since sets its bit again
+                    if (listed) atomicAnd(&dirty[k], ~listed);
+                    take = listed;
+                }
+                return (bits & ~take) != 0;
             };
-            if (kShared) {
-                for (int k = tid; k < words; k += nt) scan_word(k);
+            if (!kSummary) {
+                for (int k = tid; k < words; k += nt) list_word(k);
             } else {
                 // the summary words: a set bit marks a dirty word as possibly non-zero.
                 // A writer sets the dirty bit, then the summary bit (fence between).
@@ -193,9 +223,7 @@ __global__ void __launch_bounds__(kThreads) trees_kernel(TreeArgs a) {
                 // orders the clears before phase 2's reads of the words, so a bit set
                 // before a clear is seen in its word and one set after it leaves the
                 // summary bit set for the next round; a word left with skipped
-                // vertices gets its summary bit back.  The list spreads the words of
-                // one summary word (neighbouring vertices, often all of the frontier)
-                // over the CTA.
+                // vertices gets its summary bit back.
                 int *cnt = &s_cnt[round & 1];
                 if (tid == 0) s_cnt[(round + 1) & 1] = 0;  // read last in round - 1, before its barrier
                 for (int q = tid; q < swords; q += nt) {
@@ -212,7 +240,32 @@ __global__ void __launch_bounds__(kThreads) trees_kernel(TreeArgs a) {
                 const int m = *(volatile int *)cnt;
                 for (int i = tid; i < m; i += nt) {
                     const int k = s_list[i];
-                    if (scan_word(k)) atomicOr(&summ[k >> 5], 1u << (k & 31));
+                    if (list_word(k)) atomicOr(&summ[k >> 5], 1u << (k & 31));
+                }
+            }
+            __threadfence_block();
+            cta_sync();
+            // the listed vertices' arcs, kTreeLanes at a time
+            const int listed = min(*(volatile int *)nv, kListCap);
+            for (int i = tid / kTreeLanes; i < listed; i += nt / kTreeLanes) {
+                const int v = s_verts[i];
+                const uint32_t o1 = __ldg(a.ro + v + 1);
+                const int dv = get((uint32_t)v);
+                for (uint32_t o = __ldg(a.ro + v) + tid % kTreeLanes; o < o1; o += kTreeLanes) {
+                    const uint32_t x = __ldg(a.cols + o);
+                    const int nd = dv + __ldg(a.w + o);
+                    if (nd < get(x)) {
+                        const int old = atomicMin(&dist[x], nd);
+                        if (nd < old) {
+                            __threadfence_block();  // the new distance before the dirty bit
+                            atomicOr(&dirty[x >> 5], 1u << (x & 31));
+                            if (kSummary) {
+                                __threadfence_block();  // the dirty bit before the summary bit
+                                atomicOr(&summ[x >> 10], 1u << ((x >> 5) & 31));
+                            }
+                            mynext = nd < mynext ? nd : mynext;
+                        }
+                    }
                 }
             }
             mynext = __reduce_min_sync(0xffffffffu, mynext);
@@ -223,32 +276,45 @@ __global__ void __launch_bounds__(kThreads) trees_kernel(TreeArgs a) {
         // 2. parents by the rule, and the root's tie flag
         int tie = converged ? 0 : 1;
         for (int c = tid; c < n; c += nt) {
-            const int dc = vdist[c];
+            const int dc = get((uint32_t)c);
             int32_t slot = -1;
             if ((uint32_t)c != src && dc != INT_MAX) {
                 int bestd = INT_MAX, rival = 0;  // rival: another neighbour as near as the best
                 int shorter = 0;                 // some slot offers c a shorter path
                 uint32_t bestx = 0xffffffffu, bests = 0xffffffffu;
-                for (uint32_t o = a.ro[c]; o < a.ro[c + 1]; o++) {
-                    const uint32_t x = a.cols[o];
-                    const int dx = vdist[x];
-                    if (dx == INT_MAX) continue;
-                    // the certificate of exact distances: no slot gives c a shorter
-                    // path (with every vertex's distance that of a real path through
-                    // its parent, below, the distances are the shortest); a root
-                    // that fails it is left to the host
-                    if ((long long)dx + a.w[o] < (long long)dc) shorter = 1;
-                    if ((long long)dx + a.w[o] != (long long)dc) continue;
-                    if (dx < bestd) {
-                        bestd = dx;
-                        bestx = x;
-                        bests = a.rev[o];
-                        rival = 0;
-                    } else if (dx == bestd) {
-                        if (x == bestx)
-                            bests = a.rev[o] < bests ? a.rev[o] : bests;
-                        else
-                            rival = 1;
+                const uint32_t o1 = __ldg(a.ro + c + 1);
+                for (uint32_t ob = __ldg(a.ro + c); ob < o1; ob += 4) {  // four arcs in flight
+                    uint32_t xs[4];
+                    int dxs[4], ws[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        xs[q] = ob + q < o1 ? __ldg(a.cols + ob + q) : 0u;
+                        ws[q] = ob + q < o1 ? __ldg(a.w + ob + q) : 0;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) dxs[q] = ob + q < o1 ? get(xs[q]) : INT_MAX;
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const int dx = dxs[q];
+                        if (dx == INT_MAX) continue;
+                        // the certificate of exact distances: no slot gives c a shorter
+                        // path (with every vertex's distance that of a real path through
+                        // its parent, below, the distances are the shortest); a root
+                        // that fails it is left to the host
+                        const long long via = (long long)dx + ws[q];
+                        if (via < (long long)dc) shorter = 1;
+                        if (via != (long long)dc) continue;
+                        if (dx < bestd) {
+                            bestd = dx;
+                            bestx = xs[q];
+                            bests = __ldg(a.rev + ob + q);
+                            rival = 0;
+                        } else if (dx == bestd) {
+                            if (xs[q] == bestx)
+                                bests = min(bests, __ldg(a.rev + ob + q));
+                            else
+                                rival = 1;
+                        }
                     }
                 }
                 slot = bests == 0xffffffffu ? -1 : (int32_t)bests;
@@ -265,13 +331,18 @@ __global__ void __launch_bounds__(kThreads) trees_kernel(TreeArgs a) {
     }
 }
 
-// Dynamic shared memory for n vertices: the shared form's distances, dirty bits and
-// summary bits; the global form's list of a round's dirty words.
+constexpr int kTreeDirtyMaxN = 163840;  // 20 KB of dirty bits + 4 KB of list, eight times
+
+// Dynamic shared memory for n vertices: the shared form's distances, dirty bits and a
+// round's vertices; the other forms' vertices and dirty bits or dirty words of a round.
 inline size_t trees_smem_bytes(int n) {
     const size_t words = ((size_t)n + 31) / 32;
-    return (((size_t)n * 4 + 15) & ~(size_t)15) + words * 4 + ((words + 31) / 32) * 4;
+    return (((size_t)n * 4 + 15) & ~(size_t)15) + words * 4 + 2 * kTreeSharedList;
 }
-inline size_t trees_global_smem_bytes(int n) { return 2 * ((((size_t)n + 31) / 32 + 7) & ~(size_t)7); }
+inline size_t trees_global_smem_bytes(int n) {
+    const size_t words = ((size_t)n + 31) / 32;
+    return 4 * kTreeGlobalList + (n <= kTreeDirtyMaxN ? 4 * words : 2 * ((words + 7) & ~(size_t)7));
+}
 constexpr int kTreeGlobalMaxN = 65536 * 32;  // the global form's 16-bit word list: at most 128 KB
 
 // A launch shape of trees_kernel: CTA size, CTAs per SM (global form) and the
@@ -286,33 +357,36 @@ inline int32_t shape_delta(const TreeShape &sh, int32_t mean_w) {
     return (int32_t)(d < 1 ? 1 : d > (1ll << 30) ? (1ll << 30) : d);
 }
 
+// The kernel for a CTA size of the forms with distances in global memory.
+typedef void (*TreeKernel)(TreeArgs);
+inline TreeKernel tree_kernel(int n, int threads) {
+    const bool d = n <= kTreeDirtyMaxN;
+    switch (threads) {
+    case 128: return d ? trees_kernel<kTreeDirty, 128> : trees_kernel<kTreeGlobal, 128>;
+    case 256: return d ? trees_kernel<kTreeDirty, 256> : trees_kernel<kTreeGlobal, 256>;
+    case 512: return d ? trees_kernel<kTreeDirty, 512> : trees_kernel<kTreeGlobal, 512>;
+    default: return d ? trees_kernel<kTreeDirty, 1024> : trees_kernel<kTreeGlobal, 1024>;
+    }
+}
+
 // Launches trees_kernel in `shape` over grid CTAs (the shared form: 1024 threads,
 // smem bytes of dynamic shared memory).
 inline cudaError_t launch_trees(bool shared, const TreeShape &shape, int grid, size_t smem, cudaStream_t st,
                                 const TreeArgs &a) {
-    if (shared) {
-        trees_kernel<true, kTreeThreads><<<grid, kTreeThreads, smem, st>>>(a);
-    } else {
-        const size_t lb = trees_global_smem_bytes(a.n);
-        switch (shape.threads) {
-        case 128: trees_kernel<false, 128><<<grid, 128, lb, st>>>(a); break;
-        case 256: trees_kernel<false, 256><<<grid, 256, lb, st>>>(a); break;
-        case 512: trees_kernel<false, 512><<<grid, 512, lb, st>>>(a); break;
-        default: trees_kernel<false, 1024><<<grid, 1024, lb, st>>>(a); break;
-        }
-    }
+    if (shared)
+        trees_kernel<kTreeShared, kTreeThreads><<<grid, kTreeThreads, smem, st>>>(a);
+    else
+        tree_kernel(a.n, shape.threads)<<<grid, shape.threads <= 512 ? shape.threads : 1024,
+                                          trees_global_smem_bytes(a.n), st>>>(a);
     return cudaGetLastError();
 }
 
 inline cudaError_t set_trees_smem_limit() {
-    cudaError_t e = cudaFuncSetAttribute(trees_kernel<true, kTreeThreads>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)trees_smem_bytes(kTreeSharedMaxN));
-    const int lb = (int)trees_global_smem_bytes(kTreeGlobalMaxN);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(trees_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(trees_kernel<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(trees_kernel<false, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(trees_kernel<false, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(trees_kernel<kTreeShared, kTreeThreads>, attr, (int)trees_smem_bytes(kTreeSharedMaxN));
+    for (int threads : {128, 256, 512, 1024})
+        for (int n : {kTreeDirtyMaxN, kTreeGlobalMaxN})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(tree_kernel(n, threads), attr, (int)trees_global_smem_bytes(n));
     return e;
 }
 
