@@ -11,13 +11,15 @@
 //   1. trees_kernel (mcbgpu_sssp.cuh): distances into the chunk's distance rows,
 //      parent slots into the resident parent array (F x n' int32, kept for the
 //      lists), a tie flag per root; the host replaces the tied roots' trees.
-//   2. codes_kernel: per vertex, the child of the root its tree path runs through
-//      (its branch) or "blocked" if that path holds an FVS vertex with a smaller id
-//      than the root, by pointer jumping up the parent chains (O(n' log height)).
-//   3. cand_count_kernel: per non-tree pair of slots, the reference's test (both
-//      ends unblocked, paths meeting only at the root) as a bitmap, and a count per
-//      root; cand_write_kernel: the accepted pairs in pair order with their weights
-//      d(a) + d(b) + w, one warp per root, at offsets from a scan of the counts.
+//   2. per vertex, its branch: the child of the root its tree path runs through, or
+//      "blocked" if that path holds an FVS vertex with a smaller id than the root, by
+//      pointer jumping up the parent chains (O(n' log height)); and per non-tree pair of
+//      slots the reference's test (both ends unblocked, paths meeting only at the root)
+//      as a bitmap, and a count per root: branch_test_kernel, one CTA per root with the
+//      branches in shared memory (up to kBranchMaxN vertices), else codes_kernel and
+//      cand_count_kernel over global memory; then cand_write_kernel: the accepted pairs
+//      in pair order with their weights d(a) + d(b) + w, one warp per root, at offsets
+//      from a scan of the counts.
 // After the host has ranked all candidates:
 //   4. walk_kernel (twice): per rank, the coordinates on its two root paths and of
 //      its own edge; first the lengths, then (after a scan) the lists;
@@ -51,73 +53,152 @@ constexpr int kScanThreads = 1024;
 struct GenGraph {
     const uint32_t *ro, *rows, *cols, *rev, *pair_slot, *roots;
     const int32_t *w, *ec, *fvs;
+    const uint4 *slot_info;      // per slot: row, column, pair index
+    const uint32_t *pair_ends;   // per pair: its lower slot's row and column, 16 bits each (n <= kBranchMaxN)
     int32_t n, F;
     int64_t slots, npairs;
 };
 
-// pointer-jumping state of a vertex: bits 0-31 the ancestor it points to, 32-62 the
-// last vertex below that ancestor on its path, 63 whether the path segment between
-// them holds a blocking FVS vertex
-__device__ __forceinline__ uint64_t jpack(uint32_t anc, uint32_t top, uint32_t blk) {
-    return (uint64_t)anc | ((uint64_t)(top & 0x7fffffffu) << 32) | ((uint64_t)blk << 63);
-}
-__device__ __forceinline__ uint32_t janc(uint64_t x) { return (uint32_t)x; }
-__device__ __forceinline__ uint32_t jtop(uint64_t x) { return (uint32_t)(x >> 32) & 0x7fffffffu; }
-__device__ __forceinline__ uint32_t jblk(uint64_t x) { return (uint32_t)(x >> 63); }
-
+// A vertex's pointer starts as its parent, or as itself below the root (its branch), or
+// as "blocked" where it blocks; jumping to its pointer's pointer until that points to
+// itself (or is blocked) leaves its branch.  Pointers are updated in place: a vertex
+// reads its ancestor's whole, which is at least as far along as in the synchronous
+// scheme, so each round at least halves every remaining chain.
 constexpr int32_t kCodeRoot = -1, kCodeBlocked = -2;
 
-// Branch codes of the chunk's trees, one CTA per root.  The jump state is updated in
-// place: a vertex reads its ancestor's 64-bit state (single-copy atomic), which is at
-// least as far along as the synchronous scheme's, so each round at least halves every
-// remaining chain; rounds stop when every vertex points at the root.
+// What a vertex starts with: its pointer, with kCodeRoot / kCodeBlocked; bad: its parent
+// slot is none of its own (it is left blocked, so it joins no candidate).
+__device__ __forceinline__ int32_t first_pointer(const GenGraph &g, uint32_t v, uint32_t src, int32_t o, uint32_t &pair,
+                                                 bool &bad) {
+    pair = 0xffffffffu;
+    if (v == src) return kCodeRoot;
+    if (o < 0 || (int64_t)o >= g.slots) {
+        bad = true;
+        return kCodeBlocked;
+    }
+    const uint4 si = __ldg(g.slot_info + o);
+    if (si.y != v) {
+        bad = true;
+        return kCodeBlocked;
+    }
+    pair = si.z;
+    if (g.fvs[v] >= 0 && v < src) return kCodeBlocked;
+    return (int32_t)(si.x == src ? v : si.x);
+}
+
+// Branches and candidate test of a root in one CTA: 16-bit pointers and the tree's pairs
+// (a bit each) in shared memory, so that a pair costs its packed ends, two lookups and a
+// ballot, and nothing of a root goes through global memory but its parent slots and the
+// bitmap.  Planar-chain graph of 65k points (59.6k vertices, 130k pairs): the two kernels
+// over global memory took 3.0 us per root, this MEAS_BRANCH us.
+constexpr int kBranchMaxN = 65534;
+constexpr size_t kBranchSmemMax = 220 * 1024;
+constexpr uint16_t kRoot16 = 0xfffeu, kBlocked16 = 0xffffu;
+inline size_t branch_smem_bytes(int n, int64_t npairs) {
+    return (((size_t)n * 2 + 15) & ~(size_t)15) + 4 * (size_t)((npairs + 31) / 32);
+}
+
+__global__ void __launch_bounds__(kCodeThreads) branch_test_kernel(GenGraph g, const int32_t *__restrict__ pedge, int t0,
+                                                                   int count, uint32_t *bits, int64_t words_per_root,
+                                                                   int64_t *counts, unsigned *status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_cnt[kCodeThreads / 32];
+    const int n = g.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    volatile uint16_t *J = reinterpret_cast<volatile uint16_t *>(smem);
+    uint32_t *tree = reinterpret_cast<uint32_t *>(smem + (((size_t)n * 2 + 15) & ~(size_t)15));
+    const int words = (int)words_per_root;
+    for (int r = blockIdx.x; r < count; r += gridDim.x) {
+        const int t = t0 + r;
+        const uint32_t src = g.roots[t];
+        const int32_t *pe = pedge + (size_t)t * n;
+        for (int i = tid; i < words; i += kCodeThreads) tree[i] = 0;
+        cta_sync();
+        bool bad = false;
+        for (int v0 = tid; v0 < n; v0 += 4 * kCodeThreads) {
+            int32_t o[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) o[q] = v0 + q * kCodeThreads < n ? __ldg(pe + v0 + q * kCodeThreads) : -1;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int v = v0 + q * kCodeThreads;
+                if (v >= n) break;
+                uint32_t pair;
+                const int32_t p = first_pointer(g, (uint32_t)v, src, o[q], pair, bad);
+                J[v] = p == kCodeRoot ? kRoot16 : p == kCodeBlocked ? kBlocked16 : (uint16_t)p;
+                if (pair != 0xffffffffu) atomicOr(&tree[pair >> 5], 1u << (pair & 31u));
+            }
+        }
+        if (!cta_sync_and(!bad) && tid == 0) atomicOr(status, ST_BAD_INPUT);
+        bool done = false;
+        for (int round = 0; round < kJumpRounds && !done; round++) {
+            bool open = false;
+            for (int v = tid; v < n; v += kCodeThreads) {
+                const uint16_t p = J[v];
+                if (p >= kRoot16 || p == v) continue;
+                const uint16_t y = J[p];
+                if (y == p) continue;  // a branch
+                J[v] = y;
+                open |= y < kRoot16;
+            }
+            done = cta_sync_and(!open);
+        }
+        if (!done && tid == 0) atomicOr(status, ST_BAD_INPUT);  // a parent cycle
+        int cnt = 0;
+        uint32_t *bw = bits + (size_t)r * words_per_root;
+        for (int wi = warp; wi < words; wi += kCodeThreads / 32) {
+            const int64_t k = (int64_t)wi * 32 + lane;
+            bool acc = false;
+            if (k < g.npairs && !((tree[wi] >> lane) & 1u)) {
+                const uint32_t ab = __ldg(g.pair_ends + k);
+                const uint32_t a = ab & 0xffffu, b = ab >> 16;
+                const uint16_t ca = J[a], cb = J[b];
+                acc = ca != kBlocked16 && cb != kBlocked16 && (a == src || b == src || ca != cb);
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, acc);
+            if (lane == 0) bw[wi] = m;
+            cnt += __popc(m);
+        }
+        if (lane == 0) s_cnt[warp] = cnt;
+        cta_sync();
+        if (tid == 0) {
+            long long sum = 0;
+            for (int i = 0; i < kCodeThreads / 32; i++) sum += s_cnt[i];
+            counts[r] = sum;
+        }
+        cta_sync();
+    }
+}
+
+// Branch codes of the chunk's trees, one CTA per root, in global memory: the pointers are
+// jumped in the code array itself.
 __global__ void __launch_bounds__(kCodeThreads) codes_kernel(GenGraph g, const int32_t *__restrict__ pedge, int t0,
-                                                             int count, uint64_t *jump, int32_t *code,
-                                                             unsigned *status) {
+                                                             int count, int32_t *code, unsigned *status) {
     const int n = g.n;
     for (int r = blockIdx.x; r < count; r += gridDim.x) {
         const int t = t0 + r;
         const uint32_t src = g.roots[t];
         const int32_t *pe = pedge + (size_t)t * n;
-        volatile unsigned long long *J = reinterpret_cast<volatile unsigned long long *>(jump + (size_t)r * n);
-        int bad = 0;
+        volatile int32_t *J = code + (size_t)r * n;
+        bool bad = false;
         for (int v = threadIdx.x; v < n; v += blockDim.x) {
-            if ((uint32_t)v == src) {
-                J[v] = jpack(src, 0, 0);
-                continue;
-            }
-            const int32_t o = pe[v];
-            if (o < 0 || (int64_t)o >= g.slots || g.cols[o] != (uint32_t)v) {
-                bad = 1;  // not a tree: the vertex is left blocked, so it joins no candidate
-                J[v] = jpack(src, v, 1);
-                continue;
-            }
-            J[v] = jpack(g.rows[o], v, (g.fvs[v] >= 0 && (uint32_t)v < src) ? 1u : 0u);
+            uint32_t pair;
+            J[v] = first_pointer(g, (uint32_t)v, src, pe[v], pair, bad);
         }
-        if (!cta_sync_and(bad == 0) && threadIdx.x == 0) atomicOr(status, ST_BAD_INPUT);
+        if (!cta_sync_and(!bad) && threadIdx.x == 0) atomicOr(status, ST_BAD_INPUT);
         bool done = false;
         for (int round = 0; round < kJumpRounds && !done; round++) {
-            int open = 0;
+            bool open = false;
             for (int v = threadIdx.x; v < n; v += blockDim.x) {
-                const uint64_t x = J[v];
-                const uint32_t a = janc(x);
-                if (a == src) continue;
-                if (a >= (uint32_t)n) {  // cannot happen with checked parents; kept finite
-                    J[v] = jpack(src, v, 1);
-                    continue;
-                }
-                const uint64_t y = J[a];
-                J[v] = jpack(janc(y), jtop(y), jblk(x) | jblk(y));
-                open |= janc(y) != src;
+                const int32_t p = J[v];
+                if (p < 0 || p == v) continue;
+                const int32_t y = J[p];
+                if (y == p) continue;  // a branch
+                J[v] = y;
+                open |= y >= 0;
             }
-            done = cta_sync_and(open == 0);
+            done = cta_sync_and(!open);
         }
         if (!done && threadIdx.x == 0) atomicOr(status, ST_BAD_INPUT);  // a parent cycle
-        int32_t *cd = code + (size_t)r * n;
-        for (int v = threadIdx.x; v < n; v += blockDim.x) {
-            const uint64_t x = J[v];
-            cd[v] = (uint32_t)v == src ? kCodeRoot : (jblk(x) || janc(x) != src) ? kCodeBlocked : (int32_t)jtop(x);
-        }
         cta_sync();
     }
 }
@@ -504,8 +585,10 @@ struct mcbgpu_gen {
     // trees
     int32_t *d_pedge = nullptr;  // F x n, resident
     int32_t *d_dist = nullptr;   // chunk x n
-    int32_t *d_code = nullptr;   // chunk x n
-    uint64_t *d_jump = nullptr;  // chunk x n
+    int32_t *d_code = nullptr;   // chunk x n (without branch_shared)
+    uint4 *d_slot_info = nullptr;
+    uint32_t *d_pair_ends = nullptr;
+    bool branch_shared = false;  // branch_test_kernel
     uint32_t *d_bits = nullptr;  // chunk x words_per_root
     int32_t *d_gdist = nullptr, *d_next = nullptr;
     uint32_t *d_gdirty = nullptr, *d_gsumm = nullptr;
@@ -547,7 +630,7 @@ static void gen_free(mcbgpu_gen *g) {
     }
     cudaFree(g->d_dist_slot[1]);  // slot 0's distances are d_dist
     void *ps[] = {g->d_ro,   g->d_rows,    g->d_cols,   g->d_rev,    g->d_pairs,  g->d_roots,  g->d_w,
-                  g->d_ec,   g->d_fvs,     g->d_pedge,  g->d_dist_slot[0], g->d_code, g->d_jump, g->d_bits,
+                  g->d_ec,   g->d_fvs,     g->d_pedge,  g->d_dist_slot[0], g->d_code, g->d_slot_info, g->d_pair_ends, g->d_bits,
                   g->d_gdist, g->d_next,   g->d_gdirty, g->d_gsumm, g->d_tied,   g->d_counts, g->d_coff,   g->d_cpair,
                   g->d_cweight, g->d_nlong, g->d_status};
     for (void *p : ps) cudaFree(p);
@@ -566,6 +649,8 @@ static GenGraph graph_of(const mcbgpu_gen *g) {
     a.w = g->d_w;
     a.ec = g->d_ec;
     a.fvs = g->d_fvs;
+    a.slot_info = g->d_slot_info;
+    a.pair_ends = g->d_pair_ends;
     a.n = g->n;
     a.F = g->F;
     a.slots = g->slots;
@@ -684,8 +769,12 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     GALLOC(g->d_pedge, 4 * n * (size_t)fvs_size);
     GALLOC(g->d_dist, 4 * n * C);
     g->d_dist_slot[0] = g->d_dist;
-    GALLOC(g->d_code, 4 * n * C);
-    GALLOC(g->d_jump, 8 * n * C);
+    GALLOC(g->d_slot_info, sizeof(uint4) * (size_t)slots);
+    g->branch_shared = nodes <= kBranchMaxN && branch_smem_bytes(nodes, npairs) <= kBranchSmemMax;
+    if (g->branch_shared)
+        GALLOC(g->d_pair_ends, 4 * (size_t)npairs);
+    else
+        GALLOC(g->d_code, 4 * n * C);
     GALLOC(g->d_bits, 4 * (size_t)g->words_per_root * C);
     GALLOC(g->d_tied, C);
     GALLOC(g->d_counts, 8 * C);
@@ -727,8 +816,22 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     up(g->d_fvs, fvs_array, 4 * n);
     up(g->d_pairs, pair_slot, 4 * (size_t)npairs);
     up(g->d_roots, fvs_vertices, 4 * (size_t)fvs_size);
+    {
+        std::vector<uint4> info((size_t)slots);
+        std::vector<uint32_t> ends(g->branch_shared ? (size_t)npairs : 0);
+        for (int64_t o = 0; o < slots; o++) info[(size_t)o] = make_uint4(rows[o], cols[o], 0, 0);
+        for (int64_t k = 0; k < npairs; k++) {
+            const uint32_t o = pair_slot[k];
+            info[o].z = info[rev[o]].z = (uint32_t)k;
+            if (g->branch_shared) ends[(size_t)k] = rows[o] | (cols[o] << 16);
+        }
+        up(g->d_slot_info, info.data(), sizeof(uint4) * (size_t)slots);
+        if (g->branch_shared) up(g->d_pair_ends, ends.data(), 4 * (size_t)npairs);
+    }
     if (e == cudaSuccess) e = cudaMemset(g->d_status, 0, 4);
     if (e == cudaSuccess) e = set_trees_smem_limit();
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(branch_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBranchSmemMax);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(sort_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(int32_t) * kSortLongMax));
@@ -876,12 +979,17 @@ int mcbgpu_gen_candidates(mcbgpu_gen *g, int64_t *counts, int64_t *total, void *
     const GenGraph gg = graph_of(g);
     const int count = g->cur_count;
     const int grid = count < g->sm_count * 2 ? count : g->sm_count * 2;
-    codes_kernel<<<grid, kCodeThreads, 0, st>>>(gg, g->d_pedge, g->cur_t0, count, g->d_jump, g->d_code,
-                                                g->d_status);
-    MCB_CUDA(cudaGetLastError());
-    cand_count_kernel<<<count < g->sm_count * 4 ? count : g->sm_count * 4, kCandThreads, 0, st>>>(
-        gg, g->d_pedge, g->d_code, g->cur_t0, count, g->d_bits, g->words_per_root, g->d_counts);
-    MCB_CUDA(cudaGetLastError());
+    if (g->branch_shared) {
+        branch_test_kernel<<<grid, kCodeThreads, branch_smem_bytes(g->n, g->npairs), st>>>(
+            gg, g->d_pedge, g->cur_t0, count, g->d_bits, g->words_per_root, g->d_counts, g->d_status);
+        MCB_CUDA(cudaGetLastError());
+    } else {
+        codes_kernel<<<grid, kCodeThreads, 0, st>>>(gg, g->d_pedge, g->cur_t0, count, g->d_code, g->d_status);
+        MCB_CUDA(cudaGetLastError());
+        cand_count_kernel<<<count < g->sm_count * 4 ? count : g->sm_count * 4, kCandThreads, 0, st>>>(
+            gg, g->d_pedge, g->d_code, g->cur_t0, count, g->d_bits, g->words_per_root, g->d_counts);
+        MCB_CUDA(cudaGetLastError());
+    }
     scan_small_kernel<<<1, kScanThreads, 0, st>>>(g->d_counts, count, g->d_coff);
     MCB_CUDA(cudaGetLastError());
     MCB_CUDA(cudaMemcpyAsync(counts, g->d_counts, 8 * (size_t)count, cudaMemcpyDeviceToHost, st));

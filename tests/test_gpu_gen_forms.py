@@ -1,0 +1,41 @@
+"""Candidate generation where its forms meet: trees with distances in shared memory (up
+to 53,248 vertices), with the dirty bits alone there (up to 163,840), and neither; the
+candidate test in shared memory (up to 65,534 vertices) and over global memory.  A few
+roots of each graph, against the host's heap searches and the numpy restatement of the
+candidate test."""
+import numpy as np
+import pytest
+
+from minimumcyclebasis_gb300 import GpuGen, Problem, planar_chain_graph, random_graph
+from test_two_stage_host import root_candidates
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("make,lo,hi", [(lambda: random_graph(3000, 6000, 1, 1000, 1), 1, 53248),
+                                        (lambda: planar_chain_graph(57500, seed=2), 1, 53248),
+                                        (lambda: planar_chain_graph(60000, seed=3), 53249, 65534),
+                                        (lambda: planar_chain_graph(73000, seed=4), 65535, 163840),
+                                        (lambda: planar_chain_graph(185000, seed=5), 163841, 1 << 21)])
+def test_a_few_roots(make, lo, hi):
+    p = Problem.from_graph(make()).prepare(structure_only=True)
+    assert lo <= p.n <= hi
+    rows, cols, w, rev, _ = p.reduced_graph()
+    fa, roots = p.fvs()
+    pairs = p.pairs()
+    gen = GpuGen(p, chunk=5)
+    for t0 in (0, p.F // 2, p.F - 5):
+        tied = gen.trees(t0, 5)
+        dist, ps = p.search_trees(np.arange(t0, t0 + 5))
+        idx = np.nonzero(tied)[0]
+        if len(idx):
+            gen.put_trees(t0 + idx, dist[idx], ps[idx])
+        pi, wi, counts = gen.candidates(5)
+        at = 0
+        for i in range(5):
+            k, wk = root_candidates(int(roots[t0 + i]), dist[i], ps[i].astype(np.int64), rows, cols, w.astype(np.int64),
+                                    rev, fa, pairs)
+            assert counts[i] == len(k)
+            assert np.array_equal(pi[at:at + len(k)], k) and np.array_equal(wi[at:at + len(k)], wk)
+            at += len(k)
+    gen.close()
