@@ -53,7 +53,7 @@ constexpr int kScanThreads = 1024;
 struct GenGraph {
     const uint32_t *ro, *rows, *cols, *rev, *pair_slot, *roots;
     const int32_t *w, *ec, *fvs;
-    const uint4 *slot_info;      // per slot: row, column, pair index
+    const uint4 *slot_info;      // per slot: row, column, pair index, coordinate or -1
     const uint32_t *pair_ends;   // per pair: its lower slot's row and column, 16 bits each (n <= kBranchMaxN)
     int32_t n, F;
     int64_t slots, npairs;
@@ -90,7 +90,7 @@ __device__ __forceinline__ int32_t first_pointer(const GenGraph &g, uint32_t v, 
 // (a bit each) in shared memory, so that a pair costs its packed ends, two lookups and a
 // ballot, and nothing of a root goes through global memory but its parent slots and the
 // bitmap.  Planar-chain graph of 65k points (59.6k vertices, 130k pairs): the two kernels
-// over global memory took 3.0 us per root, this MEAS_BRANCH us.
+// over global memory took 3.0 us per root, this 0.7 us.
 constexpr int kBranchMaxN = 65534;
 constexpr size_t kBranchSmemMax = 220 * 1024;
 constexpr uint16_t kRoot16 = 0xfffeu, kBlocked16 = 0xffffu;
@@ -357,7 +357,10 @@ __device__ void candidate_features(uint16_t *f, float W, float wmed, float da, f
 
 // Per rank: the coordinates of its cycle (its own edge's, then the root paths of its
 // two ends).  Without `out`, the count into len[r] (and with `feat`, the candidate's
-// features); with it, the coordinates at out[off[r] ...] in walk order.
+// features); with it, the coordinates at out[off[r] ...] in walk order.  A hop is two
+// dependent reads (parent slot, from HBM; its row and coordinate in one 16-byte entry,
+// from L2), and the two paths are walked side by side so that theirs overlap: 1.1M
+// candidates of a 65k-point planar-chain graph, 130 hops each, 5.4 -> MEAS_WALK ms per pass.
 __global__ void __launch_bounds__(kWalkThreads) walk_kernel(GenGraph g, const int32_t *__restrict__ pedge, int64_t K,
                                                             const int32_t *__restrict__ tree,
                                                             const int32_t *__restrict__ eoff, int32_t *len,
@@ -388,21 +391,34 @@ __global__ void __launch_bounds__(kWalkThreads) walk_kernel(GenGraph g, const in
             }
             c++;
         };
-        emit(g.ec[o]);
+        const uint4 own = __ldg(g.slot_info + o);
+        emit((int32_t)own.w);
         float dist[2] = {0.0f, 0.0f};
         int hops[2] = {0, 0};
-        for (int side = 0; side < 2; side++) {
-            uint32_t x = side ? g.cols[o] : g.rows[o];
-            for (int steps = 0; x != src; steps++) {
-                const int32_t q = pe[x];
-                if (steps >= n || q < 0 || (int64_t)q >= g.slots) {
-                    atomicOr(status, ST_BAD_INPUT);
-                    break;
+        uint32_t x[2] = {own.x, own.y};
+        for (int steps = 0; x[0] != src || x[1] != src; steps++) {
+            int32_t q[2];
+#pragma unroll
+            for (int side = 0; side < 2; side++) q[side] = x[side] != src ? pe[x[side]] : -1;
+            uint4 si[2];
+#pragma unroll
+            for (int side = 0; side < 2; side++) {
+                si[side] = make_uint4(src, 0, 0, 0xffffffffu);
+                if (x[side] == src) continue;
+                if (steps >= n || q[side] < 0 || (int64_t)q[side] >= g.slots)
+                    atomicOr(status, ST_BAD_INPUT);  // the path ends here
+                else
+                    si[side] = __ldg(g.slot_info + q[side]);
+            }
+#pragma unroll
+            for (int side = 0; side < 2; side++) {
+                if (x[side] == src) continue;
+                emit((int32_t)si[side].w);
+                if (feat && q[side] >= 0 && (int64_t)q[side] < g.slots) {
+                    dist[side] += (float)g.w[q[side]];
+                    hops[side]++;
                 }
-                emit(g.ec[q]);
-                dist[side] += (float)g.w[q];
-                hops[side]++;
-                x = g.rows[q];
+                x[side] = si[side].x;
             }
         }
         if (!out) len[r] = c;
@@ -600,6 +616,10 @@ struct mcbgpu_gen {
     int32_t cur_t0 = -1, cur_count = 0;
     // lists
     int64_t K = 0, K_lists = 0, nnz = 0;
+    // list buffers, kept from one ranking to the next; their sizes in bytes
+    int64_t cap_tree = 0, cap_eoff = 0, cap_len = 0, cap_weight = 0, cap_off = 0, cap_bsum = 0, cap_coords = 0,
+            cap_longs = 0;
+    bool ranked = false;
     int32_t *d_tree = nullptr, *d_eoff = nullptr, *d_len = nullptr, *d_coords = nullptr, *d_weight = nullptr;
     int64_t *d_off = nullptr, *d_bsum = nullptr, *d_longs = nullptr;
     unsigned *d_nlong = nullptr;
@@ -607,6 +627,18 @@ struct mcbgpu_gen {
     long long bytes = 0;
     long long diverged_runs = 0;
 };
+
+// Room for `need` bytes in *p (contents are lost when it grows).
+template <typename T>
+static cudaError_t keep_room(T *&p, int64_t &cap, int64_t need) {
+    if (need <= cap) return cudaSuccess;
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+    const cudaError_t e = cudaMalloc((void **)&p, (size_t)need);
+    if (e == cudaSuccess) cap = need;
+    return e;
+}
 
 static void gen_free_lists(mcbgpu_gen *g) {
     cudaFree(g->d_tree);
@@ -617,8 +649,6 @@ static void gen_free_lists(mcbgpu_gen *g) {
     cudaFree(g->d_bsum);
     cudaFree(g->d_longs);
     cudaFree(g->d_weight);
-    g->d_tree = g->d_eoff = g->d_len = g->d_coords = g->d_weight = nullptr;
-    g->d_off = g->d_bsum = g->d_longs = nullptr;
 }
 
 static void gen_free(mcbgpu_gen *g) {
@@ -819,7 +849,7 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     {
         std::vector<uint4> info((size_t)slots);
         std::vector<uint32_t> ends(g->branch_shared ? (size_t)npairs : 0);
-        for (int64_t o = 0; o < slots; o++) info[(size_t)o] = make_uint4(rows[o], cols[o], 0, 0);
+        for (int64_t o = 0; o < slots; o++) info[(size_t)o] = make_uint4(rows[o], cols[o], 0, (uint32_t)edge_coord[o]);
         for (int64_t k = 0; k < npairs; k++) {
             const uint32_t o = pair_slot[k];
             info[o].z = info[rev[o]].z = (uint32_t)k;
@@ -1038,18 +1068,19 @@ int mcbgpu_gen_rank(mcbgpu_gen *g, int64_t K, const int32_t *tree, const int32_t
         return MCBGPU_E_STATE;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    gen_free_lists(g);
+    g->ranked = false;
     g->K = K;
     g->K_lists = 0;
     g->nnz = 0;
-    const size_t k1 = (size_t)(K > 0 ? K : 1);
+    const int64_t k1 = K > 0 ? K : 1;
     const int64_t nblk = (K + (int64_t)kScanThreads * kScanItems - 1) / ((int64_t)kScanThreads * kScanItems);
-    MCB_CUDA(cudaMalloc((void **)&g->d_tree, 4 * k1));
-    MCB_CUDA(cudaMalloc((void **)&g->d_eoff, 4 * k1));
-    MCB_CUDA(cudaMalloc((void **)&g->d_len, 4 * k1));
-    MCB_CUDA(cudaMalloc((void **)&g->d_weight, 4 * k1));
-    MCB_CUDA(cudaMalloc((void **)&g->d_off, 8 * (size_t)(K + 1)));
-    MCB_CUDA(cudaMalloc((void **)&g->d_bsum, 8 * (size_t)(nblk + 1)));
+    MCB_CUDA(keep_room(g->d_tree, g->cap_tree, 4 * k1));
+    MCB_CUDA(keep_room(g->d_eoff, g->cap_eoff, 4 * k1));
+    MCB_CUDA(keep_room(g->d_len, g->cap_len, 4 * k1));
+    MCB_CUDA(keep_room(g->d_weight, g->cap_weight, 4 * k1));
+    MCB_CUDA(keep_room(g->d_off, g->cap_off, 8 * (K + 1)));
+    MCB_CUDA(keep_room(g->d_bsum, g->cap_bsum, 8 * (nblk + 1)));
+    g->ranked = true;
     if (K == 0) return MCBGPU_OK;
     MCB_CUDA(cudaMemcpyAsync(g->d_tree, tree, 4 * (size_t)K, cudaMemcpyHostToDevice, st));
     MCB_CUDA(cudaMemcpyAsync(g->d_eoff, edge_offset, 4 * (size_t)K, cudaMemcpyHostToDevice, st));
@@ -1064,7 +1095,7 @@ int mcbgpu_gen_rank(mcbgpu_gen *g, int64_t K, const int32_t *tree, const int32_t
 }
 
 int mcbgpu_gen_build_lists(mcbgpu_gen *g, int64_t K_keep, int64_t *nnz, void *stream) {
-    if (!g || !nnz || K_keep < 0 || K_keep > g->K || !g->d_len) {
+    if (!g || !nnz || K_keep < 0 || K_keep > g->K || !g->ranked) {
         set_error("mcbgpu_gen_build_lists: invalid arguments (mcbgpu_gen_rank first)");
         return MCBGPU_E_ARG;
     }
@@ -1073,10 +1104,6 @@ int mcbgpu_gen_build_lists(mcbgpu_gen *g, int64_t K_keep, int64_t *nnz, void *st
         return MCBGPU_E_STATE;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    cudaFree(g->d_coords);
-    cudaFree(g->d_longs);
-    g->d_coords = nullptr;
-    g->d_longs = nullptr;
     g->K_lists = K_keep;
     g->nnz = 0;
     if (K_keep == 0) {
@@ -1097,14 +1124,14 @@ int mcbgpu_gen_build_lists(mcbgpu_gen *g, int64_t K_keep, int64_t *nnz, void *st
     MCB_CUDA(cudaMemcpyAsync(&total, g->d_off + K, 8, cudaMemcpyDeviceToHost, st));
     int rc = check_status(g, st, "mcbgpu_gen_build_lists (offsets)");
     if (rc) return rc;
-    MCB_CUDA(cudaMalloc((void **)&g->d_coords, 4 * (size_t)(total > 0 ? total : 1)));
+    MCB_CUDA(keep_room(g->d_coords, g->cap_coords, 4 * (total > 0 ? total : 1)));
     const GenGraph gg = graph_of(g);
     const int wgrid = (int)std::min<long long>((K + kWalkThreads - 1) / kWalkThreads, (long long)g->sm_count * 16);
     walk_kernel<<<wgrid, kWalkThreads, 0, st>>>(gg, g->d_pedge, K, g->d_tree, g->d_eoff, g->d_len, g->d_off,
                                                 g->d_coords, g->d_status, nullptr, nullptr, 1.0f);
     MCB_CUDA(cudaGetLastError());
     const unsigned long long cap_long = (unsigned long long)(K < 65536 ? K : 65536);
-    MCB_CUDA(cudaMalloc((void **)&g->d_longs, 8 * (size_t)cap_long));
+    MCB_CUDA(keep_room(g->d_longs, g->cap_longs, 8 * (int64_t)cap_long));
     MCB_CUDA(cudaMemsetAsync(g->d_nlong, 0, 4, st));
     const int sgrid = (int)std::min<long long>((K + kSortWarps - 1) / kSortWarps, (long long)g->sm_count * 8);
     sort_lists_kernel<<<sgrid, kSortWarps * 32, 0, st>>>(K, g->d_off, g->d_coords, g->d_longs, g->d_nlong, cap_long);
