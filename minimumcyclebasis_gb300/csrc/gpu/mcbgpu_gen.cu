@@ -360,7 +360,7 @@ __device__ void candidate_features(uint16_t *f, float W, float wmed, float da, f
 // features); with it, the coordinates at out[off[r] ...] in walk order.  A hop is two
 // dependent reads (parent slot, from HBM; its row and coordinate in one 16-byte entry,
 // from L2), and the two paths are walked side by side so that theirs overlap: 1.1M
-// candidates of a 65k-point planar-chain graph, 130 hops each, 5.4 -> MEAS_WALK ms per pass.
+// candidates of a 65k-point planar-chain graph, 130 hops each, 5.4 -> 4.8 ms per pass.
 __global__ void __launch_bounds__(kWalkThreads) walk_kernel(GenGraph g, const int32_t *__restrict__ pedge, int64_t K,
                                                             const int32_t *__restrict__ tree,
                                                             const int32_t *__restrict__ eoff, int32_t *len,
@@ -597,6 +597,7 @@ struct mcbgpu_gen {
     // graph
     uint32_t *d_ro = nullptr, *d_rows = nullptr, *d_cols = nullptr, *d_rev = nullptr, *d_pairs = nullptr,
              *d_roots = nullptr;
+    uint2 *d_arcs = nullptr;
     int32_t *d_w = nullptr, *d_ec = nullptr, *d_fvs = nullptr;
     // trees
     int32_t *d_pedge = nullptr;  // F x n, resident
@@ -659,7 +660,7 @@ static void gen_free(mcbgpu_gen *g) {
         cudaFree(g->d_tied_slot[k]);
     }
     cudaFree(g->d_dist_slot[1]);  // slot 0's distances are d_dist
-    void *ps[] = {g->d_ro,   g->d_rows,    g->d_cols,   g->d_rev,    g->d_pairs,  g->d_roots,  g->d_w,
+    void *ps[] = {g->d_arcs, g->d_ro,   g->d_rows,    g->d_cols,   g->d_rev,    g->d_pairs,  g->d_roots,  g->d_w,
                   g->d_ec,   g->d_fvs,     g->d_pedge,  g->d_dist_slot[0], g->d_code, g->d_slot_info, g->d_pair_ends, g->d_bits,
                   g->d_gdist, g->d_next,   g->d_gdirty, g->d_gsumm, g->d_tied,   g->d_counts, g->d_coff,   g->d_cpair,
                   g->d_cweight, g->d_nlong, g->d_status};
@@ -792,6 +793,7 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     GALLOC(g->d_cols, 4 * (size_t)slots);
     GALLOC(g->d_rev, 4 * (size_t)slots);
     GALLOC(g->d_w, 4 * (size_t)slots);
+    GALLOC(g->d_arcs, sizeof(uint2) * kArcSlots * n);
     GALLOC(g->d_ec, 4 * (size_t)slots);
     GALLOC(g->d_fvs, 4 * n);
     GALLOC(g->d_pairs, 4 * (size_t)npairs);
@@ -822,7 +824,7 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     if (g->shared_form)
         g->shapes = {{kTreeThreads, 1, 8}, {kTreeThreads, 1, 4}, {kTreeThreads, 1, 16}, {kTreeThreads, 1, 2}};
     else
-        g->shapes = {{256, 8, 4}, {256, 8, 8}, {256, 8, 2}, {256, 8, 16}, {512, 4, 8}, {128, 16, 8}};
+        g->shapes = {{256, 8, 8}, {256, 8, 4}, {256, 8, 12}, {256, 8, 16}, {512, 4, 8}, {128, 16, 8}};
     const int nchunks = (fvs_size + g->chunk - 1) / g->chunk;
     if (nchunks < 2 * (int)g->shapes.size()) g->chosen = 0;
     for (int k = 0; k < 2; k++) {
@@ -842,6 +844,10 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     up(g->d_cols, cols, 4 * (size_t)slots);
     up(g->d_rev, rev, 4 * (size_t)slots);
     up(g->d_w, weights, 4 * (size_t)slots);
+    {
+        const std::vector<uint2> arcs = arc_table(nodes, row_offsets, cols, weights);
+        up(g->d_arcs, arcs.data(), sizeof(uint2) * arcs.size());
+    }
     up(g->d_ec, edge_coord, 4 * (size_t)slots);
     up(g->d_fvs, fvs_array, 4 * n);
     up(g->d_pairs, pair_slot, 4 * (size_t)npairs);
@@ -906,6 +912,7 @@ int mcbgpu_gen_trees_submit(mcbgpu_gen *g, int32_t t0, int32_t count, void *stre
     a.cols = g->d_cols;
     a.w = g->d_w;
     a.rev = g->d_rev;
+    a.arcs = g->d_arcs;
     a.n = g->n;
     a.delta = shape_delta(shape, g->delta);
     a.roots = g->d_roots + t0;

@@ -19,8 +19,8 @@
 //      if it has not converged.  A round first lists the vertices to relax, then gives
 //      each kTreeLanes lanes, one arc at a time each: one thread per dirty word with its
 //      vertices and arcs one after the other left a few threads with all of a frontier
-//      of neighbours (planar-chain graph of 65k points: 14.8 us per root, 5.2 now; random
-//      graph of 20k vertices 3.2, 1.0 now; 2 or 8 lanes are within 8%).  Distances and dirty bits live in shared
+//      of neighbours (planar-chain graph of 65k points: 14.8 us per root, 5.2 with lists; random
+//      graph of 20k vertices 3.2, 1.0 with them; 2 or 8 lanes are within 8%).  Distances and dirty bits live in shared
 //      memory up to kTreeSharedMaxN vertices, in a per-CTA global slice beyond.  delta (the
 //      bucket width) trades rounds (each a pass over the dirty bits and a barrier)
 //      against relaxations repeated inside a bucket; the callers time a few widths
@@ -59,11 +59,30 @@ constexpr int kTreeSharedList = 4096;   // vertices listed per round: shared for
 constexpr int kTreeGlobalList = 1024;   // and global form
 constexpr int kTreeMaxCtasPerSm = 16;   // the global form's per-CTA slices are sized for this many
 
+// A vertex's first kArcSlots arcs at a fixed place, (column, weight) together: relaxing
+// is a chain of L2 reads (the vertex's distance and arcs, then its neighbours'), one
+// shorter than with the row's offsets read first (planar-chain graph of 65k points: 4.8
+// us per root with those, 3.8 with the table).  Unused entries have column
+// kNoArc; the last entry's top bit says that the vertex has more arcs (in cols / w).
+constexpr int kArcSlots = 8;
+constexpr uint32_t kNoArc = 0x7fffffffu, kMoreArcs = 0x80000000u;
+
+inline std::vector<uint2> arc_table(int32_t n, const uint32_t *ro, const uint32_t *cols, const int32_t *w) {
+    std::vector<uint2> t((size_t)n * kArcSlots, make_uint2(kNoArc, 0u));
+    for (int32_t v = 0; v < n; v++) {
+        for (uint32_t o = ro[v]; o < ro[v + 1] && o < ro[v] + kArcSlots; o++)
+            t[(size_t)v * kArcSlots + (o - ro[v])] = make_uint2(cols[o], (uint32_t)w[o]);
+        if (ro[v + 1] - ro[v] > (uint32_t)kArcSlots) t[(size_t)v * kArcSlots + kArcSlots - 1].x |= kMoreArcs;
+    }
+    return t;
+}
+
 struct TreeArgs {
     const uint32_t *ro;
     const uint32_t *cols;
     const int32_t *w;
     const uint32_t *rev;
+    const uint2 *arcs;   // n x kArcSlots: the first arcs of every vertex (arc_table)
     int32_t n;
     int32_t delta;
     const uint32_t *roots;
@@ -78,14 +97,88 @@ struct TreeArgs {
     unsigned *status;
 };
 
+// Relaxes the arcs of v (distance dv) that fall to lane `sub` of kTreeLanes: lower(x, nd)
+// is called for each, two of the fixed places at once.
+template <typename Lower>
+__device__ __forceinline__ void relax_arcs(const TreeArgs &a, uint32_t v, int dv, int sub, const Lower &lower) {
+    static_assert(kArcSlots == 2 * kTreeLanes, "two entries per lane");
+    const uint2 e0 = __ldg(a.arcs + (size_t)v * kArcSlots + sub), e1 = __ldg(a.arcs + (size_t)v * kArcSlots + kTreeLanes + sub);
+    const uint32_t x1 = e1.x & ~kMoreArcs;
+    lower(e0.x, dv + (int)e0.y, x1, dv + (int)e1.y);
+    const unsigned group = ((1u << kTreeLanes) - 1) << (threadIdx.x & 31 & ~(kTreeLanes - 1));
+    if (__shfl_sync(group, e1.x, kTreeLanes - 1, kTreeLanes) & kMoreArcs) {
+        const uint32_t o1 = __ldg(a.ro + v + 1);
+        for (uint32_t o = __ldg(a.ro + v) + kArcSlots + sub; o < o1; o += kTreeLanes)
+            lower(__ldg(a.cols + o), dv + __ldg(a.w + o), kNoArc, 0);
+    }
+}
+
+// 2. parents by the rule into the root's rows, with its distances; returns whether this
+// thread saw a tie or an inexact distance (or the distances have not converged).
+template <typename Get>
+__device__ __forceinline__ int tree_parents(const TreeArgs &a, int r, uint32_t src, const Get &get, bool converged) {
+    const int n = a.n, tid = threadIdx.x, nt = blockDim.x;
+    int tie = converged ? 0 : 1;
+    for (int c = tid; c < n; c += nt) {
+        const int dc = get((uint32_t)c);
+        int32_t slot = -1;
+        if ((uint32_t)c != src && dc != INT_MAX) {
+            int bestd = INT_MAX, rival = 0;  // rival: another neighbour as near as the best
+            int shorter = 0;                 // some slot offers c a shorter path
+            uint32_t bestx = 0xffffffffu, bests = 0xffffffffu;
+            const uint32_t o1 = __ldg(a.ro + c + 1);
+            for (uint32_t ob = __ldg(a.ro + c); ob < o1; ob += 4) {  // four arcs in flight
+                uint32_t xs[4];
+                int dxs[4], ws[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    xs[q] = ob + q < o1 ? __ldg(a.cols + ob + q) : 0u;
+                    ws[q] = ob + q < o1 ? __ldg(a.w + ob + q) : 0;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) dxs[q] = ob + q < o1 ? get(xs[q]) : INT_MAX;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int dx = dxs[q];
+                    if (dx == INT_MAX) continue;
+                    // the certificate of exact distances: no slot gives c a shorter
+                    // path (with every vertex's distance that of a real path through
+                    // its parent, below, the distances are the shortest); a root
+                    // that fails it is left to the host
+                    const long long via = (long long)dx + ws[q];
+                    if (via < (long long)dc) shorter = 1;
+                    if (via != (long long)dc) continue;
+                    if (dx < bestd) {
+                        bestd = dx;
+                        bestx = xs[q];
+                        bests = __ldg(a.rev + ob + q);
+                        rival = 0;
+                    } else if (dx == bestd) {
+                        if (xs[q] == bestx)
+                            bests = min(bests, __ldg(a.rev + ob + q));
+                        else
+                            rival = 1;
+                    }
+                }
+            }
+            slot = bests == 0xffffffffu ? -1 : (int32_t)bests;
+            if (rival || shorter || slot < 0) tie = 1;  // (no shortest-path neighbour cannot happen; left to the host)
+        } else if ((uint32_t)c != src) {
+            tie = 1;  // unreachable vertex (the graph is not connected): left to the host
+        }
+        a.dist_out[(size_t)r * n + c] = dc;
+        a.pedge_out[(size_t)r * n + c] = slot;
+    }
+    return tie;
+}
+
 // Threads per CTA: the shared-memory form runs one 1024-thread CTA per SM (its
 // distances fill the shared memory); the other forms run kThreads-thread CTAs, several
-// per SM, so that the bucket rounds of different roots overlap.  Their distances are
-// in the CTA's global slice; the dirty bits in shared memory while eight CTAs' fit an SM
-// (kTreeDirty, up to kTreeDirtyMaxN vertices), else beside the distances with a summary.
-// They wait on L2 half of their time, so a full SM of threads (32 registers, a few spills)
-// is worth more than registers: 5.2 us per root against 5.8 with 1536 threads.
-enum TreeForm { kTreeShared, kTreeDirty, kTreeGlobal };
+// per SM, so that the bucket rounds of different roots overlap: their distances are in
+// the CTA's global slice (trees_near_kernel up to kTreeNearMaxN vertices, else the dirty
+// bits too, with a summary).  They wait on L2 half of their time, so a full SM of threads
+// (32 registers, a few spills) is worth more than registers.
+enum TreeForm { kTreeShared, kTreeGlobal };
 template <int kForm, int kThreads>
 __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kThreads) trees_kernel(TreeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -106,11 +199,6 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
         dirty = reinterpret_cast<uint32_t *>(smem + (((size_t)n * 4 + 15) & ~(size_t)15));
         summ = nullptr;
         s_verts = reinterpret_cast<VertT *>(dirty + words);
-    } else if (!kSummary) {
-        dist = a.gdist + (size_t)blockIdx.x * n;
-        dirty = reinterpret_cast<uint32_t *>(smem + 4 * kTreeGlobalList);
-        summ = nullptr;
-        s_verts = reinterpret_cast<VertT *>(smem);
     } else {
         dist = a.gdist + (size_t)blockIdx.x * n;
         dirty = a.gdirty + (size_t)blockIdx.x * words;
@@ -247,101 +335,175 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
             cta_sync();
             // the listed vertices' arcs, kTreeLanes at a time
             const int listed = min(*(volatile int *)nv, kListCap);
-            for (int i = tid / kTreeLanes; i < listed; i += nt / kTreeLanes) {
-                const int v = s_verts[i];
-                const uint32_t o1 = __ldg(a.ro + v + 1);
-                const int dv = get((uint32_t)v);
-                for (uint32_t o = __ldg(a.ro + v) + tid % kTreeLanes; o < o1; o += kTreeLanes) {
-                    const uint32_t x = __ldg(a.cols + o);
-                    const int nd = dv + __ldg(a.w + o);
-                    if (nd < get(x)) {
-                        const int old = atomicMin(&dist[x], nd);
-                        if (nd < old) {
-                            __threadfence_block();  // the new distance before the dirty bit
-                            atomicOr(&dirty[x >> 5], 1u << (x & 31));
-                            if (kSummary) {
-                                __threadfence_block();  // the dirty bit before the summary bit
-                                atomicOr(&summ[x >> 10], 1u << ((x >> 5) & 31));
-                            }
-                            mynext = nd < mynext ? nd : mynext;
-                        }
+            auto improve = [&](uint32_t x, int nd) {
+                const int old = atomicMin(&dist[x], nd);
+                if (nd < old) {
+                    __threadfence_block();  // the new distance before the dirty bit
+                    atomicOr(&dirty[x >> 5], 1u << (x & 31));
+                    if (kSummary) {
+                        __threadfence_block();  // the dirty bit before the summary bit
+                        atomicOr(&summ[x >> 10], 1u << ((x >> 5) & 31));
                     }
+                    mynext = nd < mynext ? nd : mynext;
                 }
+            };
+            for (int i = tid / kTreeLanes; i < listed; i += nt / kTreeLanes) {
+                const uint32_t v = s_verts[i];
+                relax_arcs(a, v, get(v), tid % kTreeLanes, [&](uint32_t x0, int n0, uint32_t x1, int n1) {
+                    const int d0 = x0 != kNoArc ? get(x0) : INT_MIN, d1 = x1 != kNoArc ? get(x1) : INT_MIN;
+                    if (n0 < d0) improve(x0, n0);
+                    if (n1 < d1) improve(x1, n1);
+                });
             }
             mynext = __reduce_min_sync(0xffffffffu, mynext);
             if (lane == 0 && mynext != INT_MAX) atomicMin(&s_next[slot], mynext);
             cta_sync();
             lo = s_next[slot];
         }
-        // 2. parents by the rule, and the root's tie flag
-        int tie = converged ? 0 : 1;
-        for (int c = tid; c < n; c += nt) {
-            const int dc = get((uint32_t)c);
-            int32_t slot = -1;
-            if ((uint32_t)c != src && dc != INT_MAX) {
-                int bestd = INT_MAX, rival = 0;  // rival: another neighbour as near as the best
-                int shorter = 0;                 // some slot offers c a shorter path
-                uint32_t bestx = 0xffffffffu, bests = 0xffffffffu;
-                const uint32_t o1 = __ldg(a.ro + c + 1);
-                for (uint32_t ob = __ldg(a.ro + c); ob < o1; ob += 4) {  // four arcs in flight
-                    uint32_t xs[4];
-                    int dxs[4], ws[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        xs[q] = ob + q < o1 ? __ldg(a.cols + ob + q) : 0u;
-                        ws[q] = ob + q < o1 ? __ldg(a.w + ob + q) : 0;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; q++) dxs[q] = ob + q < o1 ? get(xs[q]) : INT_MAX;
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int dx = dxs[q];
-                        if (dx == INT_MAX) continue;
-                        // the certificate of exact distances: no slot gives c a shorter
-                        // path (with every vertex's distance that of a real path through
-                        // its parent, below, the distances are the shortest); a root
-                        // that fails it is left to the host
-                        const long long via = (long long)dx + ws[q];
-                        if (via < (long long)dc) shorter = 1;
-                        if (via != (long long)dc) continue;
-                        if (dx < bestd) {
-                            bestd = dx;
-                            bestx = xs[q];
-                            bests = __ldg(a.rev + ob + q);
-                            rival = 0;
-                        } else if (dx == bestd) {
-                            if (xs[q] == bestx)
-                                bests = min(bests, __ldg(a.rev + ob + q));
-                            else
-                                rival = 1;
-                        }
-                    }
-                }
-                slot = bests == 0xffffffffu ? -1 : (int32_t)bests;
-                if (rival || shorter || slot < 0) tie = 1;  // (no shortest-path neighbour cannot happen; left to the host)
-            } else if ((uint32_t)c != src) {
-                tie = 1;  // unreachable vertex (the graph is not connected): left to the host
-            }
-            a.dist_out[(size_t)r * n + c] = dc;
-            a.pedge_out[(size_t)r * n + c] = slot;
-        }
+        int tie = tree_parents(a, r, src, get, converged);
         tie = cta_sync_and(tie == 0) ? 0 : 1;
         if (tid == 0) a.tied_out[r] = tie ? 1 : 0;
         if (!converged && tid == 0) atomicOr(a.status, ST_DIVERGED);
     }
 }
 
-constexpr int kTreeDirtyMaxN = 163840;  // 20 KB of dirty bits + 4 KB of list, eight times
+// The form for distances in global memory with everything else in shared memory: two
+// bitmaps instead of one.  `near` holds the vertices to relax now (nearer than hi), `far`
+// the improved ones beyond hi.  A round relaxes all of near, and only when that is empty
+// does hi move on and far get looked at: a bucket's several rounds no longer read the
+// distances of every vertex that waits for a later one.  Planar-chain graph of 65k points:
+// 650 rounds of 125 vertices per root, 4.8 us per root (5.2 with one bitmap; 3.8 with
+// arc_table).  Bound by the chain of L2 reads of each relaxation at eight CTAs per SM
+// (512 or 128 threads per CTA: 4.6 and 5.4).
+constexpr int kTreeNearMaxN = 98304;  // 24 KB of bitmaps + 4 KB of list, eight times per SM
+
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 2048 / kThreads) trees_near_kernel(TreeArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_root, s_lo, s_nv[3];
+    const int n = a.n, words = (n + 31) >> 5;
+    uint32_t *s_verts = reinterpret_cast<uint32_t *>(smem);
+    uint32_t *near = s_verts + kTreeGlobalList, *far = near + words;
+    int32_t *dist = a.gdist + (size_t)blockIdx.x * n;
+    const int tid = threadIdx.x, lane = tid & 31;
+    auto get = [&](uint32_t v) -> int { return __ldcg(dist + v); };
+    for (;;) {
+        if (tid == 0) s_root = atomicAdd(a.next_root, 1);
+        cta_sync();
+        const int r = s_root;
+        cta_sync();  // every thread has read s_root before thread 0 writes it again
+        if (r >= a.count) return;
+        const uint32_t src = a.roots[r];  // < n, checked by the host
+        for (int v = tid; v < n; v += kThreads) dist[v] = (uint32_t)v == src ? 0 : INT_MAX;
+        for (int k = tid; k < 2 * words; k += kThreads) near[k] = 0;
+        cta_sync();
+        if (tid == 0) {
+            near[src >> 5] = 1u << (src & 31);
+            s_nv[0] = 0;
+        }
+        cta_sync();
+        bool converged = false;
+        int hi = a.delta, beyond = INT_MAX;  // beyond: this thread's smallest distance put or left in far
+        for (int it = 0; it <= 4 * n + 16; it++) {
+            int *nv = &s_nv[it % 3];
+            if (tid == 0) s_nv[(it + 1) % 3] = 0;  // read last two barriers ago
+            // the near vertices leave the bitmap for the list (those that find it full stay)
+            for (int k = tid; k < words; k += kThreads) {
+                uint32_t bits = near[k];
+                if (!bits) continue;
+                int at = atomicAdd(nv, __popc(bits));
+                while (bits && at < kTreeGlobalList) {
+                    const int b = __ffs(bits) - 1;
+                    bits &= bits - 1;
+                    s_verts[at++] = (uint32_t)((k << 5) + b);
+                }
+                near[k] = bits;
+            }
+            cta_sync();
+            const int listed = min(*(volatile int *)nv, kTreeGlobalList);
+            if (listed > 0) {
+                // their arcs, kTreeLanes at a time; bits were cleared before the barrier and
+                // distances are read after it, so a distance lowered since sets its bit again
+                auto improved = [&](uint32_t x, int nd) {
+                    __threadfence_block();  // the new distance before the bit
+                    atomicOr((nd < hi ? near : far) + (x >> 5), 1u << (x & 31));
+                    if (nd >= hi) beyond = min(beyond, nd);
+                };
+                for (int i = tid / kTreeLanes; i < listed; i += kThreads / kTreeLanes) {
+                    const uint32_t v = s_verts[i];
+                    relax_arcs(a, v, get(v), tid % kTreeLanes, [&](uint32_t x0, int n0, uint32_t x1, int n1) {
+                        const int d0 = x0 != kNoArc ? get(x0) : INT_MIN, d1 = x1 != kNoArc ? get(x1) : INT_MIN;
+                        const bool t0 = n0 < d0, t1 = n1 < d1;
+                        const int o0 = t0 ? atomicMin(&dist[x0], n0) : INT_MIN, o1 = t1 ? atomicMin(&dist[x1], n1) : INT_MIN;
+                        if (n0 < o0) improved(x0, n0);
+                        if (n1 < o1) improved(x1, n1);
+                    });
+                }
+                cta_sync();
+                continue;
+            }
+            // near is empty: the next bucket starts at far's smallest distance (or below it,
+            // where that vertex has been improved into near since: an empty bucket)
+            if (tid == 0) s_lo = INT_MAX;
+            cta_sync();
+            beyond = __reduce_min_sync(0xffffffffu, beyond);
+            if (lane == 0 && beyond != INT_MAX) atomicMin(&s_lo, beyond);
+            cta_sync();
+            const int lo = s_lo;
+            if (lo == INT_MAX) {
+                converged = true;
+                break;
+            }
+            hi = lo > INT_MAX - a.delta ? INT_MAX : lo + a.delta;
+            beyond = INT_MAX;
+            auto sort_out = [&](uint32_t v, int d) {  // out of far: into near, or back
+                if (d < hi)
+                    atomicOr(near + (v >> 5), 1u << (v & 31));
+                else {
+                    atomicOr(far + (v >> 5), 1u << (v & 31));
+                    beyond = min(beyond, d);
+                }
+            };
+            it++;
+            nv = &s_nv[it % 3];
+            if (tid == 0) s_nv[(it + 1) % 3] = 0;
+            for (int k = tid; k < words; k += kThreads) {
+                uint32_t bits = far[k];
+                if (!bits) continue;
+                far[k] = 0;
+                int at = atomicAdd(nv, __popc(bits));
+                for (; bits; bits &= bits - 1, at++) {
+                    const uint32_t v = (uint32_t)((k << 5) + __ffs(bits) - 1);
+                    if (at < kTreeGlobalList)
+                        s_verts[at] = v;
+                    else
+                        sort_out(v, get(v));  // its word is this thread's
+                }
+            }
+            cta_sync();
+            const int nfar = min(*(volatile int *)nv, kTreeGlobalList);
+            for (int i = tid; i < nfar; i += kThreads) {
+                const uint32_t v = s_verts[i];
+                sort_out(v, get(v));
+            }
+            cta_sync();
+        }
+        int tie = tree_parents(a, r, src, get, converged);
+        tie = cta_sync_and(tie == 0) ? 0 : 1;
+        if (tid == 0) a.tied_out[r] = tie ? 1 : 0;
+        if (!converged && tid == 0) atomicOr(a.status, ST_DIVERGED);
+    }
+}
 
 // Dynamic shared memory for n vertices: the shared form's distances, dirty bits and a
-// round's vertices; the other forms' vertices and dirty bits or dirty words of a round.
+// round's vertices; the other forms' vertices and bitmaps or dirty words of a round.
 inline size_t trees_smem_bytes(int n) {
     const size_t words = ((size_t)n + 31) / 32;
     return (((size_t)n * 4 + 15) & ~(size_t)15) + words * 4 + 2 * kTreeSharedList;
 }
 inline size_t trees_global_smem_bytes(int n) {
     const size_t words = ((size_t)n + 31) / 32;
-    return 4 * kTreeGlobalList + (n <= kTreeDirtyMaxN ? 4 * words : 2 * ((words + 7) & ~(size_t)7));
+    return 4 * kTreeGlobalList + (n <= kTreeNearMaxN ? 8 * words : 2 * ((words + 7) & ~(size_t)7));
 }
 constexpr int kTreeGlobalMaxN = 65536 * 32;  // the global form's 16-bit word list: at most 128 KB
 
@@ -360,12 +522,12 @@ inline int32_t shape_delta(const TreeShape &sh, int32_t mean_w) {
 // The kernel for a CTA size of the forms with distances in global memory.
 typedef void (*TreeKernel)(TreeArgs);
 inline TreeKernel tree_kernel(int n, int threads) {
-    const bool d = n <= kTreeDirtyMaxN;
+    const bool d = n <= kTreeNearMaxN;
     switch (threads) {
-    case 128: return d ? trees_kernel<kTreeDirty, 128> : trees_kernel<kTreeGlobal, 128>;
-    case 256: return d ? trees_kernel<kTreeDirty, 256> : trees_kernel<kTreeGlobal, 256>;
-    case 512: return d ? trees_kernel<kTreeDirty, 512> : trees_kernel<kTreeGlobal, 512>;
-    default: return d ? trees_kernel<kTreeDirty, 1024> : trees_kernel<kTreeGlobal, 1024>;
+    case 128: return d ? trees_near_kernel<128> : trees_kernel<kTreeGlobal, 128>;
+    case 256: return d ? trees_near_kernel<256> : trees_kernel<kTreeGlobal, 256>;
+    case 512: return d ? trees_near_kernel<512> : trees_kernel<kTreeGlobal, 512>;
+    default: return d ? trees_near_kernel<1024> : trees_kernel<kTreeGlobal, 1024>;
     }
 }
 
@@ -385,7 +547,7 @@ inline cudaError_t set_trees_smem_limit() {
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(trees_kernel<kTreeShared, kTreeThreads>, attr, (int)trees_smem_bytes(kTreeSharedMaxN));
     for (int threads : {128, 256, 512, 1024})
-        for (int n : {kTreeDirtyMaxN, kTreeGlobalMaxN})
+        for (int n : {kTreeNearMaxN, kTreeGlobalMaxN})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(tree_kernel(n, threads), attr, (int)trees_global_smem_bytes(n));
     return e;
 }

@@ -19,6 +19,7 @@ struct mcbgpu_trees {
     bool shared_form = true;
     size_t smem = 0;
     uint32_t *d_ro = nullptr, *d_cols = nullptr, *d_rev = nullptr, *d_roots = nullptr;
+    uint2 *d_arcs = nullptr;
     int32_t *d_w = nullptr, *d_dist = nullptr, *d_pedge = nullptr, *d_gdist = nullptr, *d_next = nullptr;
     uint32_t *d_gdirty = nullptr, *d_gsumm = nullptr;
     uint8_t *d_tied = nullptr;
@@ -31,6 +32,7 @@ static void trees_free(mcbgpu_trees *t) {
     cudaFree(t->d_ro);
     cudaFree(t->d_cols);
     cudaFree(t->d_rev);
+    cudaFree(t->d_arcs);
     cudaFree(t->d_roots);
     cudaFree(t->d_w);
     cudaFree(t->d_dist);
@@ -106,6 +108,7 @@ int mcbgpu_trees_create(mcbgpu_trees **out, int32_t nodes, int64_t slots, const 
     TALLOC(t->d_cols, 4 * (size_t)slots);
     TALLOC(t->d_rev, 4 * (size_t)slots);
     TALLOC(t->d_w, 4 * (size_t)slots);
+    TALLOC(t->d_arcs, sizeof(uint2) * kArcSlots * (size_t)nodes);
     TALLOC(t->d_roots, 4 * (size_t)max_roots);
     TALLOC(t->d_dist, 4 * per_root * (size_t)max_roots);
     TALLOC(t->d_pedge, 4 * per_root * (size_t)max_roots);
@@ -123,6 +126,10 @@ int mcbgpu_trees_create(mcbgpu_trees **out, int32_t nodes, int64_t slots, const 
         e = cudaMemcpy(t->d_cols, cols, 4 * (size_t)slots, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(t->d_rev, rev, 4 * (size_t)slots, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(t->d_w, weights, 4 * (size_t)slots, cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess) {
+        const std::vector<uint2> arcs = arc_table(nodes, row_offsets, cols, weights);
+        e = cudaMemcpy(t->d_arcs, arcs.data(), sizeof(uint2) * arcs.size(), cudaMemcpyHostToDevice);
     }
     // the kernel's attribute is process-wide: set to the largest shared form, so that
     // handles of different sizes can be used in any order
@@ -157,8 +164,9 @@ int mcbgpu_trees_run(mcbgpu_trees *t, const uint32_t *roots, int32_t count, int3
     a.cols = t->d_cols;
     a.w = t->d_w;
     a.rev = t->d_rev;
+    a.arcs = t->d_arcs;
     a.n = t->n;
-    const TreeShape shape = t->shared_form ? TreeShape{kTreeThreads, 1, 4} : TreeShape{256, 8, 16};
+    const TreeShape shape = t->shared_form ? TreeShape{kTreeThreads, 1, 4} : TreeShape{256, 8, 8};
     a.delta = shape_delta(shape, t->delta);
     a.roots = t->d_roots;
     a.count = count;

@@ -1,5 +1,6 @@
 """Candidate generation where its forms meet: trees with distances in shared memory (up
-to 53,248 vertices), with the dirty bits alone there (up to 163,840), and neither; the
+to 53,248 vertices), with the near and far vertices alone there (up to 98,304), and
+neither, with rows of more and of fewer arcs than the arc table's eight; the
 candidate test in shared memory (up to 65,534 vertices) and over global memory.  A few
 roots of each graph, against the host's heap searches and the numpy restatement of the
 candidate test."""
@@ -15,8 +16,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("make,lo,hi", [(lambda: random_graph(3000, 6000, 1, 1000, 1), 1, 53248),
                                         (lambda: planar_chain_graph(57500, seed=2), 1, 53248),
                                         (lambda: planar_chain_graph(60000, seed=3), 53249, 65534),
-                                        (lambda: planar_chain_graph(73000, seed=4), 65535, 163840),
-                                        (lambda: planar_chain_graph(185000, seed=5), 163841, 1 << 21)])
+                                        (lambda: planar_chain_graph(73000, seed=4), 65535, 98304),
+                                        (lambda: random_graph(125000, 250000, 1, 1000, 5), 98305, 1 << 21)])
 def test_a_few_roots(make, lo, hi):
     p = Problem.from_graph(make()).prepare(structure_only=True)
     assert lo <= p.n <= hi
