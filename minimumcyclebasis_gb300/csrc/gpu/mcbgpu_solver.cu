@@ -79,11 +79,17 @@ constexpr int kMaxWin = 32;  // the largest window (tiles per CTA and step) a sh
 // got, so a solver can time several on its own graph (mcbgpu_solver_tune).
 struct PivotShape {
     int win_early, rank_early;  // tiles per CTA and step while fewer than rank_early pivots are known
+                                // (half of it where that does not reach the expected last pivot)
     int win_mid;                // ... from rank_early on
     int rank_tail, win_tail;    // ... once rank_tail pivots are known
-    int stream_pct;             // the streaming pass reaches this percent past the last block's last pivot
+    int stream_pct;             // the streaming pass reaches this percent past the mean of the last two blocks' last pivots
 };
-constexpr PivotShape kDefaultShape = {2, 48, 8, 60, 16, 25};
+// The pass's reach: a random graph of 50k vertices (last pivots of neighbouring blocks
+// between 2M and 12M candidates deep) takes 225 ms per solve reaching 25% past the deeper
+// of the last two blocks, 214 with their mean, 211 with 0% past it (each tile not
+// streamed and not needed saves its gathers; a needed one is computed by the search),
+// 214 with 0% past the shallower; grid, RGG and planar-chain graphs do not move.
+constexpr PivotShape kDefaultShape = {2, 48, 8, 60, 16, 0};
 constexpr int kUpdRows = MCB_UPD_ROWS;    // rows per warp group in the block update (<= 32)
 constexpr unsigned long long kNone = 0xFFFFFFFFFFFFFFFFull;
 
@@ -589,11 +595,11 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
         }
         return;
     }
-    // stream stream_pct percent past the last two blocks' deepest pivot and a tile per
-    // CTA of the pivot kernel, which computes any further tile it needs
+    // stream stream_pct percent past the mean of the last two blocks' last pivots and a tile
+    // per CTA of the pivot kernel, which computes any further tile it needs
     long long pred = ntiles;
     if (e0 != 0) {
-        const long long lp = max(bs->last_pivot[0], e0 >= 128 ? bs->last_pivot[1] : 0ll) + 1;
+        const long long lp = (e0 >= 128 ? (bs->last_pivot[0] + bs->last_pivot[1]) / 2 : bs->last_pivot[0]) + 1;
         pred = (lp + lp * stream_pct / 100) / kTile + 1 + slack_tiles;
     }
     const int later = (ga.b1 > 0 ? 1 : 0) + (ga.b2 > 0 ? 1 : 0);  // the pass serves the group's later blocks too
@@ -1129,13 +1135,16 @@ __global__ void __launch_bounds__(kTile) blk_wfix_kernel(const int32_t *__restri
 // local pivots, so that a step's window is searched to its end.  Microseconds per
 // block, before / now: 32 x 32 grid 212 / 38 (10.3 steps / 1), 10k-vertex RGG 118 /
 // 30 (5.3 / 1), 100k-point planar-chain graph 88 / 31 (2.0 / 1.0), 50k-vertex
-// random graph 217 / 114 (6.9 / 3.9).  (Eliminating eight columns at a time, the first
-// row of each byte pattern by shared-memory atomics, took 17 us per merge of 465 rows.)
+// random graph 217 / 114 (6.9 / 3.9; 122 with a shorter W pass, see kDefaultShape).
+// (Eliminating eight columns at a time, the first row of each byte pattern by
+// shared-memory atomics, took 17 us per merge of 465 rows.)
 constexpr int kPivotThreads = kElimThreads;  // threads of a pivot-kernel CTA
 constexpr int kWarps = kPivotThreads / 32;
 constexpr int kMaxLocal = 64;             // local pivots a CTA can report per step (W has 64 columns)
 constexpr int kMaxGrid = 256;             // CTAs of a pivot kernel at most
-constexpr int kMissWin = 4;               // tiles per CTA and step where W is computed on the way
+// Tiles per CTA and step where W is computed on the way: 2 / 4 / 6 / 8 / 12 take 221 / 211 /
+// 207 / 207 / 211 ms on the random graph of 50k vertices.
+constexpr int kMissWin = 6;
 constexpr int kChunkTiles = 4;            // tiles of the window loaded together (kChunkRows rows per thread)
 constexpr int kChunkRows = kChunkTiles * kTile / kPivotThreads;
 
@@ -1415,6 +1424,11 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
     const long long c = blockIdx.x;
     const long long pred = ta.first ? bs->pred_tiles : bs->pair_tiles;
     const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // While the first window reaches the expected last pivot (the pass's reach less its tile
+    // per CTA) one step ends most blocks; where it does not, half of it gives the first
+    // pivots with fewer rows to merge: 50k-vertex random graph 211 -> 207 ms, but a
+    // planar-chain graph of 100k points, whose blocks end 1-2 tiles per CTA deep, 95 -> 110.
+    const int early = pred <= (long long)(sh.win_early + 1) * G || sh.win_early < 2 ? sh.win_early : sh.win_early / 2;
     unsigned gen = ld_acquire_u32(&gb->gen);
     if (tid < 64) s_basis[tid] = 0;
     long long t0 = 0;    // scan start
@@ -1426,7 +1440,7 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
         const long long cyc0 = clock64();
         // the window, the same in every CTA: the shape's while it lies in the tiles the W
         // pass computed, cut at their end; beyond it at most kMissWin tiles
-        int wsz = grank < sh.rank_early ? sh.win_early : grank >= sh.rank_tail ? sh.win_tail : sh.win_mid;
+        int wsz = grank < sh.rank_early ? early : grank >= sh.rank_tail ? sh.win_tail : sh.win_mid;
         if (t0 >= pred) wsz = min(wsz, kMissWin);
         const long long end = min(t0 + (long long)wsz * G, t0 < pred ? pred : ntiles);
         wsz = (int)((end - t0 + G - 1) / G);
