@@ -40,7 +40,15 @@ using namespace mcbgpu::elim;
 namespace {
 
 constexpr int kTile = 1024;           // candidates per tile
-constexpr int kHead = 8;              // coordinates of a list's head (one aligned 32-byte slot per candidate)
+constexpr int kHeadWords = 8;         // a list's head: one aligned 32-byte slot per candidate
+// Coordinates a head holds: 16 of 16 bits up to this N, else 8 of 32 bits.  The lists are
+// read from HBM (28M candidates of 12 coordinates on a 50k-vertex random graph), and one
+// that does not end in its head costs its offsets and 1-2 further sectors: 90 bytes a
+// candidate late in that solve, 32 with narrow heads (206 -> 197 ms per solve; 20k
+// vertices 50 -> 47).
+constexpr int kNarrowMaxN = 65535;
+template <bool kNarrow>
+constexpr int kHeadLen = kNarrow ? 16 : 8;
 constexpr int kScanThreads = 256;     // 4 candidates per thread
 constexpr int kPer = kTile / kScanThreads;
 constexpr unsigned kSpinLimit = 1u << 24;
@@ -179,20 +187,56 @@ __global__ void validate_kernel(const int64_t *__restrict__ off, const int32_t *
 
 // Smallest first coordinate per tile of 1024 candidates (lists are ascending, so a
 // tile whose value is >= the block's bound has W = 0 for every candidate).
-// head[r] = the first kHead coordinates of candidate r's list, INT_MAX past its end:
-// one aligned 32-byte slot per candidate, read by the W walks before (and mostly
-// instead of) the list itself.
+// head[r] = the first kHeadLen coordinates of candidate r's list, INT_MAX (16 bits: 65535)
+// past its end: one aligned 32-byte slot per candidate, read by the W walks before (and
+// mostly instead of) the list itself.
+template <bool kNarrow>
 __global__ void head_kernel(const int64_t *__restrict__ off, const int32_t *__restrict__ coords, long long K,
                             int32_t *head) {
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < K; r += (long long)gridDim.x * blockDim.x) {
         const int64_t a = off[r], e = off[r + 1];
-        int v[kHead];
+        int v[kHeadWords];
 #pragma unroll
-        for (int q = 0; q < kHead; q++) v[q] = a + q < e ? coords[a + q] : 0x7fffffff;
-        int4 *h = reinterpret_cast<int4 *>(head + (size_t)r * kHead);
+        for (int q = 0; q < kHeadWords; q++)
+            if (kNarrow)
+                v[q] = (int)((unsigned)(a + 2 * q < e ? coords[a + 2 * q] : 0xffff) |
+                             (unsigned)(a + 2 * q + 1 < e ? coords[a + 2 * q + 1] : 0xffff) << 16);
+            else
+                v[q] = a + q < e ? coords[a + q] : 0x7fffffff;
+        int4 *h = reinterpret_cast<int4 *>(head + (size_t)r * kHeadWords);
         h[0] = make_int4(v[0], v[1], v[2], v[3]);
         h[1] = make_int4(v[4], v[5], v[6], v[7]);
     }
+}
+
+// Candidate r's head slot: consecutive candidates' heads are consecutive, so a warp's are
+// one coalesced read, and no offset is needed unless the list goes on below the bound.
+__device__ __forceinline__ void load_head(const int32_t *__restrict__ head, long long r, int (&h)[kHeadWords]) {
+    const int4 *p = reinterpret_cast<const int4 *>(head + (size_t)r * kHeadWords);
+    const int4 a = __ldg(p), b = __ldg(p + 1);
+    h[0] = a.x;
+    h[1] = a.y;
+    h[2] = a.z;
+    h[3] = a.w;
+    h[4] = b.x;
+    h[5] = b.y;
+    h[6] = b.z;
+    h[7] = b.w;
+}
+
+// Its coordinates 8 part .. 8 part + 7 (part 1: narrow heads only).
+template <bool kNarrow>
+__device__ __forceinline__ void head_part(const int (&h)[kHeadWords], int part, int (&cv)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        cv[q] = kNarrow ? (int)(((unsigned)h[4 * part + q / 2] >> (q % 2 * 16)) & 0xffffu) : h[q];
+}
+
+// Coordinate i < kHeadLen of candidate r's head.
+template <bool kNarrow>
+__device__ __forceinline__ int head_coord(const int32_t *__restrict__ head, unsigned long long r, int64_t i) {
+    return kNarrow ? (int)__ldg(reinterpret_cast<const uint16_t *>(head + (size_t)r * kHeadWords) + i)
+                   : __ldg(head + (size_t)r * kHeadWords + i);
 }
 
 __global__ void tile_minc_kernel(const int64_t *__restrict__ off, const int32_t *__restrict__ coords, long long K,
@@ -418,6 +462,7 @@ struct PlainSlot {           // ring of four: read one launch after it was writt
 };
 constexpr int kPlainThreads = 256;
 
+template <bool kNarrow>
 __global__ void __launch_bounds__(kPlainThreads) plain_kernel(
     uint64_t *S, uint64_t *fin, int N, int P, int e, int search, const int64_t *__restrict__ off,
     const int32_t *__restrict__ coords, const int32_t *__restrict__ head, const int32_t *__restrict__ weight,
@@ -466,7 +511,7 @@ __global__ void __launch_bounds__(kPlainThreads) plain_kernel(
         if (upd) {
             unsigned par = 0;  // <C_{e-1}, S_e>
             for (int64_t i = c0 + tid; i < c1; i += kPlainThreads) {
-                const int c = i - c0 < kHead ? __ldg(head + (size_t)rp * kHead + (i - c0)) : __ldg(coords + i);
+                const int c = i - c0 < kHeadLen<kNarrow> ? head_coord<kNarrow>(head, rp, i - c0) : __ldg(coords + i);
                 if (c <= e) par ^= (unsigned)(s_S[c >> 6] >> (c & 63)) & 1u;
             }
             par = __reduce_xor_sync(0xffffffffu, par);
@@ -487,23 +532,26 @@ __global__ void __launch_bounds__(kPlainThreads) plain_kernel(
             const long long r = r0 + tid;
             unsigned par = 0;
             if (r < K) {
-                int hv[kHead];
-                const int4 a = __ldg(reinterpret_cast<const int4 *>(head + (size_t)r * kHead));
-                const int4 b = __ldg(reinterpret_cast<const int4 *>(head + (size_t)r * kHead) + 1);
-                hv[0] = a.x, hv[1] = a.y, hv[2] = a.z, hv[3] = a.w, hv[4] = b.x, hv[5] = b.y, hv[6] = b.z, hv[7] = b.w;
+                int h[kHeadWords], v[8];
+                load_head(head, r, h);
+                auto take = [&]() {
 #pragma unroll
-                for (int q = 0; q < kHead; q++)
-                    if (hv[q] <= e) par ^= (unsigned)(s_S[hv[q] >> 6] >> (hv[q] & 63)) & 1u;
-                if (hv[kHead - 1] <= e) {
+                    for (int q = 0; q < 8; q++)
+                        if (v[q] <= e) par ^= (unsigned)(s_S[v[q] >> 6] >> (v[q] & 63)) & 1u;
+                };
+                head_part<kNarrow>(h, 0, v);
+                take();
+                if (kNarrow && v[7] <= e) {
+                    head_part<kNarrow>(h, 1, v);
+                    take();
+                }
+                if (v[7] <= e) {
                     const int64_t en = __ldg(off + r + 1);
-                    for (int64_t i = __ldg(off + r) + kHead; i < en; i += kHead) {
-                        int v[kHead];
+                    for (int64_t i = __ldg(off + r) + kHeadLen<kNarrow>; i < en; i += 8) {
 #pragma unroll
-                        for (int q = 0; q < kHead; q++) v[q] = i + q < en ? __ldg(coords + i + q) : 0x7fffffff;
-#pragma unroll
-                        for (int q = 0; q < kHead; q++)
-                            if (v[q] <= e) par ^= (unsigned)(s_S[v[q] >> 6] >> (v[q] & 63)) & 1u;
-                        if (v[kHead - 1] > e) break;
+                        for (int q = 0; q < 8; q++) v[q] = i + q < en ? __ldg(coords + i + q) : 0x7fffffff;
+                        take();
+                        if (v[7] > e) break;
                     }
                 }
             }
@@ -521,7 +569,7 @@ __global__ void __launch_bounds__(kPlainThreads) plain_kernel(
         uint64_t *Sj = S + (size_t)j * P;
         unsigned par = 0;
         for (int64_t i = lane; i < c1 - c0; i += 32) {
-            const int c = i < kHead ? __ldg(head + (size_t)rp * kHead + i) : __ldg(coords + c0 + i);
+            const int c = i < kHeadLen<kNarrow> ? head_coord<kNarrow>(head, rp, i) : __ldg(coords + c0 + i);
             par ^= (unsigned)(Sj[c >> 6] >> (c & 63)) & 1u;
         }
         par = __reduce_xor_sync(0xffffffffu, par);
@@ -741,24 +789,7 @@ __device__ bool grid_barrier(GridBar *gb, unsigned nctas, unsigned &gen_local) {
 // ends the walk, and its coordinates >= bound gather nothing.  `nread` counts the
 // coordinates read.
 constexpr int kWChunk = MCB_W_CHUNK;
-static_assert(kWChunk == kHead, "the first chunk of a W walk is the list's head");
-
-// The first kHead coordinates of candidate r (INT_MAX past the end of its list), from
-// the head array: consecutive candidates' heads are consecutive 32-byte slots, so a
-// warp's first chunks are one coalesced read, and no offset is needed unless the
-// list goes on below the bound.
-__device__ __forceinline__ void load_head(const int32_t *__restrict__ head, long long r, int (&cv)[kHead]) {
-    const int4 *h = reinterpret_cast<const int4 *>(head + (size_t)r * kHead);
-    const int4 a = __ldg(h), b = __ldg(h + 1);
-    cv[0] = a.x;
-    cv[1] = a.y;
-    cv[2] = a.z;
-    cv[3] = a.w;
-    cv[4] = b.x;
-    cv[5] = b.y;
-    cv[6] = b.z;
-    cv[7] = b.w;
-}
+static_assert(kWChunk == 8, "a W walk takes a head in parts of eight");
 
 __device__ __forceinline__ uint64_t w_chunk(const int (&cv)[kWChunk], const uint64_t *__restrict__ T, int bound) {
     uint64_t tv[kWChunk];
@@ -771,21 +802,27 @@ __device__ __forceinline__ uint64_t w_chunk(const int (&cv)[kWChunk], const uint
 }
 
 // W_r = XOR of T[c] over the coordinates c < bound of candidate r's list.  The head
-// gives the first kHead coordinates; a list whose head ends below the bound goes on
+// gives the first kHeadLen coordinates; a list whose head ends below the bound goes on
 // from its offset, kWChunk coordinates at a time (independent loads), then their T
 // words (independent loads).  The list is ascending: a chunk whose last coordinate
 // is >= bound ends the walk, and its coordinates >= bound gather nothing.  `nread`
 // counts the 4-byte words read (head, offsets, further coordinates).
+template <bool kNarrow>
 __device__ __forceinline__ uint64_t w_of_candidate(long long r, const int64_t *__restrict__ off,
                                                    const int32_t *__restrict__ coords,
                                                    const int32_t *__restrict__ head,
                                                    const uint64_t *__restrict__ T, int bound, unsigned &nread) {
-    int cv[kWChunk];
-    load_head(head, r, cv);
+    int h[kHeadWords], cv[kWChunk];
+    load_head(head, r, h);
+    head_part<kNarrow>(h, 0, cv);
     uint64_t W = w_chunk(cv, T, bound);
-    nread += kHead;
-    if (cv[kHead - 1] < bound) {
-        int64_t i = __ldg(off + r) + kHead;
+    if (kNarrow && cv[kWChunk - 1] < bound) {
+        head_part<kNarrow>(h, 1, cv);
+        W ^= w_chunk(cv, T, bound);
+    }
+    nread += kHeadWords;
+    if (cv[kWChunk - 1] < bound) {
+        int64_t i = __ldg(off + r) + kHeadLen<kNarrow>;
         const int64_t e = __ldg(off + r + 1);
         nread += 2;
         while (i < e) {
@@ -801,29 +838,38 @@ __device__ __forceinline__ uint64_t w_of_candidate(long long r, const int64_t *_
 }
 
 // W of two candidates walked in lockstep (their loads overlap); rb < 0: only ra.
+template <bool kNarrow>
 __device__ __forceinline__ void w_of_two(long long ra, long long rb, const int64_t *__restrict__ off,
                                          const int32_t *__restrict__ coords, const int32_t *__restrict__ head,
                                          const uint64_t *__restrict__ T, int bound, unsigned &nread, uint64_t &Wa,
                                          uint64_t &Wb) {
-    int ca[kWChunk], cb[kWChunk];
-    load_head(head, ra, ca);
+    int ha[kHeadWords], hb[kHeadWords], ca[kWChunk], cb[kWChunk];
+    load_head(head, ra, ha);
     if (rb >= 0) {
-        load_head(head, rb, cb);
+        load_head(head, rb, hb);
     } else {
 #pragma unroll
-        for (int q = 0; q < kWChunk; q++) cb[q] = 0x7fffffff;
+        for (int q = 0; q < kHeadWords; q++) hb[q] = kNarrow ? -1 : 0x7fffffff;
     }
+    head_part<kNarrow>(ha, 0, ca);
+    head_part<kNarrow>(hb, 0, cb);
     Wa = w_chunk(ca, T, bound);
     Wb = w_chunk(cb, T, bound);
-    nread += rb >= 0 ? 2 * kHead : kHead;
+    if (kNarrow && (ca[kWChunk - 1] < bound || cb[kWChunk - 1] < bound)) {
+        head_part<kNarrow>(ha, 1, ca);
+        head_part<kNarrow>(hb, 1, cb);
+        Wa ^= w_chunk(ca, T, bound);
+        Wb ^= w_chunk(cb, T, bound);
+    }
+    nread += rb >= 0 ? 2 * kHeadWords : kHeadWords;
     int64_t ia = 0, ea = 0, ib = 0, eb = 0;
-    if (ca[kHead - 1] < bound) {
-        ia = __ldg(off + ra) + kHead;
+    if (ca[kWChunk - 1] < bound) {
+        ia = __ldg(off + ra) + kHeadLen<kNarrow>;
         ea = __ldg(off + ra + 1);
         nread += 2;
     }
-    if (rb >= 0 && cb[kHead - 1] < bound) {
-        ib = __ldg(off + rb) + kHead;
+    if (rb >= 0 && cb[kWChunk - 1] < bound) {
+        ib = __ldg(off + rb) + kHeadLen<kNarrow>;
         eb = __ldg(off + rb + 1);
         nread += 2;
     }
@@ -870,7 +916,7 @@ __device__ __forceinline__ void w_group_chunk(const int (&cv)[kWChunk], const ui
         for (int g = 0; g < kG; g++) W[g] ^= tv[q][g];
 }
 
-template <int kG>
+template <int kG, bool kNarrow>
 __device__ __forceinline__ void w_of_group(long long r, const int64_t *__restrict__ off,
                                            const int32_t *__restrict__ coords, const int32_t *__restrict__ head,
                                            const uint64_t *__restrict__ Tg, const int (&bd)[3], unsigned &nread,
@@ -878,12 +924,17 @@ __device__ __forceinline__ void w_of_group(long long r, const int64_t *__restric
     const int last = bd[kG - 1];
 #pragma unroll
     for (int g = 0; g < kG; g++) W[g] = 0;
-    int cv[kWChunk];
-    load_head(head, r, cv);
+    int h[kHeadWords], cv[kWChunk];
+    load_head(head, r, h);
+    head_part<kNarrow>(h, 0, cv);
     w_group_chunk<kG>(cv, Tg, bd, W);
-    nread += kHead;
-    if (cv[kHead - 1] < last) {
-        int64_t i = __ldg(off + r) + kHead;
+    if (kNarrow && cv[kWChunk - 1] < last) {
+        head_part<kNarrow>(h, 1, cv);
+        w_group_chunk<kG>(cv, Tg, bd, W);
+    }
+    nread += kHeadWords;
+    if (cv[kWChunk - 1] < last) {
+        int64_t i = __ldg(off + r) + kHeadLen<kNarrow>;
         const int64_t e = __ldg(off + r + 1);
         nread += 2;
         while (i < e) {
@@ -945,7 +996,7 @@ __device__ __forceinline__ void w_by_columns(const Columns &co, const uint64_t *
 #endif
 // kG > 1 (the first block of a group): also W against each later block's rows as
 // they are now (Tg, bounds bd[1..]) into Wl[0..kG-2], for blk_wfix_kernel.
-template <int kG>
+template <int kG, bool kNarrow>
 __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, const int64_t *__restrict__ off,
                                                     const int32_t *__restrict__ coords,
                                                     const int32_t *__restrict__ head,
@@ -973,7 +1024,7 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
 #if MCB_W_PREFETCH
             if (threadIdx.x == 0 && t + gridDim.x < ntiles) {  // this CTA's next tile's heads into L2
                 const long long r0 = (t + gridDim.x) * kTile, r1 = min(r0 + kTile, K);
-                if (r0 < r1) prefetch_l2(head + (size_t)r0 * kHead, 4ull * kHead * (unsigned long long)(r1 - r0));
+                if (r0 < r1) prefetch_l2(head + (size_t)r0 * kHeadWords, 4ull * kHeadWords * (unsigned long long)(r1 - r0));
             }
 #endif
             if (tile_minc[t] >= last) {  // every W of the tile is 0
@@ -986,7 +1037,7 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
             for (int g = 0; g < kG; g++) W[g] = 0;
             unsigned nread = 0;
             if (r < K) {
-                w_of_group<kG>(r, off, coords, head, Tg, bd, nread, W);
+                w_of_group<kG, kNarrow>(r, off, coords, head, Tg, bd, nread, W);
                 nb += 8ull * kG + 4ull * nread;  // kG W writes, head / offsets / coordinates read
             }
             Warr[r] = W[0];
@@ -1011,7 +1062,7 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
         uint64_t W = 0;
         unsigned nread = 0;
         if (r < K) {
-            W = w_of_candidate(r, off, coords, head, T, bound, nread);
+            W = w_of_candidate<kNarrow>(r, off, coords, head, T, bound, nread);
             nb += 8 + 4ull * nread;  // W write, head / offsets / coordinates read
         }
         Warr[r] = W;
@@ -1390,6 +1441,7 @@ __device__ void materialize_rows(const TailArgs &ta, const BlockState *bs, int b
 #endif
 // Dynamic shared memory: B's tables (16 KB) | the row list (G x kMaxLocal rows at
 // least), which the block tail reuses as scratch (P + 1 counters; kMatCols columns).
+template <bool kNarrow>
 __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kernel(
     long long K, const int64_t *__restrict__ off, const int32_t *__restrict__ coords,
     const int32_t *__restrict__ head, const int32_t *__restrict__ tile_minc, const uint64_t *__restrict__ T,
@@ -1462,7 +1514,7 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
                 const long long ra = ta_ * kTile + idx % kTile, rb = tb_ * kTile + jdx % kTile;
                 const bool va = ra < K && tile_minc[ta_] < bound, vb = rb < K && tile_minc[tb_] < bound;
                 uint64_t Wa = 0, Wb = 0;
-                if (va || vb) w_of_two(va ? ra : rb, va && vb ? rb : -1, off, coords, head, T, bound, nread, Wa, Wb);
+                if (va || vb) w_of_two<kNarrow>(va ? ra : rb, va && vb ? rb : -1, off, coords, head, T, bound, nread, Wa, Wb);
                 if (!va) {  // the walk ran on rb alone
                     Wb = Wa;
                     Wa = 0;
@@ -2331,7 +2383,11 @@ struct mcbgpu_solver {
     int32_t *d_weight = nullptr;
     int64_t *d_off = nullptr;
     int32_t *d_coords = nullptr;
-    int32_t *d_head = nullptr;     // K x kHead: each list's first coordinates (INT_MAX past its end)
+    int32_t *d_head = nullptr;     // K x kHeadWords: each list's first coordinates (head_kernel)
+    bool narrow = false;           // heads of 16-bit coordinates
+    const void *pivot_fn() const {
+        return narrow ? (const void *)blk_pivot_kernel<true> : (const void *)blk_pivot_kernel<false>;
+    }
     uint64_t *d_S = nullptr;
     uint64_t *d_C = nullptr;       // cycle vector buffer (W words)
     uint64_t *d_T = nullptr;       // 64 * P words
@@ -2620,7 +2676,8 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
     ALLOC(s->d_weight, sizeof(int32_t) * (size_t)K);
     ALLOC(s->d_off, sizeof(int64_t) * (size_t)(K + 1));
     ALLOC(s->d_coords, sizeof(int32_t) * (size_t)(nnz + 16));  // aligned 16-byte loads read up to 11 past the end
-    ALLOC(s->d_head, sizeof(int32_t) * kHead * (size_t)K);
+    s->narrow = N <= kNarrowMaxN;
+    ALLOC(s->d_head, sizeof(int32_t) * kHeadWords * (size_t)K);
     ALLOC(s->d_S, sizeof(uint64_t) * (size_t)N * s->P);
     ALLOC(s->d_C, sizeof(uint64_t) * (size_t)s->P);
     ALLOC(s->d_T, sizeof(uint64_t) * 64 * (size_t)s->P);
@@ -2710,10 +2767,10 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
         if (smem > (size_t)kPivotSmemMax) e = cudaErrorInvalidValue;
         // the attribute is the kernel's, shared by all handles: never lowered
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(blk_pivot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmemMax);
+            e = cudaFuncSetAttribute(s->pivot_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmemMax);
         int per_sm = 0;
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, blk_pivot_kernel, kPivotThreads, smem);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, s->pivot_fn(), kPivotThreads, smem);
         if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
         // CTAs beyond one per tile have nothing to scan; a few more take the tail's columns
         s->pivot_grid = (int)std::min<long long>(G, std::max<long long>((K + kTile - 1) / kTile, 8));
@@ -2808,7 +2865,7 @@ static int solver_upload(mcbgpu_solver *s, const int32_t *weight, const int64_t 
         {
             Launch L(s, KC_VALIDATE, st);
             const int hgrid = (int)std::min<long long>((s->K + 255) / 256, (long long)(s->sm_count > 0 ? s->sm_count : 148) * 16);
-            head_kernel<<<hgrid, 256, 0, st>>>(s->d_off, s->d_coords, s->K, s->d_head);
+            (s->narrow ? head_kernel<true> : head_kernel<false>)<<<hgrid, 256, 0, st>>>(s->d_off, s->d_coords, s->K, s->d_head);
         }
         int grid = (int)std::min<long long>(ntiles, (long long)(s->sm_count > 0 ? s->sm_count : 148) * 8);
         {
@@ -2956,9 +3013,10 @@ int mcbgpu_solver_run_plain(mcbgpu_solver *s, int64_t max_iterations, void *stre
             set_error("mcbgpu_solver_run_plain: support vector prefix too large for shared memory");
             return MCBGPU_E_ARG;
         }
-        if (smem > 48 * 1024) MCB_CUDA(cudaFuncSetAttribute(plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        auto *const fn = s->narrow ? plain_kernel<true> : plain_kernel<false>;
+        if (smem > 48 * 1024) MCB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         Launch L(s, KC_SEARCH, st);
-        MCB_CUDA(launch_k(s->pdl, plain_kernel, dim3(grid), dim3(kPlainThreads), smem, st, s->d_S, s->d_fin, s->N, s->P,
+        MCB_CUDA(launch_k(s->pdl, fn, dim3(grid), dim3(kPlainThreads), smem, st, s->d_S, s->d_fin, s->N, s->P,
                           (int)e, search, (const int64_t *)s->d_off, (const int32_t *)s->d_coords,
                           (const int32_t *)s->d_head, (const int32_t *)s->d_weight, s->K, s->d_ring, s->d_slots,
                           s->d_selected, s->d_bs, s->d_status));
@@ -3084,13 +3142,13 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             const BlockState *wbs = s->d_bs;
             uint64_t *nul = nullptr;
             if (nl == 2)
-                MCB_CUDA(launch_k(pdl, blk_w_kernel<3>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
+                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<3, true> : blk_w_kernel<3, false>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
                                   bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd2, Wpos[1], Wpos[2], cols));
             else if (nl == 1)
-                MCB_CUDA(launch_k(pdl, blk_w_kernel<2>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
+                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<2, true> : blk_w_kernel<2, false>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
                                   bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd1, Wpos[1], nul, cols));
             else
-                MCB_CUDA(launch_k(pdl, blk_w_kernel<1>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
+                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<1, true> : blk_w_kernel<1, false>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
                                   bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), (const uint64_t *)nullptr, 0, 0, nul,
                                   nul, cols));
         }
@@ -3131,7 +3189,7 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             PivotShape shv = sh;
             void *args[] = {&K, &off, &co, &hd, &tm, &T, (void *)&bound, &bs, &Wa, &te, &rw, &rk, &rn, &gb, &stt, &nb, &dg, &db,
                             &ta, &shv, &lcap};
-            MCB_CUDA(launch_coop(pdl, (const void *)blk_pivot_kernel, dim3(s->pivot_grid), dim3(kPivotThreads), args,
+            MCB_CUDA(launch_coop(pdl, s->pivot_fn(), dim3(s->pivot_grid), dim3(kPivotThreads), args,
                                  pivot_smem_bytes(s->pivot_grid, s->P), st));
         }
         if (s->tuning && (pos == kGroup - 1 || e0 + b >= iters)) {  // the group's last block
