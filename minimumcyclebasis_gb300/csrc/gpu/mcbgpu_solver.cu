@@ -122,7 +122,6 @@ struct BlockState {
     long long last_pivot[2];       // by block parity: rank of the block's last pivot
     long long pred_tiles;          // tiles the streaming pass computes for this block
     unsigned long long total;      // running 64-bit total weight of the basis
-    unsigned tail_ok, pad_;        // the pivot kernel's CTA 0 resolved the block
     long long pair_tiles;          // tiles the grouped streaming pass computed for the group's later blocks
     unsigned nz_count[3];          // by group (mod 3): coordinates whose T (Tg) words are not all zero
     unsigned by_columns;           // the group's W come from the column index, not from the lists
@@ -1185,8 +1184,8 @@ __global__ void __launch_bounds__(kTile) blk_wfix_kernel(const int32_t *__restri
 // pick per two CTA barriers with the tables rebuilt for each, and a CTA reports all its
 // local pivots, so that a step's window is searched to its end.  Microseconds per
 // block, before / now: 32 x 32 grid 212 / 38 (10.3 steps / 1), 10k-vertex RGG 118 /
-// 30 (5.3 / 1), 100k-point planar-chain graph 88 / 31 (2.0 / 1.0), 50k-vertex
-// random graph 217 / 114 (6.9 / 3.9; 122 with a shorter W pass, see kDefaultShape).
+// 30 (5.3 / 1), 100k-point planar-chain graph 88 / 31 (2.0 / 1.0), 50k-vertex random
+// graph 217 / 114 (6.9 / 3.9); 4-5 less since every CTA resolves the block (resolve_block).
 // (Eliminating eight columns at a time, the first row of each byte pattern by
 // shared-memory atomics, took 17 us per merge of 465 rows.)
 constexpr int kPivotThreads = kElimThreads;  // threads of a pivot-kernel CTA
@@ -1232,7 +1231,10 @@ __device__ __forceinline__ void helpers_sync(unsigned nthreads) {
 // pivot) pairs and sort them by S word (counting sort; word_end[w] = number of pairs
 // whose word is below w).  At the end the pivot index of every pair is replaced by
 // the iteration that selected it.  `hist` is shared scratch of P + 1 words.  Returns
-// false (and sets a status bit) if the block cannot be resolved.
+// false (and sets a status bit) if the block cannot be resolved.  CTA 0 does all of it;
+// the others run the b steps for the masks alone, while their first columns are read: no
+// grid barrier and no wait for CTA 0's pairs (100k-point planar-chain graph 95 -> 86 ms
+// per solve, 10k-vertex RGG 12.2 -> 11.2, 50k-vertex random graph 197 -> 193).
 #ifdef MCB_TAIL_PROFILE
 __device__ unsigned long long g_tail_prof[8];
 #define TAIL_STAMP(i) \
@@ -1247,7 +1249,7 @@ __device__ unsigned long long g_tail_prof[8];
 
 __device__ bool resolve_block(BlockState *bs, int rank, const int64_t *__restrict__ off,
                               const int32_t *__restrict__ coords, const TailArgs &ta, unsigned *hist,
-                              unsigned *status) {
+                              unsigned *status, uint64_t *s_mask) {
 #ifdef MCB_TAIL_PROFILE
     const long long t_start = clock64();
 #endif
@@ -1304,8 +1306,8 @@ __device__ bool resolve_block(BlockState *bs, int rank, const int64_t *__restric
                 }
             }
         }
-        bs->mask[lane] = m0;
-        bs->mask[32 + lane] = m1;
+        bs->mask[lane] = s_mask[lane] = m0;
+        bs->mask[32 + lane] = s_mask[32 + lane] = m1;
         TAIL_STAMP(1);
     } else {
         // warps 1..: the pivots' (coordinate, pivot) pairs, sorted by S word
@@ -1411,26 +1413,55 @@ __device__ bool resolve_block(BlockState *bs, int rank, const int64_t *__restric
 #endif
 constexpr int kMatCols = MCB_MAT_COLS;
 
-__device__ void materialize_rows(const TailArgs &ta, const BlockState *bs, int b, uint64_t *buf) {
+__device__ __forceinline__ void columns_in(const TailArgs &ta, int b, int cg, uint64_t (*s0)[kMatCols + 1], int t, int nt) {
+    const int w0 = cg * kMatCols;
+    for (int idx = t; idx < 64 * kMatCols; idx += nt) {
+        const int l = idx / kMatCols, w = idx % kMatCols;
+        s0[l][w] = (l < b && w0 + w < ta.Wb) ? ta.S[(size_t)(ta.e0 + l) * ta.P + w0 + w] : 0ull;
+    }
+}
+
+// CTA 0 takes the last groups: it comes last.
+__device__ void block_tail(const TailArgs &ta, BlockState *bs, int rank, int b, const int64_t *__restrict__ off,
+                           const int32_t *__restrict__ coords, const uint64_t *Warr, const long long *s_prank,
+                           uint64_t *buf, unsigned *status) {
     uint64_t(*s0)[kMatCols + 1] = reinterpret_cast<uint64_t(*)[kMatCols + 1]>(buf);
-    __shared__ uint64_t sm[64];
-    if (threadIdx.x < 64) sm[threadIdx.x] = (int)threadIdx.x < b ? bs->mask[threadIdx.x] : 0ull;
-    const int Wb = ta.Wb, P = ta.P, e0 = ta.e0;
-    const int ng = (Wb + kMatCols - 1) / kMatCols;
-    for (int cg = blockIdx.x; cg < ng; cg += gridDim.x) {
-        const int w0 = cg * kMatCols;
-        cta_sync();  // the masks are in place; the previous group's rows are read
-        for (int idx = threadIdx.x; idx < 64 * kMatCols; idx += blockDim.x) {
-            const int l = idx / kMatCols, w = idx % kMatCols;
-            s0[l][w] = (l < b && w0 + w < Wb) ? ta.S[(size_t)(e0 + l) * P + w0 + w] : 0ull;
+    __shared__ uint64_t s_mask[64];
+    __shared__ int s_done;
+    const int G = (int)gridDim.x, ng = (ta.Wb + kMatCols - 1) / kMatCols, tid = threadIdx.x, lane = tid & 31;
+    int cg = G - 1 - (int)blockIdx.x;
+    if (blockIdx.x == 0) {
+        if (!resolve_block(bs, rank, off, coords, ta, reinterpret_cast<unsigned *>(buf), status, s_mask)) return;
+    } else {
+        if (rank < b || cg >= ng) return;
+        if (tid < 32) {
+            uint64_t a0 = lane < b ? __ldcg(Warr + s_prank[lane]) : 0ull;
+            uint64_t a1 = 32 + lane < b ? __ldcg(Warr + s_prank[32 + lane]) : 0ull, m0, m1;
+            warp_transpose64(a0, a1);
+            int p0, p1;
+            const bool done = resolve_rows(b, a0, a1, m0, m1, p0, p1);
+            s_mask[lane] = m0;
+            s_mask[32 + lane] = m1;
+            if (lane == 0) s_done = done;
+        } else {
+            columns_in(ta, b, cg, s0, tid - 32, (int)blockDim.x - 32);
         }
         cta_sync();
-        for (int idx = threadIdx.x; idx < 64 * kMatCols; idx += blockDim.x) {
+        if (!s_done) return;
+    }
+    for (bool in = blockIdx.x != 0; cg < ng; cg += G, in = false) {
+        if (!in) {
+            cta_sync();  // the previous group's rows are read
+            columns_in(ta, b, cg, s0, tid, (int)blockDim.x);
+            cta_sync();
+        }
+        const int w0 = cg * kMatCols;
+        for (int idx = tid; idx < 64 * kMatCols; idx += blockDim.x) {
             const int k = idx / kMatCols, w = idx % kMatCols;
-            if (k < b && w0 + w < Wb) {
+            if (k < b && w0 + w < ta.Wb) {
                 uint64_t acc = 0;
-                for (uint64_t m = sm[k]; m; m &= m - 1) acc ^= s0[__ffsll((long long)m) - 1][w];
-                ta.S[(size_t)(e0 + k) * P + w0 + w] = acc;
+                for (uint64_t m = s_mask[k]; m; m &= m - 1) acc ^= s0[__ffsll((long long)m) - 1][w];
+                ta.S[(size_t)(ta.e0 + k) * ta.P + w0 + w] = acc;
             }
         }
     }
@@ -1695,27 +1726,12 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
         }
         cta_sync();
     }
-    // ---- block tail: CTA 0 resolves the block; then every CTA materialises its
-    // column groups of the final rows and their tables ----
-    long long cyc_resolve = 0, cyc_tailbar = 0, cyc_mat = 0;
+    // ---- block tail: every CTA resolves the block and writes its columns of the final rows ----
+    long long cyc_tail = 0;
     if (ok) {
         const long long c3 = clock64();
-        if (c == 0) {
-            const bool done = resolve_block(bs, grank, off, coords, ta, reinterpret_cast<unsigned *>(rows.w), status);
-            if (threadIdx.x == 0) bs->tail_ok = done ? 1u : 0u;
-        }
-        const long long c4 = clock64();
-        nbar++;
-        if (!grid_barrier(gb, G, gen)) {
-            ok = false;
-        } else {
-            const long long c5 = clock64();
-            if (*((volatile unsigned *)&bs->tail_ok)) materialize_rows(ta, bs, b, rows.w);
-            cta_sync();
-            cyc_tailbar = c5 - c4;
-            cyc_mat = clock64() - c5;
-        }
-        cyc_resolve = c4 - c3;
+        block_tail(ta, bs, grank, b, off, coords, Warr, s_prank, rows.w, status);
+        cyc_tail = clock64() - c3;
     }
     if (!ok && threadIdx.x == 0 && (*((volatile unsigned *)&gb->abort))) atomicOr(status, ST_WAIT_TIMEOUT);
     for (int d = 16; d > 0; d >>= 1) nb += __shfl_xor_sync(0xffffffffu, nb, d);
@@ -1736,9 +1752,7 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
         atomicAdd(&diag[6], (unsigned long long)cyc_scan);
         atomicAdd(&diag[7], (unsigned long long)cyc_bar);
         atomicAdd(&diag[8], (unsigned long long)cyc_merge);
-        atomicAdd(&diag[20], (unsigned long long)cyc_resolve);
-        atomicAdd(&diag[21], (unsigned long long)cyc_tailbar);
-        atomicAdd(&diag[22], (unsigned long long)cyc_mat);
+        atomicAdd(&diag[20], (unsigned long long)cyc_tail);
 #ifdef MCB_TAIL_PROFILE
         for (int i = 0; i < 6; i++) diag[24 + i] = g_tail_prof[i];
 #endif
