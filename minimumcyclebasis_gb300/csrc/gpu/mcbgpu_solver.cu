@@ -635,7 +635,21 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
                                                            uint64_t *__restrict__ Tg, GroupArgs ga) {
     griddep_wait();
     griddep_launch();
-    if (*(volatile const unsigned *)&bs->failed) {  // set by an earlier block's pivot kernel (same stream)
+    // all that is read first is read together, the first columns' rows included: a chain of
+    // reads and a launch are what bounds this kernel (10.6 -> 7.9 us on planar-chain graphs)
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5, first = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint64_t x0 = 0, y0 = 0, x1 = 0, y1 = 0, x2 = 0, y2 = 0;
+    auto load_rows = [&](int w) {
+        load_columns(S, P, e0, b, w, x0, y0);
+        if (ga.b1 > 0) load_columns(S, P, e0 + 64, ga.b1, w, x1, y1);
+        if (ga.b2 > 0) load_columns(S, P, e0 + 128, ga.b2, w, x2, y2);
+    };
+    if (first < ga.Wlast) load_rows(first);
+    const unsigned failed = __ldcg(&bs->failed);  // set by an earlier block's pivot kernel (same stream)
+    const long long lp0 = __ldcg(&bs->last_pivot[0]), lp1 = __ldcg(&bs->last_pivot[1]);
+    const unsigned before = __ldcg(&bs->nz_count[(ga.slot + 2) % 3]);
+    if (failed) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             bs->pred_tiles = 0;  // the streaming pass and its correction then cover no tile
             bs->pair_tiles = 0;
@@ -646,14 +660,14 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
     // per CTA of the pivot kernel, which computes any further tile it needs
     long long pred = ntiles;
     if (e0 != 0) {
-        const long long lp = (e0 >= 128 ? (bs->last_pivot[0] + bs->last_pivot[1]) / 2 : bs->last_pivot[0]) + 1;
+        const long long lp = (e0 >= 128 ? (lp0 + lp1) / 2 : lp0) + 1;
         pred = (lp + lp * stream_pct / 100) / kTile + 1 + slack_tiles;
     }
     const int later = (ga.b1 > 0 ? 1 : 0) + (ga.b2 > 0 ? 1 : 0);  // the pass serves the group's later blocks too
     if (later > 0 && e0 != 0) pred += pred * MCB_PAIR_MARGIN * later / 100;
     pred = pred < ntiles ? pred : ntiles;
     const bool cols = ga.nz && ga.columns &&
-                      (long long)bs->nz_count[(ga.slot + 2) % 3] * kColumnShare <= (long long)e0 + 64 * kColumnShare;
+                      (long long)before * kColumnShare <= (long long)e0 + 64 * kColumnShare;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         gb->count = 0;
         gb->abort = 0;
@@ -675,14 +689,9 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
                 W[i] = make_ulonglong2(0ull, 0ull);
         }
     }
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ga.Wlast; w += warps) {
+    for (int w = first; w < ga.Wlast; w += warps) {
         const size_t c0 = (size_t)w * 64 + lane, c1 = c0 + 32;
-        uint64_t x0, y0, x1 = 0, y1 = 0, x2 = 0, y2 = 0;
-        load_columns(S, P, e0, b, w, x0, y0);
-        if (ga.b1 > 0) load_columns(S, P, e0 + 64, ga.b1, w, x1, y1);
-        if (ga.b2 > 0) load_columns(S, P, e0 + 128, ga.b2, w, x2, y2);
+        if (w != first) load_rows(w);
         warp_transpose64(x0, y0);  // x: column 64w + lane, y: column 64w + 32 + lane
         if (w < Wb) {
             T[c0] = x0;
@@ -1496,23 +1505,24 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
     griddep_launch();
     // an earlier block ran out of candidates (flag written by an earlier launch, so
     // every CTA reads the same value and none waits at a grid barrier)
-    if (*(volatile const unsigned *)&bs->failed) return;
+    const unsigned failed = __ldcg(&bs->failed);
+    const unsigned epoch = __ldcg(&bs->epoch);
+    const int b = (int)__ldcg(&bs->b);
+    const long long pred = ta.first ? __ldcg(&bs->pred_tiles) : __ldcg(&bs->pair_tiles);
+    unsigned gen = *(volatile unsigned *)&gb->gen;  // as the previous launch left it
+    if (failed) return;
     unsigned long long n_loaded = 0, n_computed = 0, n_local = 0, n_cand = 0;
     long long cyc_scan = 0, cyc_bar = 0, cyc_merge = 0;
     unsigned long long nbar = 0;
     unsigned long long nb = 0;
-    const unsigned epoch = bs->epoch;
-    const int b = (int)bs->b;
     const long long ntiles = (K + kTile - 1) / kTile;
     const long long c = blockIdx.x;
-    const long long pred = ta.first ? bs->pred_tiles : bs->pair_tiles;
     const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // While the first window reaches the expected last pivot (the pass's reach less its tile
     // per CTA) one step ends most blocks; where it does not, half of it gives the first
     // pivots with fewer rows to merge: 50k-vertex random graph 211 -> 207 ms, but a
     // planar-chain graph of 100k points, whose blocks end 1-2 tiles per CTA deep, 95 -> 110.
     const int early = pred <= (long long)(sh.win_early + 1) * G || sh.win_early < 2 ? sh.win_early : sh.win_early / 2;
-    unsigned gen = ld_acquire_u32(&gb->gen);
     if (tid < 64) s_basis[tid] = 0;
     long long t0 = 0;    // scan start
     int grank = 0;
@@ -1529,7 +1539,7 @@ __global__ void __launch_bounds__(kPivotThreads, MCB_PIVOT_MINB) blk_pivot_kerne
         wsz = (int)((end - t0 + G - 1) / G);
         const long long tf = t0 + c * wsz;
         const int nwin = tf >= end ? 0 : (int)min((long long)wsz, end - tf);
-        if (tid < (unsigned)nwin) s_tag[tid] = ld_acquire_u32(&tile_epoch[tf + tid]);
+        if (tid < (unsigned)nwin) s_tag[tid] = __ldcg(&tile_epoch[tf + tid]);
         cta_sync();
         unsigned missmask = 0;
         for (int m = 0; m < nwin; m++)
@@ -2199,7 +2209,9 @@ __global__ void __launch_bounds__(256) near_d_kernel(const uint64_t *__restrict_
 // buffer for the next block), then takes columns [w0, w0 + kNearCols) of the block's
 // final rows into shared memory and applies S_j ^= XOR_k beta_k S_{e0+k} there to
 // every near row: one read of the final rows in all, the near rows read and written
-// once, column-contiguous.
+// once, column-contiguous.  Bound by its chain of reads and of the 64 steps: the first
+// columns are read before the betas are computed, and a step is a test and two XORs
+// (9.5 -> 7.3 us on planar-chain graphs against a parity per step and the reads after).
 constexpr int kNearCols = 32;
 constexpr int kNearBatch = 8;  // near rows per thread whose words are loaded together
 
@@ -2208,21 +2220,50 @@ __global__ void __launch_bounds__(256) near_apply_kernel(uint64_t *S, long long 
                                                         const unsigned long long *__restrict__ Dbuf,
                                                         unsigned long long *Dnext, uint64_t *beta_out,
                                                         unsigned long long *bytes) {
-    __shared__ uint64_t sg[64];
+    __shared__ __align__(16) uint64_t sg[64];  // row k: the later iterations whose gcol has bit k
     __shared__ uint64_t sbeta[kNearMaxRows];
     __shared__ uint64_t srow[65][kNearCols];  // row 64: zeros, the padding of a short batch of bits
     griddep_wait();
     griddep_launch();
-    if (threadIdx.x < 64) sg[threadIdx.x] = (int)threadIdx.x < b ? gcol[threadIdx.x] : 0;
+    // the final rows' first columns are on their way while the betas are computed
+    constexpr int kFill = (65 * kNearCols + 255) / 256;
+    uint64_t fill[kFill];
+    auto load_cols = [&](int w0) {
+#pragma unroll
+        for (int q = 0; q < kFill; q++) {
+            const int idx = threadIdx.x + q * 256, l = idx / kNearCols, x = idx % kNearCols;
+            fill[q] = l < b && w0 + x < Wb ? S[(size_t)(e0 + l) * P + w0 + x] : 0ull;
+        }
+    };
+    load_cols(blockIdx.x * kNearCols);
+    uint64_t D = threadIdx.x < nrows ? Dbuf[threadIdx.x] : 0ull;
+    if (threadIdx.x < 32) {
+        uint64_t g0 = (int)threadIdx.x < b ? gcol[threadIdx.x] : 0, g1 = (int)threadIdx.x + 32 < b ? gcol[threadIdx.x + 32] : 0;
+        warp_transpose64(g0, g1);
+        sg[threadIdx.x] = g0;
+        sg[threadIdx.x + 32] = g1;
+    }
     cta_sync();
     unsigned long long nb = 0;
-    for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
-        const uint64_t D = Dbuf[r];
-        uint64_t beta = 0;
-        for (int k = 0; k < b; k++) beta |= ((((D >> k) & 1ull) ^ (uint64_t)parity64(beta & sg[k]))) << k;
-        sbeta[r] = beta;
+    static_assert(kNearMaxRows <= 256, "a row per thread");
+    if (threadIdx.x < nrows) {
+        // iteration k's bit stands once k steps are done; it then goes to the later ones
+        unsigned dl = (unsigned)D, dh = (unsigned)(D >> 32);
+#pragma unroll 8
+        for (int k = 0; k < 32; k++) {
+            const uint64_t g = sg[k];
+            if ((dl >> k) & 1u) {
+                dl ^= (unsigned)g;
+                dh ^= (unsigned)(g >> 32);
+            }
+        }
+#pragma unroll 8
+        for (int k = 0; k < 32; k++)
+            if ((dh >> k) & 1u) dh ^= (unsigned)(sg[32 + k] >> 32);
+        const uint64_t beta = join64(dl, dh);
+        sbeta[threadIdx.x] = beta;
         if (blockIdx.x == 0) {
-            if (beta_out) beta_out[r] = beta;
+            if (beta_out) beta_out[threadIdx.x] = beta;
             nb += beta ? 16ull * (unsigned long long)Wb : 0ull;
         }
     }
@@ -2231,9 +2272,11 @@ __global__ void __launch_bounds__(256) near_apply_kernel(uint64_t *S, long long 
     cta_sync();
     const int w = threadIdx.x % kNearCols, rs = threadIdx.x / kNearCols, rstep = blockDim.x / kNearCols;
     for (int w0 = blockIdx.x * kNearCols; w0 < Wb; w0 += gridDim.x * kNearCols) {
-        for (int idx = threadIdx.x; idx < 65 * kNearCols; idx += blockDim.x) {
-            const int l = idx / kNearCols, x = idx % kNearCols;
-            srow[l][x] = (l < b && w0 + x < Wb) ? S[(size_t)(e0 + l) * P + w0 + x] : 0ull;
+        if (w0 != blockIdx.x * kNearCols) load_cols(w0);
+#pragma unroll
+        for (int q = 0; q < kFill; q++) {
+            const int idx = threadIdx.x + q * 256;
+            if (idx < 65 * kNearCols) srow[idx / kNearCols][idx % kNearCols] = fill[q];
         }
         if (threadIdx.x == 0) nb += 8ull * (unsigned long long)b * (unsigned long long)min(kNearCols, Wb - w0);
         cta_sync();
