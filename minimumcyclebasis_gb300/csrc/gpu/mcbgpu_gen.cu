@@ -360,15 +360,19 @@ __device__ void candidate_features(uint16_t *f, float W, float wmed, float da, f
 // features); with it, the coordinates at out[off[r] ...] in walk order.  A hop is two
 // dependent reads (parent slot, from HBM; its row and coordinate in one 16-byte entry,
 // from L2), and the two paths are walked side by side so that theirs overlap: 1.1M
-// candidates of a 65k-point planar-chain graph, 130 hops each, 5.4 -> 4.8 ms per pass.
+// candidates of a 65k-point planar-chain graph, 130 hops each, 5.4 -> 4.8 ms per pass, 1.3
+// by tree (tree_order_kernel).
 __global__ void __launch_bounds__(kWalkThreads) walk_kernel(GenGraph g, const int32_t *__restrict__ pedge, int64_t K,
                                                             const int32_t *__restrict__ tree,
                                                             const int32_t *__restrict__ eoff, int32_t *len,
                                                             const int64_t *__restrict__ off, int32_t *out,
                                                             unsigned *status, uint16_t *feat,
-                                                            const int32_t *__restrict__ weight, float wmed) {
+                                                            const int32_t *__restrict__ weight, float wmed,
+                                                            const int32_t *__restrict__ order, int64_t count) {
     const int n = g.n;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < K; r += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = order ? order[i] : i;
+        if (r >= K) continue;
         const int32_t t = tree[r], o = eoff[r];
         if (t < 0 || t >= g.F || o < 0 || (int64_t)o >= g.slots) {
             atomicOr(status, ST_BAD_INPUT);
@@ -429,6 +433,36 @@ __global__ void __launch_bounds__(kWalkThreads) walk_kernel(GenGraph g, const in
             candidate_features(feat + r * 16, (float)weight[r], wmed, dist[0], dist[1], (float)g.w[o], hops[0],
                                hops[1], c, (float)r / (float)K, deg_root, deg_ends);
         }
+    }
+}
+
+// The walks go tree by tree where few of them share a tree larger than L2 holds: ranks are
+// by weight, so neighbouring ones walk trees gigabytes apart, and every hop was a sector
+// of its own from HBM.  A counting sort: place[r] in its tree's group (ranks with a bad
+// tree: group F), then order[start[tree] + place[r]] = r.  The order inside a group is
+// any; the lists do not depend on it.  Two walks, by rank / by tree with the sort:
+// planar-chain graphs of 65k points (4.7 GB of parent slots, 1,060 per candidate) 9.6 /
+// 2.7 ms, 12k points (159 MB, 390) 250 / 200 us, 8k (69 MB, 290) 197 / 157 us, 4k (17 MB)
+// 117 / 97 us, which the sort's launches take back; random graphs of 20k vertices (313 MB,
+// 15) 1.82 / 2.42 ms, 8k (50 MB, 12) 271 / 368 us: the sort costs by candidate, and
+// their sectors are in L2 from other walks.
+constexpr int64_t kOrderBytes = 64 << 20;
+constexpr int64_t kOrderSlots = 64;  // parent slots per candidate from here on
+
+__global__ void __launch_bounds__(kScanThreads) tree_place_kernel(const int32_t *__restrict__ tree, int64_t K, int F,
+                                                                  int32_t *size, int32_t *place) {
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < K; r += (int64_t)gridDim.x * blockDim.x) {
+        const int t = tree[r];
+        place[r] = atomicAdd(size + (t >= 0 && t < F ? t : F), 1);
+    }
+}
+
+__global__ void __launch_bounds__(kScanThreads) tree_order_kernel(const int32_t *__restrict__ tree, int64_t K, int F,
+                                                                  const int64_t *__restrict__ start,
+                                                                  const int32_t *__restrict__ place, int32_t *order) {
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < K; r += (int64_t)gridDim.x * blockDim.x) {
+        const int t = tree[r];
+        order[start[t >= 0 && t < F ? t : F] + place[r]] = (int32_t)r;
     }
 }
 
@@ -620,7 +654,9 @@ struct mcbgpu_gen {
     // list buffers, kept from one ranking to the next; their sizes in bytes
     int64_t cap_tree = 0, cap_eoff = 0, cap_len = 0, cap_weight = 0, cap_off = 0, cap_bsum = 0, cap_coords = 0,
             cap_longs = 0;
-    bool ranked = false;
+    int64_t cap_order = 0;
+    unsigned char *d_order = nullptr;  // ranks tree by tree (mcbgpu_gen_rank), and scratch
+    bool ranked = false, ordered = false;
     int32_t *d_tree = nullptr, *d_eoff = nullptr, *d_len = nullptr, *d_coords = nullptr, *d_weight = nullptr;
     int64_t *d_off = nullptr, *d_bsum = nullptr, *d_longs = nullptr;
     unsigned *d_nlong = nullptr;
@@ -642,6 +678,7 @@ static cudaError_t keep_room(T *&p, int64_t &cap, int64_t need) {
 }
 
 static void gen_free_lists(mcbgpu_gen *g) {
+    cudaFree(g->d_order);
     cudaFree(g->d_tree);
     cudaFree(g->d_eoff);
     cudaFree(g->d_len);
@@ -1092,11 +1129,34 @@ int mcbgpu_gen_rank(mcbgpu_gen *g, int64_t K, const int32_t *tree, const int32_t
     MCB_CUDA(cudaMemcpyAsync(g->d_tree, tree, 4 * (size_t)K, cudaMemcpyHostToDevice, st));
     MCB_CUDA(cudaMemcpyAsync(g->d_eoff, edge_offset, 4 * (size_t)K, cudaMemcpyHostToDevice, st));
     MCB_CUDA(cudaMemcpyAsync(g->d_weight, weight, 4 * (size_t)K, cudaMemcpyHostToDevice, st));
+    g->ordered = false;
+    if (4 * (int64_t)g->F * g->n > kOrderBytes && (int64_t)g->F * g->n / K >= kOrderSlots && K < INT32_MAX) {
+        // [order K | start F + 2 | sums | sizes F + 1]; without the room the walks go by rank
+        const int64_t items = (int64_t)g->F + 1;
+        const int64_t ob = (items + (int64_t)kScanThreads * kScanItems - 1) / ((int64_t)kScanThreads * kScanItems);
+        const int64_t at_start = (4 * K + 15) & ~15ll, at_sums = at_start + 8 * (items + 1), at_size = at_sums + 8 * (ob + 1);
+        if (keep_room(g->d_order, g->cap_order, at_size + 4 * items) == cudaSuccess) {
+            int64_t *start = reinterpret_cast<int64_t *>(g->d_order + at_start), *sums = reinterpret_cast<int64_t *>(g->d_order + at_sums);
+            int32_t *size = reinterpret_cast<int32_t *>(g->d_order + at_size), *order = reinterpret_cast<int32_t *>(g->d_order);
+            const int ogrid = (int)std::min<long long>((K + kScanThreads - 1) / kScanThreads, (long long)g->sm_count * 8);
+            MCB_CUDA(cudaMemsetAsync(size, 0, 4 * (size_t)items, st));
+            tree_place_kernel<<<ogrid, kScanThreads, 0, st>>>(g->d_tree, K, g->F, size, g->d_len);
+            block_sums_kernel<<<(unsigned)ob, kScanThreads, 0, st>>>(size, items, sums);
+            scan_small_kernel<<<1, kScanThreads, 0, st>>>(sums, (int)ob, sums);
+            block_offsets_kernel<<<(unsigned)ob, kScanThreads, 0, st>>>(size, items, sums, start);
+            tree_order_kernel<<<ogrid, kScanThreads, 0, st>>>(g->d_tree, K, g->F, start, g->d_len, order);
+            MCB_CUDA(cudaGetLastError());
+            g->ordered = true;
+        } else {
+            (void)cudaGetLastError();
+        }
+    }
     const float wmed = (float)(weight[K / 2] > 0 ? weight[K / 2] : 1);  // the list is sorted by weight
     const GenGraph gg = graph_of(g);
     const int wgrid = (int)std::min<long long>((K + kWalkThreads - 1) / kWalkThreads, (long long)g->sm_count * 16);
     walk_kernel<<<wgrid, kWalkThreads, 0, st>>>(gg, g->d_pedge, K, g->d_tree, g->d_eoff, g->d_len, nullptr, nullptr,
-                                                g->d_status, features, g->d_weight, wmed);
+                                                g->d_status, features, g->d_weight, wmed,
+                                                g->ordered ? reinterpret_cast<const int32_t *>(g->d_order) : nullptr, K);
     MCB_CUDA(cudaGetLastError());
     return check_status(g, st, "mcbgpu_gen_rank");
 }
@@ -1133,9 +1193,11 @@ int mcbgpu_gen_build_lists(mcbgpu_gen *g, int64_t K_keep, int64_t *nnz, void *st
     if (rc) return rc;
     MCB_CUDA(keep_room(g->d_coords, g->cap_coords, 4 * (total > 0 ? total : 1)));
     const GenGraph gg = graph_of(g);
-    const int wgrid = (int)std::min<long long>((K + kWalkThreads - 1) / kWalkThreads, (long long)g->sm_count * 16);
+    const int32_t *order = g->ordered ? reinterpret_cast<const int32_t *>(g->d_order) : nullptr;
+    const int64_t walks = order ? g->K : K;  // the order is over all ranks
+    const int wgrid = (int)std::min<long long>((walks + kWalkThreads - 1) / kWalkThreads, (long long)g->sm_count * 16);
     walk_kernel<<<wgrid, kWalkThreads, 0, st>>>(gg, g->d_pedge, K, g->d_tree, g->d_eoff, g->d_len, g->d_off,
-                                                g->d_coords, g->d_status, nullptr, nullptr, 1.0f);
+                                                g->d_coords, g->d_status, nullptr, nullptr, 1.0f, order, walks);
     MCB_CUDA(cudaGetLastError());
     const unsigned long long cap_long = (unsigned long long)(K < 65536 ? K : 65536);
     MCB_CUDA(keep_room(g->d_longs, g->cap_longs, 8 * (int64_t)cap_long));
