@@ -113,7 +113,7 @@ int mcbgpu_struct_clear_memory(mcbgpu_struct *s);
  * initialize_memory (level_offsets F x (nodes+1), parent_pos and edge_offset
  * F x nodes), the map (num_edges), S (ceil(N/64) words); labels receives F x nodes
  * uint32 0/1.  Working memory is a static device array inside the library
- * (16 MiB of per-CTA label slabs + a status word) that every GPU loading the
+ * (16 MiB, the slots' bits or per-CTA label slabs, + a status word) that every GPU loading the
  * library keeps until exit; trees of more than 16 Mi vertices are rejected.  The
  * first call on a device looks up the array's device address (cudaGetSymbolAddress)
  * and should come before any stream capture.  Calls share the array: calls that
@@ -180,8 +180,8 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream);
  * after mcbgpu_solver_run.  Not with profiling on.  No counterpart in the reference
  * (its loop is host code). */
 int mcbgpu_solver_run_graph(mcbgpu_solver *s, int64_t max_iterations, void *stream);
-/* Per-iteration form over all iterations, enqueued without host synchronisation
- * (select + update per iteration). */
+/* Per-iteration form over all iterations, enqueued without host synchronisation, as one
+ * launch per iteration (select + update while profiling). */
 int mcbgpu_solver_run_plain(mcbgpu_solver *s, int64_t max_iterations, void *stream);
 /* Synchronises `stream`; copies selected[e] (rank chosen at iteration e) for the
  * iterations run, the 64-bit total weight, and checks the device status word. */
@@ -217,8 +217,8 @@ int mcbgpu_solver_kernel_stats(mcbgpu_solver *s, mcbgpu_kernel_stat *out, int ma
 int mcbgpu_solver_diagnostics(mcbgpu_solver *s, int64_t *out, int n, int reset);
 /* Search shapes of the blocked run (no counterpart in the reference, whose host scan
  * has no shape).  A shape sets the pivot search's window (W tiles a CTA scans per
- * step, by how many of the block's 64 pivots are known) and how far past the previous
- * two blocks' last pivots the W pass reaches.  Every shape gives the same result; only the time
+ * step, by how many of the block's 64 pivots are known) and how far past the mean of
+ * the previous two blocks' last pivots the W pass reaches.  Every shape gives the same result; only the time
  * differs.  A solve is cut into MCBGPU_SHAPE_SEGMENTS segments of 64-iteration
  * blocks, each with its own shape (candidate 0, the built-in default, until tuned).
  *
@@ -254,7 +254,8 @@ int mcbgpu_solve(int32_t num_coords, int64_t num_candidates, const int32_t *weig
 
 /* ---- 4. batched main loop ---------------------------------------------------
  * Many independent problems (the biconnected components of one graph, or many
- * graphs) in one persistent launch, one CTA per problem at a time.
+ * graphs) in up to four persistent launches (one per cluster size), a cluster of one to
+ * eight CTAs per problem at a time.
  * Replaces the reference's one-process-per-component loop (main.sh:19-32 runs the
  * whole mcb driver once per bicc component file); every problem's result equals
  * mcbgpu_solver_run's on the same inputs.
@@ -266,7 +267,8 @@ int mcbgpu_solve(int32_t num_coords, int64_t num_candidates, const int32_t *weig
  *   (each list ascending in [0, N_i) of its problem).  Synchronises `stream`: the
  *   offsets are checked on the device (MCBGPU_E_ARG if they are not non-decreasing
  *   from 0 to nnz).
- * run: enqueued on `stream` without host synchronisation.
+ * run: enqueued on `stream` without host synchronisation (classes of problems on
+ *   streams of the handle, forked from and joined to `stream`).
  * results: selected[sum N] (problem i's iterations at offset N_0 + ... + N_{i-1},
  *   each the candidate's rank within problem i), total_weight[count] (-1 for a
  *   problem that failed), problem_status[count] (0 = solved; may be NULL); returns

@@ -1,5 +1,5 @@
 // Batched de Pina solver: many independent problems (the biconnected components of
-// one graph, or many graphs) solved in one persistent launch.
+// one graph, or many graphs) solved in a persistent launch per cluster size.
 //
 // The reference solves one graph per process and, for a graph split into
 // biconnected components, runs the whole driver once per component file

@@ -54,7 +54,7 @@ constexpr int kPer = kTile / kScanThreads;
 constexpr unsigned kSpinLimit = 1u << 24;
 constexpr int kDiagWords = 48;  // counters of mcbgpu_solver_diagnostics (the pivot kernel's check area follows)
 // Shape parameters of the blocked search; each can be overridden at build time
-// (-DMCB_LMAX=... and so on) to sweep them.
+// (-DMCB_UPD_ROWS=... and so on) to sweep them.
 #ifndef MCB_UPD_ROWS
 #define MCB_UPD_ROWS 8
 #endif
@@ -82,9 +82,8 @@ constexpr int kGStride = kGroup == 3 ? 4 : kGroup;  // words per coordinate in t
 #endif
 constexpr int kMaxWin = 32;  // the largest window (tiles per CTA and step) a shape may use
 // The runtime shape of the blocked search (blk_pivot_kernel and the streaming pass's
-// reach).  Every shape gives the same pivots (the search is exact for any window
-// and local-pivot limit); only the time differs, by graph and by how far a solve has
-// got, so a solver can time several on its own graph (mcbgpu_solver_tune).
+// reach).  Every shape gives the same pivots (the search is exact for any window); only
+// the time differs, by graph and by how far a solve has got, so a solver can time several on its own graph (mcbgpu_solver_tune).
 struct PivotShape {
     int win_early, rank_early;  // tiles per CTA and step while fewer than rank_early pivots are known
                                 // (half of it where that does not reach the expected last pivot)
