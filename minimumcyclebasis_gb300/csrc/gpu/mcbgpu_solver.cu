@@ -56,7 +56,7 @@ constexpr int kDiagWords = 48;  // counters of mcbgpu_solver_diagnostics (the pi
 // Shape parameters of the blocked search; each can be overridden at build time
 // (-DMCB_UPD_ROWS=... and so on) to sweep them.
 #ifndef MCB_UPD_ROWS
-#define MCB_UPD_ROWS 8
+#define MCB_UPD_ROWS 4
 #endif
 #ifndef MCB_W_CHUNK
 #define MCB_W_CHUNK 8
@@ -74,7 +74,7 @@ constexpr int kGroup = MCB_GROUP;
 static_assert(kGroup >= 1 && kGroup <= 3, "MCB_GROUP must be 1, 2 or 3");
 constexpr int kGStride = kGroup == 3 ? 4 : kGroup;  // words per coordinate in the grouped transpose
 #ifndef MCB_UPD_SPLIT
-#define MCB_UPD_SPLIT 1  // warps per row group in the block update (1, 2, 4 or 8)
+#define MCB_UPD_SPLIT 2  // warps per row group in the block update (1, 2, 4 or 8)
 #endif
 
 #ifndef MCB_PDL
@@ -1838,20 +1838,21 @@ constexpr int kNzCap = MCB_NZ_CAP;
 constexpr uint16_t kDenseRow = 0xFFFFu;
 static_assert(kNzCap >= 2 && kNzCap < 0xFFFF, "MCB_NZ_CAP out of range");
 
-// D of a sparse far row from its word list: for each listed word that holds pairs
-// of this block, the row's word is read once and tested against them.  List entries
-// in batches of four (independent loads).
-__device__ __forceinline__ uint64_t sparse_D(const uint64_t *S, long long j, int P, unsigned cnt, const uint32_t *nzw,
+// The part of a sparse far row's D that falls to lane `sub` of kFarLanes, from its word
+// list: for each listed word that holds pairs of this block, the row's word is read once
+// and tested against them.  List entries in batches of four per lane (independent loads).
+constexpr int kFarLanes = 4;
+__device__ __forceinline__ uint64_t sparse_D(const uint64_t *S, long long j, int P, int sub, unsigned cnt, const uint32_t *nzw,
                                              const unsigned *__restrict__ word_end, const unsigned *__restrict__ pairs,
                                              unsigned long long &tests, unsigned long long &words) {
     const uint32_t *L = nzw + (size_t)j * kNzCap;
     const uint64_t *Sj = S + (size_t)j * P;
     uint64_t D = 0;
-    for (unsigned i = 0; i < cnt; i += 4) {
+    for (unsigned i = sub; i < cnt; i += 4 * kFarLanes) {
         uint32_t w[4];
         unsigned lo[4], hi[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) w[q] = i + q < cnt ? L[i + q] : 0xFFFFFFFFu;
+        for (int q = 0; q < 4; q++) w[q] = i + q * kFarLanes < cnt ? L[i + q * kFarLanes] : 0xFFFFFFFFu;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             lo[q] = w[q] != 0xFFFFFFFFu ? __ldg(word_end + w[q]) : 0u;
@@ -1921,7 +1922,8 @@ __global__ void __launch_bounds__(kUpdThreads) far_rows_kernel(const uint64_t *_
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long groups = (long long)gridDim.x * kUpdGroups;
     const bool dense_work = (long long)blockIdx.x * kUpdGroups * kUpdRows < (long long)ndense;
-    const bool sparse_work = (long long)blockIdx.x * kUpdThreads < (long long)nsparse + ntouch;
+    // the sparse rows go to the CTAs from the last on, the dense ones from the first on
+    const bool sparse_work = (long long)(gridDim.x - 1 - blockIdx.x) * (kUpdThreads / kFarLanes) < (long long)nsparse + ntouch;
     if (!dense_work && !sparse_work) return;  // CTA-uniform
     unsigned long long nb = 0, n_rows = 0, n_changed = 0, n_gather = 0, n_betabits = 0;
     unsigned long long n_sparse = 0, n_words = 0, n_tests = 0, n_swords = 0, n_touched = 0;
@@ -1991,32 +1993,46 @@ __global__ void __launch_bounds__(kUpdThreads) far_rows_kernel(const uint64_t *_
             n_betabits += (unsigned)__popcll(beta);
         }
     }
-    // sparse rows, then the touched unit rows, one per lane
-    const long long gw = (long long)blockIdx.x * (kUpdThreads / 32) + warp;
+    // sparse rows, then the touched unit rows, kFarLanes lanes each: a random graph's rows
+    // have up to 32 words, each a chain of three reads, and one row per lane left a few
+    // hundred warps with all of them: 97 -> 40 us per block of a 50k-vertex random graph, 192
+    // -> 167 ms per solve (with two warps per four dense rows 20 us; eight rows and one
+    // warp 39)
+    constexpr int kWarpRows = 32 / kFarLanes;
+    const int sub = lane % kFarLanes;
     const long long nwarps = (long long)gridDim.x * (kUpdThreads / 32);
+    const long long gw = nwarps - 1 - ((long long)blockIdx.x * (kUpdThreads / 32) + warp);
     const long long nall = (long long)nsparse + ntouch;
-    for (long long base = gw * 32; base < nall; base += nwarps * 32) {
-        const long long i = base + lane;
+    for (long long base = gw * kWarpRows; base < nall; base += nwarps * kWarpRows) {
+        const long long i = base + lane / kFarLanes;
         const bool touched = i >= (long long)nsparse && i < nall;
         long long j = -1;
         if (i < (long long)nsparse)
             j = __ldg(fl.sp_in + i);
         else if (touched)
             j = __ldg(fl.touch + (i - nsparse));
-        const bool keep = !touched && j >= row_begin;
+        bool keep = !touched && j >= row_begin;
         uint64_t D = 0;
         if (keep) {
             const unsigned cnt = fl.nzc[j];
-            D = sparse_D(S, j, P, cnt, fl.nzw, word_end, pairs, n_tests, n_swords);
-            n_sparse++;
-            n_words += cnt;
-            nb += 4ull + 2ull + 12ull * cnt;  // list entry, count, listed words + their two word_end entries
-        } else if (touched) {  // a unit row the scatter reached: D was scattered (never zero)
+            D = sparse_D(S, j, P, sub, cnt, fl.nzw, word_end, pairs, n_tests, n_swords);
+            if (sub == 0) {
+                n_sparse++;
+                n_words += cnt;
+                nb += 4ull + 2ull + 12ull * cnt;  // list entry, count, listed words + their two word_end entries
+            }
+        } else if (touched && sub == 0) {  // a unit row the scatter reached: D was scattered (never zero)
             D = Dfar[j];
             Dfar[j] = 0;  // ready for the next block
             unit[j] = 0;
             n_touched++;
             nb += 4ull + 16ull;
+        }
+#pragma unroll
+        for (int d = 1; d < kFarLanes; d <<= 1) D ^= __shfl_xor_sync(0xffffffffu, D, d);
+        if (sub != 0) {  // the row's first lane goes on
+            keep = false;
+            D = 0;
         }
         warp_append(keep && D == 0, (int32_t)j, fl.sp_out, fl.n_out);
         const uint64_t beta = D ? beta_of(D, gcol, b) : 0ull;
@@ -3198,13 +3214,13 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             const BlockState *wbs = s->d_bs;
             uint64_t *nul = nullptr;
             if (nl == 2)
-                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<3, true> : blk_w_kernel<3, false>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
+                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<3, true> : blk_w_kernel<3, false>, dim3(sms), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
                                   bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd2, Wpos[1], Wpos[2], cols));
             else if (nl == 1)
-                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<2, true> : blk_w_kernel<2, false>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
+                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<2, true> : blk_w_kernel<2, false>, dim3(sms), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
                                   bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd1, Wpos[1], nul, cols));
             else
-                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<1, true> : blk_w_kernel<1, false>, dim3(sms * 2), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
+                MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<1, true> : blk_w_kernel<1, false>, dim3(sms), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
                                   bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), (const uint64_t *)nullptr, 0, 0, nul,
                                   nul, cols));
         }
@@ -3290,11 +3306,14 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
                 far_scatter_kernel<<<sms * 2, 256, 0, s->st2>>>(pairs, wend, s->P, near_end, far_end, s->d_unit,
                                                                  s->d_Dfar, s->d_touch, s->d_fcnt + 4 * lout + 2,
                                                                  L.bytes());
-                // grid-stride over the listed rows: two CTAs per SM cover ~78k sparse rows per
-                // pass (a block lists ~12k at the 1M-vertex graph); more CTAs would mostly exit
-                far_rows_kernel<<<std::min(grid_for(far_end - near_end), sms * 2), kUpdThreads, 0, s->st2>>>(
+                // As many CTAs as help these two end early: the next search (whose CTAs need
+                // most of an SM's registers) and the next streaming pass (all of them) start
+                // on an SM only when theirs are gone.  50k-vertex random graph, ms per solve
+                // with 2 / 3 / 4 CTAs per SM here: 154 / 152 / 155; with 2 / 4 / 8 for the
+                // apply: 161 / 157 / 156.
+                far_rows_kernel<<<std::min(grid_for(far_end - near_end), sms * 3), kUpdThreads, 0, s->st2>>>(
                     s->d_S, near_end, s->P, b, gcol, pairs, wend, fl, s->d_Dfar, s->d_unit, L.bytes(), s->d_diag);
-                far_apply_kernel<<<sms * 2, kApplyThreads, 0, s->st2>>>(s->d_S, s->P, (int)e0, Wb, fl, L.bytes());
+                far_apply_kernel<<<sms * 8, kApplyThreads, 0, s->st2>>>(s->d_S, s->P, (int)e0, Wb, fl, L.bytes());
                 s->list_cur = lout;
             }
             if (wait_slot >= 0) MCB_CUDA(cudaStreamWaitEvent(st, s->ev_upd[wait_slot], 0));
