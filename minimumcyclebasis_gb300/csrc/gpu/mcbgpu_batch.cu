@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(kBThreads, kMinBlocks) batch_solve_kernel(
     const int gwarp = (int)crank * kBWarps + warp, nwarp = (int)csz * kBWarps;
     const unsigned full = 0xffffffffu;
 
+    cluster_sync();  // every CTA of the cluster has started: its shared memory may be written
     for (unsigned turn = 0;; turn ^= 1) {
         if (crank == 0 && tid == 0) {
             const int g = (int)atomicAdd(next, 1u);
