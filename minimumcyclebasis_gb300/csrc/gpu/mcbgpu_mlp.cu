@@ -151,12 +151,6 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas) mlp_forward_kernel(
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp == 0) tmem_alloc(&s_tmem, kTmemCols);
-    if (tid == 0) {
-        mbar_init(&bar, 1);
-        fence_mbar_init();
-    }
-    load_weights(sB, s_bw, w1, b1, w2);
     const int64_t ntiles = (count + kTileRows - 1) / kTileRows;
     // this thread's row of a tile: 16 bf16 = two 16-byte halves, loaded a tile ahead of
     // its staging
@@ -176,7 +170,15 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas) mlp_forward_kernel(
         *reinterpret_cast<uint4 *>(sA[b] + core_off(tid, 8)) = hi;
         fence_proxy_async_smem();  // generic-proxy writes -> visible to the tensor core
     };
+    // on its way while the weights are read (one tile per CTA, 60k candidates: 7.3 -> 6.6 us)
     load_row(blockIdx.x);
+    const float b2 = *b2p;
+    if (warp == 0) tmem_alloc(&s_tmem, kTmemCols);
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+    }
+    load_weights(sB, s_bw, w1, b1, w2);
     stage_row(0);
     load_row((int64_t)blockIdx.x + gridDim.x);
     tc_fence_before();
@@ -184,7 +186,6 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas) mlp_forward_kernel(
     tc_fence_after();
     if (warp == 0) tmem_relinquish();
     const uint32_t tmem = s_tmem;
-    const float b2 = *b2p;
     const uint64_t bdesc = smem_desc(sB, kLead, kStride);
     float4 bw[8];  // this thread's hidden units: 8g + 2 (lane mod 4) and the next
 #pragma unroll
