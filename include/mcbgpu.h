@@ -169,7 +169,8 @@ int mcbgpu_update(mcbgpu_solver *s, int32_t e, void *stream);
 
 /* Blocked form: iterations [0, min(max_iterations, N)) (max_iterations < 0: all),
  * enqueued on `stream` without host synchronisation.  Results via
- * mcbgpu_solver_results. */
+ * mcbgpu_solver_results.  The loop starts from the unit vectors: a handle that has
+ * run, or updated S, since its last upload or reset is reset first (on `stream`). */
 int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream);
 /* A complete solve (reset of S to the unit vectors, then the blocked run over
  * iterations [0, min(max_iterations, N))) as one CUDA graph, launched on `stream`.

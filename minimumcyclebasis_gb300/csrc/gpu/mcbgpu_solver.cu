@@ -2510,6 +2510,7 @@ struct mcbgpu_solver {
     unsigned *d_status = nullptr;
     unsigned *d_check = nullptr;   // [bad flags, longest list]
     bool uploaded = false;
+    bool fresh = false;              // as a reset leaves it: nothing has run or updated S since
     long long iters_run = 0;
     long long launches = 0;
     long long device_bytes = 0;
@@ -2869,6 +2870,7 @@ int mcbgpu_solver_reset(mcbgpu_solver *s, void *stream) {
         return MCBGPU_E_ARG;
     }
     cudaStream_t st = (cudaStream_t)stream;
+    s->fresh = false;
     if (s->N > 0) {
         int grid = s->sm_count > 0 ? s->sm_count * 4 : 256;
         {
@@ -2890,6 +2892,7 @@ int mcbgpu_solver_reset(mcbgpu_solver *s, void *stream) {
     s->list_cur = 0;
     MCB_CUDA(cudaGetLastError());
     s->iters_run = 0;
+    s->fresh = true;
     return MCBGPU_OK;
 }
 
@@ -3041,6 +3044,7 @@ int mcbgpu_update(mcbgpu_solver *s, int32_t e, void *stream) {
         return MCBGPU_E_ARG;
     }
     cudaStream_t st = (cudaStream_t)stream;
+    s->fresh = false;
     int rows = s->N - e - 1;
     int grid = (rows + 7) / 8;
     int cap = s->sm_count > 0 ? s->sm_count * 8 : 1024;
@@ -3077,6 +3081,7 @@ int mcbgpu_solver_run_plain(mcbgpu_solver *s, int64_t max_iterations, void *stre
     const int sms = s->sm_count > 0 ? s->sm_count : 64;
     const long long chunks = (s->K + kPlainThreads - 1) / kPlainThreads;
     const int grid = (int)std::min<long long>(std::max<long long>(chunks, (s->N + 7) / 8), (long long)sms * 4);
+    s->fresh = false;
     MCB_CUDA(cudaMemsetAsync(s->d_ring, 0xff, sizeof(PlainSlot) * 4, st));
     for (int64_t e = 0; e <= iters; e++) {
         const int search = e < iters ? 1 : 0;
@@ -3106,6 +3111,11 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
         set_error("mcbgpu_solver_run: candidates not uploaded");
         return MCBGPU_E_STATE;
     }
+    if (!s->fresh) {  // the loop starts at iteration 0, from the unit vectors
+        const int rc = mcbgpu_solver_reset(s, stream);
+        if (rc) return rc;
+    }
+    s->fresh = false;
     cudaStream_t caller = (cudaStream_t)stream;
     cudaStream_t st = s->st1;  // the critical path; joined back into the caller's stream at the end
     const int64_t iters = (max_iterations >= 0 && max_iterations < s->N) ? max_iterations : s->N;
@@ -3134,6 +3144,10 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
     MCB_CUDA(cudaEventRecord(s->ev_fork, caller));
     MCB_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
     MCB_CUDA(cudaStreamWaitEvent(s->st2, s->ev_fork, 0));
+    // a group clears the next group's counter of listed coordinates and appends to its own; the
+    // first one's is cleared here too, so that the list stays within its array when a caller's
+    // graph replays this run with no reset between
+    MCB_CUDA(cudaMemsetAsync(s->d_bs->nz_count, 0, sizeof s->d_bs->nz_count, st));
     struct FarRec {
         long long start;  // first row of the far update
         int slot;         // its event in ev_upd
@@ -3589,6 +3603,7 @@ int mcbgpu_solver_run_graph(mcbgpu_solver *s, int64_t max_iterations, void *stre
         s->gexec_launches = per;
         s->gexec_list_end = s->list_cur;  // the host state a replay ends in (the capture ran the loop once)
     }
+    s->fresh = false;
     MCB_CUDA(cudaGraphLaunch(s->gexec, (cudaStream_t)stream));
     s->launches += s->gexec_launches;
     s->list_cur = s->gexec_list_end;
