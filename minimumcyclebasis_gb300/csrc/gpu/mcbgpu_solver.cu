@@ -1783,8 +1783,8 @@ size_t pivot_smem_bytes(int G, int P) {
 // (coordinate, k) pairs, sorted by S word, and each pair is applied to all rows of
 // the group (independent gathers of neighbouring words); pairs whose word lies above
 // the group's last row are skipped (S_j has support [0, j]).  The warps' partial D's
-// meet in shared memory (two buffers by iteration parity, one named barrier per
-// group and iteration).  Then lane i computes, for row i of the group, beta_k =
+// meet in shared memory (two buffers in turn, one named barrier per group with a row
+// left).  Then lane i computes, for row i of the group, beta_k =
 // D_k ^ <beta_{<k}, gcol_k> (the sequential effect of the block's 64 updates); then
 // S_j ^= XOR_k beta_k S_{e0+k} through the tables, the group's warps split the
 // row's words.
@@ -1896,8 +1896,8 @@ __device__ __forceinline__ uint64_t sparse_D(const uint64_t *S, long long j, int
 // bits): the group's warps split the chosen cycles' (coordinate, k) pairs, sorted by
 // S word, and each pair is applied to all rows of the group (independent gathers);
 // pairs whose word lies above the group's last row are skipped (S_j has support [0,
-// j]).  The warps' partial D's meet in shared memory (two buffers by iteration
-// parity, one named barrier per group and iteration).  gcol, pairs and word_end are
+// j]).  The warps' partial D's meet in shared memory (two buffers in turn, one
+// named barrier per group with a row left).  gcol, pairs and word_end are
 // the block's (double-buffered by block parity, so the next block's tail can run
 // while these rows are updated).
 struct FarLists {
@@ -1931,7 +1931,7 @@ __global__ void __launch_bounds__(kUpdThreads) far_rows_kernel(const uint64_t *_
     const int gi = warp / kUpdSplit, h = warp % kUpdSplit;
     int par = 0;
     for (long long base = kUpdRows * ((long long)blockIdx.x * kUpdGroups + gi); base < (long long)ndense;
-         base += kUpdRows * groups, par ^= 1) {
+         base += kUpdRows * groups) {
         const int rows = (int)(((long long)ndense - base) < kUpdRows ? ((long long)ndense - base) : kUpdRows);
         // lane r < rows: its listed row, kept if still a far row
         const long long jr = lane < rows ? (long long)__ldg(fl.dn_in + base + lane) : -1;
@@ -1977,6 +1977,9 @@ __global__ void __launch_bounds__(kUpdThreads) far_rows_kernel(const uint64_t *_
 #pragma unroll
                 for (int q = 0; q < kUpdSplit; q++) Dmine ^= sD[par][gi][q][lane];
             }
+            // the buffers alternate with the barrier, not with the groups: after two groups with a
+            // dropped one between, one warp could write here what the other still reads
+            par ^= 1;
         }
         if (h != 0) continue;  // the group's first warp carries the rows over
         if (!keep) Dmine = 0;

@@ -1,0 +1,37 @@
+"""Rules of warp and barrier use that no run can show to be kept (a broken one goes wrong
+once in a long while), read off the kernels' sources."""
+import os
+import re
+
+from conftest import ROOT
+
+GPU = os.path.join(ROOT, "minimumcyclebasis_gb300", "csrc", "gpu")
+
+
+def kernel(file, name):
+    """The body of a function of a source file, without comments."""
+    text = open(os.path.join(GPU, file)).read()
+    text = re.sub(r"/\*.*?\*/", "", re.sub(r"//[^\n]*", "", text), flags=re.S)
+    at = text.index("{", text.index(name + "("))
+    depth = 0
+    for i in range(at, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[at:i + 1]
+    raise AssertionError(name)
+
+
+def test_far_rows_alternate_their_buffers_with_the_barrier():
+    """Two warps share a group's partial sums through sD[par] and one barrier per group
+    that has a row left.  A warp may pass the next barrier only after the other has
+    arrived there, so a buffer is safe to write again two barriers on: par has to change
+    with every barrier and with nothing else (a group without rows has no barrier)."""
+    body = kernel("mcbgpu_solver.cu", "far_rows_kernel")
+    changes = [m.start() for m in re.finditer(r"\bpar\s*(\^=|=(?!=)|\+\+|\+=)", body)]
+    assert body[changes[0] - 4:changes[0]] == "int " and len(changes) == 2
+    barrier = body.index("barrier.sync")
+    assert "barrier.sync" not in body[barrier + 1:]
+    between = body[barrier:changes[1]]
+    assert changes[1] > barrier and "continue" not in between and "break" not in between
+    # both in the block that the barrier's condition opens
+    assert between.count("}") == between.count("{")
