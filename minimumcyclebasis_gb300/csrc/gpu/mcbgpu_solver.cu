@@ -526,7 +526,11 @@ __global__ void __launch_bounds__(kPlainThreads) plain_kernel(
             for (int w = tid; w < we; w += kPlainThreads) fin[(size_t)(e & 1) * P + w] = s_S[w];
         PlainSlot *slot = ring + (e & 3);
         for (long long r0 = (long long)blockIdx.x * kPlainThreads; r0 < K; r0 += (long long)gridDim.x * kPlainThreads) {
-            if ((unsigned long long)r0 > *((volatile unsigned long long *)&slot->best)) break;  // nothing earlier is left here
+            // one lane looks for its whole warp: other CTAs lower the rank meanwhile, and lanes that
+            // saw different ranks would part here, before the ballot below
+            unsigned long long found = 0;
+            if (lane == 0) found = *((volatile unsigned long long *)&slot->best);
+            if ((unsigned long long)r0 > __shfl_sync(0xffffffffu, found, 0)) break;  // nothing earlier is left here
             const long long r = r0 + tid;
             unsigned par = 0;
             if (r < K) {

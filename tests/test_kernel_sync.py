@@ -35,3 +35,20 @@ def test_far_rows_alternate_their_buffers_with_the_barrier():
     assert changes[1] > barrier and "continue" not in between and "break" not in between
     # both in the block that the barrier's condition opens
     assert between.count("}") == between.count("{")
+
+
+def test_a_word_that_others_change_decides_for_whole_warps():
+    """A loop of warp collectives must not be left by each lane's own look at a word that
+    other CTAs change meanwhile: lanes that saw different values part, and those that stay
+    wait in the next collective for those that left.  Such a look is taken by one lane and
+    handed to the others."""
+    for file in sorted(os.listdir(GPU)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(GPU, file)).read())
+        for m in re.finditer(r"\bif \(([^;{}]*volatile[^;{}]*)\)\s*\{?\s*(break|continue|return)\b", text):
+            raise AssertionError((file, m.group(0)))
+    body = kernel("mcbgpu_solver.cu", "plain_kernel")
+    loop = body[body.index("for (long long r0"):]
+    look = re.search(r"if \(lane == 0\) (\w+) = \*\(\(volatile unsigned long long \*\)&slot->best\);", loop)
+    leave = re.search(r"if \(\(unsigned long long\)r0 > __shfl_sync\(0xffffffffu, (\w+), 0\)\) break;", loop)
+    assert look and leave and look.group(1) == leave.group(1) and look.end() < leave.start()
+    assert leave.end() < loop.index("__ballot_sync") and loop.count("slot->best") == 2  # the other: atomicMin
