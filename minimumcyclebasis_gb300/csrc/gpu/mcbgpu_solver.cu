@@ -988,8 +988,10 @@ __device__ __forceinline__ void w_by_columns(const Columns &co, const uint64_t *
         const unsigned part = it / n;
         const uint64_t *t = Tt + (size_t)kStride * c;
         const uint64_t x = t[0], y = kG > 1 ? t[kG > 1 ? 1 : 0] : 0ull, z = kG > 2 ? t[kG - 1] : 0ull;
-        const unsigned e = co.start[(size_t)c * co.segs + seg_end];
-        for (unsigned i = co.start[(size_t)c * co.segs] + part * 32 + lane; i < e; i += parts * 32) {
+        // 64 bits: a step past a column's end can pass 2^32 where the index nearly fills 32 bits
+        const unsigned long long e = co.start[(size_t)c * co.segs + seg_end];
+        for (unsigned long long i = co.start[(size_t)c * co.segs] + (unsigned long long)(part * 32 + lane); i < e;
+             i += parts * 32) {
             const unsigned r = __ldg(co.ranks + i);
             if ((long long)r >= limit) continue;
             if (x) atomicXor((unsigned long long *)W0 + r, (unsigned long long)x);
