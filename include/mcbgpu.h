@@ -336,7 +336,9 @@ int mcbgpu_trees_destroy(mcbgpu_trees *t);
  *   mcbgpu_gen_trees       the trees of FVS indices [t0, t0 + count); tied[i] = 1
  *                          where the host must search root t0 + i itself
  *                          (mcbh_search_trees), then hand its tree over with
- *   mcbgpu_gen_put_trees   (distances and parent slots, count x n', host memory);
+ *   mcbgpu_gen_put_trees   (distances and parent slots, count x n', host memory; a
+ *                          parent that is no slot of its vertex, or parents in a
+ *                          cycle, make mcbgpu_gen_candidates fail);
  *   mcbgpu_gen_candidates  the candidate test of the chunk: counts[i] candidates of
  *                          root t0 + i, *total for the chunk; then
  *   mcbgpu_gen_fetch       their pair indices (ascending per root, roots in order)

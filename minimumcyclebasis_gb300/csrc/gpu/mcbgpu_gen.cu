@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "mcbgpu_sssp.cuh"
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(kCodeThreads) branch_test_kernel(GenGraph g, c
             }
             done = cta_sync_and(!open);
         }
-        if (!done && tid == 0) atomicOr(status, ST_BAD_INPUT);  // a parent cycle
+        if (!done && tid == 0) atomicOr(status, ST_BAD_INPUT);  // deeper than any tree of checked parents
         int cnt = 0;
         uint32_t *bw = bits + (size_t)r * words_per_root;
         for (int wi = warp; wi < words; wi += kCodeThreads / 32) {
@@ -166,6 +167,47 @@ __global__ void __launch_bounds__(kCodeThreads) branch_test_kernel(GenGraph g, c
             counts[r] = sum;
         }
         cta_sync();
+    }
+}
+
+// Host-made parents (mcbgpu_gen_put_trees), one CTA per tree: each vertex's chain must reach
+// the root.  The jumps above do not show that: a vertex of a parent cycle may come to point
+// to itself, as a branch does, or to a blocking vertex of its cycle, and then stands.  Here
+// only the root stands, so a cycle stays open.  The device's own parents lie nearer to the
+// root than their children and are not checked.  Slots that are no parent's are left to
+// first_pointer().
+template <bool kShared>
+__global__ void __launch_bounds__(kCodeThreads) put_check_kernel(GenGraph g, const int32_t *__restrict__ pedge,
+                                                                 const int32_t *__restrict__ trees, int count, int t0,
+                                                                 int32_t *code, unsigned *status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    using Ptr = typename std::conditional<kShared, uint16_t, int32_t>::type;
+    const int n = g.n;
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
+        const int t = trees[i];
+        const uint32_t src = g.roots[t];
+        const int32_t *pe = pedge + (size_t)t * n;
+        volatile Ptr *J = kShared ? reinterpret_cast<volatile Ptr *>(smem)
+                                  : reinterpret_cast<volatile Ptr *>(code + (size_t)(t - t0) * n);
+        for (int v = threadIdx.x; v < n; v += blockDim.x) {
+            const int32_t o = (uint32_t)v == src ? -1 : pe[v];
+            J[v] = (Ptr)(o >= 0 && (int64_t)o < g.slots ? __ldg(g.slot_info + o).x : src);
+        }
+        cta_sync();
+        bool done = false;
+        for (int round = 0; round < kJumpRounds && !done; round++) {
+            bool open = false;
+            for (int v = threadIdx.x; v < n; v += blockDim.x) {
+                const Ptr p = J[v];
+                if ((uint32_t)p == src) continue;
+                const Ptr y = J[p];
+                J[v] = y;
+                open |= (uint32_t)y != src;
+            }
+            done = cta_sync_and(!open);
+        }
+        if (!done && threadIdx.x == 0) atomicOr(status, ST_BAD_INPUT);
+        cta_sync();  // the pointers are the next tree's
     }
 }
 
@@ -198,7 +240,7 @@ __global__ void __launch_bounds__(kCodeThreads) codes_kernel(GenGraph g, const i
             }
             done = cta_sync_and(!open);
         }
-        if (!done && threadIdx.x == 0) atomicOr(status, ST_BAD_INPUT);  // a parent cycle
+        if (!done && threadIdx.x == 0) atomicOr(status, ST_BAD_INPUT);  // deeper than any tree of checked parents
         cta_sync();
     }
 }
@@ -637,6 +679,7 @@ struct mcbgpu_gen {
     int32_t *d_pedge = nullptr;  // F x n, resident
     int32_t *d_dist = nullptr;   // chunk x n
     int32_t *d_code = nullptr;   // chunk x n (without branch_shared)
+    int32_t *d_put = nullptr;    // chunk: the trees a call of mcbgpu_gen_put_trees brings
     uint4 *d_slot_info = nullptr;
     uint32_t *d_pair_ends = nullptr;
     bool branch_shared = false;  // branch_test_kernel
@@ -698,7 +741,7 @@ static void gen_free(mcbgpu_gen *g) {
     }
     cudaFree(g->d_dist_slot[1]);  // slot 0's distances are d_dist
     void *ps[] = {g->d_arcs, g->d_ro,   g->d_rows,    g->d_cols,   g->d_rev,    g->d_pairs,  g->d_roots,  g->d_w,
-                  g->d_ec,   g->d_fvs,     g->d_pedge,  g->d_dist_slot[0], g->d_code, g->d_slot_info, g->d_pair_ends, g->d_bits,
+                  g->d_ec,   g->d_fvs,     g->d_pedge,  g->d_dist_slot[0], g->d_code, g->d_slot_info, g->d_pair_ends, g->d_put, g->d_bits,
                   g->d_gdist, g->d_next,   g->d_gdirty, g->d_gsumm, g->d_tied,   g->d_counts, g->d_coff,   g->d_cpair,
                   g->d_cweight, g->d_nlong, g->d_status};
     for (void *p : ps) cudaFree(p);
@@ -839,6 +882,7 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     GALLOC(g->d_dist, 4 * n * C);
     g->d_dist_slot[0] = g->d_dist;
     GALLOC(g->d_slot_info, sizeof(uint4) * (size_t)slots);
+    GALLOC(g->d_put, 4 * C);
     g->branch_shared = nodes <= kBranchMaxN && branch_smem_bytes(nodes, npairs) <= kBranchSmemMax;
     if (g->branch_shared)
         GALLOC(g->d_pair_ends, 4 * (size_t)npairs);
@@ -905,6 +949,8 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     if (e == cudaSuccess) e = set_trees_smem_limit();
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(branch_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBranchSmemMax);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(put_check_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kBranchMaxN);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(sort_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(int32_t) * kSortLongMax));
@@ -1027,18 +1073,33 @@ int mcbgpu_gen_put_trees(mcbgpu_gen *g, const int32_t *trees, int32_t count, con
         set_error("mcbgpu_gen_put_trees: invalid arguments");
         return MCBGPU_E_ARG;
     }
+    for (int32_t i = 0; i < count; i++)
+        if (trees[i] < g->cur_t0 || trees[i] >= g->cur_t0 + g->cur_count) {
+            set_error("mcbgpu_gen_put_trees: tree %d is not in the current chunk", (int)trees[i]);
+            return MCBGPU_E_ARG;
+        }
     cudaStream_t st = (cudaStream_t)stream;
     const size_t n = (size_t)g->n;
     for (int32_t i = 0; i < count; i++) {
         const int32_t t = trees[i];
-        if (t < g->cur_t0 || t >= g->cur_t0 + g->cur_count) {
-            set_error("mcbgpu_gen_put_trees: tree %d is not in the current chunk", (int)t);
-            return MCBGPU_E_ARG;
-        }
         MCB_CUDA(cudaMemcpyAsync(g->d_dist + (size_t)(t - g->cur_t0) * n, dist + (size_t)i * n, 4 * n,
                                  cudaMemcpyHostToDevice, st));
         MCB_CUDA(cudaMemcpyAsync(g->d_pedge + (size_t)t * n, parent_slot + (size_t)i * n, 4 * n,
                                  cudaMemcpyHostToDevice, st));
+    }
+    // a bad tree is reported with the candidates (device status)
+    const GenGraph gg = graph_of(g);
+    for (int32_t at = 0; at < count; at += g->chunk) {
+        const int32_t some = count - at < g->chunk ? count - at : g->chunk;
+        const int grid = some < g->sm_count * 2 ? some : g->sm_count * 2;
+        MCB_CUDA(cudaMemcpyAsync(g->d_put, trees + at, 4 * (size_t)some, cudaMemcpyHostToDevice, st));
+        if (g->n <= kBranchMaxN)
+            put_check_kernel<true><<<grid, kCodeThreads, 2 * n, st>>>(gg, g->d_pedge, g->d_put, some, g->cur_t0, nullptr,
+                                                                      g->d_status);
+        else
+            put_check_kernel<false><<<grid, kCodeThreads, 0, st>>>(gg, g->d_pedge, g->d_put, some, g->cur_t0, g->d_code,
+                                                                   g->d_status);
+        MCB_CUDA(cudaGetLastError());
     }
     MCB_CUDA(cudaStreamSynchronize(st));
     return MCBGPU_OK;
