@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas) mlp_forward_kernel(
         load_row(next + gridDim.x);
         ok = mbar_wait_bounded(&bar, phase, 1u << 22);
         phase ^= 1u;
+        __syncwarp();  // lanes leave the polls one by one; the aligned read wants the warp whole
         tc_fence_after();
         float z[4];  // candidates 32 warp + 8 i + lane / 4: the part of this thread's hidden units
         uint32_t acc[32];

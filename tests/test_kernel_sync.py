@@ -52,3 +52,14 @@ def test_a_word_that_others_change_decides_for_whole_warps():
     leave = re.search(r"if \(\(unsigned long long\)r0 > __shfl_sync\(0xffffffffu, (\w+), 0\)\) break;", loop)
     assert look and leave and look.group(1) == leave.group(1) and look.end() < leave.start()
     assert leave.end() < loop.index("__ballot_sync") and loop.count("slot->best") == 2  # the other: atomicMin
+
+
+def test_a_warp_is_whole_before_it_reads_tensor_memory():
+    """tcgen05.ld is a warp-aligned instruction and a thread leaves the mbarrier's polls by
+    itself, so a barrier of the warp or of the CTA stands between."""
+    for name in ("mlp_forward_kernel", "mlp_grads_kernel"):
+        body = kernel("mcbgpu_mlp.cu", name)
+        loop = body[body.index("for (int64_t tile"):]
+        wait = loop.index("mbar_wait_bounded(")
+        read = loop.index("tmem_ld", wait)
+        assert re.search(r"__syncwarp\(\)|cta_sync(_and)?\(", loop[wait:read]), name
