@@ -177,7 +177,8 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream);
  * The first call (and the first after a tuning run, a shape change or another
  * max_iterations) captures the solve on a stream of the handle and instantiates it;
  * later calls replay it.  The graph reads the handle's buffers, so a new upload
- * (same sizes) is solved by the same graph.  Results via mcbgpu_solver_results, as
+ * (same sizes) is solved by the same graph, unless it has a longer list than any
+ * before: then the next call captures again.  Results via mcbgpu_solver_results, as
  * after mcbgpu_solver_run.  Not with profiling on.  No counterpart in the reference
  * (its loop is host code). */
 int mcbgpu_solver_run_graph(mcbgpu_solver *s, int64_t max_iterations, void *stream);

@@ -2938,6 +2938,7 @@ static int solver_upload(mcbgpu_solver *s, const int32_t *weight, const int64_t 
     s->max_len = (int)chk[1];
     unsigned cap = (unsigned)(64 * (size_t)(s->max_len > 0 ? s->max_len : 1));
     if (cap > s->pair_cap) {  // resolve scratch + sorted pairs of the two block parities
+        drop_graph(s);  // it holds the old buffer and its size
         cudaFree(s->d_pairs);
         s->d_pairs = nullptr;
         MCB_CUDA(cudaMalloc((void **)&s->d_pairs, sizeof(unsigned) * 3 * (size_t)cap));
