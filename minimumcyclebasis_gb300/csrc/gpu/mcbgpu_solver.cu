@@ -2477,9 +2477,10 @@ struct mcbgpu_solver {
     uint64_t *d_Warr3 = nullptr;   // W of a group's third block
     uint64_t *d_Tg = nullptr;      // the group's blocks' rows transposed, kGStride words per coordinate
     // column index (coordinate -> ranks); absent (segs = 0) when a size needs more than 32 bits or
-    // the memory is not there
+    // the memory is short (columns_alloc, must_alloc)
     unsigned *d_colstart = nullptr, *d_colranks = nullptr, *d_colsums = nullptr;
     int col_segs = 0, col_shift = 0;
+    long long col_bytes = 0;
     int32_t *d_nz = nullptr;       // 64 P: the coordinates whose T (Tg) words are not all zero
     uint64_t *d_beta = nullptr;    // 3 x 192: update bits of the near rows of a group's first blocks
     unsigned long long *d_nearD = nullptr;  // 2 x kNearMaxRows: D of the near rows by block parity (zero between uses)
@@ -2706,6 +2707,84 @@ void free_solver(mcbgpu_solver *s) {
     delete s;
 }
 
+// The column index (three arrays), made for a handle that has everything else it needs.  It
+// only saves time, so it takes at most a quarter of the memory that is free by then: the
+// certificate's matrix, the pair buffers of a later upload and other handles find room as
+// they would without it.
+void columns_alloc(mcbgpu_solver *s) {
+    if (s->N <= 0 || s->nnz <= 0 || s->nnz >= 0xffffffffll || s->K >= 0xffffffffll) return;
+    // at most kColKeys keys; segments of a power-of-two number of ranks, whole tiles
+    const long long want = std::max<long long>(1, std::min<long long>(kColSegs, kColKeys / s->N));
+    int shift = 10;
+    while (((s->K - 1) >> shift) >= want) shift++;
+    const int segs = (int)((s->K - 1) >> shift) + 1;
+    const size_t keys = (size_t)s->N * segs;
+    const size_t sums = (keys + (size_t)kScanCta * kScanItems - 1) / ((size_t)kScanCta * kScanItems) + 1;
+    const size_t need = sizeof(unsigned) * ((size_t)s->nnz + keys + 1 + sums);
+    size_t room = 0, all = 0;
+    cudaError_t e = cudaMemGetInfo(&room, &all);
+    if (e == cudaSuccess && need > room / 4) return;  // W comes from the lists then
+    if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_colranks, sizeof(unsigned) * (size_t)s->nnz);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_colstart, sizeof(unsigned) * (keys + 1));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_colsums, sizeof(unsigned) * sums);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        cudaFree(s->d_colranks);
+        cudaFree(s->d_colstart);
+        s->d_colranks = s->d_colstart = nullptr;
+        return;
+    }
+    s->col_shift = shift;
+    s->col_segs = segs;
+    s->col_bytes = (long long)need;
+    s->device_bytes += s->col_bytes;
+}
+
+// Gives the index back (the solve's graph may use it); false if there is none.
+bool columns_drop(mcbgpu_solver *s) {
+    if (s->col_segs == 0) return false;
+    drop_graph(s);
+    cudaFree(s->d_colranks);
+    cudaFree(s->d_colstart);
+    cudaFree(s->d_colsums);
+    s->d_colranks = s->d_colstart = s->d_colsums = nullptr;
+    s->col_segs = 0;
+    s->device_bytes -= s->col_bytes;
+    s->col_bytes = 0;
+    return true;
+}
+
+// cudaMalloc of what a call cannot do without: the index makes room where there is none.
+template <typename T>
+cudaError_t must_alloc(mcbgpu_solver *s, T **p, size_t bytes) {
+    cudaError_t e = cudaMalloc((void **)p, bytes);
+    if (e == cudaErrorMemoryAllocation && columns_drop(s)) {
+        (void)cudaGetLastError();
+        e = cudaMalloc((void **)p, bytes);
+    }
+    return e;
+}
+
+// The index of the uploaded lists, enqueued on st.
+int columns_build(mcbgpu_solver *s, cudaStream_t st) {
+    if (s->col_segs == 0) return MCBGPU_OK;
+    const long long keys = (long long)s->N * s->col_segs;
+    const int cgrid = (int)std::min<long long>((s->K * kColLanes + kColThreads - 1) / kColThreads,
+                                               (long long)(s->sm_count > 0 ? s->sm_count : 148) * 8);
+    const unsigned sgrid = (unsigned)((keys + (long long)kScanCta * kScanItems - 1) / ((long long)kScanCta * kScanItems));
+    Launch L(s, KC_VALIDATE, st, 5);
+    MCB_CUDA(cudaMemsetAsync(s->d_colstart, 0, sizeof(unsigned) * (size_t)(keys + 1), st));
+    columns_kernel<false><<<cgrid, kColThreads, 0, st>>>(s->d_off, s->d_coords, s->K, s->col_segs, s->col_shift,
+                                                         s->d_colstart, nullptr);
+    scan_sums_kernel<<<sgrid, kScanCta, 0, st>>>(s->d_colstart + 1, keys, s->d_colsums);
+    scan_top_kernel<<<1, kScanCta, 0, st>>>(s->d_colsums, (int)sgrid);
+    scan_items_kernel<<<sgrid, kScanCta, 0, st>>>(s->d_colstart + 1, keys, s->d_colsums);
+    columns_kernel<true><<<cgrid, kColThreads, 0, st>>>(s->d_off, s->d_coords, s->K, s->col_segs, s->col_shift,
+                                                        s->d_colstart, s->d_colranks);
+    MCB_CUDA(cudaGetLastError());
+    return MCBGPU_OK;
+}
+
 int check_status(mcbgpu_solver *s, cudaStream_t st) {
     unsigned v = 0;
     MCB_CUDA(cudaMemcpyAsync(&v, s->d_status, sizeof v, cudaMemcpyDeviceToHost, st));
@@ -2808,28 +2887,6 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
     if (e == cudaSuccess) e = cudaMemset(s->d_unit, 1, (size_t)N > 0 ? (size_t)N : 16);
     if (e == cudaSuccess) e = cudaMemset(s->d_fcnt, 0, sizeof(unsigned) * 8);
     if (e == cudaSuccess) e = cudaMemset(s->d_word_end, 0, sizeof(unsigned) * 2 * ((size_t)s->P + 1));
-    if (e == cudaSuccess && N > 0 && nnz > 0 && nnz < 0xffffffffll && K < 0xffffffffll) {
-        // at most kColKeys keys; segments of a power-of-two number of ranks, whole tiles
-        const long long want = std::max<long long>(1, std::min<long long>(kColSegs, kColKeys / N));
-        int shift = 10;
-        while (((K - 1) >> shift) >= want) shift++;
-        s->col_shift = shift;
-        s->col_segs = (int)((K - 1) >> shift) + 1;
-        const size_t keys = (size_t)N * s->col_segs;
-        const size_t sums = (keys + (size_t)kScanCta * kScanItems - 1) / ((size_t)kScanCta * kScanItems) + 1;
-        cudaError_t ec = cudaMalloc((void **)&s->d_colranks, sizeof(unsigned) * (size_t)nnz);
-        if (ec == cudaSuccess) ec = cudaMalloc((void **)&s->d_colstart, sizeof(unsigned) * (keys + 1));
-        if (ec == cudaSuccess) ec = cudaMalloc((void **)&s->d_colsums, sizeof(unsigned) * sums);
-        if (ec == cudaSuccess) {
-            bytes += (long long)(sizeof(unsigned) * ((size_t)nnz + keys + 1 + sums));
-        } else {  // the streaming pass does without
-            (void)cudaGetLastError();
-            cudaFree(s->d_colranks);
-            cudaFree(s->d_colstart);
-            s->d_colranks = s->d_colstart = nullptr;
-            s->col_segs = 0;
-        }
-    }
     // the far update fills every SM when it runs; with the critical path (transpose,
     // streaming pass, pivot search, near update) on a higher-priority stream, the
     // block scheduler gives that path's CTAs the SMs as they free up
@@ -2869,6 +2926,7 @@ int mcbgpu_solver_create(mcbgpu_solver **out, int32_t N, int64_t K, int64_t nnz)
         return cuda_fail(e, "mcbgpu_solver_create");
     }
     s->device_bytes = bytes;
+    columns_alloc(s);
     *out = s;
     return MCBGPU_OK;
 }
@@ -2941,7 +2999,8 @@ static int solver_upload(mcbgpu_solver *s, const int32_t *weight, const int64_t 
         drop_graph(s);  // it holds the old buffer and its size
         cudaFree(s->d_pairs);
         s->d_pairs = nullptr;
-        MCB_CUDA(cudaMalloc((void **)&s->d_pairs, sizeof(unsigned) * 3 * (size_t)cap));
+        s->pair_cap = 0;
+        MCB_CUDA(must_alloc(s, &s->d_pairs, sizeof(unsigned) * 3 * (size_t)cap));
         s->device_bytes += (long long)sizeof(unsigned) * 3 * cap;
         s->pair_cap = cap;
     }
@@ -2959,22 +3018,8 @@ static int solver_upload(mcbgpu_solver *s, const int32_t *weight, const int64_t 
         }
         MCB_CUDA(cudaGetLastError());
     }
-    if (s->col_segs > 0) {
-        const long long keys = (long long)s->N * s->col_segs;
-        const int cgrid = (int)std::min<long long>((s->K * kColLanes + kColThreads - 1) / kColThreads,
-                                                   (long long)(s->sm_count > 0 ? s->sm_count : 148) * 8);
-        const unsigned sgrid = (unsigned)((keys + (long long)kScanCta * kScanItems - 1) / ((long long)kScanCta * kScanItems));
-        Launch L(s, KC_VALIDATE, st, 5);
-        MCB_CUDA(cudaMemsetAsync(s->d_colstart, 0, sizeof(unsigned) * (size_t)(keys + 1), st));
-        columns_kernel<false><<<cgrid, kColThreads, 0, st>>>(s->d_off, s->d_coords, s->K, s->col_segs, s->col_shift,
-                                                             s->d_colstart, nullptr);
-        scan_sums_kernel<<<sgrid, kScanCta, 0, st>>>(s->d_colstart + 1, keys, s->d_colsums);
-        scan_top_kernel<<<1, kScanCta, 0, st>>>(s->d_colsums, (int)sgrid);
-        scan_items_kernel<<<sgrid, kScanCta, 0, st>>>(s->d_colstart + 1, keys, s->d_colsums);
-        columns_kernel<true><<<cgrid, kColThreads, 0, st>>>(s->d_off, s->d_coords, s->K, s->col_segs, s->col_shift,
-                                                            s->d_colstart, s->d_colranks);
-        MCB_CUDA(cudaGetLastError());
-    }
+    int rc = columns_build(s, st);
+    if (rc) return rc;
     s->uploaded = true;
     return mcbgpu_solver_reset(s, stream);
 }
@@ -3422,8 +3467,9 @@ int mcbgpu_solver_verify(mcbgpu_solver *s, int64_t *violations, int64_t *first_b
     if (s->N == 0) return MCBGPU_OK;
     unsigned long long *C = nullptr, *cnt = nullptr;
     const size_t cbytes = sizeof(unsigned long long) * (size_t)s->N * s->P;
-    cudaError_t e = cudaMalloc((void **)&C, cbytes);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&cnt, 2 * sizeof(unsigned long long));
+    const bool indexed = s->col_segs > 0;
+    cudaError_t e = must_alloc(s, &C, cbytes);
+    if (e == cudaSuccess) e = must_alloc(s, &cnt, 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(C, 0, cbytes, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt + 1, 0xff, sizeof(unsigned long long), st);
@@ -3443,6 +3489,11 @@ int mcbgpu_solver_verify(mcbgpu_solver *s, int64_t *violations, int64_t *first_b
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaFree(C);
     cudaFree(cnt);
+    if (indexed && s->col_segs == 0) {  // it made room for the matrix
+        columns_alloc(s);
+        rc = columns_build(s, st);
+        if (rc) return rc;
+    }
     if (e != cudaSuccess) return cuda_fail(e, "mcbgpu_solver_verify");
     rc = check_status(s, st);
     if (rc) return rc;
