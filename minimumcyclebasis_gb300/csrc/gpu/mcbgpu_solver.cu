@@ -602,6 +602,9 @@ __global__ void cycle_vector_kernel(uint64_t *C, int W, const int64_t *__restric
 // slot 0 = T[c], slot j = bit k of S[e0+64j+k] bit c (the group's j-th later block's
 // bj rows as they are now), for the words of the group's last block (a row is zero
 // beyond its own word), and lists the coordinates whose words are not all zero.
+// (The list starts empty behind a reset, and holds each coordinate once.  In a caller's own
+// graph of a run, replayed with no reset between, an old count may be left: the list then
+// still ends with its array of 64 P entries.)
 //
 // How the group's W will be formed is decided here, from the previous group's list:
 // while fewer than 1 / kColumnShare of the coordinates are listed, from the column
@@ -716,9 +719,10 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
             unsigned at = 0;
             if (lane == 0 && (lo | hi)) at = atomicAdd(&bs->nz_count[ga.slot], (unsigned)(__popc(lo) + __popc(hi)));
             at = __shfl_sync(0xffffffffu, at, 0);
-            const unsigned below = (1u << lane) - 1u;
-            if (nx) ga.nz[at + __popc(lo & below)] = (int32_t)c0;
-            if (ny) ga.nz[at + __popc(lo) + __popc(hi & below)] = (int32_t)c1;
+            const unsigned below = (1u << lane) - 1u, cap = 64u * (unsigned)P;
+            const unsigned px = at + __popc(lo & below), py = at + __popc(lo) + __popc(hi & below);
+            if (nx && px < cap) ga.nz[px] = (int32_t)c0;
+            if (ny && py < cap) ga.nz[py] = (int32_t)c1;
         }
     }
 }
@@ -971,6 +975,7 @@ struct Columns {
     const unsigned *start;  // (N x segs) + 1
     const unsigned *ranks;
     const int32_t *nz;
+    unsigned nz_cap;
     int segs, seg_shift, slot;
 };
 
@@ -1024,7 +1029,8 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
     const long long ntiles = bs->pred_tiles;
     unsigned long long nb = (blockIdx.x == 0 && threadIdx.x == 0) ? 8ull * (unsigned long long)bound : 0ull;
     if (bs->by_columns) {
-        w_by_columns<kG>(co, kG > 1 ? Tg : T, bs->nz_count[co.slot], min(ntiles * kTile, K), Warr, Wl1, Wl2);
+        w_by_columns<kG>(co, kG > 1 ? Tg : T, min(bs->nz_count[co.slot], co.nz_cap), min(ntiles * kTile, K), Warr, Wl1,
+                         Wl2);
         for (long long t = blockIdx.x + (long long)threadIdx.x * gridDim.x; t < ntiles;
              t += (long long)blockDim.x * gridDim.x)
             tile_epoch[t] = (epoch << 1) | (tile_minc[t] >= bound ? 1u : 0u);
@@ -3199,10 +3205,6 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
     MCB_CUDA(cudaEventRecord(s->ev_fork, caller));
     MCB_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
     MCB_CUDA(cudaStreamWaitEvent(s->st2, s->ev_fork, 0));
-    // a group clears the next group's counter of listed coordinates and appends to its own; the
-    // first one's is cleared here too, so that the list stays within its array when a caller's
-    // graph replays this run with no reset between
-    MCB_CUDA(cudaMemsetAsync(s->d_bs->nz_count, 0, sizeof s->d_bs->nz_count, st));
     struct FarRec {
         long long start;  // first row of the far update
         int slot;         // its event in ev_upd
@@ -3234,6 +3236,7 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
         cols.start = s->d_colstart;
         cols.ranks = s->d_colranks;
         cols.nz = s->d_nz;
+        cols.nz_cap = 64u * (unsigned)s->P;
         cols.segs = s->col_segs;
         cols.seg_shift = s->col_shift;
         cols.slot = ga.slot;
