@@ -708,16 +708,37 @@ struct mcbgpu_gen {
     long long diverged_runs = 0;
 };
 
+template <typename T>
+static void drop_room(T *&p, int64_t &cap) {
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+}
+
 // Room for `need` bytes in *p (contents are lost when it grows).
 template <typename T>
 static cudaError_t keep_room(T *&p, int64_t &cap, int64_t need) {
     if (need <= cap) return cudaSuccess;
-    cudaFree(p);
-    p = nullptr;
-    cap = 0;
+    drop_room(p, cap);
     const cudaError_t e = cudaMalloc((void **)&p, (size_t)need);
     if (e == cudaSuccess) cap = need;
     return e;
+}
+
+// Room for what a ranking cannot do without.  Where the memory is short, the walks' order and
+// (`all`, before a new ranking) the former lists are given back for it.
+template <typename T>
+static cudaError_t must_room(mcbgpu_gen *g, T *&p, int64_t &cap, int64_t need, bool all) {
+    cudaError_t e = keep_room(p, cap, need);
+    if (e != cudaErrorMemoryAllocation) return e;
+    (void)cudaGetLastError();
+    drop_room(g->d_order, g->cap_order);
+    g->ordered = false;
+    if (all) {
+        drop_room(g->d_coords, g->cap_coords);
+        drop_room(g->d_longs, g->cap_longs);
+    }
+    return keep_room(p, cap, need);
 }
 
 static void gen_free_lists(mcbgpu_gen *g) {
@@ -1179,12 +1200,12 @@ int mcbgpu_gen_rank(mcbgpu_gen *g, int64_t K, const int32_t *tree, const int32_t
     g->nnz = 0;
     const int64_t k1 = K > 0 ? K : 1;
     const int64_t nblk = (K + (int64_t)kScanThreads * kScanItems - 1) / ((int64_t)kScanThreads * kScanItems);
-    MCB_CUDA(keep_room(g->d_tree, g->cap_tree, 4 * k1));
-    MCB_CUDA(keep_room(g->d_eoff, g->cap_eoff, 4 * k1));
-    MCB_CUDA(keep_room(g->d_len, g->cap_len, 4 * k1));
-    MCB_CUDA(keep_room(g->d_weight, g->cap_weight, 4 * k1));
-    MCB_CUDA(keep_room(g->d_off, g->cap_off, 8 * (K + 1)));
-    MCB_CUDA(keep_room(g->d_bsum, g->cap_bsum, 8 * (nblk + 1)));
+    MCB_CUDA(must_room(g, g->d_tree, g->cap_tree, 4 * k1, true));
+    MCB_CUDA(must_room(g, g->d_eoff, g->cap_eoff, 4 * k1, true));
+    MCB_CUDA(must_room(g, g->d_len, g->cap_len, 4 * k1, true));
+    MCB_CUDA(must_room(g, g->d_weight, g->cap_weight, 4 * k1, true));
+    MCB_CUDA(must_room(g, g->d_off, g->cap_off, 8 * (K + 1), true));
+    MCB_CUDA(must_room(g, g->d_bsum, g->cap_bsum, 8 * (nblk + 1), true));
     g->ranked = true;
     if (K == 0) return MCBGPU_OK;
     MCB_CUDA(cudaMemcpyAsync(g->d_tree, tree, 4 * (size_t)K, cudaMemcpyHostToDevice, st));
@@ -1252,7 +1273,7 @@ int mcbgpu_gen_build_lists(mcbgpu_gen *g, int64_t K_keep, int64_t *nnz, void *st
     MCB_CUDA(cudaMemcpyAsync(&total, g->d_off + K, 8, cudaMemcpyDeviceToHost, st));
     int rc = check_status(g, st, "mcbgpu_gen_build_lists (offsets)");
     if (rc) return rc;
-    MCB_CUDA(keep_room(g->d_coords, g->cap_coords, 4 * (total > 0 ? total : 1)));
+    MCB_CUDA(must_room(g, g->d_coords, g->cap_coords, 4 * (total > 0 ? total : 1), false));
     const GenGraph gg = graph_of(g);
     const int32_t *order = g->ordered ? reinterpret_cast<const int32_t *>(g->d_order) : nullptr;
     const int64_t walks = order ? g->K : K;  // the order is over all ranks
@@ -1261,7 +1282,7 @@ int mcbgpu_gen_build_lists(mcbgpu_gen *g, int64_t K_keep, int64_t *nnz, void *st
                                                 g->d_coords, g->d_status, nullptr, nullptr, 1.0f, order, walks);
     MCB_CUDA(cudaGetLastError());
     const unsigned long long cap_long = (unsigned long long)(K < 65536 ? K : 65536);
-    MCB_CUDA(keep_room(g->d_longs, g->cap_longs, 8 * (int64_t)cap_long));
+    MCB_CUDA(must_room(g, g->d_longs, g->cap_longs, 8 * (int64_t)cap_long, false));
     MCB_CUDA(cudaMemsetAsync(g->d_nlong, 0, 4, st));
     const int sgrid = (int)std::min<long long>((K + kSortWarps - 1) / kSortWarps, (long long)g->sm_count * 8);
     sort_lists_kernel<<<sgrid, kSortWarps * 32, 0, st>>>(K, g->d_off, g->d_coords, g->d_longs, g->d_nlong, cap_long);

@@ -1,32 +1,33 @@
 """What is optional on the device gives way where the memory is short: a solver's column index
 takes no more than a quarter of what is free, and makes room for an upload's pair buffers
-and for the certificate's matrix."""
+and for the certificate's matrix; a generation's former lists make room for the next
+ranking."""
 import numpy as np
 import pytest
 
-from minimumcyclebasis_gb300 import Solver
+from minimumcyclebasis_gb300 import GpuGen, Solver, prepare_on_device, random_graph
+from minimumcyclebasis_gb300.devprep import generate_candidates
 
 pytestmark = pytest.mark.gpu
 MB = 1 << 20
 
 
 class Squeeze:
-    """Holds all of the GPU's free memory but `leave` bytes and at most 32 MB more."""
+    """Holds all of the GPU's free memory but `leave` bytes and at most 12 MB more."""
 
     def __init__(self, leave):
         import torch
         self.torch, self.held = torch, []
         torch.cuda.empty_cache()
         size = 1 << 36
-        while size >= 16 * MB:
-            free = torch.cuda.mem_get_info()[0]
-            if free < leave + size:
-                size //= 2
-                continue
-            try:
-                self.held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
-            except torch.cuda.OutOfMemoryError:
-                size //= 2
+        while size >= 10 * MB:
+            if torch.cuda.mem_get_info()[0] >= leave + size:
+                try:
+                    self.held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+                    continue
+                except torch.cuda.OutOfMemoryError:
+                    pass
+            size = max(size // 2, 10 * MB) if size > 10 * MB else 0
 
     def __enter__(self):
         return self
@@ -99,3 +100,32 @@ def test_the_certificate_takes_the_index_s_room():
     assert np.array_equal(got, sel) and tot == total
     assert s.verify()["rank"] == N
     s.close()
+
+
+def ranked(gen, p, which):
+    """The lists of some of the ranks: offsets and coordinates."""
+    _, edge, w, tree = p.candidates()
+    gen.lists(tree[which], edge[which], w[which])
+    return gen.fetch_lists()
+
+
+def test_former_lists_make_room_for_a_ranking():
+    d, gen = prepare_on_device(random_graph(30000, 60000, 1, 1000, 4), make_solver=False, keep_gen=True)
+    p = d.problem
+    off, co = gen.fetch_lists()
+    gen.close()
+    by_length = np.argsort(np.diff(off), kind="stable")
+    short, long = np.sort(by_length[:3_700_000]), np.sort(by_length[-3_000_000:])
+    # 24 bytes per rank and 4 per coordinate: the second ranking does not fit beside the first lists
+    room = 24 * len(long) + 4 * int(np.diff(off)[long].sum())
+    need = 24 * len(short) + 4 * int(np.diff(off)[short].sum())
+    assert 24 * len(short) > 24 * len(long) + 12 * MB and need + 8 * MB < room
+    gen = GpuGen(p)
+    generate_candidates(p, gen)
+    ranked(gen, p, long)
+    with Squeeze(0):
+        got = ranked(gen, p, short)
+    assert np.array_equal(got[0], np.concatenate([[0], np.cumsum(np.diff(off)[short])]))
+    at = np.repeat(off[short] - got[0][:-1], np.diff(got[0])) + np.arange(got[0][-1])
+    assert np.array_equal(got[1], co[at])
+    gen.close()
