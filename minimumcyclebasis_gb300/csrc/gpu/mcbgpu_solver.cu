@@ -638,7 +638,8 @@ __device__ __forceinline__ void load_columns(const uint64_t *__restrict__ S, int
 __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__restrict__ S, int P, int e0, int b, int Wb,
                                                            uint64_t *__restrict__ T, BlockState *bs, long long ntiles,
                                                            GridBar *gb, long long slack_tiles, int stream_pct,
-                                                           uint64_t *__restrict__ Tg, GroupArgs ga) {
+                                                           uint64_t *__restrict__ Tg, GroupArgs ga,
+                                                           unsigned long long *bytes) {
     griddep_wait();
     griddep_launch();
     // all that is read first is read together, the first columns' rows included: a chain of
@@ -686,6 +687,11 @@ __global__ void __launch_bounds__(256) blk_transpose_kernel(const uint64_t *__re
             bs->nz_count[(ga.slot + 1) % 3] = 0;  // the next group's
             bs->by_columns = cols ? 1u : 0u;
         }
+        // rows read, their transposes written, W zeroed
+        if (bytes)
+            atomicAdd(bytes, 8ull * ((unsigned long long)(b + ga.b1 + ga.b2) * ga.Wlast + 64ull * Wb +
+                                 (later > 0 ? 64ull * kGStride * ga.Wlast : 0ull) +
+                                 (cols ? (unsigned long long)pred * kTile * (later + 1) : 0ull)));
     }
     if (cols) {
         const size_t n = (size_t)pred * kTile / 2;
@@ -965,7 +971,8 @@ __device__ __forceinline__ void w_of_group(long long r, const int64_t *__restric
 
 // W from the column index: W starts at zero, and every listed coordinate's T words are
 // added to the ranks of its column below the limit.  Warp w takes part w / n of the
-// listed coordinate w mod n's column (n listed).
+// listed coordinate w mod n's column (n listed).  Returns the bytes this thread read and
+// wrote.
 //
 // Support vectors are sparse for most of a solve: 181-235 listed coordinates of
 // 27k-82k for a pair of blocks of a planar-chain graph (100k points), 129-600 of an
@@ -980,10 +987,11 @@ struct Columns {
 };
 
 template <int kG>
-__device__ __forceinline__ void w_by_columns(const Columns &co, const uint64_t *__restrict__ Tt, unsigned n,
-                                             long long limit, uint64_t *W0, uint64_t *W1, uint64_t *W2) {
+__device__ __forceinline__ unsigned long long w_by_columns(const Columns &co, const uint64_t *__restrict__ Tt, unsigned n,
+                                                           long long limit, uint64_t *W0, uint64_t *W1, uint64_t *W2) {
     constexpr int kStride = kG == 1 ? 1 : kGStride;
-    if (n == 0 || limit <= 0) return;
+    if (n == 0 || limit <= 0) return 0;
+    unsigned long long nb = 0;
     const int lane = threadIdx.x & 31;
     const unsigned gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const unsigned parts = nw / n > 0 ? nw / n : 1u;
@@ -993,17 +1001,22 @@ __device__ __forceinline__ void w_by_columns(const Columns &co, const uint64_t *
         const unsigned part = it / n;
         const uint64_t *t = Tt + (size_t)kStride * c;
         const uint64_t x = t[0], y = kG > 1 ? t[kG > 1 ? 1 : 0] : 0ull, z = kG > 2 ? t[kG - 1] : 0ull;
+        const unsigned adds = (x ? 1u : 0u) + (y ? 1u : 0u) + (z ? 1u : 0u);
+        if (lane == 0) nb += 12 + 8 * kG;  // the coordinate, its column's ends, its words
         // 64 bits: a step past a column's end can pass 2^32 where the index nearly fills 32 bits
         const unsigned long long e = co.start[(size_t)c * co.segs + seg_end];
         for (unsigned long long i = co.start[(size_t)c * co.segs] + (unsigned long long)(part * 32 + lane); i < e;
              i += parts * 32) {
             const unsigned r = __ldg(co.ranks + i);
+            nb += 4;
             if ((long long)r >= limit) continue;
+            nb += 16 * adds;  // W read and written
             if (x) atomicXor((unsigned long long *)W0 + r, (unsigned long long)x);
             if (kG > 1 && y) atomicXor((unsigned long long *)W1 + r, (unsigned long long)y);
             if (kG > 2 && z) atomicXor((unsigned long long *)W2 + r, (unsigned long long)z);
         }
     }
+    return nb;
 }
 
 // Streaming pass: W for tiles [0, bs->pred_tiles), one candidate per thread (1024
@@ -1027,15 +1040,20 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
     griddep_launch();
     const unsigned epoch = bs->epoch;
     const long long ntiles = bs->pred_tiles;
-    unsigned long long nb = (blockIdx.x == 0 && threadIdx.x == 0) ? 8ull * (unsigned long long)bound : 0ull;
+    unsigned long long nb = 0;
     if (bs->by_columns) {
-        w_by_columns<kG>(co, kG > 1 ? Tg : T, min(bs->nz_count[co.slot], co.nz_cap), min(ntiles * kTile, K), Warr, Wl1,
-                         Wl2);
+        nb = w_by_columns<kG>(co, kG > 1 ? Tg : T, min(bs->nz_count[co.slot], co.nz_cap), min(ntiles * kTile, K), Warr,
+                              Wl1, Wl2);
         for (long long t = blockIdx.x + (long long)threadIdx.x * gridDim.x; t < ntiles;
              t += (long long)blockDim.x * gridDim.x)
             tile_epoch[t] = (epoch << 1) | (tile_minc[t] >= bound ? 1u : 0u);
+        if (bytes) {  // while profiling
+            for (int d = 16; d > 0; d >>= 1) nb += __shfl_xor_sync(0xffffffffu, nb, d);
+            if ((threadIdx.x & 31) == 0 && nb) atomicAdd(bytes, nb);
+        }
         return;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) nb = 8ull * (unsigned long long)bound;
     if (kG > 1) {
         const int bd[3] = {bound, bound1, bound2};
         const int last = bd[kG - 1];
@@ -1067,7 +1085,7 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
              t += (long long)blockDim.x * gridDim.x)
             tile_epoch[t] = (epoch << 1) | (tile_minc[t] >= bound ? 1u : 0u);
         for (int d = 16; d > 0; d >>= 1) nb += __shfl_xor_sync(0xffffffffu, nb, d);
-        if ((threadIdx.x & 31) == 0 && nb) atomicAdd(bytes, nb);
+        if ((threadIdx.x & 31) == 0 && nb && bytes) atomicAdd(bytes, nb);
         return;
     }
     // no barrier per tile: a thread moves on to its next tile as soon as its own
@@ -1089,7 +1107,7 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
     for (long long t = blockIdx.x + (long long)threadIdx.x * gridDim.x; t < ntiles; t += (long long)blockDim.x * gridDim.x)
         tile_epoch[t] = (epoch << 1) | (tile_minc[t] >= bound ? 1u : 0u);
     for (int d = 16; d > 0; d >>= 1) nb += __shfl_xor_sync(0xffffffffu, nb, d);
-    if ((threadIdx.x & 31) == 0 && nb) atomicAdd(bytes, nb);
+    if ((threadIdx.x & 31) == 0 && nb && bytes) atomicAdd(bytes, nb);
 }
 
 // A later block of a group (the j-th, j = kJ): W of every candidate the grouped pass
@@ -3266,7 +3284,8 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
                                        ga.nz && ga.columns ? (int)std::min<long long>(sms, std::max(1ll, ntiles)) : 1);
             MCB_CUDA(launch_k(pdl, blk_transpose_kernel, dim3(tgrid), dim3(256), 0, st, (const uint64_t *)s->d_S, s->P,
                               (int)e0, b, Wb, s->d_T, s->d_bs, ntiles, s->d_gbar,
-                              (long long)s->pivot_grid, sh.stream_pct, s->d_Tg, ga));
+                              (long long)s->pivot_grid, sh.stream_pct, s->d_Tg, ga,
+                              s->profiling ? L.bytes() : (unsigned long long *)nullptr));
         }
         if (ntiles > 0 && pos > 0) {
             Launch L(s, KC_WFIX, st);
@@ -3280,6 +3299,7 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
                                   s->d_tile_epoch, L.bytes()));
         } else if (ntiles > 0) {
             Launch L(s, KC_WSTREAM, st);
+            unsigned long long *nbytes = s->profiling ? L.bytes() : nullptr;
             const int64_t *woff = s->d_off;
             const int32_t *wco = s->d_coords, *whd = s->d_head, *wtm = s->d_tile_minc;
             const uint64_t *wT = s->d_T, *wTg = s->d_Tg;
@@ -3287,13 +3307,13 @@ int mcbgpu_solver_run(mcbgpu_solver *s, int64_t max_iterations, void *stream) {
             uint64_t *nul = nullptr;
             if (nl == 2)
                 MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<3, true> : blk_w_kernel<3, false>, dim3(sms), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
-                                  bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd2, Wpos[1], Wpos[2], cols));
+                                  bound, wbs, Wpos[0], s->d_tile_epoch, nbytes, wTg, bd1, bd2, Wpos[1], Wpos[2], cols));
             else if (nl == 1)
                 MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<2, true> : blk_w_kernel<2, false>, dim3(sms), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
-                                  bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), wTg, bd1, bd1, Wpos[1], nul, cols));
+                                  bound, wbs, Wpos[0], s->d_tile_epoch, nbytes, wTg, bd1, bd1, Wpos[1], nul, cols));
             else
                 MCB_CUDA(launch_k(pdl, s->narrow ? blk_w_kernel<1, true> : blk_w_kernel<1, false>, dim3(sms), dim3(kTile), 0, st, s->K, woff, wco, whd, wtm, wT,
-                                  bound, wbs, Wpos[0], s->d_tile_epoch, L.bytes(), (const uint64_t *)nullptr, 0, 0, nul,
+                                  bound, wbs, Wpos[0], s->d_tile_epoch, nbytes, (const uint64_t *)nullptr, 0, 0, nul,
                                   nul, cols));
         }
         // this block's tail rewrites the parity buffers the far update two blocks back reads
