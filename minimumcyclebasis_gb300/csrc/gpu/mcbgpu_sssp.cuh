@@ -56,7 +56,13 @@ constexpr int kTreeThreads = 1024;      // the shared-memory form's CTA
 constexpr int kTreeSharedMaxN = 53248;  // 208 KB of distances + 6.5 KB of dirty bits + 8 KB of list (of 227 KB)
 constexpr int kTreeLanes = 4;  // lanes that share a listed vertex's arcs
 constexpr int kTreeSharedList = 4096;   // vertices listed per round: shared form (16 bits each)
-constexpr int kTreeGlobalList = 1024;   // and global form
+// Global form.  A frontier of tens of thousands of vertices takes a round per list: random
+// graph of 249k vertices 120 us per root with 1024 entries and every waiting vertex's
+// distance read in every round, 79 with a full list left alone, 62 / 57 with 2048 / 3072
+// entries (70 with no list); planar-chain graph of 368k vertices 34.5 / 34.2 / 35.1, grid of
+// 160k 11.3 / 11.4 / 12.5 with 1024 / 2048 / 3072.
+constexpr int kTreeGlobalList = 2048;
+constexpr int kTreeNearList = 1024;     // and the form with two bitmaps
 constexpr int kTreeMaxCtasPerSm = 16;   // the global form's per-CTA slices are sized for this many
 
 // A vertex's first kArcSlots arcs at a fixed place, (column, weight) together: relaxing
@@ -265,6 +271,10 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
             // others stay (and their smallest distance counts for the next round), as do
             // those that find the list full.  Returns whether some vertex was left dirty.
             auto list_word = [&](int k) {
+                if (*(volatile int *)nv >= kListCap) {  // no room in this round: not looked at
+                    mynext = lo < mynext ? lo : mynext;
+                    return true;
+                }
                 const uint32_t bits = vdirty[k];
                 uint32_t take = 0;
                 for (uint32_t m = bits; m;) {  // four distances in flight
@@ -383,7 +393,7 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) trees_near_kernel(T
     __shared__ int s_root, s_lo, s_nv[3];
     const int n = a.n, words = (n + 31) >> 5;
     uint32_t *s_verts = reinterpret_cast<uint32_t *>(smem);
-    uint32_t *near = s_verts + kTreeGlobalList, *far = near + words;
+    uint32_t *near = s_verts + kTreeNearList, *far = near + words;
     int32_t *dist = a.gdist + (size_t)blockIdx.x * n;
     const int tid = threadIdx.x, lane = tid & 31;
     auto get = [&](uint32_t v) -> int { return __ldcg(dist + v); };
@@ -412,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) trees_near_kernel(T
                 uint32_t bits = near[k];
                 if (!bits) continue;
                 int at = atomicAdd(nv, __popc(bits));
-                while (bits && at < kTreeGlobalList) {
+                while (bits && at < kTreeNearList) {
                     const int b = __ffs(bits) - 1;
                     bits &= bits - 1;
                     s_verts[at++] = (uint32_t)((k << 5) + b);
@@ -420,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) trees_near_kernel(T
                 near[k] = bits;
             }
             cta_sync();
-            const int listed = min(*(volatile int *)nv, kTreeGlobalList);
+            const int listed = min(*(volatile int *)nv, kTreeNearList);
             if (listed > 0) {
                 // their arcs, kTreeLanes at a time; bits were cleared before the barrier and
                 // distances are read after it, so a distance lowered since sets its bit again
@@ -474,14 +484,14 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) trees_near_kernel(T
                 int at = atomicAdd(nv, __popc(bits));
                 for (; bits; bits &= bits - 1, at++) {
                     const uint32_t v = (uint32_t)((k << 5) + __ffs(bits) - 1);
-                    if (at < kTreeGlobalList)
+                    if (at < kTreeNearList)
                         s_verts[at] = v;
                     else
                         sort_out(v, get(v));  // its word is this thread's
                 }
             }
             cta_sync();
-            const int nfar = min(*(volatile int *)nv, kTreeGlobalList);
+            const int nfar = min(*(volatile int *)nv, kTreeNearList);
             for (int i = tid; i < nfar; i += kThreads) {
                 const uint32_t v = s_verts[i];
                 sort_out(v, get(v));
@@ -503,7 +513,7 @@ inline size_t trees_smem_bytes(int n) {
 }
 inline size_t trees_global_smem_bytes(int n) {
     const size_t words = ((size_t)n + 31) / 32;
-    return 4 * kTreeGlobalList + (n <= kTreeNearMaxN ? 8 * words : 2 * ((words + 7) & ~(size_t)7));
+    return n <= kTreeNearMaxN ? 4 * kTreeNearList + 8 * words : 4 * kTreeGlobalList + 2 * ((words + 7) & ~(size_t)7);
 }
 constexpr int kTreeGlobalMaxN = 65536 * 32;  // the global form's 16-bit word list: at most 128 KB
 
