@@ -651,7 +651,7 @@ struct mcbgpu_gen {
     int32_t n = 0, F = 0, chunk = 0, N = 0;
     int64_t slots = 0, npairs = 0, words_per_root = 0;
     int sm_count = 0;
-    bool shared_form = true;
+    TreeForm form = kTreeShared;
     size_t smem = 0;
     int delta = 1;  // the mean slot weight
     // launch shapes of the tree kernel: while tuning, call i of mcbgpu_gen_trees
@@ -879,8 +879,8 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g->sm_count, cudaDevAttrMultiProcessorCount, dev);
     const int words = (nodes + 31) / 32;
-    g->shared_form = nodes <= kTreeSharedMaxN;
-    g->smem = g->shared_form ? trees_smem_bytes(nodes) : 0;
+    g->form = tree_form(nodes, slots);
+    g->smem = g->form == kTreeShared ? trees_smem_bytes(nodes) : 0;
     const size_t n = (size_t)nodes, C = (size_t)g->chunk;
 #define GALLOC(ptr, sz)                                            \
     do {                                                           \
@@ -916,14 +916,14 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     GALLOC(g->d_next, 4);
     GALLOC(g->d_status, 4);
     GALLOC(g->d_nlong, 4);
-    if (!g->shared_form) {
+    if (g->form != kTreeShared) {
         GALLOC(g->d_gdist, 4 * n * (size_t)g->sm_count * kTreeMaxCtasPerSm);
         GALLOC(g->d_gdirty, 4 * (size_t)words * (size_t)g->sm_count * kTreeMaxCtasPerSm);
         GALLOC(g->d_gsumm, 4 * (size_t)((words + 31) / 32) * (size_t)g->sm_count * kTreeMaxCtasPerSm);
     }
     // shapes the tuner tries (the shared form: one 1024-thread CTA per SM, bucket
     // widths only); with fewer chunks than twice the shapes, the first one is kept
-    if (g->shared_form)
+    if (g->form == kTreeShared)
         g->shapes = {{kTreeThreads, 1, 8}, {kTreeThreads, 1, 4}, {kTreeThreads, 1, 16}, {kTreeThreads, 1, 2}};
     else
         g->shapes = {{256, 8, 8}, {256, 8, 4}, {256, 8, 12}, {256, 8, 16}, {512, 4, 8}, {128, 16, 8}};
@@ -1032,7 +1032,7 @@ int mcbgpu_gen_trees_submit(mcbgpu_gen *g, int32_t t0, int32_t count, void *stre
     const int cap = g->sm_count * shape.ctas_per_sm;
     const int grid = count < cap ? count : cap;
     MCB_CUDA(cudaEventRecord(g->ev_begin[k], st));
-    MCB_CUDA(launch_trees(g->shared_form, shape, grid, g->smem, st, a));
+    MCB_CUDA(launch_trees(g->form, shape, grid, g->smem, st, a));
     MCB_CUDA(cudaEventRecord(g->ev_end[k], st));
     MCB_CUDA(cudaMemcpyAsync(g->h_tied[k], g->d_tied_slot[k], (size_t)count, cudaMemcpyDeviceToHost, st));
     g->slot_t0[k] = t0;

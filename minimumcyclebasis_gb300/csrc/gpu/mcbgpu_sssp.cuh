@@ -181,10 +181,10 @@ __device__ __forceinline__ int tree_parents(const TreeArgs &a, int r, uint32_t s
 // Threads per CTA: the shared-memory form runs one 1024-thread CTA per SM (its
 // distances fill the shared memory); the other forms run kThreads-thread CTAs, several
 // per SM, so that the bucket rounds of different roots overlap: their distances are in
-// the CTA's global slice (trees_near_kernel up to kTreeNearMaxN vertices, else the dirty
-// bits too, with a summary).  They wait on L2 half of their time, so a full SM of threads
+// the CTA's global slice (trees_near_kernel by tree_form()'s rule, else the dirty bits too,
+// with a summary).  They wait on L2 half of their time, so a full SM of threads
 // (32 registers, a few spills) is worth more than registers.
-enum TreeForm { kTreeShared, kTreeGlobal };
+enum TreeForm { kTreeShared, kTreeNear, kTreeGlobal };
 template <int kForm, int kThreads>
 __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kThreads) trees_kernel(TreeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -385,7 +385,17 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
 // 650 rounds of 125 vertices per root, 4.8 us per root (5.2 with one bitmap; 3.8 with
 // arc_table).  Bound by the chain of L2 reads of each relaxation at eight CTAs per SM
 // (512 or 128 threads per CTA: 4.6 and 5.4).
-constexpr int kTreeNearMaxN = 98304;  // 24 KB of bitmaps + 4 KB of list, eight times per SM
+//
+// The line: eight CTAs' bitmaps (8 words each), lists and 1 KB of the system's must leave the
+// SM its next smaller split of shared memory and L1 (196 of 228 KB): up to 79,360 vertices.
+// Past it a random graph takes 24 us per root against 14 with the dirty bits in global
+// memory, a planar-chain graph 7.4 against 6.9.  Up to it planar-chain, grid and RGG graphs
+// gain 20-25% (60k vertices 4.0 / 5.2, 79k 5.4 / 6.7); random ones of mean degree 4.4 gain 3%
+// to 63k and lose 10% beyond (66k 11.4 / 10.0); of degree 6.3 and 8.1 they lose 10-25% from
+// the start (57k 12.9 / 11.7, 60k 19.8 / 16.9): more waits than a list holds.  So the degree
+// decides too.
+constexpr int kTreeNearMaxN = 79360;
+constexpr int kTreeNearMaxDegree = 6;
 
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, 2048 / kThreads) trees_near_kernel(TreeArgs a) {
@@ -505,15 +515,21 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) trees_near_kernel(T
     }
 }
 
+// The form for a graph of n vertices and `slots` arcs.
+inline TreeForm tree_form(int n, long long slots) {
+    if (n <= kTreeSharedMaxN) return kTreeShared;
+    return n <= kTreeNearMaxN && slots <= (long long)kTreeNearMaxDegree * n ? kTreeNear : kTreeGlobal;
+}
+
 // Dynamic shared memory for n vertices: the shared form's distances, dirty bits and a
 // round's vertices; the other forms' vertices and bitmaps or dirty words of a round.
 inline size_t trees_smem_bytes(int n) {
     const size_t words = ((size_t)n + 31) / 32;
     return (((size_t)n * 4 + 15) & ~(size_t)15) + words * 4 + 2 * kTreeSharedList;
 }
-inline size_t trees_global_smem_bytes(int n) {
+inline size_t trees_global_smem_bytes(TreeForm form, int n) {
     const size_t words = ((size_t)n + 31) / 32;
-    return n <= kTreeNearMaxN ? 4 * kTreeNearList + 8 * words : 4 * kTreeGlobalList + 2 * ((words + 7) & ~(size_t)7);
+    return form == kTreeNear ? 4 * kTreeNearList + 8 * words : 4 * kTreeGlobalList + 2 * ((words + 7) & ~(size_t)7);
 }
 constexpr int kTreeGlobalMaxN = 65536 * 32;  // the global form's 16-bit word list: at most 128 KB
 
@@ -531,8 +547,8 @@ inline int32_t shape_delta(const TreeShape &sh, int32_t mean_w) {
 
 // The kernel for a CTA size of the forms with distances in global memory.
 typedef void (*TreeKernel)(TreeArgs);
-inline TreeKernel tree_kernel(int n, int threads) {
-    const bool d = n <= kTreeNearMaxN;
+inline TreeKernel tree_kernel(TreeForm form, int threads) {
+    const bool d = form == kTreeNear;
     switch (threads) {
     case 128: return d ? trees_near_kernel<128> : trees_kernel<kTreeGlobal, 128>;
     case 256: return d ? trees_near_kernel<256> : trees_kernel<kTreeGlobal, 256>;
@@ -541,15 +557,15 @@ inline TreeKernel tree_kernel(int n, int threads) {
     }
 }
 
-// Launches trees_kernel in `shape` over grid CTAs (the shared form: 1024 threads,
+// Launches the form's kernel in `shape` over grid CTAs (the shared form: 1024 threads,
 // smem bytes of dynamic shared memory).
-inline cudaError_t launch_trees(bool shared, const TreeShape &shape, int grid, size_t smem, cudaStream_t st,
+inline cudaError_t launch_trees(TreeForm form, const TreeShape &shape, int grid, size_t smem, cudaStream_t st,
                                 const TreeArgs &a) {
-    if (shared)
+    if (form == kTreeShared)
         trees_kernel<kTreeShared, kTreeThreads><<<grid, kTreeThreads, smem, st>>>(a);
     else
-        tree_kernel(a.n, shape.threads)<<<grid, shape.threads <= 512 ? shape.threads : 1024,
-                                          trees_global_smem_bytes(a.n), st>>>(a);
+        tree_kernel(form, shape.threads)<<<grid, shape.threads <= 512 ? shape.threads : 1024,
+                                           trees_global_smem_bytes(form, a.n), st>>>(a);
     return cudaGetLastError();
 }
 
@@ -557,8 +573,10 @@ inline cudaError_t set_trees_smem_limit() {
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(trees_kernel<kTreeShared, kTreeThreads>, attr, (int)trees_smem_bytes(kTreeSharedMaxN));
     for (int threads : {128, 256, 512, 1024})
-        for (int n : {kTreeNearMaxN, kTreeGlobalMaxN})
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(tree_kernel(n, threads), attr, (int)trees_global_smem_bytes(n));
+        for (TreeForm form : {kTreeNear, kTreeGlobal})
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(tree_kernel(form, threads), attr,
+                                         (int)trees_global_smem_bytes(form, form == kTreeNear ? kTreeNearMaxN : kTreeGlobalMaxN));
     return e;
 }
 

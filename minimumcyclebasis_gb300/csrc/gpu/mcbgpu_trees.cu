@@ -16,7 +16,7 @@ struct mcbgpu_trees {
     int32_t max_roots = 0;
     int32_t delta = 1;
     int sm_count = 0;
-    bool shared_form = true;
+    TreeForm form = kTreeShared;
     size_t smem = 0;
     uint32_t *d_ro = nullptr, *d_cols = nullptr, *d_rev = nullptr, *d_roots = nullptr;
     uint2 *d_arcs = nullptr;
@@ -94,8 +94,8 @@ int mcbgpu_trees_create(mcbgpu_trees **out, int32_t nodes, int64_t slots, const 
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&t->sm_count, cudaDevAttrMultiProcessorCount, dev);
     const int words = (nodes + 31) / 32;
-    t->shared_form = nodes <= kTreeSharedMaxN;
-    t->smem = t->shared_form ? trees_smem_bytes(nodes) : 0;
+    t->form = tree_form(nodes, slots);
+    t->smem = t->form == kTreeShared ? trees_smem_bytes(nodes) : 0;
     const size_t per_root = (size_t)nodes;
 #define TALLOC(ptr, sz)                                            \
     do {                                                           \
@@ -115,7 +115,7 @@ int mcbgpu_trees_create(mcbgpu_trees **out, int32_t nodes, int64_t slots, const 
     TALLOC(t->d_tied, (size_t)max_roots);
     TALLOC(t->d_next, 4);
     TALLOC(t->d_status, 4);
-    if (!t->shared_form) {
+    if (t->form != kTreeShared) {
         TALLOC(t->d_gdist, 4 * per_root * (size_t)t->sm_count * kTreeMaxCtasPerSm);
         TALLOC(t->d_gdirty, 4 * (size_t)words * (size_t)t->sm_count * kTreeMaxCtasPerSm);
         TALLOC(t->d_gsumm, 4 * (size_t)((words + 31) / 32) * (size_t)t->sm_count * kTreeMaxCtasPerSm);
@@ -166,7 +166,7 @@ int mcbgpu_trees_run(mcbgpu_trees *t, const uint32_t *roots, int32_t count, int3
     a.rev = t->d_rev;
     a.arcs = t->d_arcs;
     a.n = t->n;
-    const TreeShape shape = t->shared_form ? TreeShape{kTreeThreads, 1, 4} : TreeShape{256, 8, 8};
+    const TreeShape shape = t->form == kTreeShared ? TreeShape{kTreeThreads, 1, 4} : TreeShape{256, 8, 8};
     a.delta = shape_delta(shape, t->delta);
     a.roots = t->d_roots;
     a.count = count;
@@ -180,7 +180,7 @@ int mcbgpu_trees_run(mcbgpu_trees *t, const uint32_t *roots, int32_t count, int3
     a.status = t->d_status;
     const int slots_ = t->sm_count * shape.ctas_per_sm;
     const int grid = count < slots_ ? count : slots_;
-    MCB_CUDA(launch_trees(t->shared_form, shape, grid, t->smem, st, a));
+    MCB_CUDA(launch_trees(t->form, shape, grid, t->smem, st, a));
     const size_t cells = (size_t)count * (size_t)t->n;
     MCB_CUDA(cudaMemcpyAsync(dist, t->d_dist, 4 * cells, cudaMemcpyDeviceToHost, st));
     MCB_CUDA(cudaMemcpyAsync(parent_slot, t->d_pedge, 4 * cells, cudaMemcpyDeviceToHost, st));
