@@ -40,7 +40,7 @@ a flushed L2.
 
 `--workload batch` measures the batched configuration instead: --batch-count graphs
 (n log-uniform in [50, 5000], average degree U[2.5, 5], w U[1, 255]) solved in one
-BatchSolver (one persistent launch, one CTA per problem), the plain GPU form (the blocked
+BatchSolver (persistent launches, one to eight CTAs per problem), the plain GPU form (the blocked
 single-problem solver, problem after problem) on a sample beside it, and the
 biconnected components of a --blocks block tree in a second batch.
 
@@ -889,7 +889,7 @@ def run_batch(args, world, rank, local, pg):
             "vs_baseline": None, "dtype": "u64", "data": "synthetic",
             "config": {"workload": BATCH_WORKLOAD % (args.batch_count, args.seed),
                        "problems": len(items), "rings_on_host": nsc, "N_max": int(Ns.max()), "N_sum": int(Ns.sum()),
-                       "K": K, "cycle_nnz": nnz, "form": "batched (one persistent launch, one CTA per problem)",
+                       "K": K, "cycle_nnz": nnz, "form": "batched (persistent launches, 1-8 CTAs per problem)",
                        "total_weight": int(tots.sum()) + host_total,
                        "l2": "inputs (%.2f GB) larger than the 129 MB L2; no flush" % ((nnz * 4 + K * 12) / 1e9),
                        "host_preparation_s": round(prep_s, 3), "host_threads": os.cpu_count()},

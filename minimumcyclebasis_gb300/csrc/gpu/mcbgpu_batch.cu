@@ -885,7 +885,7 @@ int mcbgpu_batch_upload(mcbgpu_batch *b, const int32_t *weight, const int64_t *o
     if (b->nnz > 0)
         MCB_CUDA(cudaMemcpyAsync(b->d_coords, coords, sizeof(int32_t) * (size_t)b->nnz, cudaMemcpyHostToDevice, st));
     // offsets checked on the device (non-decreasing from 0 to nnz); the longest list
-    // sizes the pair scratch; the coordinate lists are checked by the solve itself
+    // sizes the pair scratch; the coordinate lists are checked below (batch_lists_kernel)
     unsigned chk[2] = {0, 0};
     if (b->total_K > 0) {
         MCB_CUDA(cudaMemsetAsync(b->d_check, 0, sizeof chk, st));

@@ -1913,7 +1913,7 @@ __device__ __forceinline__ uint64_t sparse_D(const uint64_t *S, long long j, int
 //   far_scatter_kernel: every (coordinate c, k) pair of the block's selected cycles
 //     with c a unit far row sets bit k of Dfar[c] (first touch lists c);
 //   far_rows_kernel:    D and beta of the non-unit far rows (lists carried from update
-//     to update; sparse rows test the pairs of their listed words, one row per lane;
+//     to update; sparse rows test the pairs of their listed words, four lanes per row;
 //     dense rows gather every pair up to their own word, as the reference's update
 //     does) and of the touched unit rows; unchanged rows are carried over, changed
 //     rows go to a (row, beta) list;

@@ -14,9 +14,10 @@
 //   1. distances, label-correcting by buckets: each round takes lo = (a lower
 //      bound of) the smallest distance among dirty vertices and relaxes (atomicMin)
 //      the arcs of every dirty vertex nearer than lo + delta, marking improved heads
-//      dirty.  The dirty vertex at lo is final after its round (weights >= 1), so a
-//      root needs at most 2 (n + 1) rounds; the loop stops there and flags the root
-//      if it has not converged.  A round first lists the vertices to relax, then gives
+//      dirty.  The dirty vertex at lo is final once relaxed (weights >= 1).  The loop
+//      stops after 2 (n + 1) rounds, far more than any tree has taken, and flags the root
+//      if it has not converged (a vertex that finds the round's list full waits, so that
+//      is a check and not a bound).  A round first lists the vertices to relax, then gives
 //      each kTreeLanes lanes, one arc at a time each: one thread per dirty word with its
 //      vertices and arcs one after the other left a few threads with all of a frontier
 //      of neighbours (planar-chain graph of 65k points: 14.8 us per root, 5.2 with lists; random
@@ -250,8 +251,9 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
         // smallest distance of a skipped vertex or of an improvement made in this
         // round (at most the smallest distance left dirty, so no vertex is missed;
         // an underestimate only costs a round).  The dirty vertex at the true lo is
-        // final once relaxed (weights >= 1), so at most 2 (n + 1) rounds; the loop
-        // stops there and flags the root if it has not converged.  The round's
+        // final once relaxed (weights >= 1); it may wait while a list is full, so the
+        // number of rounds is checked: past 2 (n + 1), far more than any tree took, the
+        // root is flagged as not converged.  The round's
         // minimum goes to s_next[round % 3]: the slot read after this round's
         // barrier, reset two rounds later, when every thread has read it.
         bool converged = false;
@@ -386,11 +388,11 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
 // arc_table).  Bound by the chain of L2 reads of each relaxation at eight CTAs per SM
 // (512 or 128 threads per CTA: 4.6 and 5.4).
 //
-// The line: eight CTAs' bitmaps (8 words each), lists and 1 KB of the system's must leave the
-// SM its next smaller split of shared memory and L1 (196 of 228 KB): up to 79,360 vertices.
+// The line: eight CTAs' bitmaps (19.4 KB), lists (4 KB) and the system's 1 KB each must fit the
+// SM's last split but one of shared memory and L1 (196 of 228 KB): up to 79,360 vertices.
 // Past it a random graph takes 24 us per root against 14 with the dirty bits in global
-// memory, a planar-chain graph 7.4 against 6.9.  Up to it planar-chain, grid and RGG graphs
-// gain 20-25% (60k vertices 4.0 / 5.2, 79k 5.4 / 6.7); random ones of mean degree 4.4 gain 3%
+// memory, a planar-chain graph 7.4 against 6.9.  Up to it planar-chain and grid graphs gain
+// 15-25% (60k vertices 4.0 / 5.2, 79k 5.4 / 6.7) and RGGs nothing (5.6); random ones of mean degree 4.4 gain 3%
 // to 63k and lose 10% beyond (66k 11.4 / 10.0); of degree 6.3 and 8.1 they lose 10-25% from
 // the start (57k 12.9 / 11.7, 60k 19.8 / 16.9): more waits than a list holds.  So the degree
 // decides too.

@@ -293,7 +293,8 @@ def solve(num_coords: int, weight: np.ndarray, offsets: np.ndarray, coords: np.n
 
 
 class BatchSolver:
-    """Many independent de Pina problems in one persistent launch (one CTA per problem).
+    """Many independent de Pina problems in up to four persistent launches, a cluster of one to
+    eight CTAs per problem.
 
     `problems` is a list of (num_coords, weight, offsets, coords) tuples, each as
     Solver takes it (offsets local to the problem, starting at 0).  Every problem's
