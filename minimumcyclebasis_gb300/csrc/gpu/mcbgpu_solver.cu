@@ -1047,9 +1047,14 @@ __global__ void __launch_bounds__(kTile, MCB_W_MINB) blk_w_kernel(long long K, c
         for (long long t = blockIdx.x + (long long)threadIdx.x * gridDim.x; t < ntiles;
              t += (long long)blockDim.x * gridDim.x)
             tile_epoch[t] = (epoch << 1) | (tile_minc[t] >= bound ? 1u : 0u);
-        if (bytes) {  // while profiling
+        if (bytes) {  // while profiling; one atomic per CTA (one per warp adds 2 us to these 9)
+            __shared__ unsigned long long s_bytes;
+            if (threadIdx.x == 0) s_bytes = 0;
+            cta_sync();
             for (int d = 16; d > 0; d >>= 1) nb += __shfl_xor_sync(0xffffffffu, nb, d);
-            if ((threadIdx.x & 31) == 0 && nb) atomicAdd(bytes, nb);
+            if ((threadIdx.x & 31) == 0 && nb) atomicAdd(&s_bytes, nb);
+            cta_sync();
+            if (threadIdx.x == 0) atomicAdd(bytes, s_bytes);
         }
         return;
     }
