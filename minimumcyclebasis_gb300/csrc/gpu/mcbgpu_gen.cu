@@ -925,8 +925,12 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     // widths only); with fewer chunks than twice the shapes, the first one is kept
     if (g->form == kTreeShared)
         g->shapes = {{kTreeThreads, 1, 8}, {kTreeThreads, 1, 4}, {kTreeThreads, 1, 16}, {kTreeThreads, 1, 2}};
-    else
-        g->shapes = {{256, 8, 8}, {256, 8, 4}, {256, 8, 12}, {256, 8, 16}, {512, 4, 8}, {128, 16, 8}};
+    else {
+        g->shapes = {first_shape(g->form, nodes)};
+        for (const TreeShape sh : {TreeShape{256, 8, 8}, TreeShape{256, 8, 4}, TreeShape{256, 8, 12}, TreeShape{256, 8, 16},
+                                   TreeShape{512, 4, 8}, TreeShape{128, 16, 8}})
+            if (sh.threads != g->shapes[0].threads || sh.delta_quarters != g->shapes[0].delta_quarters) g->shapes.push_back(sh);
+    }
     const int nchunks = (fvs_size + g->chunk - 1) / g->chunk;
     if (nchunks < 2 * (int)g->shapes.size()) g->chosen = 0;
     for (int k = 0; k < 2; k++) {

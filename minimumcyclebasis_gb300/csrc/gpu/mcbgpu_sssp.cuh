@@ -41,6 +41,7 @@
 // before them diverge within warps.
 #pragma once
 
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 #include <vector>
@@ -57,12 +58,7 @@ constexpr int kTreeThreads = 1024;      // the shared-memory form's CTA
 constexpr int kTreeSharedMaxN = 53248;  // 208 KB of distances + 6.5 KB of dirty bits + 8 KB of list (of 227 KB)
 constexpr int kTreeLanes = 4;  // lanes that share a listed vertex's arcs
 constexpr int kTreeSharedList = 4096;   // vertices listed per round: shared form (16 bits each)
-// Global form.  A frontier of tens of thousands of vertices takes a round per list: random
-// graph of 249k vertices 120 us per root with 1024 entries and every waiting vertex's
-// distance read in every round, 79 with a full list left alone, 62 / 57 with 2048 / 3072
-// entries (70 with no list); planar-chain graph of 368k vertices 34.5 / 34.2 / 35.1, grid of
-// 160k 11.3 / 11.4 / 12.5 with 1024 / 2048 / 3072.
-constexpr int kTreeGlobalList = 2048;
+constexpr int kTreeGlobalList = 1024;   // global form: at least (tree_list_cap)
 constexpr int kTreeNearList = 1024;     // and the form with two bitmaps
 constexpr int kTreeMaxCtasPerSm = 16;   // the global form's per-CTA slices are sized for this many
 
@@ -92,6 +88,7 @@ struct TreeArgs {
     const uint2 *arcs;   // n x kArcSlots: the first arcs of every vertex (arc_table)
     int32_t n;
     int32_t delta;
+    int32_t list_cap;    // vertices listed per round (global form only)
     const uint32_t *roots;
     int32_t count;
     int32_t *dist_out;   // count x n
@@ -199,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
     uint32_t *dirty, *summ;
     constexpr bool kShared = kForm == kTreeShared, kSummary = kForm == kTreeGlobal;
     using VertT = typename std::conditional<kShared, uint16_t, uint32_t>::type;
-    constexpr int kListCap = kShared ? kTreeSharedList : kTreeGlobalList;
+    const int list_cap = kShared ? kTreeSharedList : a.list_cap;
     VertT *s_verts;  // the vertices of a round
     if (kShared) {
         dist = reinterpret_cast<int32_t *>(smem);
@@ -213,7 +210,7 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
         s_verts = reinterpret_cast<VertT *>(smem);
     }
     // global form: the dirty words of a round (words < 65536 entries, 16-bit)
-    uint16_t *s_list = reinterpret_cast<uint16_t *>(smem + 4 * kTreeGlobalList);
+    uint16_t *s_list = reinterpret_cast<uint16_t *>(smem + 4 * (size_t)list_cap);
     volatile int32_t *vdist = dist;
     // a distance as the CTA's atomics left it; global ones from L2, loads free to overlap
     auto get = [&](uint32_t v) -> int { return kShared ? vdist[v] : __ldcg(dist + v); };
@@ -273,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
             // others stay (and their smallest distance counts for the next round), as do
             // those that find the list full.  Returns whether some vertex was left dirty.
             auto list_word = [&](int k) {
-                if (*(volatile int *)nv >= kListCap) {  // no room in this round: not looked at
+                if (*(volatile int *)nv >= list_cap) {  // no room in this round: not looked at
                     mynext = lo < mynext ? lo : mynext;
                     return true;
                 }
@@ -300,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
                     uint32_t listed = 0;
                     for (uint32_t m = take; m; m &= m - 1, at++) {
                         const int b = __ffs(m) - 1;
-                        if (at < kListCap) {
+                        if (at < list_cap) {
                             s_verts[at] = (VertT)((k << 5) + b);
                             listed |= 1u << b;
                         } else {
@@ -346,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
             __threadfence_block();
             cta_sync();
             // the listed vertices' arcs, kTreeLanes at a time
-            const int listed = min(*(volatile int *)nv, kListCap);
+            const int listed = min(*(volatile int *)nv, list_cap);
             auto improve = [&](uint32_t x, int nd) {
                 const int old = atomicMin(&dist[x], nd);
                 if (nd < old) {
@@ -529,9 +526,9 @@ inline size_t trees_smem_bytes(int n) {
     const size_t words = ((size_t)n + 31) / 32;
     return (((size_t)n * 4 + 15) & ~(size_t)15) + words * 4 + 2 * kTreeSharedList;
 }
-inline size_t trees_global_smem_bytes(TreeForm form, int n) {
+inline size_t trees_global_smem_bytes(TreeForm form, int n, int list_cap) {
     const size_t words = ((size_t)n + 31) / 32;
-    return form == kTreeNear ? 4 * kTreeNearList + 8 * words : 4 * kTreeGlobalList + 2 * ((words + 7) & ~(size_t)7);
+    return form == kTreeNear ? 4 * kTreeNearList + 8 * words : 4 * (size_t)list_cap + 2 * ((words + 7) & ~(size_t)7);
 }
 constexpr int kTreeGlobalMaxN = 65536 * 32;  // the global form's 16-bit word list: at most 128 KB
 
@@ -559,15 +556,36 @@ inline TreeKernel tree_kernel(TreeForm form, int threads) {
     }
 }
 
+// The global form's list entries per CTA, and its shape where none is timed.  A frontier of
+// tens of thousands of vertices (random graphs) takes a round per list, so larger lists are
+// faster, until eight CTAs' lists and dirty words leave the SM a smaller L1: from 180k
+// vertices on they get half, and four CTAs of twice the threads, which keep theirs, are the
+// first choice.  Microseconds per root: no list and one thread per dirty word (as it was) /
+// 1,024 entries in eight CTAs and every waiting vertex read in every round / the rule: random
+// graphs of 104k, 166k, 249k and 332k vertices 28 / 28 / 20, 51 / 64 / 41, 73 / 121 / 54, 107 /
+// 208 / 85; of degree eight, 159k and 238k 73 / 84 / 55, 126 / 171 / 96; planar-chain graphs of
+// 166k, 242k and 368k 39 / 14 / 14, 55 / 25 / 22, 97 / 34 / 34 (with eight CTAs' lists twice as
+// long beyond 180k 276k vertices take 53 instead of 28).
+constexpr int kTreeWideN = 180000;
+inline int tree_list_cap(int n, const TreeShape &sh) {
+    const int ctas = std::max(sh.ctas_per_sm, 1);
+    return std::max(kTreeGlobalList, (n > kTreeWideN && ctas >= 8 ? 8 : 16) * kTreeGlobalList / ctas);
+}
+inline TreeShape first_shape(TreeForm form, int n) {
+    if (form == kTreeGlobal && n > kTreeWideN) return TreeShape{512, 4, 8};
+    return TreeShape{256, 8, 8};
+}
+
 // Launches the form's kernel in `shape` over grid CTAs (the shared form: 1024 threads,
 // smem bytes of dynamic shared memory).
 inline cudaError_t launch_trees(TreeForm form, const TreeShape &shape, int grid, size_t smem, cudaStream_t st,
-                                const TreeArgs &a) {
+                                TreeArgs a) {
+    a.list_cap = tree_list_cap(a.n, shape);
     if (form == kTreeShared)
         trees_kernel<kTreeShared, kTreeThreads><<<grid, kTreeThreads, smem, st>>>(a);
     else
         tree_kernel(form, shape.threads)<<<grid, shape.threads <= 512 ? shape.threads : 1024,
-                                           trees_global_smem_bytes(form, a.n), st>>>(a);
+                                           trees_global_smem_bytes(form, a.n, a.list_cap), st>>>(a);
     return cudaGetLastError();
 }
 
@@ -578,7 +596,8 @@ inline cudaError_t set_trees_smem_limit() {
         for (TreeForm form : {kTreeNear, kTreeGlobal})
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(tree_kernel(form, threads), attr,
-                                         (int)trees_global_smem_bytes(form, form == kTreeNear ? kTreeNearMaxN : kTreeGlobalMaxN));
+                                         (int)trees_global_smem_bytes(form, form == kTreeNear ? kTreeNearMaxN : kTreeGlobalMaxN,
+                                                                      2 * 8 * kTreeGlobalList));
     return e;
 }
 

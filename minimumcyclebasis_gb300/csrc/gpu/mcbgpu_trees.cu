@@ -166,7 +166,7 @@ int mcbgpu_trees_run(mcbgpu_trees *t, const uint32_t *roots, int32_t count, int3
     a.rev = t->d_rev;
     a.arcs = t->d_arcs;
     a.n = t->n;
-    const TreeShape shape = t->form == kTreeShared ? TreeShape{kTreeThreads, 1, 4} : TreeShape{256, 8, 8};
+    const TreeShape shape = t->form == kTreeShared ? TreeShape{kTreeThreads, 1, 4} : first_shape(t->form, t->n);
     a.delta = shape_delta(shape, t->delta);
     a.roots = t->d_roots;
     a.count = count;
