@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -950,15 +951,17 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
     up(g->d_cols, cols, 4 * (size_t)slots);
     up(g->d_rev, rev, 4 * (size_t)slots);
     up(g->d_w, weights, 4 * (size_t)slots);
-    {
+    try {
         const std::vector<uint2> arcs = arc_table(nodes, row_offsets, cols, weights);
         up(g->d_arcs, arcs.data(), sizeof(uint2) * arcs.size());
+    } catch (const std::bad_alloc &) {  // host memory: reported as the device's
+        e = cudaErrorMemoryAllocation;
     }
     up(g->d_ec, edge_coord, 4 * (size_t)slots);
     up(g->d_fvs, fvs_array, 4 * n);
     up(g->d_pairs, pair_slot, 4 * (size_t)npairs);
     up(g->d_roots, fvs_vertices, 4 * (size_t)fvs_size);
-    {
+    try {
         std::vector<uint4> info((size_t)slots);
         std::vector<uint32_t> ends(g->branch_shared ? (size_t)npairs : 0);
         for (int64_t o = 0; o < slots; o++) info[(size_t)o] = make_uint4(rows[o], cols[o], 0, (uint32_t)edge_coord[o]);
@@ -969,6 +972,8 @@ int mcbgpu_gen_create(mcbgpu_gen **out, int32_t nodes, int64_t slots, const uint
         }
         up(g->d_slot_info, info.data(), sizeof(uint4) * (size_t)slots);
         if (g->branch_shared) up(g->d_pair_ends, ends.data(), 4 * (size_t)npairs);
+    } catch (const std::bad_alloc &) {
+        e = cudaErrorMemoryAllocation;
     }
     if (e == cudaSuccess) e = cudaMemset(g->d_status, 0, 4);
     if (e == cudaSuccess) e = set_trees_smem_limit();

@@ -389,10 +389,10 @@ __global__ void __launch_bounds__(kThreads, kForm == kTreeShared ? 1 : 2048 / kT
 // SM's last split but one of shared memory and L1 (196 of 228 KB): up to 79,360 vertices.
 // Past it a random graph takes 24 us per root against 14 with the dirty bits in global
 // memory, a planar-chain graph 7.4 against 6.9.  Up to it planar-chain and grid graphs gain
-// 15-25% (60k vertices 4.0 / 5.2, 79k 5.4 / 6.7) and RGGs nothing (5.6); random ones of mean degree 4.4 gain 3%
-// to 63k and lose 10% beyond (66k 11.4 / 10.0); of degree 6.3 and 8.1 they lose 10-25% from
-// the start (57k 12.9 / 11.7, 60k 19.8 / 16.9): more waits than a list holds.  So the degree
-// decides too.
+// 15-25% (60k vertices 4.0 / 5.2, 79k 5.4 / 6.7) and RGGs nothing (5.6); random ones of mean
+// degree 4.4 gain 3% to 63k and lose 10% beyond (66k 11.4 / 10.0); of degree 6.3 and 8.1 they
+// lose 10-25% from the start (57k 12.9 / 11.7, 60k 19.8 / 16.9): more waits than a list
+// holds.  So the degree decides too.
 constexpr int kTreeNearMaxN = 79360;
 constexpr int kTreeNearMaxDegree = 6;
 

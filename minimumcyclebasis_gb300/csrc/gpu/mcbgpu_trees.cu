@@ -3,6 +3,7 @@
 // the kernel (mcbgpu_sssp.cuh) runs on a chunk of roots and the distances, parent
 // slots and tie flags are copied back to the host.
 #include <climits>
+#include <new>
 #include <vector>
 
 #include "mcbgpu_sssp.cuh"
@@ -128,8 +129,12 @@ int mcbgpu_trees_create(mcbgpu_trees **out, int32_t nodes, int64_t slots, const 
         if (e == cudaSuccess) e = cudaMemcpy(t->d_w, weights, 4 * (size_t)slots, cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) {
-        const std::vector<uint2> arcs = arc_table(nodes, row_offsets, cols, weights);
-        e = cudaMemcpy(t->d_arcs, arcs.data(), sizeof(uint2) * arcs.size(), cudaMemcpyHostToDevice);
+        try {
+            const std::vector<uint2> arcs = arc_table(nodes, row_offsets, cols, weights);
+            e = cudaMemcpy(t->d_arcs, arcs.data(), sizeof(uint2) * arcs.size(), cudaMemcpyHostToDevice);
+        } catch (const std::bad_alloc &) {  // host memory: reported as the device's
+            e = cudaErrorMemoryAllocation;
+        }
     }
     // the kernel's attribute is process-wide: set to the largest shared form, so that
     // handles of different sizes can be used in any order
