@@ -266,6 +266,7 @@ constexpr int kColLanes = 8;
 constexpr int kColSegs = 64;                // segments per coordinate at most
 constexpr long long kColKeys = 16ll << 20;  // (coordinate, segment) keys at most (one per coordinate at least)
 constexpr int kColThreads = 256;
+constexpr size_t kColAsk = 64 << 20;        // bytes of index up to which the free memory is not asked for (20-30 us)
 constexpr int kScanCta = 1024, kScanItems = 8;
 
 template <bool kFill>
@@ -2737,9 +2738,9 @@ void free_solver(mcbgpu_solver *s) {
 }
 
 // The column index (three arrays), made for a handle that has everything else it needs.  It
-// only saves time, so it takes at most a quarter of the memory that is free by then: the
-// certificate's matrix, the pair buffers of a later upload and other handles find room as
-// they would without it.
+// only saves time, so beyond kColAsk it takes at most a quarter of the memory that is free
+// by then: the certificate's matrix, the pair buffers of a later upload and other handles
+// find room as they would without it.
 void columns_alloc(mcbgpu_solver *s) {
     if (s->nnz <= 0 || s->nnz >= 0xffffffffll || s->K >= 0xffffffffll) return;
     // One group of blocks is one W pass: reading the lists once is less than indexing them.
@@ -2754,8 +2755,9 @@ void columns_alloc(mcbgpu_solver *s) {
     const size_t sums = (keys + (size_t)kScanCta * kScanItems - 1) / ((size_t)kScanCta * kScanItems) + 1;
     const size_t need = sizeof(unsigned) * ((size_t)s->nnz + keys + 1 + sums);
     size_t room = 0, all = 0;
-    cudaError_t e = cudaMemGetInfo(&room, &all);
-    if (e == cudaSuccess && need > room / 4) return;  // W comes from the lists then
+    cudaError_t e = cudaSuccess;
+    if (need > kColAsk) e = cudaMemGetInfo(&room, &all);
+    if (e == cudaSuccess && need > kColAsk && need > room / 4) return;  // W comes from the lists then
     if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_colranks, sizeof(unsigned) * (size_t)s->nnz);
     if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_colstart, sizeof(unsigned) * (keys + 1));
     if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_colsums, sizeof(unsigned) * sums);
